@@ -25,7 +25,8 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-r
 LINK_LIBS = ["-lcufft", "-lcuda"]
 # The FP32 pair kernels: flush denormals and use the hardware reciprocal / square-root
 # approximations (positions and forces are O(1e-3..1e3); the sums are checked against FP64).
-PER_FILE_FLAGS = {"rpy_kernels.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"]}
+PER_FILE_FLAGS = {"rpy_kernels.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
+                  "flow.cu": ["-ftz=true"]}  # reciprocal square roots
 
 
 def nvcc() -> str:

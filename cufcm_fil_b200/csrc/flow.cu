@@ -10,11 +10,11 @@
 // with S(r) f = f/|r| + r (r.f)/|r|^3, the kernel's expressions term by term.
 //
 // The reference runs one thread per flow point over 64-wide shared-memory
-// tiles.  Here: float4 source records packed once per call, 256-source tiles
-// in shared memory, two flow points per thread, the source range split over
-// gridDim.y so that a small set of flow points still fills every SM, FP32
-// blockwise TwoSum accumulation, and an FP64 reduction of the split partials
-// in a fixed order (deterministic, no atomics).
+// tiles.  Here: float4 source records packed once per call, 64-source tiles
+// in shared memory, one or two flow points per thread, the source range
+// split over gridDim.y so that a small set of flow points still fills every
+// SM, FP32 sums of one tile under a TwoSum accumulation, and an FP64 reduction
+// of the split partials in a fixed order (deterministic, no atomics).
 #include "common.cuh"
 
 #include <algorithm>
@@ -36,9 +36,9 @@ namespace cufil {
 namespace {
 
 constexpr int kFlowThreads = 128;
-constexpr int kFlowTI = 2;      // flow points per thread
-constexpr int kFlowTile = 256;  // sources per shared-memory tile
-constexpr int kFlowTargets = kFlowThreads * kFlowTI;
+constexpr int kFlowTile = 64;     // sources per shared-memory tile and per FP32 sum
+constexpr int kFlowMaxTI = 2;     // flow points per thread: 1 or 2
+constexpr int kFlowCtasPerSm = 8;
 
 struct FlowParams {
     const float *xf;                  // [3 Nf]
@@ -47,52 +47,64 @@ struct FlowParams {
     int nf, ns, split, nsplit;
 };
 
+// 1/sqrt(x) by the hardware approximation (relative error up to 2^-22.9).  The sums are FP32 over 64 sources at a time,
+// so their error stays below that of divisions and square roots under sums of 256: 4.9e-7 against 6.5e-7 (relative L2,
+// 16,000 points above 5,120 segments, FP64 the measure).  Refining each root by a Newton step changed it by 5% and took
+// 201 us for 176.
+__device__ __forceinline__ float inv_sqrt(float x) {
+    return rsqrtf(fminf(x, 3.0e38f));  // an overflowed distance contributes nothing, as 1 / infinity does
+}
+
+// One source at one flow point.  With d = x - x_s, p = dx fx + dy fy and R = (dx, dy, z + z_s), the terms are
+// gathered by vector so that the pair takes about 55 multiply-adds and two reciprocal square roots:
+//   direct   f / r + ((d.f) d + t x d) / r^3
+//   image    -f / R - (R.f) R / R^3
+//            + 2 z_s / R^5 (z (3 a R - R^2 f*) + R^2 (p e_z + f_z (dx, dy, 0))),   f* = (fx, fy, -fz), a = R.f*
+// xs.w holds 2 z_s.
 template <bool SEG, bool WALL, bool NET>
-__device__ __forceinline__ void flow_pair(float xi, float yi, float zi, const float4 &xs, const float4 &f,
+__device__ __forceinline__ void flow_pair(float xi, float yi, float zi, float z3, const float4 &xs, const float4 &f,
                                           const float4 &t, const float4 &xb, float &vx, float &vy, float &vz) {
     const float dx = xi - xs.x, dy = yi - xs.y, dz = zi - xs.z;
-    const float rm2 = 1.0f / (dx * dx + dy * dy + dz * dz);
-    const float rm1 = sqrtf(rm2);
-    const float rdf = rm2 * (dx * f.x + dy * f.y + dz * f.z);
-    vx += rm1 * (f.x + dx * rdf);
-    vy += rm1 * (f.y + dy * rdf);
-    vz += rm1 * (f.z + dz * rdf);
+    const float q2 = fmaf(dx, dx, dy * dy);
+    const float p = fmaf(dx, f.x, dy * f.y);
+    const float rm1 = inv_sqrt(fmaf(dz, dz, q2));
+    const float rm3 = rm1 * rm1 * rm1;
+    const float df = fmaf(dz, f.z, p);
+    if constexpr (SEG) {  // with the rotlet of the segment torque
+        const float cx = fmaf(t.y, dz, fmaf(-t.z, dy, df * dx));
+        const float cy = fmaf(t.z, dx, fmaf(-t.x, dz, df * dy));
+        const float cz = fmaf(t.x, dy, fmaf(-t.y, dx, df * dz));
+        vx = fmaf(rm3, cx, fmaf(rm1, f.x, vx));
+        vy = fmaf(rm3, cy, fmaf(rm1, f.y, vy));
+        vz = fmaf(rm3, cz, fmaf(rm1, f.z, vz));
+    } else {
+        const float g = rm3 * df;
+        vx = fmaf(g, dx, fmaf(rm1, f.x, vx));
+        vy = fmaf(g, dy, fmaf(rm1, f.y, vy));
+        vz = fmaf(g, dz, fmaf(rm1, f.z, vz));
+    }
     if constexpr (SEG && WALL) {  // Blake's image system (no blobs: half-space data)
         const float Rz = zi + xs.z;
-        const float R2 = dx * dx + dy * dy + Rz * Rz;
-        const float Rm1 = sqrtf(1.0f / R2);
-        const float Rdf = (dx * f.x + dy * f.y + Rz * f.z) * Rm1 * Rm1;
-        vx -= Rm1 * (f.x + dx * Rdf);
-        vy -= Rm1 * (f.y + dy * Rdf);
-        vz -= Rm1 * (f.z + Rz * Rdf);
-        const float Dxx = (3.0f * dx * dx - R2) * zi;
-        const float Dxy = 3.0f * dx * dy * zi;
-        const float Dxz = (R2 - 3.0f * Rz * zi) * dx;
-        const float Dyy = (3.0f * dy * dy - R2) * zi;
-        const float Dyz = (R2 - 3.0f * Rz * zi) * dy;
-        const float Dzx = (3.0f * Rz * zi + R2) * dx;
-        const float Dzy = (3.0f * Rz * zi + R2) * dy;
-        const float Dzz = (R2 - 3.0f * Rz * Rz) * zi;
+        const float Rm1 = inv_sqrt(fmaf(Rz, Rz, q2));
         const float Rm2 = Rm1 * Rm1;
-        const float Dfac = 2.0f * xs.z * Rm2 * Rm2 * Rm1;
-        vx += Dfac * (Dxx * f.x + Dxy * f.y + Dxz * f.z);
-        vy += Dfac * (Dxy * f.x + Dyy * f.y + Dyz * f.z);
-        vz += Dfac * (Dzx * f.x + Dzy * f.y + Dzz * f.z);
-    }
-    if constexpr (SEG) {  // rotlet of the segment torque
-        const float rm3 = rm1 * rm2;
-        vx += rm3 * (t.y * dz - t.z * dy);
-        vy += rm3 * (t.z * dx - t.x * dz);
-        vz += rm3 * (t.x * dy - t.y * dx);
+        const float Rm3 = Rm2 * Rm1;
+        const float E = xs.w * Rm3;        // 2 z_s / R^3
+        const float D = E * (z3 * Rm2);    // 6 z z_s / R^5
+        const float zf = Rz * f.z;
+        const float g = fmaf(D, p - zf, -Rm3 * (p + zf));
+        const float h = fmaf(E, f.z, g);
+        const float cp = fmaf(-E, zi, -Rm1), cm = fmaf(E, zi, -Rm1);
+        vx = fmaf(h, dx, fmaf(cp, f.x, vx));
+        vy = fmaf(h, dy, fmaf(cp, f.y, vy));
+        vz = fmaf(E, p, fmaf(g, Rz, fmaf(cm, f.z, vz)));
     }
     if constexpr (NET) {  // minus a Stokeslet of the same force at the source's body
         const float ex = xi - xb.x, ey = yi - xb.y, ez = zi - xb.z;
-        const float qm2 = 1.0f / (ex * ex + ey * ey + ez * ez);
-        const float qm1 = sqrtf(qm2);
-        const float qdf = qm2 * (ex * f.x + ey * f.y + ez * f.z);
-        vx -= qm1 * (f.x + ex * qdf);
-        vy -= qm1 * (f.y + ey * qdf);
-        vz -= qm1 * (f.z + ez * qdf);
+        const float qm1 = inv_sqrt(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
+        const float g = -(qm1 * qm1 * qm1) * fmaf(ex, f.x, fmaf(ey, f.y, ez * f.z));
+        vx = fmaf(g, ex, fmaf(-qm1, f.x, vx));
+        vy = fmaf(g, ey, fmaf(-qm1, f.y, vy));
+        vz = fmaf(g, ez, fmaf(-qm1, f.z, vz));
     }
 }
 
@@ -107,21 +119,26 @@ __device__ __forceinline__ void two_sum3(float *hi, float *lo, float ax, float a
     }
 }
 
-// grid (ceil(nf / 256), nsplit): block (x, y) sums sources [y*split, (y+1)*split)
-// of its 256 flow points.  Sources [0, nseg_src) are segments, the rest blobs.
-template <bool WALL, bool NET>
-__global__ void __launch_bounds__(kFlowThreads) flow_tile_kernel(FlowParams p, int nseg_src) {
+// grid (ceil(nf / (128 TI)), nsplit): block (x, y) sums sources [y*split, (y+1)*split)
+// of its 128 TI flow points.  Sources [0, nseg_src) are segments, the rest blobs.
+// Bound by the FP32 pipe: 16,000 points and 5,120 segments (8.2e7 pairs above the wall) take 176 us, about 51 TFLOP/s;
+// term by term with divisions and square roots, in tiles of 256 at four blocks an SM, it was 425 us.  Four points a
+// thread leave too few warps (201 us).
+template <bool WALL, bool NET, int TI>
+__global__ void __launch_bounds__(kFlowThreads, kFlowCtasPerSm) flow_tile_kernel(FlowParams p, int nseg_src) {
+    constexpr int kTargets = kFlowThreads * TI;
     __shared__ float4 s_x[kFlowTile], s_f[kFlowTile], s_t[kFlowTile], s_b[kFlowTile];
     const int j0 = blockIdx.y * p.split;
     const int j1 = min(p.ns, j0 + p.split);
-    float xi[kFlowTI], yi[kFlowTI], zi[kFlowTI];
-    float hi[kFlowTI][3], lo[kFlowTI][3];
+    float xi[TI], yi[TI], zi[TI], z3[TI];
+    float hi[TI][3], lo[TI][3];
 #pragma unroll
-    for (int k = 0; k < kFlowTI; ++k) {
-        const int i = min(static_cast<int>(blockIdx.x * kFlowTargets + k * kFlowThreads + threadIdx.x), p.nf - 1);
+    for (int k = 0; k < TI; ++k) {
+        const int i = min(static_cast<int>(blockIdx.x * kTargets + k * kFlowThreads + threadIdx.x), p.nf - 1);
         xi[k] = p.xf[3 * i];
         yi[k] = p.xf[3 * i + 1];
         zi[k] = p.xf[3 * i + 2];
+        z3[k] = 3.0f * zi[k];
 #pragma unroll
         for (int c = 0; c < 3; ++c) hi[k][c] = lo[k][c] = 0.0f;
     }
@@ -129,36 +146,47 @@ __global__ void __launch_bounds__(kFlowThreads) flow_tile_kernel(FlowParams p, i
     for (int t0 = j0; t0 < j1; t0 += kFlowTile) {
         const int nt = min(kFlowTile, j1 - t0);
         __syncthreads();
-        for (int q = threadIdx.x; q < nt; q += kFlowThreads) {
-            s_x[q] = p.sx[t0 + q];
-            s_f[q] = p.sf[t0 + q];
-            s_t[q] = (t0 + q < nseg_src) ? p.st[t0 + q] : zero4;
-            s_b[q] = NET ? p.sb[t0 + q] : zero4;
+        if (threadIdx.x < kFlowTile) {
+            const int q = threadIdx.x;
+            if (q < nt) {
+                float4 x = p.sx[t0 + q];
+                x.w = 2.0f * x.z;
+                s_x[q] = x;
+                s_f[q] = p.sf[t0 + q];
+            }
+        } else {
+            const int q = threadIdx.x - kFlowTile;
+            if (q < nt) {
+                s_t[q] = (t0 + q < nseg_src) ? p.st[t0 + q] : zero4;
+                if (NET) s_b[q] = p.sb[t0 + q];
+            }
         }
         __syncthreads();
         // Segments and blobs of this tile: two branch-free loops.
         const int nsg = max(0, min(nt, nseg_src - t0));
-        float vx[kFlowTI], vy[kFlowTI], vz[kFlowTI];
+        float vx[TI], vy[TI], vz[TI];
 #pragma unroll
-        for (int k = 0; k < kFlowTI; ++k) vx[k] = vy[k] = vz[k] = 0.0f;
+        for (int k = 0; k < TI; ++k) vx[k] = vy[k] = vz[k] = 0.0f;
+#pragma unroll 2
         for (int q = 0; q < nsg; ++q) {
-            const float4 xs = s_x[q], f = s_f[q], tq = s_t[q], xb = s_b[q];
+            const float4 xs = s_x[q], f = s_f[q], tq = s_t[q], xb = NET ? s_b[q] : zero4;
 #pragma unroll
-            for (int k = 0; k < kFlowTI; ++k)
-                flow_pair<true, WALL, NET>(xi[k], yi[k], zi[k], xs, f, tq, xb, vx[k], vy[k], vz[k]);
+            for (int k = 0; k < TI; ++k)
+                flow_pair<true, WALL, NET>(xi[k], yi[k], zi[k], z3[k], xs, f, tq, xb, vx[k], vy[k], vz[k]);
         }
+#pragma unroll 2
         for (int q = nsg; q < nt; ++q) {
-            const float4 xs = s_x[q], f = s_f[q], xb = s_b[q];
+            const float4 xs = s_x[q], f = s_f[q], xb = NET ? s_b[q] : zero4;
 #pragma unroll
-            for (int k = 0; k < kFlowTI; ++k)
-                flow_pair<false, false, NET>(xi[k], yi[k], zi[k], xs, f, zero4, xb, vx[k], vy[k], vz[k]);
+            for (int k = 0; k < TI; ++k)
+                flow_pair<false, false, NET>(xi[k], yi[k], zi[k], z3[k], xs, f, zero4, xb, vx[k], vy[k], vz[k]);
         }
 #pragma unroll
-        for (int k = 0; k < kFlowTI; ++k) two_sum3(hi[k], lo[k], vx[k], vy[k], vz[k]);
+        for (int k = 0; k < TI; ++k) two_sum3(hi[k], lo[k], vx[k], vy[k], vz[k]);
     }
 #pragma unroll
-    for (int k = 0; k < kFlowTI; ++k) {
-        const int i = static_cast<int>(blockIdx.x * kFlowTargets + k * kFlowThreads + threadIdx.x);
+    for (int k = 0; k < TI; ++k) {
+        const int i = static_cast<int>(blockIdx.x * kTargets + k * kFlowThreads + threadIdx.x);
         if (i < p.nf)
             p.partial[static_cast<size_t>(i) * p.nsplit + blockIdx.y] =
                 make_float4(hi[k][0] + lo[k][0], hi[k][1] + lo[k][1], hi[k][2] + lo[k][2], 0.0f);
@@ -210,21 +238,46 @@ __global__ void flow_pack_kernel(const float *xs, const float *fs, int ns, int n
 }
 
 struct FlowPlan {
-    int tiles, nsplit, split;
+    int ti, tiles, nsplit, split;
 };
 
-// Splits the sources so that about two waves of 256-point blocks (4 resident per
-// SM) cover the SMs, keeping at least one tile of sources per split.
-FlowPlan flow_plan(int nf, int nsrc, int num_sms) {
-    FlowPlan p{};
-    p.tiles = std::max(1, (nf + kFlowTargets - 1) / kFlowTargets);
-    const int want = std::max(1, (2 * 4 * num_sms + p.tiles - 1) / p.tiles);
-    const int max_split = std::max(1, (nsrc + kFlowTile - 1) / kFlowTile);
-    p.nsplit = std::min(want, max_split);
-    p.split = (nsrc + p.nsplit - 1) / p.nsplit;
-    p.split = ((p.split + kFlowTile - 1) / kFlowTile) * kFlowTile;
-    p.nsplit = std::max(1, (nsrc + p.split - 1) / p.split);
-    return p;
+// Flow points per thread and source splits of nf points and nsrc sources: the choice with the least estimated
+// time, waves x (per-block work), where a block's work is its sources times its points per thread plus a fixed
+// cost (staging and epilogue) worth about 24 single-point sources.  More points per thread read each staged
+// source less often (a source read from shared memory costs about 0.4 of a pair); more splits fill the SMs when
+// the points are few.  The partials (nf x nsplit) stay within `cap`, the handle's buffer.
+FlowPlan flow_plan(int nf, int nsrc, int num_sms, size_t cap) {
+    FlowPlan best{};
+    double best_cost = 1e300;
+    const int max_tiles = std::max(1, (nsrc + kFlowTile - 1) / kFlowTile);
+    for (int ti = 1; ti <= kFlowMaxTI; ti *= 2) {
+        const int per = kFlowThreads * ti;
+        const int tiles = std::max(1, (nf + per - 1) / per);
+        const long long slots = static_cast<long long>(num_sms) * kFlowCtasPerSm;
+        int last = 0;
+        for (int cand = 1; cand <= max_tiles && cand <= 1024; ++cand) {
+            const int split = kFlowTile * ((max_tiles + cand - 1) / cand);
+            const int nsplit = (nsrc + split - 1) / split;
+            if (nsplit == last) continue;
+            last = nsplit;
+            if (nsplit > 1 && static_cast<size_t>(nf) * nsplit > cap) break;
+            const long long waves = (static_cast<long long>(tiles) * nsplit + slots - 1) / slots;
+            const double cost = static_cast<double>(waves) * (split * (ti + 0.4) + 24.0);
+            if (cost < best_cost * (1.0 - 1e-9)) {
+                best_cost = cost;
+                best = FlowPlan{ti, tiles, nsplit, split};
+            }
+        }
+    }
+    return best;
+}
+
+template <int TI>
+void launch_flow_tiles(bool wall, bool net, dim3 grid, cudaStream_t st, const FlowParams &p, int ns) {
+    if (wall && net) flow_tile_kernel<true, true, TI><<<grid, kFlowThreads, 0, st>>>(p, ns);
+    else if (wall) flow_tile_kernel<true, false, TI><<<grid, kFlowThreads, 0, st>>>(p, ns);
+    else if (net) flow_tile_kernel<false, true, TI><<<grid, kFlowThreads, 0, st>>>(p, ns);
+    else flow_tile_kernel<false, false, TI><<<grid, kFlowThreads, 0, st>>>(p, ns);
 }
 
 template <typename T>
@@ -246,15 +299,13 @@ int flow_run(cf_flow *h, const float *xf, int nf, const float *xs, const float *
     flow_pack_kernel<<<(nsrc + 255) / 256, 256, 0, st>>>(xs, fs, ns, ns_pb, xb, fb, nb, nb_pb, net ? xbod : nullptr,
                                                          h->sx, h->sf, h->st, h->sb);
     CF_CHECK_LAUNCH("flow_pack_kernel");
-    const FlowPlan pl = flow_plan(nf, nsrc, h->num_sms);
+    const FlowPlan pl = flow_plan(nf, nsrc, h->num_sms, h->partial_cap);
     CF_REQUIRE(static_cast<size_t>(nf) * pl.nsplit <= h->partial_cap, "cf_flow: scratch too small");
     FlowParams p{xf, h->sx, h->sf, h->st, h->sb, h->partial, nf, nsrc, pl.split, pl.nsplit};
     const dim3 grid(pl.tiles, pl.nsplit);
     const bool wall = nb_pb == 0;  // no blobs: half-space data (flow_field_evaluator.cu:75-78)
-    if (wall && net) flow_tile_kernel<true, true><<<grid, kFlowThreads, 0, st>>>(p, ns);
-    else if (wall) flow_tile_kernel<true, false><<<grid, kFlowThreads, 0, st>>>(p, ns);
-    else if (net) flow_tile_kernel<false, true><<<grid, kFlowThreads, 0, st>>>(p, ns);
-    else flow_tile_kernel<false, false><<<grid, kFlowThreads, 0, st>>>(p, ns);
+    if (pl.ti == 2) launch_flow_tiles<2>(wall, net, grid, st, p, ns);
+    else launch_flow_tiles<1>(wall, net, grid, st, p, ns);
     CF_CHECK_LAUNCH("flow_tile_kernel");
     const double prefac = 1.0 / (8.0 * 3.14159265358979323846 * h->cfg.mu);
     flow_reduce_kernel<<<(nf + 7) / 8, 256, 0, st>>>(h->partial, nf, pl.nsplit, prefac, v);
@@ -313,9 +364,9 @@ extern "C" int cf_flow_create(const cf_flow_config *cfg, cf_flow **out) {
                               __FILE__, __LINE__)))
             break;
         const size_t nsrc = static_cast<size_t>(cfg->max_seg) + cfg->max_blob;
-        // flow_plan keeps tiles * nsplit near 8 blocks per SM, so nf * nsplit stays below this bound
-        h->partial_cap =
-            static_cast<size_t>(2 * 4 * h->num_sms + 1) * kFlowTargets + 2 * static_cast<size_t>(cfg->max_flow);
+        // one partial per point and split; flow_plan takes no more splits than fit
+        h->partial_cap = static_cast<size_t>(2 * kFlowCtasPerSm * h->num_sms + 1) * kFlowThreads +
+                         2 * static_cast<size_t>(cfg->max_flow);
         if ((rc = falloc(&h->sx, nsrc)) || (rc = falloc(&h->sf, nsrc)) || (rc = falloc(&h->st, nsrc)) ||
             (rc = falloc(&h->sb, nsrc)) || (rc = falloc(&h->partial, h->partial_cap)) ||
             (rc = falloc(&h->hx_flow, 3 * static_cast<size_t>(cfg->max_flow))) ||
