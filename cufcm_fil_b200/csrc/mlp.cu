@@ -15,7 +15,11 @@
 //   dZ1 = (dZ2 W2^T) o [A1 > 0]   dW1 = X^T dZ1    db1 = colsum dZ1
 // then one Adam step on FP32 master weights.  Reductions (loss, bias
 // gradients) are fixed-order: results do not depend on the launch.
+// Networks of widths in, H <= 256 and out <= 128 (every one the implicit step
+// attaches) run on the fused kernels of mlp_fused.cuh instead: the same
+// products of the same BF16 operands, one launch forward, three for a gradient.
 #include "common.cuh"
+#include "mlp_fused.cuh"
 #include "tc_tf32.cuh"
 
 #include <cuda_bf16.h>
@@ -25,6 +29,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <new>
 #include <random>
 #include <string>
@@ -229,6 +234,14 @@ struct cf_mlp {
     double *partial = nullptr;
     int loss_blocks = 256;
     long long step = 0;
+    // fused path (mlp_fused.cuh): operand images of the weights, transposed row operands and partial sums of a
+    // training batch
+    bool fused = false;
+    mlpk::Images im{};
+    __nv_bfloat16 *xt = nullptr, *a1t = nullptr, *a2t = nullptr, *dyt = nullptr, *dz2t = nullptr, *dz1t = nullptr;
+    float *gpart = nullptr, *db = nullptr;
+    int max_tiles = 0;
+    float *h_grads = nullptr;  // pinned: gradients, then the loss partials
     cudaStream_t stream = nullptr;
     std::vector<void *> allocations;
 };
@@ -244,6 +257,49 @@ int mlp_alloc(cf_mlp *h, T **p, size_t n) {
     return CF_OK;
 }
 
+// Splits of the weight gradients' rows: the output tiles (at most 10) times the splits fill the SMs once.
+constexpr int kGradSplits = 14;
+int grad_splits(int tiles) { return std::min(tiles, kGradSplits); }
+
+// Buffers of the fused path.  Image and operand padding is zero and stays zero: the kernels write only the true
+// entries, and a product multiplies the padding.
+int alloc_fused(cf_mlp *h) {
+    const size_t inP = mlpk::pad32(h->in), hidP = mlpk::pad32(h->hid), outP = mlpk::pad32(h->out);
+    const size_t in128 = mlpk::pad128(h->in), hid128 = mlpk::pad128(h->hid);
+    h->max_tiles = (h->max_batch + mlpk::kRows - 1) / mlpk::kRows;
+    const size_t rows = static_cast<size_t>(h->max_tiles) * mlpk::kRows;
+    auto zeros = [&](__nv_bfloat16 **p, size_t n) -> int {
+        CF_TRY(mlp_alloc(h, p, n));
+        CF_CUDA(cudaMemset(*p, 0, n * sizeof(__nv_bfloat16)));
+        return CF_OK;
+    };
+    h->im.in = h->in;
+    h->im.hid = h->hid;
+    h->im.out = h->out;
+    CF_TRY(zeros(&h->im.f1, hidP * inP));
+    CF_TRY(zeros(&h->im.f2, hidP * hidP));
+    CF_TRY(zeros(&h->im.f3, outP * hidP));
+    CF_TRY(zeros(&h->im.g3, hidP * outP));
+    CF_TRY(zeros(&h->im.g2, hidP * hidP));
+    CF_TRY(zeros(&h->xt, rows * in128));
+    CF_TRY(zeros(&h->a1t, rows * hid128));
+    CF_TRY(zeros(&h->a2t, rows * hid128));
+    CF_TRY(zeros(&h->dyt, rows * outP));
+    CF_TRY(zeros(&h->dz2t, rows * hid128));
+    CF_TRY(zeros(&h->dz1t, rows * hid128));
+    CF_TRY(mlp_alloc(h, &h->gpart, static_cast<size_t>(grad_splits(h->max_tiles)) * h->nparam));
+    CF_TRY(mlp_alloc(h, &h->db, static_cast<size_t>(h->max_tiles) * (2 * hidP + outP)));
+    CF_TRY(mlp_alloc(h, &h->partial, h->max_tiles));
+    CF_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h->h_grads), h->nparam * sizeof(float) + 8));
+    CF_CUDA(cudaFuncSetAttribute(mlpk::mlp_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(mlpk::kRowsSmem)));
+    CF_CUDA(cudaFuncSetAttribute(mlpk::mlp_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(mlpk::kRowsSmem)));
+    CF_CUDA(cudaFuncSetAttribute(mlpk::mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(mlpk::kGradSmem)));
+    return CF_OK;
+}
+
 void set_views(cf_mlp *h) {
     const long long in = h->in, hd = h->hid, out = h->out;
     float *p = h->params, *g = h->grads;
@@ -254,14 +310,94 @@ void set_views(cf_mlp *h) {
     h->gb3 = g + off[5];
 }
 
+mlpk::RowArgs row_args(const cf_mlp *h, const float *x, int n) {
+    mlpk::RowArgs a{};
+    a.x = x;
+    a.n = n;
+    a.in = h->in;
+    a.hid = h->hid;
+    a.out = h->out;
+    a.f1 = h->im.f1;
+    a.f2 = h->im.f2;
+    a.f3 = h->im.f3;
+    a.g3 = h->im.g3;
+    a.g2 = h->im.g2;
+    a.b1 = h->b1;
+    a.b2 = h->b2;
+    a.b3 = h->b3;
+    return a;
+}
+
+// The weights' images from the FP32 parameters (after these were set as a whole).
+int refresh_images(cf_mlp *h, cudaStream_t st) {
+    if (!h->fused) return CF_OK;
+    mlpk::mlp_images_kernel<<<static_cast<unsigned>((h->nparam + 255) / 256), 256, 0, st>>>(h->im, h->params, h->nparam);
+    CF_CHECK_LAUNCH("mlp_images_kernel");
+    return CF_OK;
+}
+
+// Forward + backward and the gradients (with `adam`, also the optimiser step) in three launches.
+int fused_gradients(cf_mlp *h, const float *x, const float *t, int n, const mlpk::FinishArgs *adam) {
+    cudaStream_t st = h->stream;
+    const int tiles = (n + mlpk::kRows - 1) / mlpk::kRows, splits = grad_splits(tiles);
+    mlpk::RowArgs a = row_args(h, x, n);
+    a.t = t;
+    a.xt = h->xt;
+    a.a1t = h->a1t;
+    a.a2t = h->a2t;
+    a.dyt = h->dyt;
+    a.dz2t = h->dz2t;
+    a.dz1t = h->dz1t;
+    a.db = h->db;
+    a.loss = h->partial;
+    a.scale = 1.0f / static_cast<float>(static_cast<long long>(n) * h->out);
+    CF_CUDA(launch_chained(mlpk::mlp_rows_kernel<true>, dim3(tiles), dim3(mlpk::kThreads), mlpk::kRowsSmem, st, a));
+    CF_CHECK_LAUNCH("mlp_rows_kernel");
+    mlpk::GradArgs g{h->xt, h->a1t, h->a2t, h->dyt, h->dz2t, h->dz1t, h->gpart, h->nparam, h->in, h->hid, h->out, tiles,
+                     splits};
+    const int mi = (h->in + mlpk::kChunk - 1) / mlpk::kChunk, mh = (h->hid + mlpk::kChunk - 1) / mlpk::kChunk;
+    CF_CUDA(launch_chained(mlpk::mlp_wgrad_kernel, dim3(mi * mh + mh * mh + mh, splits), dim3(mlpk::kThreads),
+                           mlpk::kGradSmem, st, g));
+    CF_CHECK_LAUNCH("mlp_wgrad_kernel");
+    mlpk::FinishArgs f{};
+    if (adam) f = *adam;
+    f.partial = h->gpart;
+    f.db = h->db;
+    f.grads = h->grads;
+    f.p = h->params;
+    f.m = h->adam_m;
+    f.v = h->adam_v;
+    f.nparam = h->nparam;
+    f.tiles = tiles;
+    f.splits = splits;
+    CF_CUDA(launch_chained(mlpk::mlp_finish_kernel, dim3(static_cast<unsigned>((h->nparam + 255) / 256)), dim3(256), 0,
+                           st, f, h->im));
+    CF_CHECK_LAUNCH("mlp_finish_kernel");
+    return CF_OK;
+}
+
 int forward(cf_mlp *h, const float *x, int n, float *y, cudaStream_t st) {
+    if (h->fused) {
+        if (n <= 0) return CF_OK;
+        mlpk::RowArgs a = row_args(h, x, n);
+        // blocks write rows of y while others read x: an output that shares memory with the input goes by way of Y
+        const size_t nx = static_cast<size_t>(n) * h->in, ny = static_cast<size_t>(n) * h->out;
+        const std::less<const float *> before;
+        const bool shared = before(x, y + ny) && before(y, x + nx);
+        a.y = shared ? h->Y : y;
+        CF_CUDA(launch_chained(mlpk::mlp_rows_kernel<false>, dim3((n + mlpk::kRows - 1) / mlpk::kRows),
+                               dim3(mlpk::kThreads), mlpk::kRowsSmem, st, a));
+        CF_CHECK_LAUNCH("mlp_rows_kernel");
+        if (shared) CF_CUDA(cudaMemcpyAsync(y, h->Y, ny * sizeof(float), cudaMemcpyDeviceToDevice, st));
+        return CF_OK;
+    }
     CF_TRY(gemm_bf16(x, h->in, 0, h->W1, h->hid, 0, h->A1, h->hid, n, h->hid, h->in, h->b1, nullptr, kEpiBiasRelu, st));
     CF_TRY(gemm_bf16(h->A1, h->hid, 0, h->W2, h->hid, 0, h->A2, h->hid, n, h->hid, h->hid, h->b2, nullptr,
                      kEpiBiasRelu, st));
     return gemm_bf16(h->A2, h->hid, 0, h->W3, h->out, 0, y, h->out, n, h->out, h->hid, h->b3, nullptr, kEpiBias, st);
 }
 
-// Forward + backward into h->grads; the loss (mean squared error) into *loss when asked (synchronises).
+// Forward + backward into h->grads by general GEMMs; the loss (mean squared error) into *loss when asked (synchronises).
 int backward(cf_mlp *h, const float *x, const float *t, int n, double *loss) {
     cudaStream_t st = h->stream;
     CF_TRY(forward(h, x, n, h->Y, st));
@@ -295,6 +431,18 @@ int backward(cf_mlp *h, const float *x, const float *t, int n, double *loss) {
         for (double v : part) s += v;
         *loss = s / static_cast<double>(cnt);
     }
+    return CF_OK;
+}
+
+// Mean squared error of the last fused gradient's batch from its tiles' sums (waits for the stream).
+int fused_loss(cf_mlp *h, int n, double *loss) {
+    const int tiles = (n + mlpk::kRows - 1) / mlpk::kRows;
+    std::vector<double> part(tiles);
+    CF_CUDA(cudaMemcpyAsync(part.data(), h->partial, sizeof(double) * tiles, cudaMemcpyDeviceToHost, h->stream));
+    CF_CUDA(cudaStreamSynchronize(h->stream));
+    double s = 0.0;
+    for (double v : part) s += v;
+    *loss = s / (static_cast<double>(n) * h->out);
     return CF_OK;
 }
 
@@ -338,13 +486,19 @@ extern "C" int cf_mlp_create(int in_dim, int hidden, int out_dim, int max_batch,
                               __FILE__, __LINE__)))
             break;
         const size_t np = h->nparam, act = static_cast<size_t>(max_batch) * hidden;
+        h->fused = in_dim <= mlpk::kMaxW && hidden <= mlpk::kMaxW && out_dim <= mlpk::kMaxOut;
         if ((rc = mlp_alloc(h, &h->params, np)) || (rc = mlp_alloc(h, &h->grads, np)) ||
-            (rc = mlp_alloc(h, &h->adam_m, np)) || (rc = mlp_alloc(h, &h->adam_v, np)) ||
-            (rc = mlp_alloc(h, &h->A1, act)) || (rc = mlp_alloc(h, &h->A2, act)) || (rc = mlp_alloc(h, &h->dZ1, act)) ||
-            (rc = mlp_alloc(h, &h->dZ2, act)) || (rc = mlp_alloc(h, &h->Y, static_cast<size_t>(max_batch) * out_dim)) ||
-            (rc = mlp_alloc(h, &h->dY, static_cast<size_t>(max_batch) * out_dim)) ||
-            (rc = mlp_alloc(h, &h->partial, h->loss_blocks)))
+            (rc = mlp_alloc(h, &h->adam_m, np)) || (rc = mlp_alloc(h, &h->adam_v, np)))
             break;
+        if ((rc = mlp_alloc(h, &h->Y, static_cast<size_t>(max_batch) * out_dim))) break;
+        if (h->fused) {
+            if ((rc = alloc_fused(h))) break;
+        } else if ((rc = mlp_alloc(h, &h->A1, act)) || (rc = mlp_alloc(h, &h->A2, act)) ||
+                   (rc = mlp_alloc(h, &h->dZ1, act)) || (rc = mlp_alloc(h, &h->dZ2, act)) ||
+                   (rc = mlp_alloc(h, &h->dY, static_cast<size_t>(max_batch) * out_dim)) ||
+                   (rc = mlp_alloc(h, &h->partial, h->loss_blocks))) {
+            break;
+        }
         set_views(h);
         // He-uniform weights from the seed, zero biases
         std::vector<float> p(np, 0.0f);
@@ -361,10 +515,16 @@ extern "C" int cf_mlp_create(int in_dim, int hidden, int out_dim, int max_batch,
             (rc = cuda_status(cudaMemset(h->adam_m, 0, np * sizeof(float)), "cudaMemset", __FILE__, __LINE__)) ||
             (rc = cuda_status(cudaMemset(h->adam_v, 0, np * sizeof(float)), "cudaMemset", __FILE__, __LINE__)))
             break;
+        // images on the handle's stream, after the legacy-stream copies above have completed
+        if ((rc = cuda_status(cudaDeviceSynchronize(), "cudaDeviceSynchronize", __FILE__, __LINE__)) ||
+            (rc = refresh_images(h, h->stream)))
+            break;
+        rc = cuda_status(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize", __FILE__, __LINE__);
     } while (0);
     if (rc != CF_OK) {
         std::string msg = cf_last_error();
         for (void *q : h->allocations) cudaFree(q);
+        if (h->h_grads) cudaFreeHost(h->h_grads);
         if (h->stream) cudaStreamDestroy(h->stream);
         delete h;
         return set_error(rc, "%s", msg.c_str());
@@ -378,6 +538,7 @@ extern "C" int cf_mlp_destroy(cf_mlp *h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void *q : h->allocations) cudaFree(q);
+    if (h->h_grads) cudaFreeHost(h->h_grads);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return CF_OK;
@@ -399,6 +560,15 @@ extern "C" int cf_mlp_gradients(cf_mlp *h, const float *x, const float *t, int n
     CF_REQUIRE(n > 0 && n <= h->max_batch, "cf_mlp_gradients: batch %d outside [1, %d]", n, h->max_batch);
     CF_CUDA(cudaSetDevice(h->device));
     double l = 0.0;
+    if (h->fused) {
+        CF_TRY(fused_gradients(h, x, t, n, nullptr));
+        if (grads)
+            CF_CUDA(cudaMemcpyAsync(h->h_grads, h->grads, sizeof(float) * h->nparam, cudaMemcpyDeviceToHost, h->stream));
+        CF_TRY(fused_loss(h, n, &l));  // waits for the stream
+        if (loss) *loss = l;
+        if (grads) std::memcpy(grads, h->h_grads, sizeof(float) * h->nparam);
+        return CF_OK;
+    }
     CF_TRY(backward(h, x, t, n, &l));
     if (loss) *loss = l;
     if (grads) {
@@ -414,11 +584,24 @@ extern "C" int cf_mlp_train_step(cf_mlp *h, const float *x, const float *t, int 
     CF_REQUIRE(n > 0 && n <= h->max_batch, "cf_mlp_train_step: batch %d outside [1, %d]", n, h->max_batch);
     CF_REQUIRE(lr > 0.0f, "cf_mlp_train_step: learning rate must be positive");
     CF_CUDA(cudaSetDevice(h->device));
+    const float b1 = 0.9f, b2 = 0.999f;
+    const float c1 = 1.0f - std::pow(b1, static_cast<float>(h->step + 1));
+    const float c2 = 1.0f - std::pow(b2, static_cast<float>(h->step + 1));
+    if (h->fused) {
+        mlpk::FinishArgs f{};
+        f.adam = 1;
+        f.lr = lr;
+        f.b1 = b1;
+        f.b2 = b2;
+        f.c1 = c1;
+        f.c2 = c2;
+        f.eps = 1e-8f;
+        CF_TRY(fused_gradients(h, x, t, n, &f));
+        h->step += 1;
+        return loss ? fused_loss(h, n, loss) : CF_OK;
+    }
     CF_TRY(backward(h, x, t, n, loss));
     h->step += 1;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.0f - std::pow(b1, static_cast<float>(h->step));
-    const float c2 = 1.0f - std::pow(b2, static_cast<float>(h->step));
     adam_kernel<<<256, 256, 0, h->stream>>>(h->params, h->grads, h->adam_m, h->adam_v, h->nparam, lr, b1, b2, c1, c2,
                                             1e-8f);
     CF_CHECK_LAUNCH("adam_kernel");
@@ -439,7 +622,9 @@ extern "C" int cf_mlp_set_params(cf_mlp *h, const float *params) {
     CF_REQUIRE(h && params, "cf_mlp_set_params: null argument");
     CF_CUDA(cudaSetDevice(h->device));
     CF_CUDA(cudaStreamSynchronize(h->stream));
-    CF_CUDA(cudaMemcpy(h->params, params, sizeof(float) * h->nparam, cudaMemcpyHostToDevice));
+    CF_CUDA(cudaMemcpyAsync(h->params, params, sizeof(float) * h->nparam, cudaMemcpyHostToDevice, h->stream));
+    CF_TRY(refresh_images(h, h->stream));
+    CF_CUDA(cudaStreamSynchronize(h->stream));
     return CF_OK;
 }
 
