@@ -157,130 +157,154 @@ __device__ __forceinline__ void load_pivot_block(const float *A, int n, int k0, 
 // Part (a) of a round: inverts pivot block K of patch p (rows and columns
 // [64K, 64K + b)) into its dinv block, zero-padded to 64 x 64; called by all
 // 256 threads of a block.  The 64x64 block D (padded with the identity beyond
-// b) is inverted in place by Gauss-Jordan elimination without pivoting in
-// registers: thread (row r = tid / 4, quarter g = tid % 4) holds D[r][16g ..
-// 16g + 15], so warp w holds rows 8w .. 8w + 7.  The pivots are taken in eight
-// panels of eight (block Gauss-Jordan, two barriers per panel instead of one
-// per pivot; the loop below says how).  Forming the inverse explicitly loses accuracy
-// when D is ill conditioned, so the result X is refined by one Newton step,
-// X <- X + X (I - D X), which squares its residual.  A zero or non-finite
-// pivot clears the patch's ok flag.
+// b) is inverted in place by block Gauss-Jordan elimination without pivoting,
+// in registers: thread (ty, tx) holds rows 4ty .. + 3 and columns 4tx .. + 3.
+// The pivots are taken in eight panels of eight: the panel's rows and columns
+// are published, warp 0 inverts the panel's 8 x 8 block by shuffles (a chain of
+// eight reciprocals), every row forms its eight coefficients (-a_r D^-1, or row
+// r of D^-1 inside the panel), and the block takes the rank-8 update
+//   x <- [x outside the panel's rows and columns] + coefficients panel.
+// Forming the inverse explicitly loses accuracy when D is ill conditioned, so
+// the result X is refined by one Newton step, X <- X + X (I - D X), which
+// squares its residual.  A zero or non-finite pivot clears the patch's ok flag.
+// The inverse is the critical path of the refresh (the next round waits for
+// it): 26.6 -> 16.4 us alone (16 blocks, 1.965 GHz), of which the elimination
+// 34 600 -> 15 900 cycles: sixteen columns of one row per thread read the panel
+// with bank conflicts, four 128-bit loads per sixteen FMAs, where a 4 x 4 tile
+// reads two without; and each warp eliminating its own panel moved sixteen
+// values per pivot by shuffles.  The Newton products take 7 700.
 // A: the patch matrix (n x n), dv: its dinv block, ok: its flag, ws: shared
 // memory of at least kInvWs floats.
 constexpr int kInvWs = 2 * kGjBlock * kInvLd;
 __device__ __noinline__ void pivot_invert(const float *A, int n, float *dv, int *ok, int K, float *ws) {
-    static_assert(kGjBlock == 64, "four threads of 16 columns per row, eight rows per warp");
+    static_assert(kGjBlock == 64, "sixteen 4 x 4 tiles a side");
     const int k0 = K * kGjBlock;
     const int b = min(kGjBlock, n - k0);
     float *X = ws, *W = ws + kGjBlock * kInvLd;  // X: the inverse; W: D, then I - D X
-    const int r = threadIdx.x >> 2, g = threadIdx.x & 3;
-    const size_t ld = patch_ld(n);
-    float v[16];
-    {
-        const float *Ar = A + (k0 + r) * ld + k0 + 16 * g;
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int c = 16 * g + q;
-            v[q] = (r < b && c < b) ? Ar[q] : (r == c ? 1.0f : 0.0f);
-        }
-    }
-    // Eight panels of eight pivots, panel m held by warp m (rows 8m .. 8m + 7): the warp eliminates the
-    // panel's pivots inside its own rows (pivot rows and column entries by shuffles, no block barrier),
-    // publishes its rows and every other row its entries in the panel's columns, and after one barrier every
-    // other row takes the rank-8 update  x <- [x outside the panel columns] - a_G panel  (block Gauss-Jordan).
-    __shared__ __align__(16) float panel[8][kGjBlock];
-    __shared__ __align__(16) float colg[kGjBlock][8];
+    constexpr int kCoefLd = kGjBlock + 4;  // the four coefficient pairs of a row land on different banks
+    __shared__ __align__(16) float rows[2][8][kGjBlock];
+    __shared__ __align__(16) float cols[2][kGjBlock][8];
+    __shared__ __align__(16) float dinv[8][8];
+    __shared__ __align__(16) float coef[8][kCoefLd];
     __shared__ int sbad;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, rl = lane >> 2;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, lane = threadIdx.x & 31;
+    const size_t ld = patch_ld(n);
+    float v[4][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int r = 4 * ty + u, c = 4 * tx;
+        // rows start on 16 bytes and the padding columns are mapped, so whole chunks inside the row stride are read
+        float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (r < b && k0 + c < static_cast<int>(ld)) q = *reinterpret_cast<const float4 *>(A + (k0 + r) * ld + k0 + c);
+        const float e[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int s = 0; s < 4; ++s) v[u][s] = (r < b && c + s < b) ? e[s] : (r == c + s ? 1.0f : 0.0f);
+        *reinterpret_cast<float4 *>(W + r * kInvLd + c) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+    }
     if (threadIdx.x == 0) sbad = 0;
 #pragma unroll 1
     for (int m = 0; m < 8; ++m) {
-        const int cg = m >> 1, half = m & 1;  // the panel's columns 8m + t: chunk cg, element 8 half + t
-        if (w == m) {
+        const int par = m & 1;
+        const bool prow = (ty >> 1) == m, pcol = (tx >> 1) == m;
+        if (prow)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                *reinterpret_cast<float4 *>(&rows[par][4 * (ty & 1) + u][4 * tx]) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+        if (pcol)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                *reinterpret_cast<float4 *>(&cols[par][4 * ty + u][4 * (tx & 1)]) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+        __syncthreads();
+        if (threadIdx.x < 32) {  // warp 0: the panel's 8 x 8 block, lane (row lane / 4, columns 2 (lane % 4), + 1)
+            float2 d = *reinterpret_cast<const float2 *>(&cols[par][8 * m + (lane >> 2)][2 * (lane & 3)]);
             bool bad = false;
 #pragma unroll
             for (int t = 0; t < 8; ++t) {
-                float p[16];
-#pragma unroll
-                for (int q = 0; q < 16; ++q) p[q] = __shfl_sync(0xffffffffu, v[q], 4 * t + g);  // pivot row
-                const float mine = half ? v[8 + t] : v[t];
-                const float f = __shfl_sync(0xffffffffu, mine, (lane & ~3) | cg);  // this row's entry, column k
-                const float piv = __shfl_sync(0xffffffffu, mine, 4 * t + cg);
-                bad |= !(fabsf(piv) > 0.0f) || !isfinite(piv);
-                const float ip = __frcp_rn(piv);
-                // v <- a v + b p with (a, b) = (0, 1/piv) in the pivot row, (1, -f/piv) elsewhere; the pivot
-                // column takes b itself
-                const bool own = rl == t;
+                const float mine = (t & 1) ? d.y : d.x;
+                const float piv = __shfl_sync(0xffffffffu, mine, 4 * t + (t >> 1));
+                const float f = __shfl_sync(0xffffffffu, mine, (lane & ~3) | (t >> 1));
+                const float px = __shfl_sync(0xffffffffu, d.x, 4 * t + (lane & 3)), py = __shfl_sync(0xffffffffu, d.y, 4 * t + (lane & 3));
+                float ip;
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ip) : "f"(piv));
+                bad |= !(fabsf(piv) > 0.0f) || !(fabsf(piv) < INFINITY);
+                const bool own = (lane >> 2) == t, here = (lane & 3) == (t >> 1);
                 const float a = own ? 0.0f : 1.0f, bq = own ? ip : -f * ip;
-#pragma unroll
-                for (int q = 0; q < 16; ++q) v[q] = fmaf(bq, p[q], a * v[q]);
-                if (g == cg) {
-                    if (half) v[8 + t] = bq;
-                    else v[t] = bq;
-                }
+                const float nx = fmaf(bq, px, a * d.x), ny = fmaf(bq, py, a * d.y);
+                d.x = (here && !(t & 1)) ? bq : nx;
+                d.y = (here && (t & 1)) ? bq : ny;
             }
+            *reinterpret_cast<float2 *>(&dinv[lane >> 2][2 * (lane & 3)]) = d;
             if (bad) sbad = 1;
-#pragma unroll
-            for (int q = 0; q < 16; q += 4)
-                *reinterpret_cast<float4 *>(&panel[rl][16 * g + q]) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-        } else if (g == cg) {
-            const float4 a0 = half ? make_float4(v[8], v[9], v[10], v[11]) : make_float4(v[0], v[1], v[2], v[3]);
-            const float4 a1 = half ? make_float4(v[12], v[13], v[14], v[15]) : make_float4(v[4], v[5], v[6], v[7]);
-            *reinterpret_cast<float4 *>(&colg[r][0]) = a0;
-            *reinterpret_cast<float4 *>(&colg[r][4]) = a1;
         }
         __syncthreads();
-        if (w != m) {
-            const float4 a0 = *reinterpret_cast<const float4 *>(&colg[r][0]);
-            const float4 a1 = *reinterpret_cast<const float4 *>(&colg[r][4]);
-            const float ag[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            if (g == cg) {  // the panel's columns are replaced, not updated
+        {  // two of the row's eight coefficients: -a_r D^-1 outside the panel, row r of D^-1 inside
+            const int r = threadIdx.x >> 2, s = 2 * (threadIdx.x & 3);
+            float cx = 0.0f, cy = 0.0f;
+            if ((r >> 3) == m) {
+                cx = dinv[r & 7][s];
+                cy = dinv[r & 7][s + 1];
+            } else {
+                const float4 a0 = *reinterpret_cast<const float4 *>(&cols[par][r][0]), a1 = *reinterpret_cast<const float4 *>(&cols[par][r][4]);
+                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    if (half) v[8 + q] = 0.0f;
-                    else v[q] = 0.0f;
+                for (int t = 0; t < 8; ++t) {
+                    const float2 e = *reinterpret_cast<const float2 *>(&dinv[t][s]);
+                    cx = fmaf(-av[t], e.x, cx);
+                    cy = fmaf(-av[t], e.y, cy);
                 }
             }
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-#pragma unroll
-                for (int q = 0; q < 16; q += 4) {
-                    const float4 pp = *reinterpret_cast<const float4 *>(&panel[t][16 * g + q]);
-                    v[q] = fmaf(-ag[t], pp.x, v[q]);
-                    v[q + 1] = fmaf(-ag[t], pp.y, v[q + 1]);
-                    v[q + 2] = fmaf(-ag[t], pp.z, v[q + 2]);
-                    v[q + 3] = fmaf(-ag[t], pp.w, v[q + 3]);
-                }
-            }
+            coef[s][r] = cx;
+            coef[s + 1][r] = cy;
         }
-        __syncthreads();  // panel and colg are rewritten by the next panel
-    }
-    const bool bad = sbad != 0;
+        __syncthreads();
+        if (prow)
 #pragma unroll
-    for (int q = 0; q < 16; q += 4)
-        *reinterpret_cast<float4 *>(X + r * kInvLd + 16 * g + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-    // Newton step: W = D, then W = I - D X, then X + X W straight to dv
-    load_pivot_block(A, n, k0, b, W);
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int s = 0; s < 4; ++s) v[u][s] = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+            const float4 p4 = *reinterpret_cast<const float4 *>(&rows[par][t][4 * tx]);
+            const float4 c4 = *reinterpret_cast<const float4 *>(&coef[t][4 * ty]);
+            const float p[4] = {p4.x, p4.y, p4.z, p4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int s = 0; s < 4; ++s) v[u][s] = fmaf(c[u], p[s], v[u][s]);
+        }
+        if (pcol)  // the panel's columns hold the coefficients themselves
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const float4 c4 = *reinterpret_cast<const float4 *>(&coef[4 * (tx & 1) + s][4 * ty]);
+                v[0][s] = c4.x;
+                v[1][s] = c4.y;
+                v[2][s] = c4.z;
+                v[3][s] = c4.w;
+            }
+    }
+    const int r0 = 4 * ty, c0 = 4 * tx;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        *reinterpret_cast<float4 *>(X + (r0 + u) * kInvLd + c0) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
     __syncthreads();
     float acc[4][4];
     block_gemm64(W, X, acc);
     __syncthreads();
-    const int r0 = 4 * (threadIdx.x >> 4), c0 = 4 * (threadIdx.x & 15);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int w = 0; w < 4; ++w) W[(r0 + u) * kInvLd + c0 + w] = (r0 + u == c0 + w ? 1.0f : 0.0f) - acc[u][w];
+        for (int q = 0; q < 4; ++q) W[(r0 + u) * kInvLd + c0 + q] = (r0 + u == c0 + q ? 1.0f : 0.0f) - acc[u][q];
     __syncthreads();
     block_gemm64(X, W, acc);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const int rr = r0 + u, c = c0 + w;
-            dv[rr * kGjBlock + c] = (rr < b && c < b) ? X[rr * kInvLd + c] + acc[u][w] : 0.0f;
+        for (int q = 0; q < 4; ++q) {
+            const int rr = r0 + u, c = c0 + q;
+            dv[rr * kGjBlock + c] = (rr < b && c < b) ? v[u][q] + acc[u][q] : 0.0f;
         }
     if (threadIdx.x == 0) {
-        if (bad) *ok = 0;
+        if (sbad) *ok = 0;
         else if (K == 0) *ok = 1;
     }
 }
