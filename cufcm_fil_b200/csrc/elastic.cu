@@ -51,7 +51,8 @@ struct cf_elastic {
     float *v = nullptr;  // [6N]
     double *jinv = nullptr;  // [F][6S][6S]
     double *err = nullptr, *nerr = nullptr, *upd = nullptr, *C = nullptr, *D = nullptr, *dots = nullptr,
-           *scal = nullptr;
+           *dpart = nullptr;  // dots: of one iteration's residual with the pairs; dpart: the filaments' shares
+    unsigned int *counter = nullptr;
     int *flags = nullptr, *h_flags = nullptr;
     int last_iters = 0, total_iters = 0, max_iters = 0, steps = 0;
     bool stepped = false;
@@ -265,17 +266,19 @@ __device__ inline void moment_derivative(const ElDev &d, const Q4 &q1, const Q4 
     }
 }
 
-// Robot arm: x_k = x_{k-1} + DL/2 (t_{k-1} + t_k) from the base (one thread).
-__device__ inline void robot_arm(const ElDev &d, int m) {
+// Robot arm: x_k = x_{k-1} + DL/2 (t_{k-1} + t_k) from the base.  Called by all threads of a block of 32: the tangents in
+// parallel into tan [S][3] (shared), then one thread per component adds along the filament.
+__device__ inline void robot_arm(const ElDev &d, int m, double (*tan)[3]) {
     const int S = d.S;
-    double *x = d.x + 3 * m * S;
-    const double *q = d.q + 4 * m * S;
-    double t1[3], t2[3];
-    qtan(qload(q), t1);
-    for (int k = 1; k < S; ++k) {
-        qtan(qload(q + 4 * k), t2);
-        for (int c = 0; c < 3; ++c) x[3 * k + c] = x[3 * (k - 1) + c] + 0.5 * d.DL * (t1[c] + t2[c]);
-        for (int c = 0; c < 3; ++c) t1[c] = t2[c];
+    for (int k = threadIdx.x; k < S; k += blockDim.x) qtan(qload(d.q + 4 * (static_cast<size_t>(m) * S + k)), tan[k]);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double *x = d.x + 3 * static_cast<size_t>(m) * S + threadIdx.x;
+        double a = x[0];
+        for (int k = 1; k < S; ++k) {
+            a = a + 0.5 * d.DL * (tan[k - 1][threadIdx.x] + tan[k][threadIdx.x]);
+            x[3 * k] = a;
+        }
     }
 }
 
@@ -285,6 +288,7 @@ __device__ inline void robot_arm(const ElDev &d, int m) {
 // base with u = 0 (accept_state_from_rigid_body); positions by the robot arm; the multipliers are
 // extrapolated linearly (step 2) or quadratically (step 3 on).  One block of 32 threads per filament.
 __global__ void el_initial_guess_kernel(ElDev d, int nt) {
+    __shared__ double tan[kMaxSeg][3];
     const int m = blockIdx.x, S = d.S;
     for (int k = threadIdx.x; k < S; k += blockDim.x) {
         const int i = m * S + k;
@@ -334,13 +338,13 @@ __global__ void el_initial_guess_kernel(ElDev d, int nt) {
         extrap(d.clp, d.clpm1, d.clpm2, 3 * m + threadIdx.x);
     }
     __syncthreads();
-    if (threadIdx.x == 0) robot_arm(d, m);
+    robot_arm(d, m, tan);
 }
 
 // filament::update (filament.cpp:2174-2206): multipliers += their updates, u_k += update and
-// q_k = exp(u_k) q_k^{n-1} for k >= 1, then the robot arm.  One block of 32 threads per filament.
-__global__ void el_update_kernel(ElDev d, const double *du) {
-    const int m = blockIdx.x, S = d.S;
+// q_k = exp(u_k) q_k^{n-1} for k >= 1, then the robot arm (all 32 threads of the filament's block).
+__device__ inline void apply_update(const ElDev &d, int m, const double *du, double (*tan)[3]) {
+    const int S = d.S;
     const double *w = du + static_cast<size_t>(6) * S * m;
     for (int k = threadIdx.x; k < S; k += blockDim.x) {
         if (k == 0) {
@@ -357,16 +361,20 @@ __global__ void el_update_kernel(ElDev d, const double *du) {
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) robot_arm(d, m);
+    robot_arm(d, m, tan);
+    __syncthreads();
 }
 
 // internal_forces_and_torques (filament.cpp:1745-1853) for instability cilia: FP64 forces and
 // torques f [6N], then their FP32 copy (with the barrier forces added by el_barrier_kernel) for the
 // pair kernel.  One block per filament, one thread per link; the link terms are collected in
-// shared memory and added segment by segment in the reference's order.
-__global__ void el_forces_kernel(ElDev d, int nt) {
+// shared memory and added segment by segment in the reference's order.  With du, the state first takes
+// that Broyden update.
+__global__ void el_forces_kernel(ElDev d, int nt, const double *du) {
     __shared__ double lk[kMaxSeg][12];  // per link: force on k, torque on k, force on k+1, torque on k+1
+    __shared__ double tan[kMaxSeg][3];
     const int m = blockIdx.x, S = d.S;
+    if (du) apply_update(d, m, du, tan);
     const int i0 = m * S;
     for (int k = threadIdx.x; k < S - 1; k += blockDim.x) {
         const double *lam = d.lam + 3 * (m * (S - 1) + k);
@@ -425,48 +433,97 @@ __global__ void el_forces_kernel(ElDev d, int nt) {
 // a repulsion growing as the fourth power of the overlap within 1.1 (a_i + a_j) of another segment
 // (not the segment itself nor its neighbours in the same filament) and within DL/2 of the wall;
 // added in FP64 to the internal forces and packed as FP32 for the pair kernel.  A block takes 16
-// targets; its threads split the sources sixteen ways (split c takes every sixteenth of each
-// 1024-source tile staged in shared memory), screen the pairs on the FP32 positions with a margin and
-// evaluate the few within reach in FP64; the sixteen partial sums are added in a fixed order.
+// targets.  Sources are taken in tiles of 1024: its threads first keep, in order, those within reach
+// of the targets' bounding box (one test per source instead of one per pair; the targets are
+// neighbours along a filament, so few pass), then split the kept ones sixteen ways, screen the pairs
+// on the FP32 positions with a margin and evaluate those within reach in FP64; the sixteen partial
+// sums are added in a fixed order.  Bound by the chain of tiles: 256 filaments of 20 take 11 us, where
+// screening every pair without the bounding box took 37.
 constexpr int kBarTargets = 16, kBarSplit = 16, kBarThreads = kBarTargets * kBarSplit, kBarTile = 1024;
+constexpr float kBarReach = 2.22f;  // above 1.1 (a_i + a_j) = 2.2 by more than the FP32 rounding of positions
 __global__ void __launch_bounds__(kBarThreads) el_barrier_kernel(ElDev d) {
     __shared__ float4 sx[kBarTile];
+    __shared__ int sj[kBarTile];
+    __shared__ int woff[kBarThreads / 32 + 1];
     __shared__ double part[kBarSplit][kBarTargets][3];
     const int t = threadIdx.x % kBarTargets, c = threadIdx.x / kBarTargets;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i = blockIdx.x * kBarTargets + t;
     const bool live = i < d.N;
+    const float4 xf = d.x4[min(i, d.N - 1)];
     double xi[3] = {0.0, 0.0, 0.0}, fb[3] = {0.0, 0.0, 0.0};
-    float4 xf = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (live) {
         for (int q = 0; q < 3; ++q) xi[q] = d.x[3 * i + q];
-        xf = d.x4[i];
         if (c == 0 && xi[2] < 0.5 * d.DL) {
-            const double w = fmin(1.0, 1.0 - (xi[2] - 1.0) / (0.5 * d.DL - 1.0));
-            fb[2] = d.frep * w * w * w * w;
+            const double w4 = fmin(1.0, 1.0 - (xi[2] - 1.0) / (0.5 * d.DL - 1.0));
+            fb[2] = d.frep * w4 * w4 * w4 * w4;
         }
+    }
+    // the targets' box, grown by the reach (every warp holds all sixteen targets in its lanes)
+    float lo[3] = {xf.x, xf.y, xf.z}, hi[3] = {xf.x, xf.y, xf.z};
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            lo[q] = fminf(lo[q], __shfl_xor_sync(0xffffffffu, lo[q], o));
+            hi[q] = fmaxf(hi[q], __shfl_xor_sync(0xffffffffu, hi[q], o));
+        }
+    for (int q = 0; q < 3; ++q) {
+        lo[q] -= kBarReach;
+        hi[q] += kBarReach;
     }
     const int fi = live ? i / d.S : -1;
     for (int j0 = 0; j0 < d.N; j0 += kBarTile) {
         const int nj = min(kBarTile, d.N - j0);
         __syncthreads();
-        for (int q = threadIdx.x; q < nj; q += kBarThreads) sx[q] = d.x4[j0 + q];
+        int kept = 0;  // thread-contiguous runs of four sources keep the list in source order
+        float4 p[4];
+        bool in[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int jj = 4 * threadIdx.x + q;
+            p[q] = jj < nj ? d.x4[j0 + jj] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            // a NaN position is kept: the test below then rejects it, as it rejects NaN distances
+            in[q] = jj < nj && !(p[q].x < lo[0] || p[q].x > hi[0] || p[q].y < lo[1] || p[q].y > hi[1] || p[q].z < lo[2] ||
+                                 p[q].z > hi[2]);
+            kept += in[q] ? 1 : 0;
+        }
+        int upto = kept;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += u;
+        }
+        if (lane == 31) woff[w] = upto;
+        __syncthreads();
+        int at = upto - kept, total = 0;
+        for (int q = 0; q < kBarThreads / 32; ++q) {
+            if (q < w) at += woff[q];
+            total += woff[q];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (in[q]) {
+                sx[at] = p[q];
+                sj[at++] = j0 + 4 * threadIdx.x + q;
+            }
         __syncthreads();
         if (!live) continue;
-        for (int jj = c; jj < nj; jj += kBarSplit) {
-            const float4 sj = sx[jj];
-            const float ex = xf.x - sj.x, ey = xf.y - sj.y, ez = xf.z - sj.z;
+        for (int jj = c; jj < total; jj += kBarSplit) {
+            const float4 xs = sx[jj];
+            const float ex = xf.x - xs.x, ey = xf.y - xs.y, ez = xf.z - xs.z;
             if (ex * ex + ey * ey + ez * ez >= 4.9f) continue;  // screen: (1.1 * 2a)^2 = 4.84, with margin
-            const int js = j0 + jj;
+            const int js = sj[jj];
             const double dx = xi[0] - d.x[3 * js], dy = xi[1] - d.x[3 * js + 1], dz = xi[2] - d.x[3 * js + 2];
             const double r2 = dx * dx + dy * dy + dz * dz;
             if (r2 >= 4.84) continue;
             if (fi == js / d.S && abs(i - js) <= 1) continue;
             const double r = sqrt(r2);
-            double w = fmin(1.0, 1.0 - 5.0 * (r - 2.0));
-            w = d.frep * w * w * w * w;
-            fb[0] += w * dx / r;
-            fb[1] += w * dy / r;
-            fb[2] += w * dz / r;
+            double w4 = fmin(1.0, 1.0 - 5.0 * (r - 2.0));
+            w4 = d.frep * w4 * w4 * w4 * w4;
+            fb[0] += w4 * dx / r;
+            fb[1] += w4 * dy / r;
+            fb[2] += w4 * dz / r;
         }
     }
     for (int q = 0; q < 3; ++q) part[c][t][q] = fb[q];
@@ -692,149 +749,242 @@ __global__ void el_jacobian_kernel(ElDev d, int nt) {
     }
 }
 
-// In-place Gauss-Jordan inversion with partial pivoting of each filament's 6S x 6S block (FP64,
-// held in shared memory); a zero pivot column sets the non-finite flag.  Per pivot, three barriers:
-// warp 0 finds the pivot row; the pivot row, row k and the pivot column are saved; then the row
-// interchange, the scaling of the pivot row and the rank-one update are one pass in which every element
-// is written from its own old value and the saved vectors, over a 2-D split of the matrix (warp w takes
-// rows w, w + 16, ..., its lanes consecutive columns).
-constexpr int kInvThreads = 512;
-__global__ void __launch_bounds__(kInvThreads) el_invert_kernel(ElDev d, int *flags) {
+// In-place Gauss-Jordan inversion with partial pivoting of each filament's 6S x 6S block (FP64, held in
+// shared memory); a zero pivot column sets the non-finite flag.  Eight pivots (a panel of eight
+// columns) at a time, without moving rows:
+//   (a) every row's eight entries of the panel sit in one thread's registers.  Per pivot, each warp
+//       finds its largest unused entry (two 32-bit warp maxima over the bits of |a|) and publishes that
+//       row's entries; after one barrier every thread picks the largest of the warps' rows and updates
+//       its own row, which leaves the panel's columns of the partly inverted matrix;
+//   (b) the eight pivot rows are copied out, and every other column takes the rank-8 update
+//       A[r][c] = (r a pivot row ? 0 : A[r][c]) + sum_s P[r][s] A_old[p_s][c], P the panel's columns:
+//       a warp holds its share of the eight rows in registers and reads and writes each row once.
+// After the last panel, row p_k of A holds solution row k and column k belongs to equation p_k, so
+// inverse[k][p_j] = A[p_k][j].
+//
+// Bound by shared memory: the matrix moves twice per panel, 2 x 115 KB x 15 at S = 20, where one pivot
+// at a time moves it 120 times: 256 blocks of 120 x 120 (two waves) take 314 us, one at a time 800.
+constexpr int kInvThreads = 512, kInvPanel = 8, kInvRowWarps = (6 * kMaxSeg + 31) / 32;
+__host__ __device__ constexpr size_t inv_smem_doubles(int n) { return static_cast<size_t>(n) * n + 2 * kInvPanel * n; }
+// Barrier among the first `threads` threads (whole warps).
+__device__ __forceinline__ void row_barrier(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+__global__ void __launch_bounds__(kInvThreads, 1) el_invert_kernel(ElDev d, int *flags) {
     extern __shared__ double A[];
-    __shared__ int piv_row[6 * kMaxSeg];
-    __shared__ double colk[6 * kMaxSeg], prow_s[6 * kMaxSeg], rowk_s[6 * kMaxSeg];
-    __shared__ int sp;
+    __shared__ double cand[2][kInvRowWarps][kInvPanel + 1];  // each warp's candidate row and 1 / pivot, by pivot parity
+    __shared__ unsigned long long key[2][kInvRowWarps];      // bits of its |pivot|
+    __shared__ int crow[2][kInvRowWarps], piv_row[6 * kMaxSeg], singular_s;
+    __shared__ unsigned char rank_of[6 * kMaxSeg];           // position in the current panel of a pivot row, or 255
     const int m = blockIdx.x, n = 6 * d.S;
+    double *P = A + static_cast<size_t>(n) * n;  // [n][8] panel columns
+    double *X = P + kInvPanel * n;               // [8][n] pivot rows before the update
     double *J = d.jinv + static_cast<size_t>(m) * n * n;
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) A[e] = J[e];
+    for (int e = threadIdx.x; e < n * n / 2; e += blockDim.x)  // n * n is a multiple of 36
+        reinterpret_cast<double2 *>(A)[e] = reinterpret_cast<const double2 *>(J)[e];
+    if (threadIdx.x == 0) singular_s = 0;
     __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    bool singular = false;
-    for (int k = 0; k < n; ++k) {
-        if (w == 0) {  // pivot: the largest |A[r][k]|, r >= k (lowest index among ties)
-            double best = -1.0;
-            int bi = k;
-            for (int r = k + lane; r < n; r += 32) {
-                const double a = fabs(A[r * n + k]);
-                if (a > best) {
-                    best = a;
-                    bi = r;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int row_warps = (n + 31) / 32, row = threadIdx.x;
+    const bool holds = row < n;
+    bool used = !holds;
+    for (int K = 0; K < n; K += kInvPanel) {
+        const int kb = min(kInvPanel, n - K);
+        if (w < row_warps) {  // (a), by the warps that hold the rows
+            double v[kInvPanel];
+            if (holds) rank_of[row] = 255;
+#pragma unroll
+            for (int q = 0; q < kInvPanel; ++q) v[q] = (holds && q < kb) ? A[row * n + K + q] : 0.0;
+            bool singular = false;
+#pragma unroll
+            for (int t = 0; t < kInvPanel; ++t) {
+                if (t >= kb || singular) continue;  // uniform over these warps
+                const int par = t & 1;
+                const double a = fabs(v[t]), inv_own = 1.0 / v[t];
+                const unsigned long long bits = (used || !(a == a)) ? 0ull : static_cast<unsigned long long>(__double_as_longlong(a));
+                const unsigned hi = static_cast<unsigned>(bits >> 32);
+                const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+                const unsigned lo = hi == mh ? static_cast<unsigned>(bits) : 0u;
+                const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+                const unsigned who = __ballot_sync(0xffffffffu, hi == mh && lo == ml && !used);
+                if (who != 0u && lane == __ffs(who) - 1) {
+                    key[par][w] = bits;
+                    crow[par][w] = row;
+#pragma unroll
+                    for (int q = 0; q < kInvPanel; ++q) cand[par][w][q] = v[q];
+                    cand[par][w][kInvPanel] = inv_own;
+                } else if (who == 0u && lane == 0) {
+                    key[par][w] = 0ull;
+                }
+                row_barrier(32 * row_warps);
+                int best = 0;
+                unsigned long long bk = key[par][0];
+                for (int q = 1; q < row_warps; ++q) {
+                    const unsigned long long kq = key[par][q];
+                    if (kq > bk) {
+                        bk = kq;
+                        best = q;
+                    }
+                }
+                if (bk == 0ull) {
+                    singular = true;
+                    continue;
+                }
+                const int p = crow[par][best];
+                const double inv = cand[par][best][kInvPanel];
+                if (row == p) {
+                    used = true;
+                    piv_row[K + t] = p;
+                    rank_of[p] = static_cast<unsigned char>(t);
+#pragma unroll
+                    for (int q = 0; q < kInvPanel; ++q) v[q] = q == t ? inv : v[q] * inv;
+                } else {
+                    const double f = -v[t] * inv;
+#pragma unroll
+                    for (int q = 0; q < kInvPanel; ++q) v[q] = q == t ? f : fma(f, cand[par][best][q], v[q]);
                 }
             }
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_down_sync(0xffffffffu, best, o);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) {
-                    best = ob;
-                    bi = oi;
+            if (singular && row == 0) singular_s = 1;
+            if (holds) {
+                double2 *o = reinterpret_cast<double2 *>(P + row * kInvPanel);
+#pragma unroll
+                for (int q = 0; q < kInvPanel; q += 2) o[q / 2] = make_double2(q < kb ? v[q] : 0.0, q + 1 < kb ? v[q + 1] : 0.0);
+            }
+        }
+        __syncthreads();  // piv_row, rank_of and P are complete
+        if (singular_s) break;
+        for (int e = threadIdx.x; e < kInvPanel * n; e += blockDim.x) {
+            const int t = e / n, c = e - t * n;
+            X[e] = t < kb ? A[piv_row[K + t] * n + c] : 0.0;
+        }
+        __syncthreads();
+        constexpr int kSpan = 4;  // (b): 128 columns at a time, four a lane, the warp's share of X in registers
+        for (int c0 = lane; c0 < n; c0 += 32 * kSpan) {
+            double x[kSpan][kInvPanel];
+#pragma unroll
+            for (int u = 0; u < kSpan; ++u)
+#pragma unroll
+                for (int t = 0; t < kInvPanel; ++t) x[u][t] = c0 + 32 * u < n ? X[t * n + c0 + 32 * u] : 0.0;
+            for (int r = w; r < n; r += kInvThreads / 32) {
+                const bool own = rank_of[r] != 255;
+                const double2 *pr = reinterpret_cast<const double2 *>(P + r * kInvPanel);
+                const double2 p0 = pr[0], p1 = pr[1], p2 = pr[2], p3 = pr[3];
+                const double pv[kInvPanel] = {p0.x, p0.y, p1.x, p1.y, p2.x, p2.y, p3.x, p3.y};
+                double *Ar = A + r * n + c0;
+#pragma unroll
+                for (int u = 0; u < kSpan; ++u) {
+                    const int c = c0 + 32 * u;
+                    if (c < n) {
+                        double a = own ? 0.0 : Ar[32 * u];
+#pragma unroll
+                        for (int t = 0; t < kInvPanel; ++t) a = fma(pv[t], x[u][t], a);
+                        Ar[32 * u] = (c >= K && c < K + kb) ? P[r * kInvPanel + c - K] : a;
+                    }
                 }
             }
-            if (lane == 0) {
-                sp = (best > 0.0) ? bi : -1;
-                piv_row[k] = sp < 0 ? k : sp;
-            }
-        }
-        __syncthreads();
-        const int p = sp;
-        if (p < 0) {
-            singular = true;
-            break;
-        }
-        // save the scaled pivot row (old row p times 1/pivot, 1/pivot in column k), old row k and the pivot
-        // column with rows k and p interchanged
-        const double inv = 1.0 / A[p * n + k];
-        for (int c = threadIdx.x; c < n; c += blockDim.x) {
-            prow_s[c] = (c == k) ? inv : A[p * n + c] * inv;
-            rowk_s[c] = A[k * n + c];
-        }
-        for (int r = threadIdx.x; r < n; r += blockDim.x) colk[r] = A[(r == k ? p : (r == p ? k : r)) * n + k];
-        __syncthreads();
-        // every element from its own old value and the saved vectors: row k becomes the scaled pivot row, every
-        // other row (row p holding old row k after the interchange) loses its pivot-column entry times it; the
-        // lane that wrote a row's column-k entry then replaces it by -entry / pivot
-        for (int r = w; r < n; r += nw) {
-            double *Ar = A + r * n;
-            if (r == k) {
-                for (int c = lane; c < n; c += 32) Ar[c] = prow_s[c];
-                continue;
-            }
-            const double fr = colk[r];
-            const double *src = (r == p) ? rowk_s : Ar;
-            for (int c = lane; c < n; c += 32) Ar[c] = fma(-fr, prow_s[c], src[c]);
-            if (lane == (k & 31)) Ar[k] = -fr * inv;
         }
         __syncthreads();
     }
-    if (singular) {
+    if (singular_s) {
         if (threadIdx.x == 0) atomicOr(flags, kNonFinite);
         return;
     }
-    // undo the row interchanges as column interchanges, last first
-    for (int k = n - 1; k >= 0; --k) {
-        const int p = piv_row[k];
-        if (p != k)
-            for (int r = threadIdx.x; r < n; r += blockDim.x) {
-                const double t = A[r * n + k];
-                A[r * n + k] = A[r * n + p];
-                A[r * n + p] = t;
-            }
-        __syncthreads();
+    for (int r = w; r < n; r += kInvThreads / 32) {
+        const double *Ar = A + piv_row[r] * n;
+        for (int c = lane; c < n; c += 32) J[static_cast<size_t>(r) * n + piv_row[c]] = Ar[c];
     }
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) J[e] = A[e];
 }
 
-// out_m = s * Jinv_m in_m per filament (swimmer::jacobian_inv_mult); one warp per row.
-__global__ void el_jinv_mult_kernel(ElDev d, const double *in, double *out, double s) {
+// Rows r = first, first + step, ... of s * Jinv x for one filament, four rows of a warp in flight; write(r, value).
+template <class Write>
+__device__ __forceinline__ void jinv_rows(const double *__restrict__ J, const double *x, int n, double s, int w, int nw,
+                                          int lane, Write write) {
+    constexpr int kRows = 4;
+    for (int r0 = kRows * w; r0 < n; r0 += kRows * nw) {
+        double a[kRows] = {0.0, 0.0, 0.0, 0.0};
+        const double2 *Jr = reinterpret_cast<const double2 *>(J + static_cast<size_t>(r0) * n);  // n is a multiple of 6
+        const double2 *x2 = reinterpret_cast<const double2 *>(x);
+        for (int c = lane; c < n / 2; c += 32) {
+            const double2 xv = x2[c];
+#pragma unroll
+            for (int q = 0; q < kRows; ++q)
+                if (r0 + q < n) {
+                    const double2 j = __ldg(Jr + static_cast<size_t>(q) * (n / 2) + c);
+                    a[q] = fma(j.x, xv.x, fma(j.y, xv.y, a[q]));
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < kRows; ++q) {
+            const double v = warp_sum(a[q]);
+            if (lane == 0 && r0 + q < n) write(r0 + q, s * v);
+        }
+    }
+}
+
+// First update of a step: out_m = s * Jinv_m in_m (swimmer::jacobian_inv_mult); one block per filament.
+__global__ void __launch_bounds__(512) el_jinv_mult_kernel(ElDev d, const double *in, double *out, double s) {
+    __shared__ __align__(16) double x[6 * kMaxSeg];
     const int m = blockIdx.x, n = 6 * d.S;
-    const double *J = d.jinv + static_cast<size_t>(m) * n * n;
-    const double *x = in + static_cast<size_t>(m) * n;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int r = w; r < n; r += nw) {
+    for (int c = threadIdx.x; c < n; c += blockDim.x) x[c] = in[static_cast<size_t>(m) * n + c];
+    __syncthreads();
+    double *o = out + static_cast<size_t>(m) * n;
+    jinv_rows(d.jinv + static_cast<size_t>(m) * n * n, x, n, s, threadIdx.x >> 5, blockDim.x >> 5, threadIdx.x & 31,
+              [&](int r, double v) { o[r] = v; });
+}
+
+// The products of one Broyden iteration (broyden_solver::end_of_iter), one block per filament: the raw new column
+// -conf Jinv nerr into Ck, the raw difference nerr - err into Dk, and the filament's share of <nerr, D_i>, i < k, of
+// |Dk|^2 and of <nerr, Dk>.  The block arriving last sums the filaments' shares in order into dots[0 .. k + 1].
+__global__ void __launch_bounds__(512) el_column_kernel(ElDev d, const double *err, const double *nerr, const double *D,
+                                                        double *Ck, double *Dk, double s, int k, double *part,
+                                                        double *dots, unsigned int *counter) {
+    __shared__ __align__(16) double x[6 * kMaxSeg];
+    __shared__ double sd[6 * kMaxSeg];
+    __shared__ int last;
+    const int m = blockIdx.x, n = 6 * d.S, nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t at = static_cast<size_t>(m) * n;
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
+        x[c] = nerr[at + c];
+        sd[c] = x[c] - err[at + c];
+        Dk[at + c] = sd[c];
+    }
+    __syncthreads();
+    jinv_rows(d.jinv + at * n, x, n, s, w, nw, lane, [&](int r, double v) { Ck[at + r] = v; });
+    for (int i = w; i < k + 2; i += nw) {
+        const double *col = i < k ? D + static_cast<size_t>(i) * d.NB + at : sd;
+        const double *other = i == k ? sd : x;
         double a = 0.0;
-        for (int c = lane; c < n; c += 32) a += J[static_cast<size_t>(r) * n + c] * x[c];
+        for (int c = lane; c < n; c += 32) a += other[c] * col[c];
         a = warp_sum(a);
-        if (lane == 0) out[static_cast<size_t>(m) * n + r] = s * a;
+        if (lane == 0) part[static_cast<size_t>(m) * (k + 2) + i] = a;
     }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = w; i < k + 2; i += nw) {
+        double a = 0.0;
+        for (int f = lane; f < d.F; f += 32) a += __ldcg(part + static_cast<size_t>(f) * (k + 2) + i);
+        a = warp_sum(a);
+        if (lane == 0) dots[i] = a;
+    }
+    if (threadIdx.x == 0) *counter = 0u;
 }
 
-// dots[i] = <vec, D_i>, i < k (one block per column, fixed-order block sum).
-__global__ void el_dots_kernel(const double *vec, const double *D, size_t ld, int len, double *dots) {
-    __shared__ double sm32[32];
-    const double *col = D + static_cast<size_t>(blockIdx.x) * ld;
-    double a = 0.0;
-    for (int i = threadIdx.x; i < len; i += blockDim.x) a += vec[i] * col[i];
-    a = block_sum(a, sm32);
-    if (threadIdx.x == 0) dots[blockIdx.x] = a;
-}
-
-// out -= sum_i dots[i] C_i, i = 0..k-1 in order (the reference's sequential column updates).
-__global__ void el_sub_cols_kernel(double *out, const double *C, size_t ld, const double *dots, int k, int len) {
+// The finished pair and the next update (broyden_solver::end_of_iter, find_update): C_k = (raw - sum_i <nerr, D_i> C_i)
+// / |D_k| (i in order), D_k /= |D_k|, and, err being the new residual from here on,
+// update = -conf Jinv err - sum_{i <= k} <err, D_i> C_i = (the undivided C_k) - <err, D_k> C_k.
+__global__ void el_pair_kernel(double *Ck, double *Dk, const double *C, size_t ld, const double *dots, int k, int len,
+                               double *upd) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= len) return;
-    double a = out[i];
+    double a = Ck[i];
     for (int j = 0; j < k; ++j) a -= dots[j] * C[static_cast<size_t>(j) * ld + i];
-    out[i] = a;
-}
-
-// D_k = nerr - err and its norm into scal[0] (one block).
-__global__ void el_diff_norm_kernel(const double *nerr, const double *err, double *Dk, int len, double *scal) {
-    __shared__ double sm32[32];
-    double a = 0.0;
-    for (int i = threadIdx.x; i < len; i += blockDim.x) {
-        const double t = nerr[i] - err[i];
-        Dk[i] = t;
-        a += t * t;
-    }
-    a = block_sum(a, sm32);
-    if (threadIdx.x == 0) scal[0] = sqrt(a);
-}
-
-__global__ void el_scale2_kernel(double *a, double *b, int len, const double *scal) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= len) return;
-    const double s = scal[0];
-    a[i] /= s;
-    b[i] /= s;
+    const double norm = sqrt(dots[k]);
+    const double c = a / norm;
+    Ck[i] = c;
+    Dk[i] /= norm;
+    upd[i] = a - (dots[k + 1] / norm) * c;
 }
 
 // ------------------------------------------------------------ host side
@@ -889,12 +1039,12 @@ ElDev dev(const cf_elastic *h) {
 
 int grid_for(int n, int t) { return std::max(1, (n + t - 1) / t); }
 
-// forces, barrier forces, the 6x6 wall mobility and the residual into e; the flags word is
+// with `update`, that update of the state; forces, barrier forces, the 6x6 wall mobility and the residual into e; the flags word is
 // cleared first and left on the device.
-int evaluate(cf_elastic *h, int nt, double *e) {
+int evaluate(cf_elastic *h, int nt, const double *update, double *e) {
     cudaStream_t st = h->stream;
     const ElDev d = dev(h);
-    el_forces_kernel<<<h->F, 32, 0, st>>>(d, nt);
+    el_forces_kernel<<<h->F, 32, 0, st>>>(d, nt, update);
     CF_CHECK_LAUNCH("el_forces_kernel");
     el_barrier_kernel<<<grid_for(h->N, kBarTargets), kBarThreads, 0, st>>>(d);
     CF_CHECK_LAUNCH("el_barrier_kernel");
@@ -912,7 +1062,11 @@ int evaluate(cf_elastic *h, int nt, double *e) {
     bd.ns = h->N;
     bd.as = 1.0f;
     bd.mu = 1.0f;
-    CF_TRY(rpy_block_product(bd, h->scratch, h->scratch_cap, h->flags + 1, h->v, 6, kOutWrite, h->num_sms, st));
+    // The tile kernel, not the symmetric one: the tethering and inextensibility multipliers carry the product's FP32
+    // rounding amplified a thousandfold, so another order of summation would move the forces by more than 2e-5.
+    const RpyPlan plan = rpy_plan(h->N, h->N, 6, 6, h->num_sms);
+    CF_TRY(rpy_launch_tiles(bd, plan, h->scratch, h->flags + 1, st));
+    CF_TRY(rpy_launch_reduce_f32(bd, plan, h->scratch, h->v, 6, kOutWrite, st, h->flags + 1));
     CF_CUDA(cudaMemsetAsync(h->flags, 0, sizeof(int), st));
     el_errors_kernel<<<grid_for(h->N, 256), 256, 0, st>>>(d, nt, h->tol, e, h->flags);
     CF_CHECK_LAUNCH("el_errors_kernel");
@@ -935,45 +1089,28 @@ int prepare_jacobian(cf_elastic *h, int nt) {
     const ElDev d = dev(h);
     el_jacobian_kernel<<<h->F, 64, 0, h->stream>>>(d, nt);
     CF_CHECK_LAUNCH("el_jacobian_kernel");
-    const size_t smem = sizeof(double) * 36 * h->S * h->S;
+    const size_t smem = sizeof(double) * inv_smem_doubles(6 * h->S);
     el_invert_kernel<<<h->F, kInvThreads, smem, h->stream>>>(d, h->flags);
     CF_CHECK_LAUNCH("el_invert_kernel");
     return CF_OK;
 }
 
-// update = -conf Jinv err - sum_i <err, D_i> C_i (broyden_solver::find_update)
-int find_update(cf_elastic *h, int iter) {
-    cudaStream_t st = h->stream;
-    const ElDev d = dev(h);
-    el_jinv_mult_kernel<<<h->F, 256, 0, st>>>(d, h->err, h->upd, -h->conf);
+// The step's first update, -conf Jinv err (broyden_solver::find_update without pairs).
+int first_update(cf_elastic *h) {
+    el_jinv_mult_kernel<<<h->F, 512, 0, h->stream>>>(dev(h), h->err, h->upd, -h->conf);
     CF_CHECK_LAUNCH("el_jinv_mult_kernel");
-    if (iter > 0) {
-        el_dots_kernel<<<iter, 512, 0, st>>>(h->err, h->D, h->NB, h->NB, h->dots);
-        CF_CHECK_LAUNCH("el_dots_kernel");
-        el_sub_cols_kernel<<<grid_for(h->NB, 256), 256, 0, st>>>(h->upd, h->C, h->NB, h->dots, iter, h->NB);
-        CF_CHECK_LAUNCH("el_sub_cols_kernel");
-    }
     return CF_OK;
 }
 
-// The new rank-one pair (broyden_solver::end_of_iter): C_k = (-conf Jinv nerr - sum_i <nerr, D_i> C_i)/|D_k|,
-// D_k = (nerr - err)/|D_k|; then err <-> nerr.
+// The new rank-one pair and the next update from it (broyden_solver::end_of_iter, find_update); then err <-> nerr.
 int end_of_iter(cf_elastic *h, int iter) {
     cudaStream_t st = h->stream;
-    const ElDev d = dev(h);
     double *Ck = h->C + static_cast<size_t>(iter) * h->NB, *Dk = h->D + static_cast<size_t>(iter) * h->NB;
-    el_jinv_mult_kernel<<<h->F, 256, 0, st>>>(d, h->nerr, Ck, -h->conf);
-    CF_CHECK_LAUNCH("el_jinv_mult_kernel");
-    if (iter > 0) {
-        el_dots_kernel<<<iter, 512, 0, st>>>(h->nerr, h->D, h->NB, h->NB, h->dots);
-        CF_CHECK_LAUNCH("el_dots_kernel");
-        el_sub_cols_kernel<<<grid_for(h->NB, 256), 256, 0, st>>>(Ck, h->C, h->NB, h->dots, iter, h->NB);
-        CF_CHECK_LAUNCH("el_sub_cols_kernel");
-    }
-    el_diff_norm_kernel<<<1, 1024, 0, st>>>(h->nerr, h->err, Dk, h->NB, h->scal);
-    CF_CHECK_LAUNCH("el_diff_norm_kernel");
-    el_scale2_kernel<<<grid_for(h->NB, 256), 256, 0, st>>>(Ck, Dk, h->NB, h->scal);
-    CF_CHECK_LAUNCH("el_scale2_kernel");
+    el_column_kernel<<<h->F, 512, 0, st>>>(dev(h), h->err, h->nerr, h->D, Ck, Dk, -h->conf, iter, h->dpart, h->dots,
+                                           h->counter);
+    CF_CHECK_LAUNCH("el_column_kernel");
+    el_pair_kernel<<<grid_for(h->NB, 128), 128, 0, st>>>(Ck, Dk, h->C, h->NB, h->dots, iter, h->NB, h->upd);
+    CF_CHECK_LAUNCH("el_pair_kernel");
     std::swap(h->err, h->nerr);
     return CF_OK;
 }
@@ -1073,19 +1210,14 @@ extern "C" int cf_elastic_create(const cf_elastic_config *cfg, cf_elastic **out)
             (rc = el_alloc(h, &h->jinv, static_cast<size_t>(F) * 36 * S * S)) || (rc = el_alloc(h, &h->err, NB)) ||
             (rc = el_alloc(h, &h->nerr, NB)) || (rc = el_alloc(h, &h->upd, NB)) ||
             (rc = el_alloc(h, &h->C, NB * h->maxb)) || (rc = el_alloc(h, &h->D, NB * h->maxb)) ||
-            (rc = el_alloc(h, &h->dots, static_cast<size_t>(h->maxb))) || (rc = el_alloc(h, &h->scal, 1)) ||
+            (rc = el_alloc(h, &h->dots, static_cast<size_t>(h->maxb) + 2)) ||
+            (rc = el_alloc(h, &h->dpart, static_cast<size_t>(F) * (h->maxb + 2))) ||
+            (rc = el_alloc(h, &h->counter, 1)) ||
             (rc = el_alloc(h, &h->flags, 2)))
             break;
-        RpyBlockDesc bd{};
-        bd.wall = 1;
-        bd.vd = 6;
-        bd.fd = 6;
-        bd.self_set = 1;
-        bd.nt = bd.ns = h->N;
-        bd.xt = bd.xs = h->x4;
-        h->scratch_cap = rpy_plan_for(bd, h->num_sms).scratch_float4;
+        h->scratch_cap = rpy_plan(h->N, h->N, 6, 6, h->num_sms).scratch_float4;
         if ((rc = el_alloc(h, &h->scratch, h->scratch_cap))) break;
-        const size_t inv_smem = sizeof(double) * 36 * S * S;
+        const size_t inv_smem = sizeof(double) * inv_smem_doubles(6 * S);
         if ((rc = cuda_status(cudaFuncSetAttribute(el_invert_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    static_cast<int>(inv_smem)),
                               "cudaFuncSetAttribute", __FILE__, __LINE__)))
@@ -1125,7 +1257,9 @@ extern "C" int cf_elastic_create(const cf_elastic_config *cfg, cf_elastic **out)
             (rc = up(h->pert, pert.data(), 6 * F)) || (rc = up(h->base, cfg->base_pos, 3 * F)) ||
             (rc = up(h->f, zeros.data(), 6 * N)))
             break;
-        if ((rc = cuda_status(cudaMemset(h->flags, 0, 2 * sizeof(int)), "cudaMemset", __FILE__, __LINE__))) break;
+        if ((rc = cuda_status(cudaMemset(h->flags, 0, 2 * sizeof(int)), "cudaMemset", __FILE__, __LINE__)) ||
+            (rc = cuda_status(cudaMemset(h->counter, 0, sizeof(unsigned int)), "cudaMemset", __FILE__, __LINE__)))
+            break;
     } while (0);
     if (rc != CF_OK) {
         const std::string msg = cf_last_error();
@@ -1144,22 +1278,20 @@ extern "C" int cf_elastic_step(cf_elastic *h, int nt, int *broyden_iters) {
     cudaStream_t st = h->stream;
     el_initial_guess_kernel<<<h->F, 32, 0, st>>>(dev(h), nt);
     CF_CHECK_LAUNCH("el_initial_guess_kernel");
-    CF_TRY(evaluate(h, nt, h->err));
+    CF_TRY(evaluate(h, nt, nullptr, h->err));
     int fl = 0;
     CF_TRY(read_flags(h, &fl));
     if (fl & kNonFinite) return set_error(CF_NONFINITE, "cf_elastic: non-finite residual at step %d", nt);
     bool too_large = (fl & kTooLarge) != 0;
     if (too_large) {
         CF_TRY(prepare_jacobian(h, nt));
+        CF_TRY(first_update(h));
         CF_TRY(read_flags(h, &fl));
         if (fl & kNonFinite) return set_error(CF_NONFINITE, "cf_elastic: singular approximate Jacobian at step %d", nt);
     }
     int iter = 0;
     while (too_large && iter < h->maxb) {
-        CF_TRY(find_update(h, iter));
-        el_update_kernel<<<h->F, 32, 0, st>>>(dev(h), h->upd);
-        CF_CHECK_LAUNCH("el_update_kernel");
-        CF_TRY(evaluate(h, nt, h->nerr));
+        CF_TRY(evaluate(h, nt, h->upd, h->nerr));
         CF_TRY(read_flags(h, &fl));
         if (fl & kNonFinite) {
             h->last_iters = iter + 1;
@@ -1227,7 +1359,7 @@ extern "C" int cf_elastic_first_evaluation(cf_elastic *h, int nt, double *err_ou
     CF_CUDA(cudaSetDevice(h->device));
     el_initial_guess_kernel<<<h->F, 32, 0, h->stream>>>(dev(h), nt);
     CF_CHECK_LAUNCH("el_initial_guess_kernel");
-    CF_TRY(evaluate(h, nt, h->err));
+    CF_TRY(evaluate(h, nt, nullptr, h->err));
     CF_TRY(prepare_jacobian(h, nt));
     int fl = 0;
     CF_TRY(read_flags(h, &fl));
