@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <new>
+#include <vector>
 
 struct cf_mobility {
     cf_mobility_config cfg{};
@@ -19,7 +20,7 @@ struct cf_mobility {
     float *x_blobs = nullptr, *f_blobs = nullptr, *v_blobs = nullptr;
     // float4 particle records used by the kernels.
     float4 *xs4 = nullptr, *fs4 = nullptr, *ts4 = nullptr;
-    float4 *xb4 = nullptr, *fb4 = nullptr;
+    float4 *xb4 = nullptr, *fb4 = nullptr;  // right behind the segments' records: both are one set too
     // Partial sums of the split-source products.
     float4 *scratch = nullptr;
     size_t scratch_cap = 0;
@@ -147,12 +148,33 @@ int eval_bs(cf_mobility *h, float *v_blobs, cudaStream_t st) {
     return product(h, desc_bs(h), v_blobs, 3, h->cfg.seg_dof == 3 ? kOutAdd : kOutWrite, st);
 }
 
+// Torque-carrying particles of the handle's set.
+int set_n6(const cf_mobility_config &c) { return c.seg_dof == 6 ? c.n_seg : 0; }
+// Segments and blobs as one set of equal spheres (above the wall the blocks do not depend on the radii).
+bool one_set(const cf_mobility_config &c) {
+    return (c.wall || c.seg_radius == c.blob_radius) && rpy_set_symmetric(c.n_seg + c.n_blob, set_n6(c));
+}
+
+// The full product from the callers' layouts (device).
+int eval_full(cf_mobility *h, float *v_segs, float *v_blobs, cudaStream_t st);
+int apply_full(cf_mobility *h, const float *x_segs, const float *x_blobs, const float *f_segs, const float *f_blobs,
+               float *v_segs, float *v_blobs, cudaStream_t st) {
+    const cf_mobility_config &c = h->cfg;
+    CF_TRY(pack_sets_to_float4(x_segs, f_segs, x_blobs, f_blobs, c.n_seg, c.n_blob, h->xs4, h->fs4, h->ts4, st));
+    return eval_full(h, v_segs, v_blobs, st);
+}
+
 int eval_full(cf_mobility *h, float *v_segs, float *v_blobs, cudaStream_t st) {
+    const cf_mobility_config &c = h->cfg;
+    if (c.n_seg > 0 && c.n_blob > 0 && one_set(c)) {  // the four blocks in one symmetric product
+        RpySetDesc d{c.wall, c.seg_dof, c.n_seg, c.n_seg + c.n_blob, h->xs4, h->fs4, h->ts4,
+                     static_cast<float>(c.seg_radius), static_cast<float>(c.mu)};
+        return rpy_set_product(d, h->scratch, h->scratch_cap, v_segs, v_blobs, h->num_sms, st);
+    }
     CF_TRY(eval_ss(h, v_segs, st));
     CF_TRY(eval_sb(h, v_segs, st));
     CF_TRY(eval_bb(h, v_blobs, st));
-    if (h->cfg.n_blob > 0 && h->cfg.n_seg > 0)
-        CF_TRY(product(h, desc_bs(h), v_blobs, 3, kOutAdd, st));
+    if (c.n_blob > 0 && c.n_seg > 0) CF_TRY(product(h, desc_bs(h), v_blobs, 3, kOutAdd, st));
     return CF_OK;
 }
 
@@ -190,15 +212,19 @@ extern "C" int cf_mobility_create(const cf_mobility_config *cfg, cf_mobility **o
         const size_t ns = cfg->n_seg, nb = cfg->n_blob;
         if ((rc = dalloc(&h->x_segs, 3 * ns)) || (rc = dalloc(&h->f_segs, 6 * ns)) || (rc = dalloc(&h->v_segs, 6 * ns)) ||
             (rc = dalloc(&h->x_blobs, 3 * nb)) || (rc = dalloc(&h->f_blobs, 3 * nb)) ||
-            (rc = dalloc(&h->v_blobs, 3 * nb)) || (rc = dalloc(&h->xs4, ns)) || (rc = dalloc(&h->fs4, ns)) ||
-            (rc = dalloc(&h->ts4, ns)) || (rc = dalloc(&h->xb4, nb)) || (rc = dalloc(&h->fb4, nb)) ||
-            (rc = dalloc(&h->err, 1)))
+            (rc = dalloc(&h->v_blobs, 3 * nb)) || (rc = dalloc(&h->xs4, ns + nb)) || (rc = dalloc(&h->fs4, ns + nb)) ||
+            (rc = dalloc(&h->ts4, ns)) || (rc = dalloc(&h->err, 1)))
             break;
+        h->xb4 = h->xs4 + ns;
+        h->fb4 = h->fs4 + ns;
         // Partials buffer: the largest of the four block products' plans.
         const int sd = cfg->seg_dof, n_s = cfg->n_seg, n_b = cfg->n_blob;
-        const RpyPlan plans[6] = {rpy_plan(n_s, n_s, sd, sd, h->num_sms), rpy_plan(n_s, n_b, sd, 3, h->num_sms),
-                                  rpy_plan(n_b, n_b, 3, 3, h->num_sms), rpy_plan(n_b, n_s, 3, sd, h->num_sms),
-                                  rpy_plan_sym(n_s, h->num_sms), rpy_plan_sym(n_b, h->num_sms)};
+        const int n6 = set_n6(*cfg);
+        std::vector<RpyPlan> plans = {rpy_plan(n_s, n_s, sd, sd, h->num_sms), rpy_plan(n_s, n_b, sd, 3, h->num_sms),
+                                      rpy_plan(n_b, n_b, 3, 3, h->num_sms), rpy_plan(n_b, n_s, 3, sd, h->num_sms),
+                                      rpy_plan_sym(n_b, 0, h->num_sms)};
+        if (n6 == 0 || rpy_set_symmetric(n_s, n6)) plans.push_back(rpy_plan_sym(n_s, n6, h->num_sms));
+        if (n_s > 0 && n_b > 0 && one_set(*cfg)) plans.push_back(rpy_plan_sym(n_s + n_b, n6, h->num_sms));
         h->scratch_cap = 1;
         for (const RpyPlan &pl : plans) h->scratch_cap = std::max(h->scratch_cap, pl.scratch_float4);
         if ((rc = dalloc(&h->scratch, h->scratch_cap))) break;
@@ -226,8 +252,8 @@ extern "C" int cf_mobility_destroy(cf_mobility *h) {
     cudaSetDevice(h->cfg.device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void *p : {(void *)h->x_segs, (void *)h->f_segs, (void *)h->v_segs, (void *)h->x_blobs, (void *)h->f_blobs,
-                    (void *)h->v_blobs, (void *)h->xs4, (void *)h->fs4, (void *)h->ts4, (void *)h->xb4,
-                    (void *)h->fb4, (void *)h->scratch, (void *)h->err})
+                    (void *)h->v_blobs, (void *)h->xs4, (void *)h->fs4, (void *)h->ts4, (void *)h->scratch,
+                    (void *)h->err})
         if (p) cudaFree(p);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
@@ -360,8 +386,5 @@ extern "C" int cf_apply_mobility_device(cf_mobility *h, const float *d_x_segs, c
     CF_CUDA(cudaSetDevice(h->cfg.device));
     // A null stream is CUDA's legacy default stream, as for any runtime call.
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    CF_TRY(pack_set_to_float4(d_x_segs, d_f_segs, h->xs4, h->fs4, h->ts4, ns, st));
-    CF_TRY(pack_xyz_to_float4(d_x_blobs, h->xb4, nb, st));
-    CF_TRY(pack_xyz_to_float4(d_f_blobs, h->fb4, nb, st));
-    return eval_full(h, d_v_segs, d_v_blobs, st);
+    return apply_full(h, d_x_segs, d_x_blobs, d_f_segs, d_f_blobs, d_v_segs, d_v_blobs, st);
 }

@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "rpy_kernels.cuh"
 #include "rpy_pairs.cuh"
+#include "rpy_sym6.cuh"
 #include "tma.cuh"
 
 #include <algorithm>
@@ -172,23 +173,31 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rpy_tile_kernel(TilePara
 }
 
 // ---------------------------------------------------------------------------
-// Symmetric wall kernel for the segment-segment block (targets == sources, 3x3).
-// The grand mobility is symmetric, so each unordered pair is evaluated once and
-// applied in both directions (wall_pair_sym_f32).  Work unit: one warp and one
-// pair of 32-particle tiles (I <= J) of the upper triangle.  The warp's lanes
-// own the 32 targets of tile I; the 32 sources of tile J, with the accumulators
-// of their own velocities, rotate around the warp by one lane per step, so after
-// 32 steps every lane has met every source and every source accumulator is back
-// in its home lane.  Diagonal tiles are evaluated one-sided (j != i).  Each
-// target receives exactly one partial per tile, written to
-// partial[i * nb + tile] -- no atomics, deterministic.
+// Symmetric kernel for a set of particles acting on themselves: segments with or
+// without torques and spins, blobs after them, above the wall or (equal spheres)
+// unbounded.  The grand mobility is symmetric, so each unordered pair is evaluated
+// once and applied in both directions (rpy_pairs.cuh, rpy_sym6.cuh).  Work unit:
+// one warp and one pair of 32-particle tiles (I <= J) of the upper triangle.  The
+// warp's lanes own the 32 targets of tile I; the 32 sources of tile J, with the
+// accumulators of their own velocities, rotate around the warp by one lane per
+// step, so after 32 steps every lane has met every source and every source
+// accumulator is back in its home lane.  Diagonal tiles are evaluated one-sided
+// (j != i; the other direction's results are dropped).  Each target receives exactly
+// one partial per tile (RpyPlan says where) -- no atomics, deterministic; the
+// reduction adds the self blocks.
+//
+// Bound by instruction issue (3x3: 84 FP32 instructions and 9 shuffles a pair; 6x6
+// above the wall: about 200 and 21, where two one-sided evaluations take about 600).
+// A product above the wall: 20,480 segments 880 us; 5,120 with torques 127 us, by tiles 214.
 struct SymParams {
     const float4 *x;
     const float4 *f;
+    const float4 *t;  // torques of particles [0, n6)
     float4 *partial;
-    int n, nb;
+    int n, n6, nb;
     long long items;
     float a, inv_mu;  // unbounded form: the common radius and 1 / viscosity
+    const int *gate;  // may be null: nothing is done where *gate is zero
 };
 
 __device__ __forceinline__ void sym_item(long long t, int nb, int &I, int &J) {
@@ -214,69 +223,104 @@ __device__ __forceinline__ void sym_load(const SymParams &p, int idx, int lane, 
     }
 }
 
-// WALL false: the same scheme for the unbounded product of equal spheres (free_pair_sym_f32); the diagonal
-// tiles then add each target's own self mobility, which the one-sided loop (j != i) leaves out.
-template <bool WALL>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) rpy_sym_kernel(SymParams p) {
-    chain_wait();  // launched as a programmatic dependent of the packing launch
+// One pair of tiles.  SI, SJ: tile I, J holds particles with torques and spins (a tile that also holds others gives
+// those zero torques, and their spins are dropped).
+template <bool WALL, bool SI, bool SJ>
+__device__ __forceinline__ void sym_tiles(const SymParams &p, const FreeSym6 &k, int I, int J, int lane) {
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
     const int src_lane = (lane + 1) & 31;
+    const int i = I * 32 + lane, j = J * 32 + lane;
+    constexpr int NI = SI ? 6 : 3, NJ = SJ ? 6 : 3;
+    float4 xi, fi4, xs, fs4;
+    sym_load(p, i, lane, xi, fi4);
+    sym_load(p, j, lane, xs, fs4);
+    float fi[NI] = {fi4.x, fi4.y, fi4.z}, fs[NJ] = {fs4.x, fs4.y, fs4.z}, vi[NI] = {}, vs[NJ] = {};
+    if constexpr (SI)
+        if (i < p.n6) {
+            const float4 t = p.t[i];
+            fi[3] = t.x;
+            fi[4] = t.y;
+            fi[5] = t.z;
+        }
+    if constexpr (SJ)
+        if (j < p.n6) {
+            const float4 t = p.t[j];
+            fs[3] = t.x;
+            fs[4] = t.y;
+            fs[5] = t.z;
+        }
+    auto rotate = [&](float &v) { v = __shfl_sync(full, v, src_lane); };
+    auto rotate_source = [&] {
+        rotate(xs.x);
+        rotate(xs.y);
+        rotate(xs.z);
+#pragma unroll
+        for (int c = 0; c < NJ; ++c) rotate(fs[c]);
+    };
+    auto pair = [&](float *vj) {
+        const float dx = xi.x - xs.x, dy = xi.y - xs.y, dz = xi.z - xs.z;
+        if constexpr (!SI && !SJ) {
+            if constexpr (WALL) wall_pair_sym_f32(dx, dy, dz, xi.z, xs.z, fs, fi, vi, vj);
+            else free_pair_sym_f32(dx, dy, dz, k.t, fs, fi, vi, vj);
+        } else {
+            if constexpr (WALL) wall_pair_sym6_f32<SI, SJ>(dx, dy, dz, xi.z, xs.z, fs, fi, vi, vj);
+            else free_pair_sym6_f32<SI, SJ>(dx, dy, dz, k, fs, fi, vi, vj);
+        }
+    };
+    auto place = [&](int q, int tile) {
+        return p.partial + (q < p.n6 ? 2 * (static_cast<size_t>(q) * p.nb + tile)
+                                     : static_cast<size_t>(p.n6 + q) * p.nb + tile);
+    };
+    auto store = [&](int q, int tile, const float *v, bool spins) {
+        if (q >= p.n) return;
+        float4 *o = place(q, tile);
+        o[0] = make_float4(v[0], v[1], v[2], 0.0f);
+        if (spins && q < p.n6) o[1] = make_float4(v[3], v[4], v[5], 0.0f);
+    };
+    if (I == J) {
+#pragma unroll 1
+        for (int step = 1; step < 32; ++step) {
+            rotate_source();
+            float drop[NJ] = {};
+            pair(drop);
+        }
+        store(i, I, vi, SI);
+    } else {
+#pragma unroll(SI || SJ ? 1 : 2)
+        for (int step = 0; step < 32; ++step) {
+            pair(vs);
+            rotate_source();
+#pragma unroll
+            for (int c = 0; c < NJ; ++c) rotate(vs[c]);
+        }
+        store(i, J, vi, SI);
+        store(j, I, vs, SJ);
+    }
+}
+
+// DOF6: the first p.n6 > 0 particles have torques and spins (5 blocks per SM for their registers).
+constexpr int kSym6CtasPerSm = 5;
+template <bool WALL, bool DOF6>
+__global__ void __launch_bounds__(kThreads, DOF6 ? kSym6CtasPerSm : kCtasPerSm) rpy_sym_kernel(SymParams p) {
+    chain_wait();  // launched as a programmatic dependent of the packing launch
+    if (p.gate && *p.gate == 0) return;
+    FreeSym6 k{};
+    if constexpr (!WALL) {
+        if constexpr (DOF6) k = free_sym6(p.a, p.inv_mu);
+        else k.t = free_sym(p.a, p.inv_mu);
+    }
+    const int lane = threadIdx.x & 31;
     const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
     for (long long t = static_cast<long long>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5); t < p.items;
          t += nwarps) {
         int I, J;
         sym_item(t, p.nb, I, J);
-        const int i = I * 32 + lane;
-        const int j = J * 32 + lane;
-        float4 xi, fi, xs, fs;
-        sym_load(p, i, lane, xi, fi);
-        sym_load(p, j, lane, xs, fs);
-        const float fiv[3] = {fi.x, fi.y, fi.z};
-        float vi[3] = {0.0f, 0.0f, 0.0f};
-        if (I == J) {
-#pragma unroll 1
-            for (int step = 1; step < 32; ++step) {
-                xs.x = __shfl_sync(full, xs.x, src_lane);
-                xs.y = __shfl_sync(full, xs.y, src_lane);
-                xs.z = __shfl_sync(full, xs.z, src_lane);
-                fs.x = __shfl_sync(full, fs.x, src_lane);
-                fs.y = __shfl_sync(full, fs.y, src_lane);
-                fs.z = __shfl_sync(full, fs.z, src_lane);
-                const float fsv[3] = {fs.x, fs.y, fs.z};
-                if constexpr (WALL)
-                    wall_pair_f32<3, 3>(xi.x - xs.x, xi.y - xs.y, xi.z - xs.z, xi.z, xs.z, fsv, vi);
-                else
-                    free_pair_f32<3, 3>(xi.x - xs.x, xi.y - xs.y, xi.z - xs.z, p.a, p.a, p.inv_mu, fsv, vi);
-            }
-            if constexpr (!WALL) {  // the self mobility of the target
-                const float self = p.inv_mu / (6.0f * 3.14159265358979f * p.a);
-                vi[0] += self * fi.x;
-                vi[1] += self * fi.y;
-                vi[2] += self * fi.z;
-            }
-            if (i < p.n) p.partial[static_cast<size_t>(i) * p.nb + I] = make_float4(vi[0], vi[1], vi[2], 0.0f);
+        if constexpr (DOF6) {  // uniform over the warp; J >= I, so J has torques only if I has
+            if (J * 32 < p.n6) sym_tiles<WALL, true, true>(p, k, I, J, lane);
+            else if (I * 32 < p.n6) sym_tiles<WALL, true, false>(p, k, I, J, lane);
+            else sym_tiles<WALL, false, false>(p, k, I, J, lane);
         } else {
-            float vs[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll 2
-            for (int step = 0; step < 32; ++step) {
-                const float fsv[3] = {fs.x, fs.y, fs.z};
-                if constexpr (WALL)
-                    wall_pair_sym_f32(xi.x - xs.x, xi.y - xs.y, xi.z - xs.z, xi.z, xs.z, fsv, fiv, vi, vs);
-                else
-                    free_pair_sym_f32(xi.x - xs.x, xi.y - xs.y, xi.z - xs.z, p.a, p.inv_mu, fsv, fiv, vi, vs);
-                xs.x = __shfl_sync(full, xs.x, src_lane);
-                xs.y = __shfl_sync(full, xs.y, src_lane);
-                xs.z = __shfl_sync(full, xs.z, src_lane);
-                fs.x = __shfl_sync(full, fs.x, src_lane);
-                fs.y = __shfl_sync(full, fs.y, src_lane);
-                fs.z = __shfl_sync(full, fs.z, src_lane);
-                vs[0] = __shfl_sync(full, vs[0], src_lane);
-                vs[1] = __shfl_sync(full, vs[1], src_lane);
-                vs[2] = __shfl_sync(full, vs[2], src_lane);
-            }
-            if (i < p.n) p.partial[static_cast<size_t>(i) * p.nb + J] = make_float4(vi[0], vi[1], vi[2], 0.0f);
-            if (j < p.n) p.partial[static_cast<size_t>(j) * p.nb + I] = make_float4(vs[0], vs[1], vs[2], 0.0f);
+            sym_tiles<WALL, false, false>(p, k, I, J, lane);
         }
     }
 }
@@ -423,6 +467,76 @@ __global__ void rpy_reduce_kernel(ReduceParams p) {
     }
 }
 
+// The same for a whole set after the symmetric kernel: segments [0, n_seg) into out (stride 6), blobs into out_b
+// (stride 3); the self blocks, which that kernel leaves out, are added here.
+struct SetReduceParams {
+    const float4 *partial, *x, *f, *t;
+    float *out, *out_b;
+    int n, n_seg, n6, nb;
+    float self_t, self_r;  // unbounded: 1 / (6 pi mu a), 1 / (8 pi mu a^3)
+};
+template <bool WALL>
+__global__ void __launch_bounds__(256) rpy_set_reduce_kernel(SetReduceParams p) {
+    chain_wait();
+    const int lane = threadIdx.x & 31, i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i >= p.n) return;
+    const bool six = i < p.n6;
+    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (six) {
+        const float4 *pt = p.partial + 2 * static_cast<size_t>(i) * p.nb;
+        for (int s = lane; s < p.nb; s += 32) {
+            const float4 a = __ldcs(pt + 2 * s), b = __ldcs(pt + 2 * s + 1);
+            v[0] += a.x;
+            v[1] += a.y;
+            v[2] += a.z;
+            v[3] += b.x;
+            v[4] += b.y;
+            v[5] += b.z;
+        }
+    } else {
+        const float4 *pt = p.partial + static_cast<size_t>(p.n6 + i) * p.nb;
+        for (int s = lane; s < p.nb; s += 32) {
+            const float4 a = __ldcs(pt + s);
+            v[0] += a.x;
+            v[1] += a.y;
+            v[2] += a.z;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        if (c >= 3 && !six) continue;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
+    }
+    if (lane != 0) return;
+    const float4 f4 = p.f[i];
+    float f[6] = {f4.x, f4.y, f4.z, 0.f, 0.f, 0.f}, vs[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (six) {
+        const float4 t4 = p.t[i];
+        f[3] = t4.x;
+        f[4] = t4.y;
+        f[5] = t4.z;
+    }
+    if constexpr (WALL) {
+        if (six) wall_self_f32<6, 6>(p.x[i].z, f, vs);
+        else wall_self_f32<3, 3>(p.x[i].z, f, vs);
+    } else {
+        for (int c = 0; c < 3; ++c) {
+            vs[c] = p.self_t * f[c];
+            vs[3 + c] = p.self_r * f[3 + c];
+        }
+    }
+    if (i < p.n_seg) {
+        float *o = p.out + 6 * static_cast<size_t>(i);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) o[c] = (c < 3 || six) ? static_cast<float>(v[c] + vs[c]) : 0.0f;
+    } else {
+        float *o = p.out_b + 3 * static_cast<size_t>(i - p.n_seg);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) o[c] = static_cast<float>(v[c] + vs[c]);
+    }
+}
+
 __global__ void pack_xyz_kernel(const float *__restrict__ a, float4 *__restrict__ o, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) o[i] = make_float4(a[3 * i], a[3 * i + 1], a[3 * i + 2], 0.0f);
@@ -446,6 +560,25 @@ __global__ void pack_set_kernel(const float *__restrict__ x, const float *__rest
         fo[i] = make_float4(ft[6 * i], ft[6 * i + 1], ft[6 * i + 2], 0.0f);
         if (to) to[i] = make_float4(ft[6 * i + 3], ft[6 * i + 4], ft[6 * i + 5], 0.0f);
     }
+}
+
+// Segments, then blobs, of a mobility handle in one launch.
+__global__ void pack_sets_kernel(const float *__restrict__ xs, const float *__restrict__ fs, const float *__restrict__ xb,
+                                 const float *__restrict__ fb, int n_seg, int n, float4 *__restrict__ xo,
+                                 float4 *__restrict__ fo, float4 *__restrict__ to) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float *x, *f;
+    if (i < n_seg) {
+        x = xs + 3 * static_cast<size_t>(i);
+        f = fs + 6 * static_cast<size_t>(i);
+        to[i] = make_float4(f[3], f[4], f[5], 0.0f);
+    } else {
+        x = xb + 3 * static_cast<size_t>(i - n_seg);
+        f = fb + 3 * static_cast<size_t>(i - n_seg);
+    }
+    xo[i] = make_float4(x[0], x[1], x[2], 0.0f);
+    fo[i] = make_float4(f[0], f[1], f[2], 0.0f);
 }
 
 // Raises the dynamic shared-memory cap of one instantiation once per device.
@@ -515,14 +648,16 @@ int launch_reduce_t(const ReduceParams &p, cudaStream_t st) {
 
 }  // namespace
 
-RpyPlan rpy_plan_sym(int n, int num_sms) {
+RpyPlan rpy_plan_sym(int n, int n6, int num_sms) {
     RpyPlan pl{};
     pl.sym = 1;
+    pl.n6 = n6;
     pl.ti = 1;
     const int nb = std::max(1, (n + 31) / 32);
     pl.nb = nb;
     pl.items = static_cast<long long>(nb) * (nb + 1) / 2;
-    const long long max_warps = static_cast<long long>(std::max(1, num_sms)) * kCtasPerSm * (kThreads / 32);
+    const int per_sm = n6 > 0 ? kSym6CtasPerSm : kCtasPerSm;
+    const long long max_warps = static_cast<long long>(std::max(1, num_sms)) * per_sm * (kThreads / 32);
     const long long per_warp = (pl.items + max_warps - 1) / max_warps;  // balanced: every warp does per_warp items
     const long long warps = (pl.items + per_warp - 1) / per_warp;
     pl.grid = static_cast<int>((warps + (kThreads / 32) - 1) / (kThreads / 32));
@@ -530,8 +665,20 @@ RpyPlan rpy_plan_sym(int n, int num_sms) {
     pl.nsplit = nb;  // partials per target
     pl.split = 32;
     pl.smem = 0;
-    pl.scratch_float4 = static_cast<size_t>(nb) * std::max(n, 1);
+    pl.scratch_float4 = static_cast<size_t>(nb) * std::max(n + n6, 1);
     return pl;
+}
+
+// Without torques the symmetric kernel serves every set.  With them it was faster at every size measured (320
+// particles above the wall 11.3 us, by tiles 18.5; 1,000: 11.9 and 20.2; 5,120: 127 and 214; without a wall 9.7 and
+// 20.9, 9.7 and 22.4, 71 and 102); sets below kSym6MinParticles stay with the tile kernel, whose bounded wait for its
+// bulk copies is what their callers see as CF_TIMEOUT.
+// One partial per particle and tile is n^2 / 2 bytes (twice that with torques): sets whose partials would pass 4 GB stay
+// with the tile kernel, except the 3x3 product of one set.
+constexpr int kSym6MinParticles = 512;
+constexpr size_t kSetMaxPartials = static_cast<size_t>(1) << 28;
+bool rpy_set_symmetric(int n, int n6) {
+    return (n6 == 0 || n >= kSym6MinParticles) && static_cast<size_t>((n + 31) / 32) * (n + n6) <= kSetMaxPartials;
 }
 
 RpyPlan rpy_plan(int nt, int ns, int vd, int fd, int num_sms) {
@@ -601,8 +748,12 @@ int rpy_launch_tiles(const RpyBlockDesc &d, const RpyPlan &plan, float4 *scratch
         p.items = plan.items;
         p.a = d.at;
         p.inv_mu = 1.0f / d.mu;
-        if (d.wall) CF_CUDA(launch_chained(rpy_sym_kernel<true>, dim3(plan.grid), dim3(kThreads), 0, st, p));
-        else CF_CUDA(launch_chained(rpy_sym_kernel<false>, dim3(plan.grid), dim3(kThreads), 0, st, p));
+        p.gate = d.gate;
+        p.t = d.ts;
+        p.n6 = plan.n6;
+        auto kern = d.wall ? (plan.n6 ? rpy_sym_kernel<true, true> : rpy_sym_kernel<true, false>)
+                           : (plan.n6 ? rpy_sym_kernel<false, true> : rpy_sym_kernel<false, false>);
+        CF_CUDA(launch_chained(kern, dim3(plan.grid), dim3(kThreads), 0, st, p));
         CF_CHECK_LAUNCH("rpy_sym_kernel");
         return CF_OK;
     }
@@ -661,6 +812,15 @@ int pack_set_to_float4(const float *aos3, const float *aos6, float4 *x, float4 *
     return CF_OK;
 }
 
+int pack_sets_to_float4(const float *x_segs, const float *f_segs, const float *x_blobs, const float *f_blobs, int n_seg,
+                        int n_blob, float4 *x, float4 *force, float4 *torque, cudaStream_t st) {
+    const int n = n_seg + n_blob;
+    if (n <= 0) return CF_OK;
+    pack_sets_kernel<<<(n + 127) / 128, 128, 0, st>>>(x_segs, f_segs, x_blobs, f_blobs, n_seg, n, x, force, torque);
+    CF_CHECK_LAUNCH("pack_sets_kernel");
+    return CF_OK;
+}
+
 int pack_ft6_to_float4(const float *aos6, float4 *force, float4 *torque, int n, cudaStream_t st) {
     if (n <= 0) return CF_OK;
     pack_ft6_kernel<<<(n + 255) / 256, 256, 0, st>>>(aos6, force, torque, n);
@@ -669,11 +829,47 @@ int pack_ft6_to_float4(const float *aos6, float4 *force, float4 *torque, int n, 
 }
 
 RpyPlan rpy_plan_for(const RpyBlockDesc &d, int num_sms) {
-    if (d.wall && d.self_set && d.vd == 3 && d.fd == 3 && d.nt == d.ns && d.xt == d.xs)
-        return rpy_plan_sym(d.nt, num_sms);
-    if (!d.wall && d.vd == 3 && d.fd == 3 && d.nt == d.ns && d.xt == d.xs && d.at == d.as)  // equal spheres
-        return rpy_plan_sym(d.nt, num_sms);
+    const bool itself = d.nt == d.ns && d.xt == d.xs && (d.wall ? d.self_set != 0 : d.at == d.as);  // equal spheres
+    const int n6 = d.vd == 6 ? d.nt : 0;
+    if (itself && d.vd == d.fd && (n6 == 0 || rpy_set_symmetric(d.nt, n6))) return rpy_plan_sym(d.nt, n6, num_sms);
     return rpy_plan(d.nt, d.ns, d.vd, d.fd, num_sms);
+}
+
+int rpy_set_product(const RpySetDesc &s, float4 *scratch, size_t scratch_cap, float *v_segs, float *v_blobs, int num_sms,
+                    cudaStream_t st) {
+    RpyBlockDesc d{};
+    d.wall = s.wall;
+    d.vd = d.fd = 3;
+    d.self_set = 1;
+    d.xt = d.xs = s.x;
+    d.nt = d.ns = s.n;
+    d.at = d.as = s.a;
+    d.fs = s.f;
+    d.ts = s.t;
+    d.mu = s.mu;
+    const int n6 = s.seg_dof == 6 ? s.n_seg : 0;
+    const RpyPlan plan = rpy_plan_sym(s.n, n6, num_sms);
+    if (plan.scratch_float4 > scratch_cap)
+        return set_error(CF_EINVAL, "rpy: scratch too small (%zu < %zu float4)", scratch_cap, plan.scratch_float4);
+    CF_TRY(rpy_launch_tiles(d, plan, scratch, nullptr, st));
+    SetReduceParams p;
+    p.partial = scratch;
+    p.x = s.x;
+    p.f = s.f;
+    p.t = s.t;
+    p.out = v_segs;
+    p.out_b = v_blobs;
+    p.n = s.n;
+    p.n_seg = s.n_seg;
+    p.n6 = n6;
+    p.nb = plan.nb;
+    const double pi = 3.14159265358979323846;
+    p.self_t = static_cast<float>(1.0 / (6.0 * pi * s.mu * s.a));
+    p.self_r = static_cast<float>(1.0 / (8.0 * pi * s.mu * s.a * s.a * s.a));
+    auto kern = s.wall ? rpy_set_reduce_kernel<true> : rpy_set_reduce_kernel<false>;
+    CF_CUDA(launch_chained(kern, dim3((s.n + 7) / 8), dim3(256), 0, st, p));
+    CF_CHECK_LAUNCH("rpy_set_reduce_kernel");
+    return CF_OK;
 }
 
 int rpy_block_product(const RpyBlockDesc &d, float4 *scratch, size_t scratch_cap, int *dev_err, float *out_f,
@@ -682,8 +878,18 @@ int rpy_block_product(const RpyBlockDesc &d, float4 *scratch, size_t scratch_cap
     RpyPlan plan = rpy_plan_for(d, num_sms);
     if (plan.scratch_float4 > scratch_cap)
         return set_error(CF_EINVAL, "rpy: scratch too small (%zu < %zu float4)", scratch_cap, plan.scratch_float4);
+    if (plan.sym && mode == kOutWrite && (stride == 6 || (stride == 3 && d.vd == 3))) {
+        const bool segs = stride == 6;
+        RpySetDesc s{d.wall, d.vd, segs ? d.nt : 0, d.nt, d.xs, d.fs, d.ts, d.as, d.mu};
+        return rpy_set_product(s, scratch, scratch_cap, segs ? out_f : nullptr, segs ? nullptr : out_f, num_sms, st);
+    }
+    if (plan.sym) {  // accumulating self products do not occur; the general kernel serves them
+        plan = rpy_plan(d.nt, d.ns, d.vd, d.fd, num_sms);
+        if (plan.scratch_float4 > scratch_cap)
+            return set_error(CF_EINVAL, "rpy: scratch too small (%zu < %zu float4)", scratch_cap, plan.scratch_float4);
+    }
     if (d.ns > 0) CF_TRY(rpy_launch_tiles(d, plan, scratch, dev_err, st));
-    return rpy_launch_reduce_f32(d, plan, scratch, out_f, stride, mode, st, plan.sym ? nullptr : dev_err);
+    return rpy_launch_reduce_f32(d, plan, scratch, out_f, stride, mode, st, dev_err);
 }
 
 }  // namespace cufil

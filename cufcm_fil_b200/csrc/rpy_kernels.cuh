@@ -33,10 +33,12 @@ struct RpyBlockDesc {
     int ns;
     float as;             // source radius (unbounded only)
     float mu;             // viscosity (unbounded only)
+    const int *gate;      // may be null; the symmetric 3x3 kernel does nothing where *gate is zero
 };
 
 struct RpyPlan {
-    int sym;       // 1: symmetric warp-tile kernel (wall, segments on segments, 3x3)
+    int sym;       // 1: symmetric warp-tile kernel (a set on itself)
+    int n6;        // symmetric: the first n6 particles have torques and spins
     int nb;        // symmetric: 32-particle tiles
     long long items;  // symmetric: tile pairs of the upper triangle
     int grid;      // symmetric: CTAs
@@ -56,8 +58,23 @@ RpyPlan rpy_plan(int nt, int ns, int vd, int fd, int num_sms);
 // Same with at most max_nsplit source splits (bounded partials buffer); the
 // split count never drops below ceil(ns / 2048).
 RpyPlan rpy_plan_capped(int nt, int ns, int vd, int fd, int num_sms, int max_nsplit);
-// Plan of the symmetric kernel for n particles acting on themselves.
-RpyPlan rpy_plan_sym(int n, int num_sms);
+// Plan of the symmetric kernel for n particles acting on themselves, the first n6 with torques and spins.  Its partials
+// are target-major: particle i < n6 has nb pairs (velocity, spin) at 2 nb i, particle i >= n6 nb velocities at
+// 2 nb n6 + nb (i - n6).
+RpyPlan rpy_plan_sym(int n, int n6, int num_sms);
+
+// The full product of one particle set on itself through the symmetric kernel: segments [0, n_seg) (with torques and
+// spins when seg_dof is 6) followed by blobs, the wall or equal radii `a`.  Velocities into v_segs [6 n_seg] (spins zero
+// for seg_dof 3) and v_blobs [3 (n - n_seg)].
+struct RpySetDesc {
+    int wall, seg_dof, n_seg, n;
+    const float4 *x, *f, *t;  // [n], [n], [n_seg]
+    float a, mu;
+};
+// Whether that is the faster way for n particles, n6 of them with torques, and its partials stay bounded.
+bool rpy_set_symmetric(int n, int n6);
+int rpy_set_product(const RpySetDesc &d, float4 *scratch, size_t scratch_cap, float *v_segs, float *v_blobs, int num_sms,
+                    cudaStream_t st);
 // The plan rpy_block_product uses for d (symmetric when d allows it).
 RpyPlan rpy_plan_for(const RpyBlockDesc &d, int num_sms);
 
@@ -108,6 +125,10 @@ int pack_ft6_to_float4(const float *aos6, float4 *force, float4 *torque, int n, 
 // Both of the above for one particle set (positions [3n], forces + torques [6n]) in one launch.
 int pack_set_to_float4(const float *aos3, const float *aos6, float4 *x, float4 *force, float4 *torque, int n,
                        cudaStream_t st);
+
+// Segments then blobs (either may be empty) from the reference's layouts into consecutive float4 records, in one launch.
+int pack_sets_to_float4(const float *x_segs, const float *f_segs, const float *x_blobs, const float *f_blobs, int n_seg,
+                        int n_blob, float4 *x, float4 *force, float4 *torque, cudaStream_t st);
 
 // Full product V_t (=|+=) M F_s with the right staging; convenience wrapper.
 int rpy_block_product(const RpyBlockDesc &d, float4 *scratch, size_t scratch_cap, int *dev_err, float *out_f,

@@ -253,101 +253,105 @@ namespace cufil {
 // Both directions of one wall pair from a single block evaluation.
 //   d = x_i - x_j, hz = z_i + z_j; fj, fi: source forces of j and i.
 //   vi += M(i <- j) fj,  vj += M(j <- i) fi = M(i <- j)^T fi.
-// The grand mobility is symmetric, so the image block is written as
-//   M = c6 [k0 I + a d' d'^T + b d' z^T + c z d'^T + k4 z z^T],  d' = (dx, dy, hz),
-// with the coefficients of the reference's wall branch (cuda_functions.cu:118-150)
-// regrouped: a = alpha w^2, b = beta w, c = gamma w^2 hz (w = 1/|d'|).
+// The grand mobility is symmetric; the block is
+//   M = A I + B d d^T + k0 I + a d' d'^T + b d' z^T + c z d'^T + e z z^T,  d' = (dx, dy, hz),
+// with the coefficients of the reference's wall branch (cuda_functions.cu:118-150) as polynomials in
+// u = 1/|d'|^2, E = hz^2 u and P = z_i z_j u.  Where the reference has h = z_j / hz, the products that occur are
+// h hz = z_j, h (1 - h) E = P and h^2 E = z_j^2 u, so no division is left:
+//   k0 = -w (3/4 + 3/2 P + u ((1 - 3E) / 2 - u (1 - 5E) / 2)) / 6 pi,            w = 1/|d'|
+//   a  = -w u (3/4 - 9/2 P + u G) / 6 pi,                                        G = 5/2 u (1 - 7E) - 3/2 (1 - 5E)
+//   b  =  w u (3/2 z_j + hz (u (2G + 5u) - 9P)) / 6 pi
+//   c  =  w u (3/2 z_j - 5 hz u^2) / 6 pi
+//   e  = -w u (3 z_j^2 + 3E + u (2 - 15E)) / 6 pi
+// The kernel is bound by instruction issue: 84 FP32 instructions and two reciprocal square roots for both
+// directions; written with the reference's factors it was 109, three and a division (20,480 segments 994 us a
+// product, 880 so).
 __device__ __forceinline__ void wall_pair_sym_f32(float dx, float dy, float dz, float zi, float zj, const float *fj,
                                                   const float *fi, float *vi, float *vj) {
     const float c6 = RpyConst::inv6pi;
     const float c8 = RpyConst::inv8pi;
-    const float q2 = dx * dx + dy * dy;
-    // free space: M = A I + B d d^T (even in d)
+    const float q2 = fmaf(dx, dx, dy * dy);
+    // free space: A I + B d d^T (even in d)
     const float s = rsqrtf(fmaf(dz, dz, q2));
     const float s2 = s * s;
     const float g = c8 * s;
     const float A = g * fmaf(2.0f / 3.0f, s2, 1.0f);
-    const float B = g * fmaf(-2.0f, s2, 1.0f) * s2;
+    const float B = (g * s2) * fmaf(-2.0f, s2, 1.0f);
     // image system
     const float hz = zi + zj;
-    const float hz2 = hz * hz;
-    const float w = rsqrtf(q2 + hz2);
-    const float w2 = w * w, w3 = w2 * w, w5 = w3 * w2;
-    const float h = __fdividef(zj, hz);
-    const float hm = 1.0f - h;
-    const float ez2 = w2 * hz2;
-    const float hh = h * hm;
-    const float t5 = fmaf(-5.0f, ez2, 1.0f);
-    const float w075 = 0.75f * w;
-    const float hw15 = 1.5f * h * w;
-    const float k0 = -(w075 * fmaf(2.0f * hh, ez2, 1.0f) + 0.5f * (w3 * fmaf(-3.0f, ez2, 1.0f) - w5 * t5));
-    const float al = -(w075 * fmaf(-6.0f * hh, ez2, 1.0f) - 1.5f * w3 * t5 + 2.5f * w5 * fmaf(-7.0f, ez2, 1.0f));
-    const float be = (hz * w) * (hw15 * fmaf(-6.0f * hm, ez2, 1.0f) - 3.0f * w3 * t5 + 5.0f * w5 * fmaf(-7.0f, ez2, 2.0f));
-    const float ga = hw15 - 5.0f * w5;
-    const float de = -((3.0f * h * h * w + 3.0f * w3) * ez2 + fmaf(-15.0f, ez2, 2.0f) * w5);
-    const float K0 = c6 * k0;
-    const float a = c6 * al * w2;
-    const float b = c6 * be * w;
-    const float c = c6 * ga * w2 * hz;
-    const float e = c6 * de;
+    const float w = rsqrtf(fmaf(hz, hz, q2));
+    const float u = w * w;
+    const float cw = c6 * w, cu = cw * u;
+    const float hu = hz * u, E = hz * hu;
+    const float P = (zi * zj) * u;
+    const float n5 = fmaf(7.5f, E, -1.5f);  // -3/2 (1 - 5E)
+    const float u5 = 5.0f * u;
+    const float G = fmaf(0.5f * u5, fmaf(-7.0f, E, 1.0f), n5);
+    const float k0 = fmaf(u, fmaf(u * (1.0f / 3.0f), n5, fmaf(-1.5f, E, 0.5f)), fmaf(1.5f, P, 0.75f));
+    const float AK = fmaf(-cw, k0, A);
+    const float a = -cu * fmaf(u, G, fmaf(-4.5f, P, 0.75f));
+    const float z15 = 1.5f * zj;
+    const float b = cu * fmaf(-9.0f * P, hz, fmaf(hu, fmaf(2.0f, G, u5), z15));
+    const float c = cu * fmaf(-u5, hu, z15);
+    const float e = -cu * fmaf(2.0f * z15, zj, fmaf(u, fmaf(-15.0f, E, 2.0f), 3.0f * E));
+    const float AKe = AK + e;
     // i <- j
     {
-        const float dF = dx * fj[0] + dy * fj[1] + dz * fj[2];
-        const float dpF = dx * fj[0] + dy * fj[1] + hz * fj[2];
-        const float t0 = B * dF;
-        const float t1 = a * dpF + b * fj[2];
-        const float t2 = c * dpF + e * fj[2];
-        const float AK = A + K0;
-        vi[0] += AK * fj[0] + t0 * dx + t1 * dx;
-        vi[1] += AK * fj[1] + t0 * dy + t1 * dy;
-        vi[2] += AK * fj[2] + t0 * dz + t1 * hz + t2;
+        const float p = fmaf(dx, fj[0], dy * fj[1]);
+        const float dp = fmaf(hz, fj[2], p);
+        const float t0 = B * fmaf(dz, fj[2], p);
+        const float t1 = fmaf(a, dp, b * fj[2]);
+        const float t = t0 + t1;
+        vi[0] = fmaf(t, dx, fmaf(AK, fj[0], vi[0]));
+        vi[1] = fmaf(t, dy, fmaf(AK, fj[1], vi[1]));
+        vi[2] = fmaf(c, dp, fmaf(t1, hz, fmaf(t0, dz, fmaf(AKe, fj[2], vi[2]))));
     }
     // j <- i (transpose)
     {
-        const float dF = dx * fi[0] + dy * fi[1] + dz * fi[2];
-        const float dpF = dx * fi[0] + dy * fi[1] + hz * fi[2];
-        const float t0 = B * dF;
-        const float t1 = a * dpF + c * fi[2];
-        const float t2 = b * dpF + e * fi[2];
-        const float AK = A + K0;
-        vj[0] += AK * fi[0] + t0 * dx + t1 * dx;
-        vj[1] += AK * fi[1] + t0 * dy + t1 * dy;
-        vj[2] += AK * fi[2] + t0 * dz + t1 * hz + t2;
+        const float p = fmaf(dx, fi[0], dy * fi[1]);
+        const float dp = fmaf(hz, fi[2], p);
+        const float t0 = B * fmaf(dz, fi[2], p);
+        const float t1 = fmaf(a, dp, c * fi[2]);
+        const float t = t0 + t1;
+        vj[0] = fmaf(t, dx, fmaf(AK, fi[0], vj[0]));
+        vj[1] = fmaf(t, dy, fmaf(AK, fi[1], vj[1]));
+        vj[2] = fmaf(b, dp, fmaf(t1, hz, fmaf(t0, dz, fmaf(AKe, fi[2], vj[2]))));
     }
 }
 
-// Unbounded RPY pair of two equal spheres (radius a) in both directions: the block M = A I + B u u^T is the
-// same for i <- j and j <- i (u changes sign, u u^T does not), so one evaluation serves both.  Branches as in
-// free_pair_f32 with ai = aj = a (far; overlapping, with dmin = 0; coincident: the self mobility).
-__device__ __forceinline__ void free_pair_sym_f32(float dx, float dy, float dz, float a, float inv_mu, const float *fj,
-                                                  const float *fi, float *vi, float *vj) {
+// Unbounded RPY pair of two equal spheres (radius a) in both directions: the block M = A I + B d d^T is the
+// same for i <- j and j <- i, so one evaluation serves both.  Branches as in free_pair_f32 with ai = aj = a (far;
+// overlapping, with dmin = 0; coincident: the self mobility); the far one needs a single reciprocal square root,
+// and the others are a rare branch on top of it.
+//   a2 = a^2, c8 = 1 / (8 pi mu), c6 = 1 / (6 pi mu a)
+struct FreeSym {
+    float a4, k, c8, c6, ia;  // (2a)^2, 2 a^2 / 3, 1 / (8 pi mu), 1 / (6 pi mu a), 1 / a
+};
+__device__ __forceinline__ FreeSym free_sym(float a, float inv_mu) {
     const float pi = 3.14159265358979f;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    const float r = sqrtf(r2);
-    const float s = 1.0f / (r + 1e-20f);
-    const float ux = dx * s, uy = dy * s, uz = dz * s;
-    float A, Bc;
-    if (r > 2.0f * a) {
-        const float q = s * s * (2.0f * a * a) * (1.0f / 3.0f);
-        const float c = s * inv_mu * (1.0f / (8.0f * pi));
-        A = (1.0f + q) * c;
-        Bc = (1.0f - 3.0f * q) * c;
-    } else if (r > 0.0f) {
-        const float c = inv_mu / (6.0f * pi * a * a);
-        A = (a - (9.0f / 32.0f) * r) * c;
-        Bc = (3.0f / 32.0f) * r * c;
-    } else {
-        A = inv_mu / (6.0f * pi * a);
-        Bc = 0.0f;
+    return FreeSym{4.0f * a * a, a * a * (2.0f / 3.0f), inv_mu / (8.0f * pi), inv_mu / (6.0f * pi * a), 1.0f / a};
+}
+__device__ __forceinline__ void free_pair_sym_f32(float dx, float dy, float dz, const FreeSym &q, const float *fj,
+                                                  const float *fi, float *vi, float *vj) {
+    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    const float s = rsqrtf(r2);
+    const float s2 = s * s;
+    const float g = q.c8 * s;
+    float A = g * fmaf(q.k, s2, 1.0f);
+    float B = (g * s2) * fmaf(-3.0f * q.k, s2, 1.0f);
+    if (r2 <= q.a4) {
+        const float r = r2 > 0.0f ? r2 * s : 0.0f;
+        A = q.c6 * fmaf(-9.0f / 32.0f * q.ia, r, 1.0f);
+        B = r2 > 0.0f ? q.c6 * q.ia * (3.0f / 32.0f) * s : 0.0f;
     }
-    const float tj = Bc * (ux * fj[0] + uy * fj[1] + uz * fj[2]);
-    const float ti = Bc * (ux * fi[0] + uy * fi[1] + uz * fi[2]);
-    vi[0] += A * fj[0] + tj * ux;
-    vi[1] += A * fj[1] + tj * uy;
-    vi[2] += A * fj[2] + tj * uz;
-    vj[0] += A * fi[0] + ti * ux;
-    vj[1] += A * fi[1] + ti * uy;
-    vj[2] += A * fi[2] + ti * uz;
+    const float tj = B * fmaf(dx, fj[0], fmaf(dy, fj[1], dz * fj[2]));
+    const float ti = B * fmaf(dx, fi[0], fmaf(dy, fi[1], dz * fi[2]));
+    vi[0] = fmaf(tj, dx, fmaf(A, fj[0], vi[0]));
+    vi[1] = fmaf(tj, dy, fmaf(A, fj[1], vi[1]));
+    vi[2] = fmaf(tj, dz, fmaf(A, fj[2], vi[2]));
+    vj[0] = fmaf(ti, dx, fmaf(A, fi[0], vj[0]));
+    vj[1] = fmaf(ti, dy, fmaf(A, fi[1], vj[1]));
+    vj[2] = fmaf(ti, dz, fmaf(A, fi[2], vj[2]));
 }
 
 }  // namespace cufil
