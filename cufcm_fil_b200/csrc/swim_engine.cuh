@@ -9,7 +9,7 @@
 //                   positions from the body-frame references (swimmer.cpp:440-458);
 //   kinematics      the Fulford-Blake beat in each filament's frame (kinematics_kernel);
 //   precon matrix   swimmer::make_precon_mat (swimmer.cpp:1175-1349), the 6x6 body Schur
-//                   matrix, on the host in FP64 and inverted there;
+//                   matrix and its inverse, in FP64;
 //   RHS             -q_phase, -q_angle rows (mobility_solver.cpp:284-420), zero elsewhere;
 //   solve           right-preconditioned GMRES on the saddle system
 //                   [3N lambda | 3B blob forces | V, Omega | N_fil phase rates | N_fil angle rates]
@@ -19,11 +19,35 @@
 //                        force and torque balance rows, and the filament rate rows;
 //                     P: apply_preconditioner_new's body branch (:1244-1475);
 //   body update     x += dt V, q = lie_exp(dt Omega) q (cilia_sim_main.cu:700-716).
-// The Krylov vectors live on the device in FP64; the Hessenberg and Givens
-// bookkeeping runs on the host (classical Gram-Schmidt with one
-// re-orthogonalisation, one synchronisation per iteration).  The pair products
-// are the FP32 tile kernel with compensated sums (rpy_kernels.cu).
+// Everything runs on the device; the host only enqueues.  A GMRES iteration is eight
+// launches (classical Gram-Schmidt with one re-orthogonalisation); the block that
+// finishes the last of them does the Givens step and decides whether the solve goes
+// on, and the kernels of an iteration enqueued past that point return at once, so
+// the host enqueues one iteration ahead instead of waiting for each.  The pair
+// products are the FP32 symmetric warp-tile kernel (rpy_kernels.cu).  A step of 256
+// filaments on 2,562 blobs takes 1.56 ms, of which the pair products are about half;
+// with the host waiting for each iteration's dot products, the frames and the 6 x 6
+// body matrix formed on the host and 19 launches an iteration it took 2.60 ms.
 #pragma once
+
+namespace cufil {
+namespace swim {
+// State of one solve.
+struct SwimCtl {
+    int run;         // 1 while GMRES iterates
+    int apply;       // what the solve does to sol: 0 nothing, 1 adds the correction, 2 replaces sol by it, 3 zeroes sol
+    int status;      // CF_OK, CF_NOT_CONVERGED, CF_NONFINITE
+    int iters, zero_guess, singular;
+    double norm_rhs, relres, inv_scale;
+};
+// What the host reads back: two control records in turn, the body's velocity and the wait flag.
+struct SwimReport {
+    SwimCtl ctl[2];
+    double bv[6];
+    int err;
+};
+}  // namespace swim
+}  // namespace cufil
 
 struct cf_swim {
     cf_swim_config cfg{};
@@ -35,14 +59,18 @@ struct cf_swim {
     std::vector<double> fil_ref;  // [3F] filament bases in the body frame
     std::vector<double> blob_ref; // [3B] blobs in the body frame
     double bx[3] = {0, 0, 0}, bq[4] = {1, 0, 0, 0}, bv[6] = {0, 0, 0, 0, 0, 0};
-    double *Rfil = nullptr, *xb = nullptr, *body = nullptr, *aux = nullptr, *kinv = nullptr, *gram_h = nullptr;
+    double *d_qref = nullptr, *d_fil_ref = nullptr, *d_blob_ref = nullptr;  // the same on the device
+    double *Rfil = nullptr, *xb = nullptr, *body = nullptr, *aux = nullptr, *kinv = nullptr;
     float4 *x4all = nullptr, *f4all = nullptr, *scratch = nullptr;
-    float *u = nullptr;
     size_t scratch_cap = 0;
     int *err = nullptr;
-    double *rhs = nullptr, *sol = nullptr, *w = nullptr, *z = nullptr, *t = nullptr, *Q = nullptr, *hb = nullptr;
-    double *dpart = nullptr;          // chunk partials of swim_dots_kernel [(max_iter + 1) * kSwimChunks]
-    unsigned int *dcount = nullptr;   // its arrival counter (zero between launches)
+    double *rhs = nullptr, *sol = nullptr, *w = nullptr, *z = nullptr, *t = nullptr, *Q = nullptr;
+    double *h1 = nullptr, *h2 = nullptr, *H = nullptr, *cs = nullptr, *sn = nullptr, *beta = nullptr, *y = nullptr;
+    double *part = nullptr;           // block partials of the sums that span blocks
+    unsigned int *counter = nullptr;  // their arrival counter (zero between launches)
+    cufil::swim::SwimCtl *ctl = nullptr;
+    cufil::swim::SwimReport *h_rep = nullptr;  // pinned: control records and body velocity read back
+    cudaEvent_t ev[2] = {};
     int last_iters = 0, last_status = CF_OK;
     double last_relres = 0.0;
     bool stepped = false;
@@ -53,12 +81,12 @@ namespace cufil {
 namespace swim {
 
 // ------------------------------------------------------------ quaternions
-// Host FP64 quaternions (scalar first), as src/general/quaternion.cpp defines them.
+// FP64 quaternions (scalar first), as src/general/quaternion.cpp defines them.
 struct Quat {
     double s, v[3];
 };
 
-Quat qmul(const Quat &a, const Quat &b) {  // operator*= (quaternion.cpp:104-118)
+__host__ __device__ inline Quat qmul(const Quat &a, const Quat &b) {  // operator*= (quaternion.cpp:104-118)
     Quat r;
     r.s = a.s * b.s - (a.v[0] * b.v[0] + a.v[1] * b.v[1] + a.v[2] * b.v[2]);
     r.v[0] = a.s * b.v[0] + b.s * a.v[0] + a.v[1] * b.v[2] - a.v[2] * b.v[1];
@@ -96,7 +124,7 @@ void qnormal(const Quat &q, double n[3]) {  // normal (:271-277)
     n[2] = 2.0 * (q.v[1] * q.v[2] + q.s * q.v[0]);
 }
 
-void qrot(const Quat &q, double R[9]) {  // rot_mat (:305-345), row-major
+__host__ __device__ inline void qrot(const Quat &q, double R[9]) {  // rot_mat (:305-345), row-major
     const double x = q.v[0], y = q.v[1], zc = q.v[2], s = q.s;
     R[0] = 1.0 - 2.0 * y * y - 2.0 * zc * zc;
     R[4] = 1.0 - 2.0 * x * x - 2.0 * zc * zc;
@@ -144,17 +172,21 @@ Quat filament_frame(const double *dir_in) {
 }
 
 // 6x6 inverse by Gauss-Jordan with partial pivoting (row-major, FP64); false if singular.
-bool invert6(double *A) {
+__device__ inline bool invert6(double *A) {
     double M[6][12];
     for (int i = 0; i < 6; ++i)
         for (int j = 0; j < 12; ++j) M[i][j] = j < 6 ? A[6 * i + j] : (j - 6 == i ? 1.0 : 0.0);
     for (int c = 0; c < 6; ++c) {
         int p = c;
         for (int r = c + 1; r < 6; ++r)
-            if (std::fabs(M[r][c]) > std::fabs(M[p][c])) p = r;
-        if (M[p][c] == 0.0 || !std::isfinite(M[p][c])) return false;
+            if (fabs(M[r][c]) > fabs(M[p][c])) p = r;
+        if (M[p][c] == 0.0 || !isfinite(M[p][c])) return false;
         if (p != c)
-            for (int j = 0; j < 12; ++j) std::swap(M[p][j], M[c][j]);
+            for (int j = 0; j < 12; ++j) {
+                const double t = M[p][j];
+                M[p][j] = M[c][j];
+                M[c][j] = t;
+            }
         const double inv = 1.0 / M[c][c];
         for (int j = 0; j < 12; ++j) M[c][j] *= inv;
         for (int r = 0; r < 6; ++r)
@@ -190,209 +222,440 @@ __device__ __forceinline__ long long swim_row(const SwimParams &p, int i) {
     return i < p.N ? 3LL * i : p.o_blob + 3LL * (i - p.N);
 }
 
-__global__ void swim_pack_positions_kernel(const float4 *seg, const double *xb, int N, int B, float4 *all) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < N) all[i] = seg[i];
-    else if (i < N + B)
-        all[i] = make_float4(static_cast<float>(xb[3 * (i - N)]), static_cast<float>(xb[3 * (i - N) + 1]),
-                             static_cast<float>(xb[3 * (i - N) + 2]), 0.0f);
+// Sums of NV values over a block of kSwT threads: value c's total in thread c (fixed order).
+constexpr int kSwT = 128;
+template <int NV>
+__device__ __forceinline__ double block_sums(const double (&v)[NV], double (*sm)[NV]) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+        const double s = warp_sum(v[c]);
+        if (lane == 0) sm[w][c] = s;
+    }
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x < NV)
+        for (int q = 0; q < kSwT / 32; ++q) t += sm[q][threadIdx.x];
+    return t;
 }
 
-__global__ void swim_pack_forces_kernel(SwimParams p, const double *v, float4 *f4) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.N + p.B) return;
-    const long long r = swim_row(p, i);
-    f4[i] = make_float4(static_cast<float>(v[r]), static_cast<float>(v[r + 1]), static_cast<float>(v[r + 2]), 0.0f);
+// The particles of a block of the per-filament kernels: block m < F holds filament m, the blocks after them kSwT
+// blobs each.
+__device__ __forceinline__ void swim_range(const SwimParams &p, int blk, int &lo, int &hi) {
+    if (blk < p.F) {
+        lo = blk * p.nseg;
+        hi = lo + p.nseg;
+    } else {
+        lo = p.N + (blk - p.F) * kSwT;
+        hi = min(p.N + p.B, lo + kSwT);
+    }
 }
 
-// Particle rows of A v: u - V - Omega x r, and for segments - phi_dot k_phi - theta_dot k_theta.
-__global__ void swim_rows_kernel(SwimParams p, const double *v, const float *u, double *out) {
+// Totals over the blocks of NV values each left in part[block][NV], by the block that arrives last; value c in
+// thread c * (kSwT / NV) ... handled by warp c % 4, in a fixed order, into out[c] (shared).
+template <int NV>
+__device__ __forceinline__ bool swim_totals(double *part, unsigned int *counter, int *flag, double *out) {
+    if (!arrive_last(counter, gridDim.x, flag)) return false;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int c = w; c < NV; c += kSwT / 32) {
+        double t = 0.0;
+        for (int b = lane; b < static_cast<int>(gridDim.x); b += 32) t += __ldcg(part + static_cast<size_t>(b) * NV + c);
+        t = warp_sum(t);
+        if (lane == 0) out[c] = t;
+    }
+    if (threadIdx.x == 0) *counter = 0u;
+    __syncthreads();
+    return true;
+}
+
+// Body frame of the current body state (swimmer::initial_guess, swimmer.cpp:433-466; the filaments' quaternions follow
+// the body's): filament frames and bases, blob positions, body centre.
+struct BodyState {
+    double x[3], q[4];
+};
+__global__ void swim_frames_kernel(BodyState b, int F, int B, const double *qref, const double *fil_ref,
+                                   const double *blob_ref, double *R, double *base, double *xb, double *body) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const Quat qb{b.q[0], {b.q[1], b.q[2], b.q[3]}};
+    double Rb[9];
+    qrot(qb, Rb);
+    if (i < 3) body[i] = b.x[i];
+    if (i < F) {
+        const Quat qr{qref[4 * i], {qref[4 * i + 1], qref[4 * i + 2], qref[4 * i + 3]}};
+        qrot(qmul(qb, qr), R + 9 * static_cast<size_t>(i));
+    }
+    const double *ref = i < F ? fil_ref + 3 * static_cast<size_t>(i) : blob_ref + 3 * static_cast<size_t>(i - F);
+    double *out = i < F ? base + 3 * static_cast<size_t>(i) : xb + 3 * static_cast<size_t>(i - F);
+    if (i < F + B)
+        for (int c = 0; c < 3; ++c) out[c] = b.x[c] + Rb[3 * c] * ref[0] + Rb[3 * c + 1] * ref[1] + Rb[3 * c + 2] * ref[2];
+}
+
+// Start of a step after the kinematics: pair-kernel positions, the driving rows -q_phase, -(q_angle - spring term)
+// (the other rows of the right-hand side stay zero), and swimmer::make_precon_mat (swimmer.cpp:1175-1349, dynamic
+// phase and angle): the per-filament sums v_phi, u_phi, v_theta, u_theta and Gram entries that the preconditioner
+// reuses, and the inverse of the 6x6 body Schur matrix
+//   6 pi [ n I      S(d)^T ]  -  6 pi sum_m [v u]^T C_m^-1 [v u],   S(d) w = w x d,
+//        [ S(d)  -S(d)S(d) ]
+// whose particle sums are the first and second moments of d = x - x_body.  kinv is left untouched and ctl->singular set
+// when the matrix cannot be inverted.
+constexpr int kPreMoments = 9, kPreValues = kPreMoments + 21;  // sums of d and d d^T; lower triangle of the C terms
+__global__ void __launch_bounds__(kSwT) swim_begin_kernel(SwimParams p, SimDev d, float4 *x4all, double *rhs, double *aux,
+                                                          double *gram, double *kinv, double *part,
+                                                          unsigned int *counter, SwimCtl *ctl) {
+    __shared__ double sm[kSwT / 32][15];
+    __shared__ double mom[kPreMoments + 15], tot[kPreValues];
+    __shared__ int flag;
+    int lo, hi;
+    swim_range(p, blockIdx.x, lo, hi);
+    const bool fil = static_cast<int>(blockIdx.x) < p.F;
+    double m9[kPreMoments] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    double f15[15] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // vp, up, vt, ut, c11, c22, c12
+    for (int i = lo + threadIdx.x; i < hi; i += kSwT) {
+        double r[3];
+        swim_diff(p, i, r);
+        for (int c = 0; c < 3; ++c) m9[c] += r[c];
+        m9[3] += r[0] * r[0];
+        m9[4] += r[1] * r[1];
+        m9[5] += r[2] * r[2];
+        m9[6] += r[0] * r[1];
+        m9[7] += r[0] * r[2];
+        m9[8] += r[1] * r[2];
+        if (fil) {
+            x4all[i] = d.x4[i];
+            const double *a = p.kp + 3 * static_cast<size_t>(i), *b = p.ka + 3 * static_cast<size_t>(i);
+            for (int c = 0; c < 3; ++c) {
+                f15[c] += a[c];
+                f15[6 + c] += b[c];
+            }
+            f15[3] += r[1] * a[2] - r[2] * a[1];
+            f15[4] += r[2] * a[0] - r[0] * a[2];
+            f15[5] += r[0] * a[1] - r[1] * a[0];
+            f15[9] += r[1] * b[2] - r[2] * b[1];
+            f15[10] += r[2] * b[0] - r[0] * b[2];
+            f15[11] += r[0] * b[1] - r[1] * b[0];
+            f15[12] += a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+            f15[13] += b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
+            f15[14] += a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+        } else {
+            const double *x = p.xb + 3 * static_cast<size_t>(i - p.N);
+            x4all[i] = make_float4(static_cast<float>(x[0]), static_cast<float>(x[1]), static_cast<float>(x[2]), 0.0f);
+        }
+    }
+    const double t15 = block_sums<15>(f15, sm);
+    if (threadIdx.x < 15) mom[kPreMoments + threadIdx.x] = t15;
+    __syncthreads();
+    {
+        double (*sm9)[kPreMoments] = reinterpret_cast<double (*)[kPreMoments]>(sm);
+        const double t9 = block_sums<kPreMoments>(m9, sm9);
+        if (threadIdx.x < kPreMoments) mom[threadIdx.x] = t9;
+    }
+    __syncthreads();
+    double *mine = part + static_cast<size_t>(blockIdx.x) * kPreValues;
+    if (threadIdx.x < kPreMoments) mine[threadIdx.x] = mom[threadIdx.x];
+    if (threadIdx.x < 21) {  // entry (i, j), j <= i, of this filament's C term
+        int i = 0, j = threadIdx.x;
+        while (j > i) j -= ++i;
+        double v = 0.0;
+        if (fil) {
+            const double *f = mom + kPreMoments;
+            const double c11 = f[12], c22 = f[13], c12 = f[14], det = c11 * c22 - c12 * c12;
+            const double i11 = c22 / det, i22 = c11 / det, i12 = -c12 / det;
+            const double pi_ = f[i], pj = f[j], ti = f[6 + i], tj = f[6 + j];  // (v, u) of phi, then of theta
+            v = pi_ * pj * i11 + pi_ * tj * i12 + ti * pj * i12 + ti * tj * i22;
+        }
+        mine[kPreMoments + threadIdx.x] = v;
+    }
+    if (fil) {
+        const int m = blockIdx.x;
+        if (threadIdx.x < 12) aux[12 * static_cast<size_t>(m) + threadIdx.x] = mom[kPreMoments + threadIdx.x];
+        if (threadIdx.x < 3) gram[3 * static_cast<size_t>(m) + threadIdx.x] = mom[kPreMoments + 12 + threadIdx.x];
+        if (threadIdx.x == 0) {
+            const double w0 = d.omega0[m] * 0.5 / 3.14159265358979323846;
+            double q_angle = cyclic_spline(d.phase[m], d.angle_refs, d.n_angle_refs) * w0;
+            q_angle -= d.spring * d.omega0[m] * d.L * d.L * d.L * d.angle[m];
+            rhs[p.o_phase + m] = -cyclic_spline(d.phase[m], d.phase_refs, d.n_phase_refs) * w0;
+            rhs[p.o_angle + m] = -q_angle;
+        }
+    }
+    if (!swim_totals<kPreValues>(part, counter, &flag, tot) || threadIdx.x != 0) return;
+    double K[36];
+    for (double &v : K) v = 0.0;
+    const double s[3] = {tot[0], tot[1], tot[2]};
+    const double mm[3][3] = {{tot[3], tot[6], tot[7]}, {tot[6], tot[4], tot[8]}, {tot[7], tot[8], tot[5]}};
+    const double tr = tot[3] + tot[4] + tot[5];
+    const double rc[3][3] = {{0.0, s[2], -s[1]}, {-s[2], 0.0, s[0]}, {s[1], -s[0], 0.0}};  // S(sum of d)
+    for (int i = 0; i < 3; ++i) {
+        K[7 * i] = static_cast<double>(p.N + p.B);
+        for (int j = 0; j < 3; ++j) {
+            K[6 * i + 3 + j] = rc[i][j];
+            K[6 * (3 + i) + j] = -rc[i][j];
+            K[6 * (3 + i) + 3 + j] = (i == j ? tr : 0.0) - mm[i][j];
+        }
+    }
+    for (int i = 0, e = kPreMoments; i < 6; ++i)
+        for (int j = 0; j <= i; ++j, ++e) {
+            K[6 * i + j] -= tot[e];
+            if (i != j) K[6 * j + i] -= tot[e];
+        }
+    for (double &v : K) v *= kSwimMobInv;
+    if (invert6(K)) {
+        for (int q = 0; q < 36; ++q) kinv[q] = K[q];
+        ctl->singular = 0;
+    } else {
+        ctl->singular = 1;
+    }
+}
+
+// Rows of A v that need v alone, and the pair kernel's forces: f4 = float(v), out[phase, angle] = -K^T lambda_m per
+// filament, out[body] = minus the total force and torque (about the body centre) of every particle.
+__device__ __forceinline__ void swim_tail_add(const SwimParams &p, int i, const double *f, double (&acc)[8]) {
+    double r[3];
+    swim_diff(p, i, r);
+    acc[0] += f[0];
+    acc[1] += f[1];
+    acc[2] += f[2];
+    acc[3] += r[1] * f[2] - r[2] * f[1];
+    acc[4] += r[2] * f[0] - r[0] * f[2];
+    acc[5] += r[0] * f[1] - r[1] * f[0];
+    if (i < p.N)
+        for (int c = 0; c < 3; ++c) {
+            acc[6] += p.kp[3 * static_cast<size_t>(i) + c] * f[c];
+            acc[7] += p.ka[3 * static_cast<size_t>(i) + c] * f[c];
+        }
+}
+__device__ __forceinline__ void swim_tail_end(const SwimParams &p, const double (&acc)[8], double (*sm)[8], int *flag,
+                                              double *out, double *part, unsigned int *counter, double *tot) {
+    const double t = block_sums<8>(acc, sm);
+    const int m = blockIdx.x;
+    if (threadIdx.x < 6) part[static_cast<size_t>(m) * 6 + threadIdx.x] = t;
+    else if (threadIdx.x < 8 && m < p.F) out[(threadIdx.x == 6 ? p.o_phase : p.o_angle) + m] = -t;
+    if (swim_totals<6>(part, counter, flag, tot) && threadIdx.x < 6) out[p.o_body + threadIdx.x] = -tot[threadIdx.x];
+}
+__global__ void __launch_bounds__(kSwT) swim_tail_kernel(SwimParams p, const double *v, float4 *f4, double *out,
+                                                         double *part, unsigned int *counter) {
+    __shared__ double sm[kSwT / 32][8], tot[6];
+    __shared__ int flag;
+    chain_wait();
+    int lo, hi;
+    swim_range(p, blockIdx.x, lo, hi);
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int i = lo + threadIdx.x; i < hi; i += kSwT) {
+        const double *f = v + swim_row(p, i);
+        f4[i] = make_float4(static_cast<float>(f[0]), static_cast<float>(f[1]), static_cast<float>(f[2]), 0.0f);
+        swim_tail_add(p, i, f, acc);
+    }
+    swim_tail_end(p, acc, sm, &flag, out, part, counter, tot);
+}
+
+// ---- preconditioner (apply_preconditioner_new, body branch, mobility_solver.cpp:1244-1475), two launches
+// (a) q = src * scale (the new basis vector); per filament (-r_rate - K^T M^-1 r_1) through its 2x2 C^-1, left in the
+// rate rows of z; over all blocks the body's -r_2 - K^T M^-1 r_1 - the filaments' B terms, then the 6x6 solve into the
+// body rows of z.  gate: the launch does nothing where *gate is zero; ctl: scale and, for the first iteration after a
+// discarded guess, rhs in place of src.
+__global__ void __launch_bounds__(kSwT) swim_pre_a_kernel(SwimParams p, const int *gate, const SwimCtl *ctl,
+                                                          const double *src, const double *rhs, double *q, double *z,
+                                                          double *part, unsigned int *counter) {
+    __shared__ double sm[kSwT / 32][8], t8[8], tot[6];
+    __shared__ int flag;
+    chain_wait();
+    if (gate && *gate == 0) return;
+    const double sc = ctl ? ctl->inv_scale : 1.0;
+    if (rhs && ctl->zero_guess) src = rhs;
+    int lo, hi;
+    swim_range(p, blockIdx.x, lo, hi);
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int i = lo + threadIdx.x; i < hi; i += kSwT) {
+        const long long row = swim_row(p, i);
+        double f[3];
+        for (int c = 0; c < 3; ++c) {
+            const double v = src[row + c] * sc;
+            q[row + c] = v;
+            f[c] = kSwimMobInv * v;
+        }
+        swim_tail_add(p, i, f, acc);
+    }
+    const double t = block_sums<8>(acc, sm);
+    if (threadIdx.x < 8) t8[threadIdx.x] = t;
+    __syncthreads();
+    const int m = blockIdx.x;
+    if (threadIdx.x < 6) {
+        double v = t8[threadIdx.x];
+        if (m < p.F) {
+            const double qp = src[p.o_phase + m] * sc, qa = src[p.o_angle + m] * sc;
+            const double c11 = p.gram[3 * m], c22 = p.gram[3 * m + 1], c12 = p.gram[3 * m + 2];
+            const double det = c11 * c22 - c12 * c12;
+            const double i11 = c22 / det, i22 = c11 / det, i12 = -c12 / det;
+            const double a = -qp - t8[6], b = -qa - t8[7];
+            const double ph = i11 * a + i12 * b, an = i12 * a + i22 * b;
+            const double *ax = p.aux + 12 * static_cast<size_t>(m);  // v_phi, u_phi, v_theta, u_theta
+            v += ph * ax[threadIdx.x] + an * ax[6 + threadIdx.x];
+            if (threadIdx.x == 0) {
+                q[p.o_phase + m] = qp;
+                q[p.o_angle + m] = qa;
+                z[p.o_phase + m] = ph;
+                z[p.o_angle + m] = an;
+            }
+        }
+        part[static_cast<size_t>(m) * 6 + threadIdx.x] = v;
+    }
+    if (!swim_totals<6>(part, counter, &flag, tot)) return;
+    if (threadIdx.x < 6) {
+        const double r = src[p.o_body + threadIdx.x] * sc;
+        q[p.o_body + threadIdx.x] = r;
+        tot[threadIdx.x] = -r - tot[threadIdx.x];
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        double v = 0.0;
+        for (int c = 0; c < 6; ++c) v += p.kinv[6 * threadIdx.x + c] * tot[c];
+        z[p.o_body + threadIdx.x] = v;
+    }
+}
+
+// (b) the rates, divided by 6 pi mu a, minus C^-1 B^T of the body solution; s1 = M^-1 (r_1 + K s_2) on the particle
+// rows.  With out, also the tail of A z (swim_tail_kernel).
+__global__ void __launch_bounds__(kSwT) swim_pre_b_kernel(SwimParams p, const int *gate, const double *q, double *z,
+                                                          float4 *f4, double *out, double *part, unsigned int *counter) {
+    __shared__ double sm[kSwT / 32][8], tot[6];
+    __shared__ int flag;
+    chain_wait();
+    if (gate && *gate == 0) return;
+    int lo, hi;
+    swim_range(p, blockIdx.x, lo, hi);
+    const int m = blockIdx.x;
+    double V[3], W[3], ph = 0.0, an = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        V[c] = z[p.o_body + c];
+        W[c] = z[p.o_body + 3 + c];
+    }
+    if (m < p.F) {
+        const double c11 = p.gram[3 * m], c22 = p.gram[3 * m + 1], c12 = p.gram[3 * m + 2];
+        const double det = c11 * c22 - c12 * c12;
+        const double i11 = c22 / det, i22 = c11 / det, i12 = -c12 / det;
+        const double *a = p.aux + 12 * static_cast<size_t>(m);
+        double vpV = 0, vtV = 0, upW = 0, utW = 0;
+        for (int c = 0; c < 3; ++c) {
+            vpV += a[c] * V[c];
+            upW += a[3 + c] * W[c];
+            vtV += a[6 + c] * V[c];
+            utW += a[9 + c] * W[c];
+        }
+        ph = z[p.o_phase + m] / kSwimMobInv - (i11 * vpV + i12 * vtV + i11 * upW + i12 * utW);
+        an = z[p.o_angle + m] / kSwimMobInv - (i12 * vpV + i22 * vtV + i12 * upW + i22 * utW);
+    }
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int i = lo + threadIdx.x; i < hi; i += kSwT) {
+        const long long row = swim_row(p, i);
+        double r[3];
+        swim_diff(p, i, r);
+        const double k[3] = {V[0] + W[1] * r[2] - W[2] * r[1], V[1] + W[2] * r[0] - W[0] * r[2],
+                             V[2] + W[0] * r[1] - W[1] * r[0]};
+        double f[3];
+        for (int c = 0; c < 3; ++c) {
+            double v = k[c];
+            if (i < p.N) v += ph * p.kp[3 * static_cast<size_t>(i) + c] + an * p.ka[3 * static_cast<size_t>(i) + c];
+            f[c] = kSwimMobInv * q[row + c] + kSwimMobInv * v;
+            z[row + c] = f[c];
+        }
+        if (out) {
+            f4[i] = make_float4(static_cast<float>(f[0]), static_cast<float>(f[1]), static_cast<float>(f[2]), 0.0f);
+            swim_tail_add(p, i, f, acc);
+        }
+    }
+    __syncthreads();  // every thread has read the rates as step (a) left them
+    if (threadIdx.x == 0 && m < p.F) {
+        z[p.o_phase + m] = ph;
+        z[p.o_angle + m] = an;
+    }
+    if (out) swim_tail_end(p, acc, sm, &flag, out, part, counter, tot);
+}
+
+// Particle rows of A v, one warp each: the FP64 sum of the particle's pair partials and its self mobility, minus V + Omega x r, and for
+// segments minus phi_dot k_phi + theta_dot k_theta.
+__global__ void __launch_bounds__(256) swim_rows_kernel(SwimParams p, const int *gate, const float4 *__restrict__ partial,
+                                                        int nb, const double *v, double *out) {
+    chain_wait();
+    if (gate && *gate == 0) return;
+    const int lane = threadIdx.x & 31, i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= p.N + p.B) return;
+    double o[3] = {0.0, 0.0, 0.0};
+    const float4 *pt = partial + static_cast<size_t>(i) * nb;
+    for (int s = lane; s < nb; s += 32) {
+        const float4 q = __ldcs(pt + s);
+        o[0] += q.x;
+        o[1] += q.y;
+        o[2] += q.z;
+    }
+    for (int c = 0; c < 3; ++c) o[c] = warp_sum(o[c]);
+    if (lane != 0) return;
     double r[3];
     swim_diff(p, i, r);
     const double *V = v + p.o_body, *W = v + p.o_body + 3;
     const double wr[3] = {W[1] * r[2] - W[2] * r[1], W[2] * r[0] - W[0] * r[2], W[0] * r[1] - W[1] * r[0]};
     const long long row = swim_row(p, i);
-    double o[3];
-    for (int c = 0; c < 3; ++c) o[c] = static_cast<double>(u[3 * i + c]) - V[c] - wr[c];
+    for (int c = 0; c < 3; ++c) o[c] += v[row + c] / kSwimMobInv - (V[c] + wr[c]);
     if (i < p.N) {
         const int m = i / p.nseg;
         const double ph = v[p.o_phase + m], an = v[p.o_angle + m];
-        for (int c = 0; c < 3; ++c) o[c] -= ph * p.kp[3 * i + c] + an * p.ka[3 * i + c];
+        for (int c = 0; c < 3; ++c) o[c] -= ph * p.kp[3 * static_cast<size_t>(i) + c] + an * p.ka[3 * static_cast<size_t>(i) + c];
     }
     for (int c = 0; c < 3; ++c) out[row + c] = o[c];
 }
 
-// Filament rows of A v: -K_phi^T lambda_m, -K_theta^T lambda_m (one block per filament).
-__global__ void swim_fil_rows_kernel(SwimParams p, const double *v, double *out) {
-    __shared__ double sm32[32];
-    const int m = blockIdx.x;
-    const int nb = 3 * p.nseg;
-    double dp = 0.0, da = 0.0;
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-        const long long r = 3LL * m * p.nseg + j;
-        dp += p.kp[r] * v[r];
-        da += p.ka[r] * v[r];
-    }
-    dp = block_sum(dp, sm32);
-    da = block_sum(da, sm32);
-    if (threadIdx.x == 0) {
-        out[p.o_phase + m] = -dp;
-        out[p.o_angle + m] = -da;
-    }
-}
-
-// Body rows of A v: minus the total force and torque (about the body centre) of every segment and blob (one block).
-__global__ void swim_body_rows_kernel(SwimParams p, const double *v, double *out) {
-    __shared__ double sm32[32];
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < p.N + p.B; i += blockDim.x) {
-        double r[3];
-        swim_diff(p, i, r);
-        const double *f = v + swim_row(p, i);
-        acc[0] += f[0];
-        acc[1] += f[1];
-        acc[2] += f[2];
-        acc[3] += r[1] * f[2] - r[2] * f[1];
-        acc[4] += r[2] * f[0] - r[0] * f[2];
-        acc[5] += r[0] * f[1] - r[1] * f[0];
-    }
-    for (int c = 0; c < 6; ++c) {
-        const double s = block_sum(acc[c], sm32);
-        if (threadIdx.x == 0) out[p.o_body + c] = -s;
-        __syncthreads();
-    }
-}
-
-// The driving rows: -q_phase, -(q_angle - spring term) per filament (one thread each).
-__global__ void swim_rhs_kernel(SwimParams p, SimDev d, double *rhs) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= p.F) return;
-    const double w0 = d.omega0[m] * 0.5 / 3.14159265358979323846;
-    double q_angle = cyclic_spline(d.phase[m], d.angle_refs, d.n_angle_refs) * w0;
-    q_angle -= d.spring * d.omega0[m] * d.L * d.L * d.L * d.angle[m];
-    const double q_phase = cyclic_spline(d.phase[m], d.phase_refs, d.n_phase_refs) * w0;
-    rhs[p.o_phase + m] = -q_phase;
-    rhs[p.o_angle + m] = -q_angle;
-}
-
-// ---- preconditioner (apply_preconditioner_new, body branch, mobility_solver.cpp:1244-1475)
-// (1) M^-1 r_1 on the particle rows.
-__global__ void swim_pc_scale_kernel(SwimParams p, const double *r, double *out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.N + p.B) return;
-    const long long row = swim_row(p, i);
-    for (int c = 0; c < 3; ++c) out[row + c] = kSwimMobInv * r[row + c];
-}
-
-// (2) per filament: (-r_rate - K^T M^-1 r_1), through the filament's 2x2 C^-1 (one block per filament).
-__global__ void swim_pc_fil1_kernel(SwimParams p, const double *r, double *out) {
-    __shared__ double sm32[32];
-    const int m = blockIdx.x;
-    const int nb = 3 * p.nseg;
-    double dp = 0.0, da = 0.0;
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-        const long long k = 3LL * m * p.nseg + j;
-        dp += p.kp[k] * out[k];
-        da += p.ka[k] * out[k];
-    }
-    dp = block_sum(dp, sm32);
-    da = block_sum(da, sm32);
-    if (threadIdx.x == 0) {
-        const double ph = -r[p.o_phase + m] - dp, an = -r[p.o_angle + m] - da;
-        const double c11 = p.gram[3 * m], c22 = p.gram[3 * m + 1], c12 = p.gram[3 * m + 2];
-        const double det = c11 * c22 - c12 * c12;
-        const double i11 = c22 / det, i22 = c11 / det, i12 = -c12 / det;
-        out[p.o_phase + m] = i11 * ph + i12 * an;
-        out[p.o_angle + m] = i12 * ph + i22 * an;
-    }
-}
-
-// (3) the body: -r_2 - K^T M^-1 r_1 - the filaments' B terms, then the 6x6 solve (one block).
-__global__ void swim_pc_body_kernel(SwimParams p, const double *r, double *out) {
-    __shared__ double sm32[32];
-    __shared__ double bsum[6];
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < p.N + p.B; i += blockDim.x) {
-        double d3[3];
-        swim_diff(p, i, d3);
-        const double *f = out + swim_row(p, i);
-        acc[0] += f[0];
-        acc[1] += f[1];
-        acc[2] += f[2];
-        acc[3] += d3[1] * f[2] - d3[2] * f[1];
-        acc[4] += d3[2] * f[0] - d3[0] * f[2];
-        acc[5] += d3[0] * f[1] - d3[1] * f[0];
-    }
-    for (int m = threadIdx.x; m < p.F; m += blockDim.x) {
-        const double ph = out[p.o_phase + m], an = out[p.o_angle + m];
-        const double *a = p.aux + 12 * m;  // v_phi, u_phi, v_theta, u_theta
-        for (int c = 0; c < 3; ++c) {
-            acc[c] += ph * a[c] + an * a[6 + c];
-            acc[3 + c] += ph * a[3 + c] + an * a[9 + c];
-        }
-    }
-    for (int c = 0; c < 6; ++c) {
-        const double s = block_sum(acc[c], sm32);
-        if (threadIdx.x == 0) bsum[c] = -r[p.o_body + c] - s;
-        __syncthreads();
-    }
-    if (threadIdx.x < 6) {
-        double v = 0.0;
-        for (int c = 0; c < 6; ++c) v += p.kinv[6 * threadIdx.x + c] * bsum[c];
-        out[p.o_body + threadIdx.x] = v;
-    }
-}
-
-// (4) the rates: divided by 6 pi mu a, minus C^-1 B^T of the body solution (one thread per filament).
-__global__ void swim_pc_fil2_kernel(SwimParams p, double *out) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= p.F) return;
-    const double c11 = p.gram[3 * m], c22 = p.gram[3 * m + 1], c12 = p.gram[3 * m + 2];
-    const double det = c11 * c22 - c12 * c12;
-    const double i11 = c22 / det, i22 = c11 / det, i12 = -c12 / det;
-    const double *a = p.aux + 12 * m;
-    const double *V = out + p.o_body, *W = out + p.o_body + 3;
-    double vpV = 0, vtV = 0, upW = 0, utW = 0;
-    for (int c = 0; c < 3; ++c) {
-        vpV += a[c] * V[c];
-        upW += a[3 + c] * W[c];
-        vtV += a[6 + c] * V[c];
-        utW += a[9 + c] * W[c];
-    }
-    const double ph = out[p.o_phase + m] / kSwimMobInv, an = out[p.o_angle + m] / kSwimMobInv;
-    out[p.o_phase + m] = ph - (i11 * vpV + i12 * vtV + i11 * upW + i12 * utW);
-    out[p.o_angle + m] = an - (i12 * vpV + i22 * vtV + i12 * upW + i22 * utW);
-}
-
-// (5) s1 = M^-1 (r_1 + K s_2) on the particle rows.
-__global__ void swim_pc_add_kernel(SwimParams p, double *out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.N + p.B) return;
-    double r[3];
-    swim_diff(p, i, r);
-    const double *V = out + p.o_body, *W = out + p.o_body + 3;
-    double k[3] = {V[0] + W[1] * r[2] - W[2] * r[1], V[1] + W[2] * r[0] - W[0] * r[2],
-                   V[2] + W[0] * r[1] - W[1] * r[0]};
-    if (i < p.N) {
-        const int m = i / p.nseg;
-        const double ph = out[p.o_phase + m], an = out[p.o_angle + m];
-        for (int c = 0; c < 3; ++c) k[c] += ph * p.kp[3 * i + c] + an * p.ka[3 * i + c];
-    }
-    const long long row = swim_row(p, i);
-    for (int c = 0; c < 3; ++c) out[row + c] += kSwimMobInv * k[c];
-}
-
 // ---- Krylov vector kernels (rows [0, n))
-// h[j] = <Q_j, w> for j < k1 (with `root`, h[0] = sqrt(<w, w>) for Q = w, k1 = 1).  Block (c, j) sums the
-// rows of chunk c with four independent accumulators; the block arriving last sums every j's chunks in a
-// fixed order (part: k1 x kSwimChunks partials, counter: zero on entry, reset by that block).
+// r0 = rhs - A x0 in place of A x0 in w; the block arriving last decides how the solve starts (mobility_solver.cpp:
+// 2216-2424): zero right-hand side -> zero solution; a good guess is kept; a guess worse than zero is discarded.
+__global__ void __launch_bounds__(kSwT) swim_start_kernel(const double *rhs, double *w, int n, double tol, SwimCtl *ctl,
+                                                          double *beta, double *part, unsigned int *counter) {
+    __shared__ double sm[kSwT / 32][2], tot[2];
+    __shared__ int flag;
+    chain_wait();
+    double acc[2] = {0.0, 0.0};
+    for (int i = blockIdx.x * kSwT + threadIdx.x; i < n; i += gridDim.x * kSwT) {
+        const double b = rhs[i], r = b - w[i];
+        w[i] = r;
+        acc[0] += r * r;
+        acc[1] += b * b;
+    }
+    const double t = block_sums<2>(acc, sm);
+    if (threadIdx.x < 2) part[2 * static_cast<size_t>(blockIdx.x) + threadIdx.x] = t;
+    if (!swim_totals<2>(part, counter, &flag, tot) || threadIdx.x != 0) return;
+    double b0 = sqrt(tot[0]);
+    const double nr = sqrt(tot[1]);
+    ctl->run = 0;
+    ctl->apply = 0;
+    ctl->iters = 0;
+    ctl->zero_guess = 0;
+    ctl->status = CF_OK;
+    ctl->norm_rhs = nr;
+    ctl->relres = b0 / nr;
+    if (ctl->singular) return;
+    if (!isfinite(nr) || !isfinite(b0)) {
+        ctl->status = CF_NONFINITE;
+    } else if (nr == 0.0) {
+        ctl->apply = 3;
+        ctl->relres = 0.0;
+    } else if (!(b0 <= tol * nr)) {
+        if (b0 > nr) {
+            ctl->zero_guess = 1;
+            b0 = nr;
+        }
+        ctl->run = 1;
+        ctl->inv_scale = 1.0 / b0;
+        beta[0] = b0;
+    }
+}
+
+// h[j] = <Q_j, w> for j < k1.  Block (c, j) sums the rows of chunk c with four independent accumulators; the block
+// arriving last sums every j's chunks in a fixed order (part: k1 x kSwimChunks partials).
 constexpr int kSwimChunks = 16;
-__global__ void __launch_bounds__(256) swim_dots_kernel(const double *Q, long long ldq, const double *w, int n,
-                                                        double *part, unsigned int *counter, double *h, int root) {
+__global__ void __launch_bounds__(256) swim_dots_kernel(const int *gate, const double *Q, long long ldq, const double *w,
+                                                        int n, double *part, unsigned int *counter, double *h) {
     __shared__ double sm32[32];
     __shared__ int last;
+    chain_wait();
+    if (*gate == 0) return;
     const int c = blockIdx.x, j = blockIdx.y;
     const int chunk = (n + kSwimChunks - 1) / kSwimChunks;
     const int r0 = c * chunk, r1 = min(n, r0 + chunk);
@@ -412,34 +675,144 @@ __global__ void __launch_bounds__(256) swim_dots_kernel(const double *Q, long lo
     for (int jj = threadIdx.x; jj < static_cast<int>(gridDim.y); jj += blockDim.x) {
         double t = 0.0;
         for (int cc = 0; cc < kSwimChunks; ++cc) t += __ldcg(&part[jj * kSwimChunks + cc]);
-        h[jj] = root ? sqrt(t) : t;
+        h[jj] = t;
     }
     if (threadIdx.x == 0) *counter = 0;
 }
 
-// w -= sum_j h[j] Q_j (j < k1)
-__global__ void swim_sub_basis_kernel(double *w, const double *Q, long long ldq, const double *h, int k1, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double s = 0.0;
-    for (int j = 0; j < k1; ++j) s += h[j] * Q[static_cast<long long>(j) * ldq + i];
-    w[i] -= s;
+// w -= sum_j h[j] Q_j (j < k1).  In the final pass (h1 given) also |w|, and by the block arriving last the Givens step
+// of column k1 - 1 of the Hessenberg matrix, h1 + h (mobility_solver.cpp:2462-2515), and the stopping decision.
+struct SwimGivens {
+    double *H, *cs, *sn, *beta;
+    const double *h1;
+    int ldh, max_iter;
+    double tol;
+};
+__global__ void __launch_bounds__(kSwT) swim_sub_kernel(const int *gate, double *w, const double *Q, long long ldq,
+                                                        const double *h, int k1, int n, SwimGivens g, SwimCtl *ctl,
+                                                        double *part, unsigned int *counter) {
+    __shared__ double sm[kSwT / 32][1], tot[1];
+    __shared__ int flag;
+    chain_wait();
+    if (*gate == 0) return;
+    const int i = blockIdx.x * kSwT + threadIdx.x;
+    double acc[1] = {0.0};
+    if (i < n) {
+        double s0 = 0.0, s1 = 0.0;
+        int j = 0;
+        for (; j + 1 < k1; j += 2) {
+            s0 += h[j] * Q[static_cast<long long>(j) * ldq + i];
+            s1 += h[j + 1] * Q[static_cast<long long>(j + 1) * ldq + i];
+        }
+        if (j < k1) s0 += h[j] * Q[static_cast<long long>(j) * ldq + i];
+        const double v = w[i] - (s0 + s1);
+        w[i] = v;
+        acc[0] = v * v;
+    }
+    if (!g.h1) return;
+    const double t = block_sums<1>(acc, sm);
+    if (threadIdx.x == 0) part[blockIdx.x] = t;
+    if (!swim_totals<1>(part, counter, &flag, tot)) return;
+    double *col = g.H + static_cast<size_t>(k1 - 1) * g.ldh;  // column k1 - 1, rows 0 .. k1
+    for (int r = threadIdx.x; r < k1; r += kSwT) col[r] = g.h1[r] + h[r];
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const double qn = sqrt(tot[0]);
+    ctl->iters = k1;
+    if (!isfinite(qn)) {
+        ctl->run = 0;
+        ctl->status = CF_NONFINITE;
+        ctl->relres = qn;
+        return;
+    }
+    for (int r = 1; r < k1; ++r) {
+        const double a = g.cs[r - 1] * col[r - 1] + g.sn[r - 1] * col[r];
+        col[r] = g.cs[r - 1] * col[r] - g.sn[r - 1] * col[r - 1];
+        col[r - 1] = a;
+    }
+    const double a = col[k1 - 1];
+    double c, s;
+    if (qn == 0.0) {
+        c = 1.0;
+        s = 0.0;
+    } else if (fabs(qn) > fabs(a)) {
+        const double tt = a / qn;
+        s = 1.0 / sqrt(1.0 + tt * tt);
+        c = tt * s;
+    } else {
+        const double tt = qn / a;
+        c = (a > 0 ? 1.0 : -1.0) / sqrt(1.0 + tt * tt);
+        s = tt * c;
+    }
+    g.cs[k1 - 1] = c;
+    g.sn[k1 - 1] = s;
+    col[k1 - 1] = c * a + s * qn;
+    col[k1] = 0.0;
+    const double bk = g.beta[k1 - 1];
+    g.beta[k1] = -s * bk;
+    g.beta[k1 - 1] = c * bk;
+    const double rel = fabs(s * bk) / ctl->norm_rhs;
+    ctl->relres = rel;
+    ctl->inv_scale = qn != 0.0 ? 1.0 / qn : 1.0;
+    if (rel <= g.tol || k1 == g.max_iter) {
+        ctl->run = 0;
+        ctl->status = rel <= g.tol ? CF_OK : CF_NOT_CONVERGED;
+        ctl->apply = ctl->zero_guess ? 2 : 1;
+    }
 }
 
-// dst = a * src + b * dst2 (dst2 may alias dst; b = 0 ignores it)
-__global__ void swim_axpby_kernel(double *dst, double a, const double *src, double b, const double *dst2, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    dst[i] = a * src[i] + (b != 0.0 ? b * dst2[i] : 0.0);
+// H y = beta by one block, column oriented (mobility_solver.cpp:2520-2537).
+__global__ void __launch_bounds__(256) swim_backsub_kernel(const SwimCtl *ctl, const double *H, int ldh,
+                                                           const double *beta, double *y) {
+    chain_wait();
+    if (ctl->apply != 1 && ctl->apply != 2) return;
+    const int k = ctl->iters;
+    for (int r = threadIdx.x; r < k; r += blockDim.x) y[r] = beta[r];
+    __syncthreads();
+    for (int i = k - 1; i >= 0; --i) {
+        const double *col = H + static_cast<size_t>(i) * ldh;
+        if (threadIdx.x == 0) y[i] /= col[i];
+        __syncthreads();
+        const double yi = y[i];
+        for (int r = threadIdx.x; r < i; r += blockDim.x) y[r] -= col[r] * yi;
+        __syncthreads();
+    }
 }
 
-// t = sum_j y[j] Q_j (j < k)
-__global__ void swim_combine_kernel(double *t, const double *Q, long long ldq, const double *y, int k, int n) {
+// t = sum_j y_j Q_j
+__global__ void __launch_bounds__(256) swim_combine_kernel(const SwimCtl *ctl, double *t, const double *Q, long long ldq,
+                                                           const double *y, int n) {
+    chain_wait();
+    if (ctl->apply != 1 && ctl->apply != 2) return;
+    const int k = ctl->iters;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double s = 0.0;
-    for (int j = 0; j < k; ++j) s += y[j] * Q[static_cast<long long>(j) * ldq + i];
-    t[i] = s;
+    double s0 = 0.0, s1 = 0.0;
+    int j = 0;
+    for (; j + 1 < k; j += 2) {
+        s0 += y[j] * Q[static_cast<long long>(j) * ldq + i];
+        s1 += y[j + 1] * Q[static_cast<long long>(j + 1) * ldq + i];
+    }
+    if (j < k) s0 += y[j] * Q[static_cast<long long>(j) * ldq + i];
+    t[i] = s0 + s1;
+}
+
+__global__ void swim_set_step_kernel(LoopCtl *lc, int nt) { lc->nt = nt; }
+
+// sol as ctl->apply says, and the rates that the next step advances with.
+__global__ void swim_finish_kernel(SwimParams p, const SwimCtl *ctl, const double *z, double *sol, int n,
+                                   double *phase_dot, double *angle_dot) {
+    chain_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int a = ctl->apply;
+    double v = sol[i];
+    if (a == 1) v += z[i];
+    else if (a == 2) v = z[i];
+    else if (a == 3) v = 0.0;
+    sol[i] = v;
+    if (i >= p.o_phase && i < p.o_phase + p.F) phase_dot[i - p.o_phase] = v;
+    if (i >= p.o_angle && i < p.o_angle + p.F) angle_dot[i - p.o_angle] = v;
 }
 
 // ------------------------------------------------------------ host side
@@ -482,14 +855,12 @@ SwimParams swim_params(const cf_swim *h) {
 }
 
 int swim_grid(int n) { return std::max(1, (n + 255) / 256); }
+int swim_blocks(const cf_swim *h) { return h->F + (h->B + kSwT - 1) / kSwT; }
 
-// out = A v (system_matrix_mult_new, body branch)
-int swim_matvec(cf_swim *h, const double *v, double *out) {
+// Particle rows of out = A v once f4 holds v's forces (system_matrix_mult_new, body branch).
+int swim_rows(cf_swim *h, const double *v, double *out, const int *gate) {
     cudaStream_t st = h->stream;
-    const SwimParams p = swim_params(h);
     const int np = h->N + h->B;
-    swim_pack_forces_kernel<<<swim_grid(np), 256, 0, st>>>(p, v, h->f4all);
-    CF_CHECK_LAUNCH("swim_pack_forces_kernel");
     RpyBlockDesc d{};
     d.wall = 0;
     d.vd = 3;
@@ -504,293 +875,101 @@ int swim_matvec(cf_swim *h, const double *v, double *out) {
     d.ns = np;
     d.as = 1.0f;
     d.mu = 1.0f;
-    CF_TRY(rpy_block_product(d, h->scratch, h->scratch_cap, h->err, h->u, 3, kOutWrite, h->num_sms, st));
-    swim_rows_kernel<<<swim_grid(np), 256, 0, st>>>(p, v, h->u, out);
+    d.gate = gate;
+    const RpyPlan plan = rpy_plan_for(d, h->num_sms);  // equal spheres on themselves: the symmetric kernel
+    CF_TRY(rpy_launch_tiles(d, plan, h->scratch, h->err, st));
+    CF_CUDA(launch_chained(swim_rows_kernel, dim3((np + 7) / 8), dim3(256), 0, st, swim_params(h), gate,
+                           static_cast<const float4 *>(h->scratch), plan.nsplit, v, out));
     CF_CHECK_LAUNCH("swim_rows_kernel");
-    swim_fil_rows_kernel<<<h->F, 64, 0, st>>>(p, v, out);
-    CF_CHECK_LAUNCH("swim_fil_rows_kernel");
-    swim_body_rows_kernel<<<1, 1024, 0, st>>>(p, v, out);
-    CF_CHECK_LAUNCH("swim_body_rows_kernel");
     return CF_OK;
 }
 
-// out = P r (apply_preconditioner_new, body branch)
-int swim_precond(cf_swim *h, const double *r, double *out) {
+// out = A v
+int swim_matvec(cf_swim *h, const double *v, double *out) {
+    CF_CUDA(launch_chained(swim_tail_kernel, dim3(swim_blocks(h)), dim3(kSwT), 0, h->stream, swim_params(h), v, h->f4all,
+                           out, h->part, h->counter));
+    CF_CHECK_LAUNCH("swim_tail_kernel");
+    return swim_rows(h, v, out, nullptr);
+}
+
+// q = the vector preconditioned, z = P q; with out also the tail of A z.
+int swim_precond(cf_swim *h, const int *gate, const SwimCtl *ctl, const double *src, const double *rhs, double *q,
+                 double *z, double *out) {
     cudaStream_t st = h->stream;
     const SwimParams p = swim_params(h);
-    const int np = h->N + h->B;
-    swim_pc_scale_kernel<<<swim_grid(np), 256, 0, st>>>(p, r, out);
-    CF_CHECK_LAUNCH("swim_pc_scale_kernel");
-    swim_pc_fil1_kernel<<<h->F, 64, 0, st>>>(p, r, out);
-    CF_CHECK_LAUNCH("swim_pc_fil1_kernel");
-    swim_pc_body_kernel<<<1, 1024, 0, st>>>(p, r, out);
-    CF_CHECK_LAUNCH("swim_pc_body_kernel");
-    swim_pc_fil2_kernel<<<swim_grid(h->F), 256, 0, st>>>(p, out);
-    CF_CHECK_LAUNCH("swim_pc_fil2_kernel");
-    swim_pc_add_kernel<<<swim_grid(np), 256, 0, st>>>(p, out);
-    CF_CHECK_LAUNCH("swim_pc_add_kernel");
+    const dim3 grid(swim_blocks(h));
+    CF_CUDA(launch_chained(swim_pre_a_kernel, grid, dim3(kSwT), 0, st, p, gate, ctl, src, rhs, q, z, h->part, h->counter));
+    CF_CHECK_LAUNCH("swim_pre_a_kernel");
+    CF_CUDA(launch_chained(swim_pre_b_kernel, grid, dim3(kSwT), 0, st, p, gate, static_cast<const double *>(q), z, h->f4all,
+                           out, h->part, h->counter));
+    CF_CHECK_LAUNCH("swim_pre_b_kernel");
     return CF_OK;
 }
 
 int swim_sync(cf_swim *h) {
+    CF_CUDA(cudaMemcpyAsync(&h->h_rep->err, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CF_CUDA(cudaStreamSynchronize(h->stream));
-    int flags = 0;
-    CF_CUDA(cudaMemcpy(&flags, h->err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flags) {
-        CF_CUDA(cudaMemset(h->err, 0, sizeof(int)));
-        return set_error(CF_TIMEOUT, "swim: a bounded device wait gave up (flags 0x%x)", flags);
+    if (h->h_rep->err) {
+        CF_CUDA(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream));
+        return set_error(CF_TIMEOUT, "swim: a bounded device wait gave up (flags 0x%x)", h->h_rep->err);
     }
     return CF_OK;
 }
 
-// Body frame of the current body state: filament frames, bases and blob positions to the device
-// (swimmer::initial_guess, swimmer.cpp:433-466; the filaments' quaternions follow the body's).
-int swim_frames(cf_swim *h) {
-    const int F = h->F, B = h->B;
-    double Rb[9];
-    const Quat qb{h->bq[0], {h->bq[1], h->bq[2], h->bq[3]}};
-    qrot(qb, Rb);
-    std::vector<double> R(9 * static_cast<size_t>(F)), base(3 * static_cast<size_t>(F)), xb(3 * static_cast<size_t>(B));
-    for (int m = 0; m < F; ++m) {
-        const Quat qr{h->qref[4 * m], {h->qref[4 * m + 1], h->qref[4 * m + 2], h->qref[4 * m + 3]}};
-        qrot(qmul(qb, qr), &R[9 * m]);
-        for (int c = 0; c < 3; ++c)
-            base[3 * m + c] = h->bx[c] + Rb[3 * c] * h->fil_ref[3 * m] + Rb[3 * c + 1] * h->fil_ref[3 * m + 1] +
-                              Rb[3 * c + 2] * h->fil_ref[3 * m + 2];
-    }
-    for (int k = 0; k < B; ++k)
-        for (int c = 0; c < 3; ++c)
-            xb[3 * k + c] = h->bx[c] + Rb[3 * c] * h->blob_ref[3 * k] + Rb[3 * c + 1] * h->blob_ref[3 * k + 1] +
-                            Rb[3 * c + 2] * h->blob_ref[3 * k + 2];
-    cudaStream_t st = h->stream;
-    CF_CUDA(cudaMemcpyAsync(h->Rfil, R.data(), R.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    CF_CUDA(cudaMemcpyAsync(const_cast<double *>(h->d.base), base.data(), base.size() * sizeof(double),
-                            cudaMemcpyHostToDevice, st));
-    if (B) CF_CUDA(cudaMemcpyAsync(h->xb, xb.data(), xb.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    CF_CUDA(cudaMemcpyAsync(h->body, h->bx, 3 * sizeof(double), cudaMemcpyHostToDevice, st));
-    CF_CUDA(cudaStreamSynchronize(st));  // the host vectors go out of scope
-    return CF_OK;
-}
-
-// swimmer::make_precon_mat (swimmer.cpp:1175-1349, dynamic phase and angle) on the host in FP64, with the
-// per-filament sums v_phi, u_phi, v_theta, u_theta that the preconditioner reuses.
-int swim_precon_matrix(cf_swim *h) {
-    const int F = h->F, nseg = h->nseg, N = h->N, B = h->B;
-    std::vector<double> x(3 * static_cast<size_t>(N)), kp(3 * static_cast<size_t>(N)), ka(3 * static_cast<size_t>(N));
-    cudaStream_t st = h->stream;
-    CF_CUDA(cudaMemcpyAsync(x.data(), h->d.xd, x.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CF_CUDA(cudaMemcpyAsync(kp.data(), h->d.kp, kp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CF_CUDA(cudaMemcpyAsync(ka.data(), h->d.ka, ka.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CF_CUDA(cudaStreamSynchronize(st));
-    const double mob = kSwimMobInv;
-    double K[36] = {0};
-    const double eye = static_cast<double>(N) * mob + static_cast<double>(B) * mob;
-    K[0] = K[7] = K[14] = eye;
-    auto add_r = [&](const double *d3) {
-        // rcross(d) (matrix.cpp:665-679): rcross(d) w = w x d
-        const double rc[9] = {0.0, d3[2], -d3[1], -d3[2], 0.0, d3[0], d3[1], -d3[0], 0.0};
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j) {
-                K[6 * i + 3 + j] += mob * rc[3 * i + j];
-                double rr = 0.0;
-                for (int q = 0; q < 3; ++q) rr += rc[3 * i + q] * rc[3 * q + j];
-                K[6 * (3 + i) + 3 + j] -= mob * rr;
-            }
-    };
-    for (int i = 0; i < N; ++i) {
-        const double d3[3] = {x[3 * i] - h->bx[0], x[3 * i + 1] - h->bx[1], x[3 * i + 2] - h->bx[2]};
-        add_r(d3);
-    }
-    double Rb[9];
-    qrot(Quat{h->bq[0], {h->bq[1], h->bq[2], h->bq[3]}}, Rb);
-    for (int k = 0; k < B; ++k) {
-        double d3[3];
-        for (int c = 0; c < 3; ++c)
-            d3[c] = Rb[3 * c] * h->blob_ref[3 * k] + Rb[3 * c + 1] * h->blob_ref[3 * k + 1] +
-                    Rb[3 * c + 2] * h->blob_ref[3 * k + 2];
-        add_r(d3);
-    }
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) K[6 * (3 + i) + j] = -K[6 * i + 3 + j];
-    double C[36] = {0};
-    std::vector<double> aux(12 * static_cast<size_t>(F));
-    std::vector<double> gram(3 * static_cast<size_t>(F));
-    for (int m = 0; m < F; ++m) {
-        double c11 = 0, c22 = 0, c12 = 0, vp[3] = {0, 0, 0}, up[3] = {0, 0, 0}, vt[3] = {0, 0, 0}, ut[3] = {0, 0, 0};
-        for (int k = 0; k < nseg; ++k) {
-            const int i = m * nseg + k;
-            const double *a = &kp[3 * i], *b = &ka[3 * i];
-            const double d3[3] = {x[3 * i] - h->bx[0], x[3 * i + 1] - h->bx[1], x[3 * i + 2] - h->bx[2]};
-            for (int c = 0; c < 3; ++c) {
-                vp[c] += a[c];
-                vt[c] += b[c];
-            }
-            up[0] += d3[1] * a[2] - d3[2] * a[1];
-            up[1] += d3[2] * a[0] - d3[0] * a[2];
-            up[2] += d3[0] * a[1] - d3[1] * a[0];
-            ut[0] += d3[1] * b[2] - d3[2] * b[1];
-            ut[1] += d3[2] * b[0] - d3[0] * b[2];
-            ut[2] += d3[0] * b[1] - d3[1] * b[0];
-            c11 += a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
-            c22 += b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
-            c12 += a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
-        }
-        const double det = c11 * c22 - c12 * c12;
-        const double i11 = c22 / det, i22 = c11 / det, i12 = -c12 / det;
-        for (int i = 0; i < 3; ++i)
-            for (int j = 0; j < 3; ++j) {
-                C[6 * i + j] += vp[i] * vp[j] * i11 + vp[i] * vt[j] * i12 + vt[i] * vp[j] * i12 + vt[i] * vt[j] * i22;
-                C[6 * (3 + i) + j] +=
-                    up[i] * vp[j] * i11 + up[i] * vt[j] * i12 + ut[i] * vp[j] * i12 + ut[i] * vt[j] * i22;
-                C[6 * (3 + i) + 3 + j] +=
-                    up[i] * up[j] * i11 + up[i] * ut[j] * i12 + ut[i] * up[j] * i12 + ut[i] * ut[j] * i22;
-            }
-        for (int c = 0; c < 3; ++c) {
-            aux[12 * m + c] = vp[c];
-            aux[12 * m + 3 + c] = up[c];
-            aux[12 * m + 6 + c] = vt[c];
-            aux[12 * m + 9 + c] = ut[c];
-        }
-        gram[3 * m] = c11;
-        gram[3 * m + 1] = c22;
-        gram[3 * m + 2] = c12;
-    }
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) C[6 * i + 3 + j] = C[6 * (3 + j) + i];
-    for (int q = 0; q < 36; ++q) K[q] -= mob * C[q];
-    if (!invert6(K)) return set_error(CF_NONFINITE, "cf_swim: the body's 6x6 preconditioner matrix is singular");
-    CF_CUDA(cudaMemcpyAsync(h->kinv, K, sizeof(K), cudaMemcpyHostToDevice, st));
-    CF_CUDA(cudaMemcpyAsync(h->aux, aux.data(), aux.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    CF_CUDA(cudaMemcpyAsync(h->d.gram, gram.data(), gram.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    CF_CUDA(cudaStreamSynchronize(st));
-    return CF_OK;
-}
-
-// out[j] = <Q_j, w> for j < k1 (Q rows n apart), or with `root` out[0] = |w| for Q = w, k1 = 1.
-int swim_dots(cf_swim *h, const double *Q, const double *w, int k1, double *out, int root) {
-    swim_dots_kernel<<<dim3(kSwimChunks, k1), 256, 0, h->stream>>>(Q, h->n, w, h->n, h->dpart, h->dcount, out, root);
-    CF_CHECK_LAUNCH("swim_dots_kernel");
-    return CF_OK;
-}
-
-// Right-preconditioned GMRES on A sol = rhs with the warm start in sol (mobility_solver.cpp:2187-2669):
-// zero RHS -> zero solution; a good guess is kept; a guess worse than zero is discarded.
+// Right-preconditioned GMRES on A sol = rhs with the warm start in sol (mobility_solver.cpp:2187-2669), then the
+// solution's update.  The control record of iteration i - 1 is looked at after iteration i was enqueued, so the device
+// always has work queued; the at most one iteration enqueued past the end does nothing (its kernels see run = 0).
 int swim_gmres(cf_swim *h) {
-    const int n = h->n;
+    const int n = h->n, M = h->max_iter, sub_grid = (n + kSwT - 1) / kSwT;
     cudaStream_t st = h->stream;
     const long long ldq = n;
-    const int g = swim_grid(n);
-    // hb layout: [0, M+1) h1, [M+1, 2M+2) h2, [2M+2] norm, [2M+3] |rhs|, [2M+4..) y
-    const int M = h->max_iter;
-    double *h1 = h->hb, *h2 = h->hb + (M + 1), *nrm = h->hb + 2 * (M + 1), *nrhs = nrm + 1, *yd = nrm + 2;
-    CF_TRY(swim_dots(h, h->rhs, h->rhs, 1, nrhs, 1));
+    const int *run = &h->ctl->run;
     CF_TRY(swim_matvec(h, h->sol, h->w));
-    swim_axpby_kernel<<<g, 256, 0, st>>>(h->w, 1.0, h->rhs, -1.0, h->w, n);  // r0 = rhs - A x0
-    CF_CHECK_LAUNCH("swim_axpby_kernel");
-    CF_TRY(swim_dots(h, h->w, h->w, 1, nrm, 1));
-    double nb[2];
-    CF_CUDA(cudaMemcpyAsync(nb, nrm, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CF_TRY(swim_sync(h));
-    double beta0 = nb[0];
-    const double nr = nb[1];
-    h->last_iters = 0;
-    if (!std::isfinite(nr) || !std::isfinite(beta0)) {
-        h->last_status = CF_NONFINITE;
-        h->last_relres = beta0 / nr;
-        return CF_OK;
-    }
-    if (nr == 0.0) {
-        CF_CUDA(cudaMemsetAsync(h->sol, 0, sizeof(double) * n, st));
-        h->last_status = CF_OK;
-        h->last_relres = 0.0;
-        return CF_OK;
-    }
-    if (beta0 <= h->cfg.gmres_tol * nr) {
-        h->last_status = CF_OK;
-        h->last_relres = beta0 / nr;
-        return CF_OK;
-    }
-    if (beta0 > nr) {  // the initial guess is worse than zero
-        CF_CUDA(cudaMemsetAsync(h->sol, 0, sizeof(double) * n, st));
-        CF_CUDA(cudaMemcpyAsync(h->w, h->rhs, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-        beta0 = nr;
-    }
-    swim_axpby_kernel<<<g, 256, 0, st>>>(h->Q, 1.0 / beta0, h->w, 0.0, nullptr, n);
-    CF_CHECK_LAUNCH("swim_axpby_kernel");
-    std::vector<double> H(static_cast<size_t>(M + 1) * (M + 1), 0.0), cs(M), sn(M), beta(M + 1, 0.0);
-    beta[0] = beta0;
-    std::vector<double> hh(2 * (M + 1) + 1);
-    int it = 0;
-    double rel = 1.0;
-    for (it = 1; it <= M; ++it) {
-        const int k1 = it;  // basis vectors Q_0 .. Q_{it-1}
-        CF_TRY(swim_precond(h, h->Q + static_cast<long long>(it - 1) * ldq, h->z));
-        CF_TRY(swim_matvec(h, h->z, h->w));
-        CF_TRY(swim_dots(h, h->Q, h->w, k1, h1, 0));
-        swim_sub_basis_kernel<<<g, 256, 0, st>>>(h->w, h->Q, ldq, h1, k1, n);
-        CF_CHECK_LAUNCH("swim_sub_basis_kernel");
-        CF_TRY(swim_dots(h, h->Q, h->w, k1, h2, 0));
-        swim_sub_basis_kernel<<<g, 256, 0, st>>>(h->w, h->Q, ldq, h2, k1, n);
-        CF_CHECK_LAUNCH("swim_sub_basis_kernel");
-        CF_TRY(swim_dots(h, h->w, h->w, 1, nrm, 1));
-        CF_CUDA(cudaMemcpyAsync(hh.data(), h->hb, hh.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-        CF_TRY(swim_sync(h));
-        const double qn = hh[2 * (M + 1)];
-        double *col = &H[static_cast<size_t>(it - 1) * (M + 1)];  // column it-1, rows 0..it
-        for (int i = 0; i < it; ++i) col[i] = hh[i] + hh[(M + 1) + i];
-        col[it] = qn;
-        if (!std::isfinite(qn)) {
-            h->last_iters = it;
-            h->last_status = CF_NONFINITE;
-            h->last_relres = qn;
-            return CF_OK;
+    CF_CUDA(launch_chained(swim_start_kernel, dim3(2 * h->num_sms), dim3(kSwT), 0, st, static_cast<const double *>(h->rhs),
+                           h->w, n, h->cfg.gmres_tol, h->ctl, h->beta, h->part, h->counter));
+    CF_CHECK_LAUNCH("swim_start_kernel");
+    for (int it = 1; it <= M; ++it) {
+        const double *src = h->w, *rhs = it == 1 ? h->rhs : nullptr, *Q = h->Q;
+        double *q = h->Q + static_cast<long long>(it - 1) * ldq;
+        CF_TRY(swim_precond(h, run, h->ctl, src, rhs, q, h->z, h->w));
+        CF_TRY(swim_rows(h, h->z, h->w, run));
+        const double *wv = h->w;
+        for (int pass = 0; pass < 2; ++pass) {
+            double *hh = pass == 0 ? h->h1 : h->h2;
+            CF_CUDA(launch_chained(swim_dots_kernel, dim3(kSwimChunks, it), dim3(256), 0, st, run, Q, ldq, wv, n, h->part,
+                                   h->counter, hh));
+            CF_CHECK_LAUNCH("swim_dots_kernel");
+            SwimGivens g{h->H, h->cs, h->sn, h->beta, pass == 0 ? nullptr : h->h1, M + 1, M, h->cfg.gmres_tol};
+            CF_CUDA(launch_chained(swim_sub_kernel, dim3(sub_grid), dim3(kSwT), 0, st, run, h->w, Q, ldq,
+                                   static_cast<const double *>(hh), it, n, g, h->ctl, h->part, h->counter));
+            CF_CHECK_LAUNCH("swim_sub_kernel");
         }
-        swim_axpby_kernel<<<g, 256, 0, st>>>(h->Q + static_cast<long long>(it) * ldq, qn != 0.0 ? 1.0 / qn : 1.0,
-                                             h->w, 0.0, nullptr, n);
-        CF_CHECK_LAUNCH("swim_axpby_kernel");
-        // previous rotations, then the new one (the oracle's and the reference's Givens recurrence)
-        for (int i = 1; i < it; ++i) {
-            const double tmp = cs[i - 1] * col[i - 1] + sn[i - 1] * col[i];
-            col[i] = cs[i - 1] * col[i] - sn[i - 1] * col[i - 1];
-            col[i - 1] = tmp;
+        CF_CUDA(cudaMemcpyAsync(&h->h_rep->ctl[it & 1], h->ctl, sizeof(SwimCtl), cudaMemcpyDeviceToHost, st));
+        CF_CUDA(cudaEventRecord(h->ev[it & 1], st));
+        if (it > 1) {
+            CF_CUDA(cudaEventSynchronize(h->ev[(it - 1) & 1]));
+            if (!h->h_rep->ctl[(it - 1) & 1].run) break;
         }
-        const double a = col[it - 1], b = col[it];
-        if (b == 0.0) {
-            cs[it - 1] = 1.0;
-            sn[it - 1] = 0.0;
-        } else if (std::fabs(b) > std::fabs(a)) {
-            const double tt = a / b;
-            sn[it - 1] = (b > 0 ? 1.0 : -1.0) / std::sqrt(1.0 + tt * tt);
-            cs[it - 1] = tt * sn[it - 1];
-        } else {
-            const double tt = b / a;
-            cs[it - 1] = (a > 0 ? 1.0 : -1.0) / std::sqrt(1.0 + tt * tt);
-            sn[it - 1] = tt * cs[it - 1];
-        }
-        col[it - 1] = cs[it - 1] * a + sn[it - 1] * b;
-        col[it] = 0.0;
-        beta[it] = -sn[it - 1] * beta[it - 1];
-        beta[it - 1] = cs[it - 1] * beta[it - 1];
-        rel = std::fabs(beta[it]) / nr;
-        if (rel <= h->cfg.gmres_tol || it == M) break;
     }
-    if (it > M) it = M;
-    std::vector<double> y(it, 0.0);
-    for (int i = it - 1; i >= 0; --i) {
-        double s = beta[i];
-        for (int j = i + 1; j < it; ++j) s -= H[static_cast<size_t>(j) * (M + 1) + i] * y[j];
-        y[i] = s / H[static_cast<size_t>(i) * (M + 1) + i];
-    }
-    CF_CUDA(cudaMemcpyAsync(yd, y.data(), it * sizeof(double), cudaMemcpyHostToDevice, st));
-    swim_combine_kernel<<<g, 256, 0, st>>>(h->t, h->Q, ldq, yd, it, n);
+    const SwimCtl *ctl = h->ctl;
+    CF_CUDA(launch_chained(swim_backsub_kernel, dim3(1), dim3(256), 0, st, ctl, static_cast<const double *>(h->H), M + 1,
+                           static_cast<const double *>(h->beta), h->y));
+    CF_CHECK_LAUNCH("swim_backsub_kernel");
+    CF_CUDA(launch_chained(swim_combine_kernel, dim3(swim_grid(n)), dim3(256), 0, st, ctl, h->t,
+                           static_cast<const double *>(h->Q), ldq, static_cast<const double *>(h->y), n));
     CF_CHECK_LAUNCH("swim_combine_kernel");
-    CF_TRY(swim_precond(h, h->t, h->z));
-    swim_axpby_kernel<<<g, 256, 0, st>>>(h->sol, 1.0, h->z, 1.0, h->sol, n);
-    CF_CHECK_LAUNCH("swim_axpby_kernel");
+    CF_TRY(swim_precond(h, &h->ctl->apply, nullptr, h->t, nullptr, h->w, h->z, nullptr));
+    CF_CUDA(launch_chained(swim_finish_kernel, dim3(swim_grid(n)), dim3(256), 0, st, swim_params(h),
+                           ctl, static_cast<const double *>(h->z), h->sol, n,
+                           h->d.phase_dot, h->d.angle_dot));
+    CF_CHECK_LAUNCH("swim_finish_kernel");
+    CF_CUDA(cudaMemcpyAsync(&h->h_rep->ctl[0], h->ctl, sizeof(SwimCtl), cudaMemcpyDeviceToHost, st));
+    CF_CUDA(cudaMemcpyAsync(h->h_rep->bv, h->sol + h->o_body, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
     CF_TRY(swim_sync(h));
-    h->last_iters = it;
-    h->last_relres = rel;
-    h->last_status = rel <= h->cfg.gmres_tol ? CF_OK : CF_NOT_CONVERGED;
+    const SwimCtl &c = h->h_rep->ctl[0];
+    h->last_iters = c.iters;
+    h->last_relres = c.relres;
+    h->last_status = c.status;
     return CF_OK;
 }
 
@@ -798,6 +977,12 @@ void swim_release(cf_swim *h) {
     cudaSetDevice(h->device);
     for (void *p : h->allocations) cudaFree(p);
     h->allocations.clear();
+    if (h->h_rep) cudaFreeHost(h->h_rep);
+    h->h_rep = nullptr;
+    for (cudaEvent_t &e : h->ev) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
     if (h->stream) cudaStreamDestroy(h->stream);
     h->stream = nullptr;
 }
@@ -894,7 +1079,10 @@ extern "C" int cf_swim_create(const cf_swim_config *cfg, cf_swim **out) {
             if (cfg->phase0) ph[m] = cfg->phase0[m];
             if (cfg->angle0) an[m] = cfg->angle0[m];
         }
-        const size_t N = h->N, np = h->N + h->B, nv = h->n;
+        const size_t N = h->N, np = h->N + h->B, nv = h->n, mi = h->max_iter;
+        // block partials: the begin kernel's sums, the dot products' chunks, the norms
+        const size_t npart = std::max({static_cast<size_t>(swim_blocks(h)) * kPreValues, (mi + 1) * kSwimChunks,
+                                       (nv + kSwT - 1) / kSwT, 4 * static_cast<size_t>(h->num_sms)});
         if ((rc = swim_upload(h, const_cast<double **>(&d.s_table), cfg->s_values_ref,
                               static_cast<size_t>(d.s_rows) * d.s_cols)) ||
             (rc = swim_upload(h, const_cast<double **>(&d.phase_refs), cfg->gen_phase_force_refs, d.n_phase_refs)) ||
@@ -911,15 +1099,29 @@ extern "C" int cf_swim_create(const cf_swim_config *cfg, cf_swim **out) {
             (rc = swim_alloc(h, &h->xb, 3 * static_cast<size_t>(h->B))) || (rc = swim_alloc(h, &h->body, 3)) ||
             (rc = swim_alloc(h, &h->aux, 12 * static_cast<size_t>(F))) || (rc = swim_alloc(h, &h->kinv, 36)) ||
             (rc = swim_alloc(h, &h->x4all, np)) || (rc = swim_alloc(h, &h->f4all, np)) ||
-            (rc = swim_alloc(h, &h->u, 3 * np)) || (rc = swim_alloc(h, &h->err, 1)) ||
+            (rc = swim_alloc(h, &h->err, 1)) ||
+            (rc = swim_upload(h, &h->d_qref, h->qref.data(), h->qref.size())) ||
+            (rc = swim_upload(h, &h->d_fil_ref, h->fil_ref.data(), h->fil_ref.size())) ||
+            (rc = swim_upload(h, &h->d_blob_ref, h->blob_ref.data(), h->blob_ref.size())) ||
             (rc = swim_alloc(h, &h->rhs, nv)) || (rc = swim_alloc(h, &h->sol, nv)) || (rc = swim_alloc(h, &h->w, nv)) ||
             (rc = swim_alloc(h, &h->z, nv)) || (rc = swim_alloc(h, &h->t, nv)) ||
             (rc = swim_alloc(h, &h->Q, static_cast<size_t>(h->max_iter + 1) * nv)) ||
-            (rc = swim_alloc(h, &h->hb, 3 * static_cast<size_t>(h->max_iter + 1) + 4)) ||
-            (rc = swim_alloc(h, &h->dpart, static_cast<size_t>(h->max_iter + 1) * kSwimChunks)) ||
-            (rc = swim_alloc(h, &h->dcount, 1)))
+            (rc = swim_alloc(h, &h->h1, mi + 1)) || (rc = swim_alloc(h, &h->h2, mi + 1)) ||
+            (rc = swim_alloc(h, &h->H, (mi + 1) * (mi + 1))) || (rc = swim_alloc(h, &h->cs, mi + 1)) ||
+            (rc = swim_alloc(h, &h->sn, mi + 1)) || (rc = swim_alloc(h, &h->beta, mi + 1)) || (rc = swim_alloc(h, &h->y, mi + 1)) ||
+            (rc = swim_alloc(h, &h->part, npart)) || (rc = swim_alloc(h, &h->counter, 1)) ||
+            (rc = swim_alloc(h, &h->ctl, 1)))
             break;
-        if ((rc = cuda_status(cudaMemset(h->dcount, 0, sizeof(unsigned int)), "cudaMemset", __FILE__, __LINE__))) break;
+        if ((rc = cuda_status(cudaMemset(h->counter, 0, sizeof(unsigned int)), "cudaMemset", __FILE__, __LINE__)) ||
+            (rc = cuda_status(cudaMemset(h->ctl, 0, sizeof(SwimCtl)), "cudaMemset", __FILE__, __LINE__)) ||
+            (rc = cuda_status(cudaMemset(h->rhs, 0, sizeof(double) * nv), "cudaMemset", __FILE__, __LINE__)) ||
+            (rc = cuda_status(cudaMallocHost(reinterpret_cast<void **>(&h->h_rep), sizeof(SwimReport)),
+                              "cudaMallocHost", __FILE__, __LINE__)) ||
+            (rc = cuda_status(cudaEventCreateWithFlags(&h->ev[0], cudaEventDisableTiming), "cudaEventCreate", __FILE__,
+                              __LINE__)) ||
+            (rc = cuda_status(cudaEventCreateWithFlags(&h->ev[1], cudaEventDisableTiming), "cudaEventCreate", __FILE__,
+                              __LINE__)))
+            break;
         d.Rfil = h->Rfil;
         RpyBlockDesc bd{};
         bd.wall = 0;
@@ -957,30 +1159,28 @@ extern "C" int cf_swim_step(cf_swim *h, int nt, int *iters, double *relres) {
     CF_CUDA(cudaSetDevice(h->device));
     cudaStream_t st = h->stream;
     SimDev &d = h->d;
-    CF_TRY(swim_frames(h));
-    LoopCtl lc{};
-    lc.nt = nt;
-    CF_CUDA(cudaMemcpyAsync(d.lc, &lc, sizeof(lc), cudaMemcpyHostToDevice, st));
+    BodyState body;
+    for (int c = 0; c < 3; ++c) body.x[c] = h->bx[c];
+    for (int c = 0; c < 4; ++c) body.q[c] = h->bq[c];
+    swim_frames_kernel<<<swim_grid(h->F + h->B), 256, 0, st>>>(body, h->F, h->B, h->d_qref, h->d_fil_ref, h->d_blob_ref,
+                                                               h->Rfil, const_cast<double *>(d.base), h->xb, h->body);
+    CF_CHECK_LAUNCH("swim_frames_kernel");
+    swim_set_step_kernel<<<1, 1, 0, st>>>(d.lc, nt);
+    CF_CHECK_LAUNCH("swim_set_step_kernel");
     const int ns = h->nseg;
     const int threads = std::min(256, std::max(64, (3 * ns + 31) / 32 * 32));
     const size_t kin_smem = sizeof(double) * (2 * (10 * ns + 1) + ns);
     kinematics_kernel<<<h->F, threads, kin_smem, st>>>(d);
     CF_CHECK_LAUNCH("kinematics_kernel");
-    swim_pack_positions_kernel<<<swim_grid(h->N + h->B), 256, 0, st>>>(d.x4, h->xb, h->N, h->B, h->x4all);
-    CF_CHECK_LAUNCH("swim_pack_positions_kernel");
-    CF_TRY(swim_precon_matrix(h));  // synchronises
     const SwimParams p = swim_params(h);
-    CF_CUDA(cudaMemsetAsync(h->rhs, 0, sizeof(double) * h->n, st));
-    swim_rhs_kernel<<<swim_grid(h->F), 256, 0, st>>>(p, d, h->rhs);
-    CF_CHECK_LAUNCH("swim_rhs_kernel");
+    swim_begin_kernel<<<swim_blocks(h), kSwT, 0, st>>>(p, d, h->x4all, h->rhs, h->aux, d.gram, h->kinv, h->part,
+                                                       h->counter, h->ctl);
+    CF_CHECK_LAUNCH("swim_begin_kernel");
     CF_TRY(swim_gmres(h));
+    if (h->h_rep->ctl[0].singular)
+        return set_error(CF_NONFINITE, "cf_swim: the body's 6x6 preconditioner matrix is singular");
     h->stepped = true;
-    // the rates the next step advances with, and the body's velocity for its update
-    const size_t fb = sizeof(double) * h->F;
-    CF_CUDA(cudaMemcpyAsync(d.phase_dot, h->sol + h->o_phase, fb, cudaMemcpyDeviceToDevice, st));
-    CF_CUDA(cudaMemcpyAsync(d.angle_dot, h->sol + h->o_angle, fb, cudaMemcpyDeviceToDevice, st));
-    CF_CUDA(cudaMemcpyAsync(h->bv, h->sol + h->o_body, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CF_CUDA(cudaStreamSynchronize(st));
+    for (int c = 0; c < 6; ++c) h->bv[c] = h->h_rep->bv[c];
     if (iters) *iters = h->last_iters;
     if (relres) *relres = h->last_relres;
     if (h->last_status == CF_NONFINITE)
@@ -1064,7 +1264,7 @@ extern "C" int cf_swim_apply_preconditioner(cf_swim *h, const double *in, double
     CF_REQUIRE(h && in && out && h->stepped, "cf_swim_apply_preconditioner: bad arguments or no step yet");
     CF_CUDA(cudaSetDevice(h->device));
     CF_CUDA(cudaMemcpyAsync(h->t, in, sizeof(double) * h->n, cudaMemcpyHostToDevice, h->stream));
-    CF_TRY(swim_precond(h, h->t, h->z));
+    CF_TRY(swim_precond(h, nullptr, nullptr, h->t, nullptr, h->w, h->z, nullptr));
     CF_CUDA(cudaMemcpyAsync(out, h->z, sizeof(double) * h->n, cudaMemcpyDeviceToHost, h->stream));
     return swim_sync(h);
 }
