@@ -186,9 +186,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rpy_tile_kernel(TilePara
 // one partial per tile (RpyPlan says where) -- no atomics, deterministic; the
 // reduction adds the self blocks.
 //
-// Bound by instruction issue (3x3: 84 FP32 instructions and 9 shuffles a pair; 6x6
-// above the wall: about 200 and 21, where two one-sided evaluations take about 600).
-// A product above the wall: 20,480 segments 880 us; 5,120 with torques 127 us, by tiles 214.
+// This kernel serves the sets with torques (the one below those without).  Bound by
+// instruction issue: above the wall about 200 FP32 instructions and 21 shuffles a pair
+// of particles with torques, where two one-sided evaluations take about 600.
+// 5,120 particles with torques above the wall take 127 us a product, by tiles 214.
 struct SymParams {
     const float4 *x;
     const float4 *f;
@@ -260,8 +261,8 @@ __device__ __forceinline__ void sym_tiles(const SymParams &p, const FreeSym6 &k,
     auto pair = [&](float *vj) {
         const float dx = xi.x - xs.x, dy = xi.y - xs.y, dz = xi.z - xs.z;
         if constexpr (!SI && !SJ) {
-            if constexpr (WALL) wall_pair_sym_f32(dx, dy, dz, xi.z, xs.z, fs, fi, vi, vj);
-            else free_pair_sym_f32(dx, dy, dz, k.t, fs, fi, vi, vj);
+            if constexpr (WALL) wall_pair_sym<float>(dx, dy, dz, xi.z, xs.z, fs, fi, vi, vj);
+            else free_pair_sym<float>(dx, dy, dz, k.t, fs, fi, vi, vj);
         } else {
             if constexpr (WALL) wall_pair_sym6_f32<SI, SJ>(dx, dy, dz, xi.z, xs.z, fs, fi, vi, vj);
             else free_pair_sym6_f32<SI, SJ>(dx, dy, dz, k, fs, fi, vi, vj);
@@ -298,30 +299,133 @@ __device__ __forceinline__ void sym_tiles(const SymParams &p, const FreeSym6 &k,
     }
 }
 
-// DOF6: the first p.n6 > 0 particles have torques and spins (5 blocks per SM for their registers).
+// The first p.n6 > 0 particles have torques and spins (5 blocks per SM for their registers).
 constexpr int kSym6CtasPerSm = 5;
-template <bool WALL, bool DOF6>
-__global__ void __launch_bounds__(kThreads, DOF6 ? kSym6CtasPerSm : kCtasPerSm) rpy_sym_kernel(SymParams p) {
+template <bool WALL>
+__global__ void __launch_bounds__(kThreads, kSym6CtasPerSm) rpy_sym6_kernel(SymParams p) {
     chain_wait();  // launched as a programmatic dependent of the packing launch
     if (p.gate && *p.gate == 0) return;
     FreeSym6 k{};
-    if constexpr (!WALL) {
-        if constexpr (DOF6) k = free_sym6(p.a, p.inv_mu);
-        else k.t = free_sym(p.a, p.inv_mu);
-    }
+    if constexpr (!WALL) k = free_sym6(p.a, p.inv_mu);
     const int lane = threadIdx.x & 31;
     const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
     for (long long t = static_cast<long long>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5); t < p.items;
          t += nwarps) {
         int I, J;
         sym_item(t, p.nb, I, J);
-        if constexpr (DOF6) {  // uniform over the warp; J >= I, so J has torques only if I has
-            if (J * 32 < p.n6) sym_tiles<WALL, true, true>(p, k, I, J, lane);
-            else if (I * 32 < p.n6) sym_tiles<WALL, true, false>(p, k, I, J, lane);
-            else sym_tiles<WALL, false, false>(p, k, I, J, lane);
-        } else {
-            sym_tiles<WALL, false, false>(p, k, I, J, lane);
+        // uniform over the warp; J >= I, so J has torques only if I has
+        if (J * 32 < p.n6) sym_tiles<WALL, true, true>(p, k, I, J, lane);
+        else if (I * 32 < p.n6) sym_tiles<WALL, true, false>(p, k, I, J, lane);
+        else sym_tiles<WALL, false, false>(p, k, I, J, lane);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same without torques, two sources a lane in packed arithmetic.  Work unit: one warp, the 32 targets of tile I
+// and the 64 sources of tiles 2K and 2K + 1, K >= I / 2.  The sources lie in shared memory as packed pairs (source l of
+// one tile with source l of the other), so a lane reads the pair of step s at l + s, and only the accumulators of the
+// sources rotate.  In the units K = I / 2 the tile meets itself: those pairs are evaluated one-sided and a particle
+// never meets itself; an odd I leaves the other half empty there.
+//
+// Every particle receives one partial per tile, as above: FP32 sums are of 32 terms.
+//
+// Bound by the FP32 pipe, at 81% of it (86 packed instructions for both directions of two pairs): a product of 20,480
+// segments above the wall takes 690 us; 880 us with one source a lane and its position and force rotating by shuffles.
+// The loop alone: 3.01 ms for 10^9 pairs, one scalar source 3.60, two rotating packed ones 3.13.
+constexpr int kSym3CtasPerSm = 4;
+using Sym3Smem = ulonglong2[3][64];
+
+__device__ __forceinline__ void sym3_unit(long long t, int nb, int &I, int &K) {
+    const int nk = (nb + 1) / 2;
+    int T;
+    sym_item(t >> 1, nk, T, K);
+    I = 2 * T + static_cast<int>(t & 1);
+}
+
+// store(particle, tile, velocity)
+template <bool WALL, class Store>
+__device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const float4 *__restrict__ f, int n, int nb,
+                                           const FreeSym &k, int I, int K, int lane, Sym3Smem &sm, Store store) {
+    if (I >= nb) return;
+    const unsigned full = 0xffffffffu;
+    const int src_lane = (lane + 1) & 31;
+    const bool own = K == I >> 1, odd_own = own && (I & 1);
+    const int i = I * 32 + lane, ja = odd_own ? i : K * 64 + lane, jb = odd_own ? n : K * 64 + 32 + lane;
+    auto load = [&](int idx, float apart, float4 &xv, float4 &fv) {
+        if (idx < n) {
+            xv = x[idx];
+            fv = f[idx];
+        } else {  // inert: far from everything and from each other, no force
+            xv = make_float4(1.0e5f * static_cast<float>(lane + 1), apart, 1.0e4f, 0.0f);
+            fv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
+    };
+    float4 xi, fi4, xa, fa, xb, fb;
+    load(i, 0.0f, xi, fi4);
+    load(ja, 1.0e5f, xa, fa);
+    load(jb, 2.0e5f, xb, fb);
+    const ulonglong2 q0 = make_ulonglong2(pack2(xa.x, xb.x).v, pack2(xa.y, xb.y).v),
+                     q1 = make_ulonglong2(pack2(xa.z, xb.z).v, pack2(fa.x, fb.x).v),
+                     q2 = make_ulonglong2(pack2(fa.y, fb.y).v, pack2(fa.z, fb.z).v);
+    __syncwarp();  // the last unit's reads
+    sm[0][lane] = sm[0][lane + 32] = q0;
+    sm[1][lane] = sm[1][lane + 32] = q1;
+    sm[2][lane] = sm[2][lane + 32] = q2;
+    __syncwarp();
+    const F2 tx = splat<F2>(xi.x), ty = splat<F2>(xi.y), tz = splat<F2>(xi.z);
+    const F2 fi[3] = {splat<F2>(fi4.x), splat<F2>(fi4.y), splat<F2>(fi4.z)};
+    F2 vi[3] = {}, vj[3] = {};
+    auto pair = [&](F2 sx, F2 sy, F2 sz, const F2 *fj) {
+        if constexpr (WALL) wall_pair_sym<F2>(vsub(tx, sx), vsub(ty, sy), vsub(tz, sz), tz, sz, fj, fi, vi, vj);
+        else free_pair_sym<F2>(vsub(tx, sx), vsub(ty, sy), vsub(tz, sz), k, fj, fi, vi, vj);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) vj[c].v = __shfl_sync(full, vj[c].v, src_lane);
+    };
+    if (!own) {
+#pragma unroll 8
+        for (int s = 0; s < 32; ++s) {
+            const ulonglong2 a = sm[0][lane + s], b = sm[1][lane + s], c = sm[2][lane + s];
+            const F2 fj[3] = {F2{b.y}, F2{c.x}, F2{c.y}};
+            pair(F2{a.x}, F2{a.y}, F2{b.x}, fj);
+        }
+    } else {
+#pragma unroll 1
+        for (int s = 0; s < 32; ++s) {
+            const ulonglong2 a = sm[0][lane + s], b = sm[1][lane + s], c = sm[2][lane + s];
+            F2 sx{a.x}, fj[3] = {F2{b.y}, F2{c.x}, F2{c.y}};
+            if (s == 0) {
+                // at step 0 the own tile's half is the particle itself: an inert one instead
+                sx = pack2(-1.0e5f * static_cast<float>(lane + 1), unpack2(sx).y);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) fj[q] = pack2(0.0f, unpack2(fj[q]).y);
+            }
+            pair(sx, F2{a.y}, F2{b.x}, fj);
+        }
+    }
+    auto lo = [](F2 a) { return unpack2(a).x; };
+    auto hi = [](F2 a) { return unpack2(a).y; };
+    if (i < n) {  // two partials: their sum is left to FP64
+        store(i, odd_own ? I : 2 * K, make_float4(lo(vi[0]), lo(vi[1]), lo(vi[2]), 0.0f));
+        if (!odd_own && 2 * K + 1 < nb) store(i, 2 * K + 1, make_float4(hi(vi[0]), hi(vi[1]), hi(vi[2]), 0.0f));
+    }
+    if (ja < n && !own) store(ja, I, make_float4(lo(vj[0]), lo(vj[1]), lo(vj[2]), 0.0f));
+    if (jb < n) store(jb, I, make_float4(hi(vj[0]), hi(vj[1]), hi(vj[2]), 0.0f));
+}
+
+template <bool WALL>
+__global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_sym3_kernel(SymParams p) {
+    __shared__ Sym3Smem sm[kThreads / 32];
+    chain_wait();  // launched as a programmatic dependent of the packing launch
+    if (p.gate && *p.gate == 0) return;
+    FreeSym k{};
+    if constexpr (!WALL) k = free_sym(p.a, p.inv_mu);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
+    auto store = [&](int q, int slot, float4 v) { p.partial[static_cast<size_t>(q) * p.nb + slot] = v; };
+    for (long long t = static_cast<long long>(blockIdx.x) * (kThreads / 32) + w; t < p.items; t += nwarps) {
+        int I, K;
+        sym3_unit(t, p.nb, I, K);
+        sym3_tiles<WALL>(p.x, p.f, p.n, p.nb, k, I, K, lane, sm[w], store);
     }
 }
 
@@ -333,14 +437,12 @@ __global__ void __launch_bounds__(kThreads, DOF6 ? kSym6CtasPerSm : kCtasPerSm) 
 // stored slot-major per array, partial[poff + slot * n + i] (slot = the other
 // tile of the pair), so that both these writes and the per-segment reduction
 // that reads them are coalesced.
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) rpy_wall_sym_batch_kernel(SymBatchParams p) {
+__global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_wall_sym_batch_kernel(SymBatchParams p) {
+    __shared__ Sym3Smem sm[kThreads / 32];
     chain_wait();
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int src_lane = (lane + 1) & 31;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
-    for (long long t = static_cast<long long>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5); t < p.items;
-         t += nwarps) {
+    for (long long t = static_cast<long long>(blockIdx.x) * (kThreads / 32) + w; t < p.items; t += nwarps) {
         int lo = 0, hi = p.B - 1;  // last array whose first item <= t
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -349,54 +451,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rpy_wall_sym_batch_kerne
         }
         const int b = lo;
         if (p.active && !p.active[b]) continue;
-        const int nb = p.nb[b];
-        SymParams q;
-        q.x = p.x + p.seg0[b];
-        q.f = p.f + p.seg0[b];
-        q.partial = p.partial + p.poff[b];
-        q.n = p.n[b];
-        q.nb = nb;
-        int I, J;
-        sym_item(t - p.item0[b], nb, I, J);
-        const int i = I * 32 + lane;
-        const int j = J * 32 + lane;
-        float4 xi, fi, xs, fs;
-        sym_load(q, i, lane, xi, fi);
-        sym_load(q, j, lane, xs, fs);
-        const float fiv[3] = {fi.x, fi.y, fi.z};
-        float vi[3] = {0.0f, 0.0f, 0.0f};
-        if (I == J) {
-#pragma unroll 1
-            for (int step = 1; step < 32; ++step) {
-                xs.x = __shfl_sync(full, xs.x, src_lane);
-                xs.y = __shfl_sync(full, xs.y, src_lane);
-                xs.z = __shfl_sync(full, xs.z, src_lane);
-                fs.x = __shfl_sync(full, fs.x, src_lane);
-                fs.y = __shfl_sync(full, fs.y, src_lane);
-                fs.z = __shfl_sync(full, fs.z, src_lane);
-                const float fsv[3] = {fs.x, fs.y, fs.z};
-                wall_pair_f32<3, 3>(xi.x - xs.x, xi.y - xs.y, xi.z - xs.z, xi.z, xs.z, fsv, vi);
-            }
-            if (i < q.n) q.partial[static_cast<size_t>(I) * q.n + i] = make_float4(vi[0], vi[1], vi[2], 0.0f);
-        } else {
-            float vs[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll 2
-            for (int step = 0; step < 32; ++step) {
-                const float fsv[3] = {fs.x, fs.y, fs.z};
-                wall_pair_sym_f32(xi.x - xs.x, xi.y - xs.y, xi.z - xs.z, xi.z, xs.z, fsv, fiv, vi, vs);
-                xs.x = __shfl_sync(full, xs.x, src_lane);
-                xs.y = __shfl_sync(full, xs.y, src_lane);
-                xs.z = __shfl_sync(full, xs.z, src_lane);
-                fs.x = __shfl_sync(full, fs.x, src_lane);
-                fs.y = __shfl_sync(full, fs.y, src_lane);
-                fs.z = __shfl_sync(full, fs.z, src_lane);
-                vs[0] = __shfl_sync(full, vs[0], src_lane);
-                vs[1] = __shfl_sync(full, vs[1], src_lane);
-                vs[2] = __shfl_sync(full, vs[2], src_lane);
-            }
-            if (i < q.n) q.partial[static_cast<size_t>(J) * q.n + i] = make_float4(vi[0], vi[1], vi[2], 0.0f);
-            if (j < q.n) q.partial[static_cast<size_t>(I) * q.n + j] = make_float4(vs[0], vs[1], vs[2], 0.0f);
-        }
+        const int n = p.n[b], nb = p.nb[b];
+        float4 *partial = p.partial + p.poff[b];
+        auto store = [&](int q, int slot, float4 v) { partial[static_cast<size_t>(slot) * n + q] = v; };
+        int I, K;
+        sym3_unit(t - p.item0[b], nb, I, K);
+        sym3_tiles<true>(p.x + p.seg0[b], p.f + p.seg0[b], n, nb, FreeSym{}, I, K, lane, sm[w], store);
     }
 }
 
@@ -655,8 +715,8 @@ RpyPlan rpy_plan_sym(int n, int n6, int num_sms) {
     pl.ti = 1;
     const int nb = std::max(1, (n + 31) / 32);
     pl.nb = nb;
-    pl.items = static_cast<long long>(nb) * (nb + 1) / 2;
-    const int per_sm = n6 > 0 ? kSym6CtasPerSm : kCtasPerSm;
+    pl.items = n6 > 0 ? static_cast<long long>(nb) * (nb + 1) / 2 : rpy_sym_items(nb);
+    const int per_sm = n6 > 0 ? kSym6CtasPerSm : kSym3CtasPerSm;
     const long long max_warps = static_cast<long long>(std::max(1, num_sms)) * per_sm * (kThreads / 32);
     const long long per_warp = (pl.items + max_warps - 1) / max_warps;  // balanced: every warp does per_warp items
     const long long warps = (pl.items + per_warp - 1) / per_warp;
@@ -751,10 +811,10 @@ int rpy_launch_tiles(const RpyBlockDesc &d, const RpyPlan &plan, float4 *scratch
         p.gate = d.gate;
         p.t = d.ts;
         p.n6 = plan.n6;
-        auto kern = d.wall ? (plan.n6 ? rpy_sym_kernel<true, true> : rpy_sym_kernel<true, false>)
-                           : (plan.n6 ? rpy_sym_kernel<false, true> : rpy_sym_kernel<false, false>);
+        auto kern = d.wall ? (plan.n6 ? rpy_sym6_kernel<true> : rpy_sym3_kernel<true>)
+                           : (plan.n6 ? rpy_sym6_kernel<false> : rpy_sym3_kernel<false>);
         CF_CUDA(launch_chained(kern, dim3(plan.grid), dim3(kThreads), 0, st, p));
-        CF_CHECK_LAUNCH("rpy_sym_kernel");
+        CF_CHECK_LAUNCH("rpy_sym kernel");
         return CF_OK;
     }
     const bool self = d.self_set != 0;
@@ -920,6 +980,6 @@ int rpy_launch_sym_batch(const SymBatchParams &p, int grid, cudaStream_t st) {
     return CF_OK;
 }
 
-int rpy_sym_batch_max_grid(int num_sms) { return std::max(1, num_sms) * kCtasPerSm; }
+int rpy_sym_batch_max_grid(int num_sms) { return std::max(1, num_sms) * kSym3CtasPerSm; }
 
 }  // namespace cufil

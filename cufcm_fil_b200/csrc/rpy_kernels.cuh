@@ -89,7 +89,7 @@ int rpy_launch_tiles(const RpyBlockDesc &d, const RpyPlan &plan, float4 *scratch
 // Batched symmetric wall products (segments on segments, 3x3) of B independent
 // particle sets stored back to back.  Per array b: particles [seg0[b], seg0[b]+n[b])
 // of x/f, nb[b] = ceil(n[b]/32) tiles, partials at partial + poff[b] laid out
-// slot-major, [tile * n[b] + i], and work items [item0[b], item0[b+1]) (item0[B] == items).
+// slot-major, [tile * n[b] + i], and rpy_sym_items(nb[b]) work items [item0[b], item0[b+1]) (item0[B] == items).
 struct SymBatchParams {
     const float4 *x;
     const float4 *f;
@@ -101,6 +101,10 @@ struct SymBatchParams {
     long long items;
 };
 int rpy_launch_sym_batch(const SymBatchParams &p, int grid, cudaStream_t st);
+// Work items of a force-only set of nb tiles.
+__host__ __device__ constexpr long long rpy_sym_items(int nb) {
+    return static_cast<long long>((nb + 1) / 2) * ((nb + 1) / 2 + 1);
+}
 // Largest useful grid of the batched kernel (one resident wave).
 int rpy_sym_batch_max_grid(int num_sms);
 

@@ -13,6 +13,8 @@
 
 #include <cuda_runtime.h>
 
+#include "packed.cuh"
+
 namespace cufil {
 
 struct RpyConst {
@@ -263,59 +265,57 @@ namespace cufil {
 //   b  =  w u (3/2 z_j + hz (u (2G + 5u) - 9P)) / 6 pi
 //   c  =  w u (3/2 z_j - 5 hz u^2) / 6 pi
 //   e  = -w u (3 z_j^2 + 3E + u (2 - 15E)) / 6 pi
-// The kernel is bound by instruction issue: 84 FP32 instructions and two reciprocal square roots for both
-// directions; written with the reference's factors it was 109, three and a division (20,480 segments 994 us a
-// product, 880 so).
-__device__ __forceinline__ void wall_pair_sym_f32(float dx, float dy, float dz, float zi, float zj, const float *fj,
-                                                  const float *fi, float *vi, float *vj) {
-    const float c6 = RpyConst::inv6pi;
-    const float c8 = RpyConst::inv8pi;
-    const float q2 = fmaf(dx, dx, dy * dy);
+// 86 FP32 instructions and two reciprocal square roots for both directions; written with the reference's factors it
+// was 109, three and a division (a product of 20,480 segments took 994 us so, 880 without the division, both scalar).
+template <class T>
+__device__ __forceinline__ void wall_pair_sym(T dx, T dy, T dz, T zi, T zj, const T *fj, const T *fi, T *vi, T *vj) {
+    auto k = [](float c) { return splat<T>(c); };
+    const T q2 = vfma(dx, dx, vmul(dy, dy));
     // free space: A I + B d d^T (even in d)
-    const float s = rsqrtf(fmaf(dz, dz, q2));
-    const float s2 = s * s;
-    const float g = c8 * s;
-    const float A = g * fmaf(2.0f / 3.0f, s2, 1.0f);
-    const float B = (g * s2) * fmaf(-2.0f, s2, 1.0f);
-    // image system
-    const float hz = zi + zj;
-    const float w = rsqrtf(fmaf(hz, hz, q2));
-    const float u = w * w;
-    const float cw = c6 * w, cu = cw * u;
-    const float hu = hz * u, E = hz * hu;
-    const float P = (zi * zj) * u;
-    const float n5 = fmaf(7.5f, E, -1.5f);  // -3/2 (1 - 5E)
-    const float u5 = 5.0f * u;
-    const float G = fmaf(0.5f * u5, fmaf(-7.0f, E, 1.0f), n5);
-    const float k0 = fmaf(u, fmaf(u * (1.0f / 3.0f), n5, fmaf(-1.5f, E, 0.5f)), fmaf(1.5f, P, 0.75f));
-    const float AK = fmaf(-cw, k0, A);
-    const float a = -cu * fmaf(u, G, fmaf(-4.5f, P, 0.75f));
-    const float z15 = 1.5f * zj;
-    const float b = cu * fmaf(-9.0f * P, hz, fmaf(hu, fmaf(2.0f, G, u5), z15));
-    const float c = cu * fmaf(-u5, hu, z15);
-    const float e = -cu * fmaf(2.0f * z15, zj, fmaf(u, fmaf(-15.0f, E, 2.0f), 3.0f * E));
-    const float AKe = AK + e;
+    const T s = rsqrt_approx(vfma(dz, dz, q2));
+    const T s2 = vmul(s, s);
+    const T g = vmul(k(RpyConst::inv8pi), s);
+    const T A = vmul(g, vfma(k(2.0f / 3.0f), s2, k(1.0f)));
+    const T B = vmul(vmul(g, s2), vfma(k(-2.0f), s2, k(1.0f)));
+    // image system; cw = -w / 6 pi, cu = cw u (the signs of the brackets below are turned accordingly)
+    const T hz = vadd(zi, zj);
+    const T w = rsqrt_approx(vfma(hz, hz, q2));
+    const T u = vmul(w, w);
+    const T cw = vmul(k(-RpyConst::inv6pi), w), cu = vmul(cw, u);
+    const T hu = vmul(hz, u), E = vmul(hz, hu);
+    const T P = vmul(vmul(zi, zj), u);
+    const T n5 = vfma(k(7.5f), E, k(-1.5f));  // -3/2 (1 - 5E)
+    const T u5 = vmul(k(5.0f), u);
+    const T G = vfma(u5, vfma(k(-3.5f), E, k(0.5f)), n5);
+    const T k0 = vfma(u, vfma(vmul(u, k(1.0f / 3.0f)), n5, vfma(k(-1.5f), E, k(0.5f))), vfma(k(1.5f), P, k(0.75f)));
+    const T AK = vfma(cw, k0, A);
+    const T a = vmul(cu, vfma(u, G, vfma(k(-4.5f), P, k(0.75f))));
+    const T z15 = vmul(k(-1.5f), zj);
+    const T b = vmul(cu, vfma(vmul(k(9.0f), P), hz, vfma(vmul(k(-1.0f), hu), vfma(k(2.0f), G, u5), z15)));
+    const T c = vmul(cu, vfma(u5, hu, z15));
+    const T e = vmul(cu, vfma(vmul(k(-2.0f), z15), zj, vfma(u, vfma(k(-15.0f), E, k(2.0f)), vmul(k(3.0f), E))));
+    const T AKe = vadd(AK, e);
     // i <- j
     {
-        const float p = fmaf(dx, fj[0], dy * fj[1]);
-        const float dp = fmaf(hz, fj[2], p);
-        const float t0 = B * fmaf(dz, fj[2], p);
-        const float t1 = fmaf(a, dp, b * fj[2]);
-        const float t = t0 + t1;
-        vi[0] = fmaf(t, dx, fmaf(AK, fj[0], vi[0]));
-        vi[1] = fmaf(t, dy, fmaf(AK, fj[1], vi[1]));
-        vi[2] = fmaf(c, dp, fmaf(t1, hz, fmaf(t0, dz, fmaf(AKe, fj[2], vi[2]))));
+        const T p = vfma(dx, fj[0], vmul(dy, fj[1]));
+        const T dp = vfma(hz, fj[2], p);
+        const T t0 = vmul(B, vfma(dz, fj[2], p));
+        const T t1 = vfma(a, dp, vmul(b, fj[2]));
+        const T t = vadd(t0, t1);
+        vi[0] = vfma(t, dx, vfma(AK, fj[0], vi[0]));
+        vi[1] = vfma(t, dy, vfma(AK, fj[1], vi[1]));
+        vi[2] = vfma(c, dp, vfma(t1, hz, vfma(t0, dz, vfma(AKe, fj[2], vi[2]))));
     }
     // j <- i (transpose)
     {
-        const float p = fmaf(dx, fi[0], dy * fi[1]);
-        const float dp = fmaf(hz, fi[2], p);
-        const float t0 = B * fmaf(dz, fi[2], p);
-        const float t1 = fmaf(a, dp, c * fi[2]);
-        const float t = t0 + t1;
-        vj[0] = fmaf(t, dx, fmaf(AK, fi[0], vj[0]));
-        vj[1] = fmaf(t, dy, fmaf(AK, fi[1], vj[1]));
-        vj[2] = fmaf(b, dp, fmaf(t1, hz, fmaf(t0, dz, fmaf(AKe, fi[2], vj[2]))));
+        const T p = vfma(dx, fi[0], vmul(dy, fi[1]));
+        const T dp = vfma(hz, fi[2], p);
+        const T t0 = vmul(B, vfma(dz, fi[2], p));
+        const T t1 = vfma(a, dp, vmul(c, fi[2]));
+        const T t = vadd(t0, t1);
+        vj[0] = vfma(t, dx, vfma(AK, fi[0], vj[0]));
+        vj[1] = vfma(t, dy, vfma(AK, fi[1], vj[1]));
+        vj[2] = vfma(b, dp, vfma(t1, hz, vfma(t0, dz, vfma(AKe, fi[2], vj[2]))));
     }
 }
 
@@ -331,27 +331,45 @@ __device__ __forceinline__ FreeSym free_sym(float a, float inv_mu) {
     const float pi = 3.14159265358979f;
     return FreeSym{4.0f * a * a, a * a * (2.0f / 3.0f), inv_mu / (8.0f * pi), inv_mu / (6.0f * pi * a), 1.0f / a};
 }
-__device__ __forceinline__ void free_pair_sym_f32(float dx, float dy, float dz, const FreeSym &q, const float *fj,
-                                                  const float *fi, float *vi, float *vj) {
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    const float s = rsqrtf(r2);
-    const float s2 = s * s;
-    const float g = q.c8 * s;
-    float A = g * fmaf(q.k, s2, 1.0f);
-    float B = (g * s2) * fmaf(-3.0f * q.k, s2, 1.0f);
-    if (r2 <= q.a4) {
-        const float r = r2 > 0.0f ? r2 * s : 0.0f;
-        A = q.c6 * fmaf(-9.0f / 32.0f * q.ia, r, 1.0f);
-        B = r2 > 0.0f ? q.c6 * q.ia * (3.0f / 32.0f) * s : 0.0f;
+// One overlapping pair's A and B.
+__device__ __forceinline__ void free_overlap(const FreeSym &q, float r2, float s, float &A, float &B) {
+    const float r = r2 > 0.0f ? r2 * s : 0.0f;
+    A = q.c6 * fmaf(-9.0f / 32.0f * q.ia, r, 1.0f);
+    B = r2 > 0.0f ? q.c6 * q.ia * (3.0f / 32.0f) * s : 0.0f;
+}
+__device__ __forceinline__ void free_near(const FreeSym &q, float r2, float s, float &A, float &B) {
+    if (r2 <= q.a4) free_overlap(q, r2, s, A, B);
+}
+__device__ __forceinline__ void free_near(const FreeSym &q, F2 r2, F2 s, F2 &A, F2 &B) {
+    const float2 r = unpack2(r2);
+    if (fminf(r.x, r.y) <= q.a4) {
+        const float2 sv = unpack2(s);
+        float2 Av = unpack2(A), Bv = unpack2(B);
+        if (r.x <= q.a4) free_overlap(q, r.x, sv.x, Av.x, Bv.x);
+        if (r.y <= q.a4) free_overlap(q, r.y, sv.y, Av.y, Bv.y);
+        A = pack2(Av.x, Av.y);
+        B = pack2(Bv.x, Bv.y);
     }
-    const float tj = B * fmaf(dx, fj[0], fmaf(dy, fj[1], dz * fj[2]));
-    const float ti = B * fmaf(dx, fi[0], fmaf(dy, fi[1], dz * fi[2]));
-    vi[0] = fmaf(tj, dx, fmaf(A, fj[0], vi[0]));
-    vi[1] = fmaf(tj, dy, fmaf(A, fj[1], vi[1]));
-    vi[2] = fmaf(tj, dz, fmaf(A, fj[2], vi[2]));
-    vj[0] = fmaf(ti, dx, fmaf(A, fi[0], vj[0]));
-    vj[1] = fmaf(ti, dy, fmaf(A, fi[1], vj[1]));
-    vj[2] = fmaf(ti, dz, fmaf(A, fi[2], vj[2]));
+}
+template <class T>
+__device__ __forceinline__ void free_pair_sym(T dx, T dy, T dz, const FreeSym &q, const T *fj, const T *fi, T *vi,
+                                              T *vj) {
+    auto k = [](float c) { return splat<T>(c); };
+    const T r2 = vfma(dx, dx, vfma(dy, dy, vmul(dz, dz)));
+    const T s = rsqrt_approx(r2);
+    const T s2 = vmul(s, s);
+    const T g = vmul(k(q.c8), s);
+    T A = vmul(g, vfma(k(q.k), s2, k(1.0f)));
+    T B = vmul(vmul(g, s2), vfma(k(-3.0f * q.k), s2, k(1.0f)));
+    free_near(q, r2, s, A, B);
+    const T tj = vmul(B, vfma(dx, fj[0], vfma(dy, fj[1], vmul(dz, fj[2]))));
+    const T ti = vmul(B, vfma(dx, fi[0], vfma(dy, fi[1], vmul(dz, fi[2]))));
+    vi[0] = vfma(tj, dx, vfma(A, fj[0], vi[0]));
+    vi[1] = vfma(tj, dy, vfma(A, fj[1], vi[1]));
+    vi[2] = vfma(tj, dz, vfma(A, fj[2], vi[2]));
+    vj[0] = vfma(ti, dx, vfma(A, fi[0], vj[0]));
+    vj[1] = vfma(ti, dy, vfma(A, fi[1], vj[1]));
+    vj[2] = vfma(ti, dz, vfma(A, fi[2], vj[2]));
 }
 
 }  // namespace cufil

@@ -44,7 +44,7 @@ constexpr int kMinDotsChunk = 1024;
 
 // Launch shapes chosen by the autotuner (or the defaults).
 struct Tuning {
-    int pair_ctas_per_sm = 8;   // pair kernel residency target
+    int pair_ctas_per_sm = 4;   // pair kernel residency target (its launch bound)
     int dots_chunk = 4096;      // rows per dot-product item
     int dots_blocks_per_sm = 2;
     int update_blocks_per_sm = 8;
@@ -723,7 +723,7 @@ int engine_init(Engine *e, const cf_sim_config *cfgs, int B) {
         seg += a.N;
         voff += a.vlen;
         poff += static_cast<long long>(a.N) * a.nb;
-        item0 += static_cast<long long>(a.nb) * (a.nb + 1) / 2;
+        item0 += rpy_sym_items(a.nb);
         mi_max = std::max(mi_max, a.max_iter);
     }
     CF_REQUIRE(voff < (1LL << 31), "cf_batch_create: the batch vectors exceed 2^31 rows");
