@@ -8,6 +8,7 @@
 #include "rpy_kernels.cuh"
 
 #include <algorithm>
+#include <functional>
 #include <new>
 #include <vector>
 
@@ -155,11 +156,26 @@ bool one_set(const cf_mobility_config &c) {
     return (c.wall || c.seg_radius == c.blob_radius) && rpy_set_symmetric(c.n_seg + c.n_blob, set_n6(c));
 }
 
-// The full product from the callers' layouts (device).
+bool overlap(const float *a, size_t na, const float *b, size_t nb) {
+    return na > 0 && nb > 0 && std::less<const float *>()(a, b + nb) && std::less<const float *>()(b, a + na);
+}
+
+// The full product from the callers' layouts (device).  The direct kernel reads inputs while others are written, so
+// velocities that share memory with an input take the packed way.
 int eval_full(cf_mobility *h, float *v_segs, float *v_blobs, cudaStream_t st);
 int apply_full(cf_mobility *h, const float *x_segs, const float *x_blobs, const float *f_segs, const float *f_blobs,
                float *v_segs, float *v_blobs, cudaStream_t st) {
     const cf_mobility_config &c = h->cfg;
+    const size_t ns = c.n_seg, nb = c.n_blob;
+    auto shared = [&](const float *v, size_t n) {
+        return overlap(v, n, x_segs, 3 * ns) || overlap(v, n, f_segs, 6 * ns) || overlap(v, n, x_blobs, 3 * nb) ||
+               overlap(v, n, f_blobs, 3 * nb);
+    };
+    if (set_n6(c) == 0 && c.n_seg + c.n_blob <= kRpyDirectMax && one_set(c) && !shared(v_segs, 6 * ns) &&
+        !shared(v_blobs, 3 * nb))
+        return rpy_direct_product(c.wall, x_segs, f_segs, x_blobs, f_blobs, c.n_seg, c.n_blob,
+                                  static_cast<float>(c.n_seg ? c.seg_radius : c.blob_radius), static_cast<float>(c.mu),
+                                  v_segs, v_blobs, st);
     CF_TRY(pack_sets_to_float4(x_segs, f_segs, x_blobs, f_blobs, c.n_seg, c.n_blob, h->xs4, h->fs4, h->ts4, st));
     return eval_full(h, v_segs, v_blobs, st);
 }

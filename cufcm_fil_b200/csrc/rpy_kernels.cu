@@ -597,6 +597,65 @@ __global__ void __launch_bounds__(256) rpy_set_reduce_kernel(SetReduceParams p) 
     }
 }
 
+// Small sets of force-only particles, one launch: four warps per target, their lanes over the sources (FP32 sums of at
+// most kRpyDirectMax / 128 terms a lane, then FP64), reading and writing the callers' layouts.  What it saves is the
+// packing, the partials and two launches; what it costs is evaluating each pair twice, so it stops paying where the
+// pairs outweigh the launches: above the wall 320 particles take 2.9 us, 7.9 by the symmetric kernel; 1,020 6.6 and
+// 8.5; 1,520 12.0 and 11.0 (without a wall 2.7 and 7.9, 4.9 and 7.9, 8.0 and 9.6, and at 2,040 13.3 and 10.9).  Bound
+// by the latency of a lane's chain of pairs: with one warp per target it was 6.0 us at 320, 10.4 at 640.
+constexpr int kDirectWarps = 4;  // the last sum below is written for four
+struct DirectParams {
+    const float *xs, *fs, *xb, *fb;
+    float *vs, *vb;
+    int ns, n;
+    float a, inv_mu, self_t;
+};
+template <bool WALL>
+__global__ void __launch_bounds__(256) rpy_direct_kernel(DirectParams p) {
+    constexpr int kLanes = 32 * kDirectWarps;
+    __shared__ double part[256 / 32][3];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rank = threadIdx.x % kLanes;
+    const int target = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes, i = min(target, p.n - 1);
+    auto position = [&](int q) { return q < p.ns ? p.xs + 3 * q : p.xb + 3 * (q - p.ns); };
+    auto force = [&](int q) { return q < p.ns ? p.fs + 6 * q : p.fb + 3 * (q - p.ns); };
+    FreeSym k{};
+    if constexpr (!WALL) k = free_sym(p.a, p.inv_mu);
+    const float *xi = position(i);
+    const float x = xi[0], y = xi[1], z = xi[2];
+    float v[3] = {0.0f, 0.0f, 0.0f};
+    const float none[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll 2
+    for (int j = rank; j < p.n; j += kLanes) {
+        const float *xj = position(j), *fj = force(j);
+        const float f[3] = {fj[0], fj[1], fj[2]};
+        const float px = xj[0], py = xj[1], pz = xj[2];
+        if (j == i) continue;
+        float drop[3] = {0.0f, 0.0f, 0.0f};
+        if constexpr (WALL) wall_pair_sym<float>(x - px, y - py, z - pz, z, pz, f, none, v, drop);
+        else free_pair_sym<float>(x - px, y - py, z - pz, k, f, none, v, drop);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double s = v[c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) part[w][c] = s;
+    }
+    __syncthreads();
+    if (rank != 0 || target >= p.n) return;
+    const float *fi = force(i);
+    const float f[3] = {fi[0], fi[1], fi[2]};
+    float self[3] = {0.0f, 0.0f, 0.0f};
+    if constexpr (WALL) wall_self_f32<3, 3>(z, f, self);
+    else
+        for (int c = 0; c < 3; ++c) self[c] = p.self_t * f[c];
+    float *o = i < p.ns ? p.vs + 6 * static_cast<size_t>(i) : p.vb + 3 * static_cast<size_t>(i - p.ns);
+    for (int c = 0; c < 3; ++c)
+        o[c] = static_cast<float>((part[w][c] + part[w + 1][c]) + (part[w + 2][c] + part[w + 3][c]) + self[c]);
+    if (i < p.ns)
+        for (int c = 3; c < 6; ++c) o[c] = 0.0f;
+}
+
 __global__ void pack_xyz_kernel(const float *__restrict__ a, float4 *__restrict__ o, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) o[i] = make_float4(a[3 * i], a[3 * i + 1], a[3 * i + 2], 0.0f);
@@ -855,6 +914,18 @@ int rpy_launch_reduce_f32(const RpyBlockDesc &d, const RpyPlan &plan, const floa
     if (d.vd == 6 && d.fd == 3) return ws ? launch_reduce_t<true, 6, 3>(p, st) : launch_reduce_t<false, 6, 3>(p, st);
     if (d.vd == 3 && d.fd == 6) return ws ? launch_reduce_t<true, 3, 6>(p, st) : launch_reduce_t<false, 3, 6>(p, st);
     return set_error(CF_EINVAL, "rpy: unsupported dof pair %d/%d", d.vd, d.fd);
+}
+
+int rpy_direct_product(int wall, const float *x_segs, const float *f_segs, const float *x_blobs, const float *f_blobs,
+                       int n_seg, int n_blob, float a, float mu, float *v_segs, float *v_blobs, cudaStream_t st) {
+    DirectParams p{x_segs, f_segs, x_blobs, f_blobs, v_segs, v_blobs, n_seg, n_seg + n_blob, a, 1.0f / mu,
+                   static_cast<float>(1.0 / (6.0 * 3.14159265358979323846 * mu * a))};
+    if (p.n <= 0) return CF_OK;
+    const int per_block = 256 / (32 * kDirectWarps), blocks = (p.n + per_block - 1) / per_block;
+    if (wall) rpy_direct_kernel<true><<<blocks, 256, 0, st>>>(p);
+    else rpy_direct_kernel<false><<<blocks, 256, 0, st>>>(p);
+    CF_CHECK_LAUNCH("rpy_direct_kernel");
+    return CF_OK;
 }
 
 int pack_xyz_to_float4(const float *aos3, float4 *out, int n, cudaStream_t st) {

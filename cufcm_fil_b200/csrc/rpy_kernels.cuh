@@ -123,6 +123,12 @@ int rpy_launch_reduce_f32(const RpyBlockDesc &d, const RpyPlan &plan, const floa
 // (cf_set_wait_limit); the default is the full limit.
 unsigned rpy_wait_limit();
 
+// The full product of a small set of force-only particles (the wall, or equal radii) in one launch, straight from and to
+// the reference's layouts: segments x [3 n_seg], f [6 n_seg], v [6 n_seg] (spins zero), blobs x, f, v [3 n_blob].
+constexpr int kRpyDirectMax = 1280;  // largest n_seg + n_blob (see rpy_kernels.cu)
+int rpy_direct_product(int wall, const float *x_segs, const float *f_segs, const float *x_blobs, const float *f_blobs,
+                       int n_seg, int n_blob, float a, float mu, float *v_segs, float *v_blobs, cudaStream_t st);
+
 // Packing helpers between the reference's AoS host layouts and float4 arrays.
 int pack_xyz_to_float4(const float *aos3, float4 *out, int n, cudaStream_t st);
 int pack_ft6_to_float4(const float *aos6, float4 *force, float4 *torque, int n, cudaStream_t st);
