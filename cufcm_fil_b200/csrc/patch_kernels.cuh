@@ -368,9 +368,10 @@ __global__ void __launch_bounds__(256) gj_prep_kernel(PatchDev P, int K) {
         }
         return;
     }
-    // D^-1, 16-byte loads, stored transposed
+    // D^-1, 16-byte loads, stored transposed: a warp takes 32 rows, so that its stores do not share banks (with the
+    // lanes along the rows eight of them did: 14.2 us a round, 12.9 so)
     for (int e4 = threadIdx.x; e4 < kGjBlock * kGjBlock / 4; e4 += blockDim.x) {
-        const int r = e4 >> 4, c4 = 4 * (e4 & 15);
+        const int r = e4 & 63, c4 = 4 * (e4 >> 6);
         const float4 v = *reinterpret_cast<const float4 *>(dv + r * kGjBlock + c4);
         DvT[c4][r] = v.x;
         DvT[c4 + 1][r] = v.y;
@@ -386,9 +387,9 @@ __global__ void __launch_bounds__(256) gj_prep_kernel(PatchDev P, int K) {
             if (s_ < b && j0 + c4 < static_cast<int>(ld)) v = *reinterpret_cast<const float4 *>(A + (k0 + s_) * ld + j0 + c4);
             *reinterpret_cast<float4 *>(&Us[s_][c4]) = v;
         }
-    } else {  // j0 + 64 <= k0: U[s][c] = A[j0 + c][k0 + s], rows of A read contiguously, stored transposed
+    } else {  // j0 + 64 <= k0: U[s][c] = A[j0 + c][k0 + s], rows of A stored transposed
         for (int e4 = threadIdx.x; e4 < kGjTile * kGjBlock / 4; e4 += blockDim.x) {
-            const int c = e4 >> 4, s4 = 4 * (e4 & 15);
+            const int c = e4 & 63, s4 = 4 * (e4 >> 6);
             float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (k0 + s4 < static_cast<int>(ld)) v = *reinterpret_cast<const float4 *>(A + (j0 + c) * ld + k0 + s4);
             Us[s4][c] = v.x;
@@ -485,11 +486,11 @@ __device__ __forceinline__ GjTile gj_tile(const PatchDev &P, int K, int T, int i
 // Stage of the update: the tile's split operands as the prep pass left them
 // (A = the pivot-row copies of its row tile, B = the scaled pivot rows of its
 // column tile, each a TF32 high part and an FP32 remainder in the canonical
-// layout, 4 x 16 KB).  The old values are read from global memory by the
-// epilogue.  One stage per block and two blocks per SM: one block's copies
-// overlap the other's products and stores.
+// layout, 4 x 16 KB), and behind it the product tile on its way from tensor
+// memory to the rows of A.  Two blocks per SM.
 constexpr int kUpStage = 4 * tc::kOperandFloats;
-constexpr size_t kUpdateSmem = kUpStage * sizeof(float);
+constexpr int kUpLd = kGjTile + 4;  // 16-byte rows
+constexpr size_t kUpdateSmem = (kUpStage + kGjTile * kUpLd) * sizeof(float);
 
 // Issues the 16-byte copies of a tile's operands into `stage` (contiguous blocks: 8 + 8 chunks per thread;
 // the pivot rows need B only).
@@ -514,29 +515,32 @@ __device__ __forceinline__ void gj_issue_tile(const PatchDev &P, const GjTile &t
 // per SM) take tiles from a per-round counter.  The tile product C^T rbuf runs
 // on the tensor cores (tc_tf32.cuh: the operands as the prep pass split them,
 // three TF32 products accumulated in FP32 in tensor memory, issued by one
-// thread and committed to an mbarrier).  Read-back: warp w holds tile rows
-// 16 (w % 4) .. + 15 in lanes 0-15 and columns 32 (w / 4) .. + 31; each lane
-// pair (l, l + 16) then splits the 32 columns, so every thread writes 16
-// columns of one row.  The block that takes a patch's diagonal tile
-// (K + 1, K + 1) inverts it for the next round right after its update, while
-// the other blocks go on with the rest.  A wait for the products that gives up
-// (bounded) marks the tile's patch unusable -- it falls back to the
-// block-diagonal preconditioner -- and the block computes no further products.
-// Dynamic shared memory: kUpdateSmem.
+// thread and committed to an mbarrier).  A tile is a chain of waits (operands,
+// products, read-back), so the chain is overlapped: the next tile is drawn
+// while the operands land and its copies start as soon as the products have
+// read theirs, and the products go through shared memory so that the rows of A
+// are read and written 256 contiguous bytes at a time: a round of 16 patches of
+// 992 unknowns takes 33 us, 41 without, of which the chain diagonal tile ->
+// inversion is about 22.
+// The block that takes a patch's diagonal tile (K + 1, K + 1) inverts it for
+// the next round right after its update, while the other blocks go on with the
+// rest.  A wait for the products that gives up (bounded) marks the tile's patch
+// unusable -- it falls back to the block-diagonal preconditioner -- and the
+// block computes no further products.  Dynamic shared memory: kUpdateSmem.
 __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, int T, int *counter) {
     static_assert(kGjTile == 64 && kGjBlock == 64 && tc::kTileMN == 64 && tc::kTileK == 64, "64-wide tiles");
     static_assert(kUpStage >= kInvWs, "the inversion reuses the stage");
     extern __shared__ __align__(128) float usm[];
-    __shared__ int next_item;
+    __shared__ int next_item[2];  // drawn ahead; drawn after an inversion
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tbase;
     __shared__ int tc_ok, dead;
     chain_wait();
     const int total = P.np * (T * (T + 1) / 2);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) next_item = atomicAdd(counter, 1);
+    if (threadIdx.x == 0) next_item[0] = atomicAdd(counter, 1);
     __syncthreads();
-    int item = next_item;
+    const int item = next_item[0];
     if (item >= total) return;
     if (warp == 0) tc::tmem_alloc(&tbase, tc::kTmemCols);
     if (threadIdx.x == 0) {
@@ -550,113 +554,141 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, in
     const uint32_t tmem = tbase;
     uint32_t products = 0;  // completed phases of `bar`
     const float *Ab = usm, *Bb = usm + 2 * tc::kOperandFloats;
-    // this thread's output: tile row tr, columns tc0 .. tc0 + 15
-    const int tr = 16 * (warp & 3) + (lane & 15), tc0 = 32 * (warp >> 2) + 16 * (lane >> 4);
-    while (item < total) {
-        const GjTile cur = gj_tile(P, K, T, item);
-        if (cur.valid) {
-            gj_issue_tile(P, cur, usm);
-            cp_async_commit();
-            const int n = cur.n, ld = patch_ld(n);
-            const int i = cur.row0 + tr, j = cur.col0 + tc0;
-            float *Arow = P.A + P.moff[cur.p] + static_cast<size_t>(i) * ld + j;
-            // the old values, while the operands land (the pivot columns and rows are overwritten)
-            float res[16];
+    float *Ct = usm + kUpStage;
+    // this thread's output: rows tr + 16 k, columns tc4 .. + 3
+    const int tr = threadIdx.x >> 4, tc4 = 4 * (threadIdx.x & 15);
+    GjTile cur = gj_tile(P, K, T, item);
+    if (cur.valid) {
+        gj_issue_tile(P, cur, usm);
+        cp_async_commit();
+    }
+    for (;;) {
+        int drawn = 0;
+        if (threadIdx.x == 0 && !cur.diag) drawn = atomicAdd(counter, 1);
+        const int n = cur.n, ld = patch_ld(n);
+        const int i0 = cur.row0 + tr, j = cur.col0 + tc4;
+        float *Arow = P.A + P.moff[cur.p] + static_cast<size_t>(i0) * ld + j;
+        float res[4][4] = {};
+        // the old values, while the operands land (the pivot columns and rows are overwritten)
+        if (cur.valid && !cur.prow && !cur.pcol && j < ld) {
 #pragma unroll
-            for (int q = 0; q < 16; ++q) res[q] = 0.0f;
-            if (!cur.prow && !cur.pcol && i < n) {
-#pragma unroll
-                for (int q = 0; q < 16; q += 4) {
-                    if (j + q < ld) {
-                        const float4 o4 = *reinterpret_cast<const float4 *>(Arow + q);
-                        res[q] = o4.x;
-                        res[q + 1] = o4.y;
-                        res[q + 2] = o4.z;
-                        res[q + 3] = o4.w;
-                    }
+            for (int k = 0; k < 4; ++k)
+                if (i0 + 16 * k < n) {
+                    const float4 o4 = *reinterpret_cast<const float4 *>(Arow + static_cast<size_t>(16 * k) * ld);
+                    res[k][0] = o4.x;
+                    res[k][1] = o4.y;
+                    res[k][2] = o4.z;
+                    res[k][3] = o4.w;
                 }
-            }
-            cp_async_wait<0>();
-            tc::fence_proxy_async();  // the operands are visible to the tensor cores
-            tc::fence_before_sync();
-            __syncthreads();
-            tc::fence_after_sync();
-            bool have = true;
+        }
+        if (threadIdx.x == 0) next_item[0] = drawn;
+        cp_async_wait<0>();
+        tc::fence_proxy_async();  // the operands are visible to the tensor cores
+        tc::fence_before_sync();
+        __syncthreads();
+        tc::fence_after_sync();
+        int next = next_item[0];
+        const bool stopped = dead != 0;
+        if (cur.valid && !cur.prow && !stopped && threadIdx.x == 0) {
+            tc::issue_tile_products(tmem, Ab, Ab + tc::kOperandFloats, Bb, Bb + tc::kOperandFloats);
+            tc::commit(&bar);
+        }
+        GjTile nxt{};
+        if (next < total && !cur.diag) nxt = gj_tile(P, K, T, next);
+        if (cur.valid) {
             if (cur.prow) {  // the pivot rows: the scaled pivot rows themselves (row0 == k0), high + low parts
 #pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    const int e = tc::canon(tc0 + q, tr);
-                    res[q] = Bb[e] + Bb[tc::kOperandFloats + e];
-                }
-            } else if (dead) {
-                have = false;
-            } else {
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int e = tc::canon(tc4 + q, tr + 16 * k);
+                        res[k][q] = Bb[e] + Bb[tc::kOperandFloats + e];
+                    }
+            } else if (!stopped) {
                 if (threadIdx.x == 0) {
-                    tc::issue_tile_products(tmem, Ab, Ab + tc::kOperandFloats, Bb, Bb + tc::kOperandFloats);
-                    tc::commit(&bar);
                     bool ok = mbar_wait_bounded(&bar, products & 1u);
                     if (!ok) ok = mbar_wait_bounded(&bar, products & 1u);  // drain before going on
                     tc_ok = ok ? 1 : 0;
-                    if (!ok) {
-                        dead = 1;
-                        P.ok[cur.p] = 0;
-                    }
                 }
                 ++products;
-                __syncthreads();
-                tc::fence_after_sync();
-                have = tc_ok != 0;
-                if (have) {
-                    float v[32];
-                    tc::tmem_ld32(tc::tmem_addr(tmem, warp, 32 * (warp >> 2)), v);
-                    // lanes l and l + 16 share row l's 32 columns: l keeps 0..15, l + 16 takes 16..31
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        const float hi16 = __shfl_sync(0xffffffffu, v[16 + q], lane & 15);
-                        res[q] -= (lane < 16) ? v[q] : hi16;
-                    }
-                    tc::fence_before_sync();
-                }
-            }
-            if (have) {
-                // the patch's last round writes its final values: a non-finite one marks the inverse unusable
-                const bool last = (K + 1) * kGjBlock >= n;
-                bool bad = false;
-                if (i < n) {
-#pragma unroll
-                    for (int q = 0; q < 16; q += 4) {
-                        if (j + q + 3 < n) {
-                            *reinterpret_cast<float4 *>(Arow + q) = make_float4(res[q], res[q + 1], res[q + 2], res[q + 3]);
-                        } else {  // the row's last, partial chunk: nothing beyond column n - 1
-#pragma unroll
-                            for (int u = 0; u < 4; ++u)
-                                if (j + q + u < n) Arow[q + u] = res[q + u];
-                        }
-                    }
-                    if (last)
-#pragma unroll
-                        for (int q = 0; q < 16; ++q) bad |= (j + q < n) && !isfinite(res[q]);
-                }
-                if (bad) P.ok[cur.p] = 0;
-                if (last && cur.row0 < cur.col0 && i < n) {
-                    // final values: also the transposed tile of the lower block triangle (A^-1 is symmetric)
-                    float *At = P.A + P.moff[cur.p] + i;
-#pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        if (j + q < n) At[static_cast<size_t>(j + q) * ld] = res[q];
-                }
-            } else if (threadIdx.x == 0) {
-                P.ok[cur.p] = 0;
-            }
-            if (cur.diag) {  // the tile is final for round K + 1: invert it now (its writes are the block's own)
-                __syncthreads();
-                pivot_invert_patch(P, cur.p, K + 1, usm);
             }
         }
-        __syncthreads();  // every thread is done with the stage and with next_item
-        if (threadIdx.x == 0) next_item = atomicAdd(counter, 1);
+        __syncthreads();  // the stage has been read
+        tc::fence_after_sync();
+        const bool product = cur.valid && !cur.prow, have = !product || (!stopped && tc_ok != 0);
+        if (nxt.valid) gj_issue_tile(P, nxt, usm);
+        cp_async_commit();
+        if (product && have) {
+            // row m of the product lies in lane m % 16 of warps m / 16 and m / 16 + 4 (32 columns each)
+            float v[32];
+            tc::tmem_ld32(tc::tmem_addr(tmem, warp, 32 * (warp >> 2)), v);
+            if (lane < 16) {
+                float4 *o = reinterpret_cast<float4 *>(Ct + (16 * (warp & 3) + lane) * kUpLd + 32 * (warp >> 2));
+#pragma unroll
+                for (int q = 0; q < 8; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            }
+            tc::fence_before_sync();
+        }
         __syncthreads();
-        item = next_item;
+        if (product && !have && threadIdx.x == 0) {
+            P.ok[cur.p] = 0;
+            dead = 1;
+        }
+        if (cur.valid && have) {
+            if (product)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float4 v4 = *reinterpret_cast<const float4 *>(Ct + (tr + 16 * k) * kUpLd + tc4);
+                    res[k][0] -= v4.x;
+                    res[k][1] -= v4.y;
+                    res[k][2] -= v4.z;
+                    res[k][3] -= v4.w;
+                }
+            // the patch's last round writes its final values: a non-finite one marks the inverse unusable
+            const bool last = (K + 1) * kGjBlock >= n, mirror = last && cur.row0 < cur.col0;
+            bool bad = false;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (i0 + 16 * k >= n) continue;
+                float *o = Arow + static_cast<size_t>(16 * k) * ld;
+                if (j + 3 < n) {
+                    *reinterpret_cast<float4 *>(o) = make_float4(res[k][0], res[k][1], res[k][2], res[k][3]);
+                } else {  // the row's last, partial chunk: nothing beyond column n - 1
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (j + q < n) o[q] = res[k][q];
+                }
+                if (last)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) bad |= (j + q < n) && !isfinite(res[k][q]);
+            }
+            if (bad) P.ok[cur.p] = 0;
+            if (mirror) {  // final values: also the transposed tile of the lower block triangle (A^-1 is symmetric)
+                __syncthreads();
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    *reinterpret_cast<float4 *>(Ct + (tr + 16 * k) * kUpLd + tc4) =
+                        make_float4(res[k][0], res[k][1], res[k][2], res[k][3]);
+                __syncthreads();
+                for (int e = threadIdx.x; e < kGjTile * kGjTile; e += blockDim.x) {
+                    const int c = e >> 6, r = e & 63;
+                    if (cur.row0 + r < n && cur.col0 + c < n)
+                        P.A[P.moff[cur.p] + static_cast<size_t>(cur.col0 + c) * ld + cur.row0 + r] = Ct[r * kUpLd + c];
+                }
+            }
+        }
+        if (cur.diag) {  // the tile is final for round K + 1: invert it now (its writes are the block's own).  The
+            __syncthreads();  // inversion works in the stage, so the next tile is drawn and copied after it
+            if (cur.valid) pivot_invert_patch(P, cur.p, K + 1, usm);
+            if (threadIdx.x == 0) next_item[1] = atomicAdd(counter, 1);
+            __syncthreads();
+            next = next_item[1];
+            if (next < total) nxt = gj_tile(P, K, T, next);
+            if (nxt.valid) gj_issue_tile(P, nxt, usm);
+            cp_async_commit();
+        }
+        if (next >= total) break;
+        cur = nxt;
     }
     tc::fence_before_sync();
     __syncthreads();
