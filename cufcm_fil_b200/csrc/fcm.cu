@@ -11,12 +11,14 @@
 //   sort back                 sortback (CUFCM_SOLVER.cu:493-515)
 // Differences in the execution, not the mathematics: one warp per particle for
 // spread and gather with the particle's 1-D Gaussian tables in that warp's
-// shared memory (no block barriers); the three components' FFTs batched in one
-// cuFFT plan each way; the Stokes projector applied in place to the spectra;
+// shared memory (no block barriers); the transforms and the projector in five
+// passes over the used rows of the grid (fcm_fft.cuh, which says when; else cuFFT,
+// batched over the components, and stokes_kernel);
 // the near-field correction one-sided over all 27 neighbour cells (every pair
 // is visited from both ends, so no atomics and a deterministic result); and
 // results scattered straight back to input order instead of a second sort.
 #include "common.cuh"
+#include "fcm_fft.cuh"
 
 #include <cub/cub.cuh>
 #include <cufft.h>
@@ -45,6 +47,14 @@ struct cf_fcm {
     int *cell_start = nullptr, *cell_end = nullptr;
     void *sort_tmp = nullptr;
     size_t sort_tmp_bytes = 0;
+    // transforms: fcm_fft.cuh, or (grids it does not take) cuFFT plans
+    bool own_fft = false;
+    cufil::fftk::Grid g{};
+    void *fft_tables = nullptr;
+    unsigned char *flags = nullptr;  // counts, row and plane flags (cleared by one memset per apply)
+    size_t flag_bytes = 0;
+    int *row_list = nullptr;         // used rows, then used planes
+    int num_sms = CF_B200_SMS;
     cufftHandle plan_fwd = 0, plan_inv = 0;
     bool have_fwd = false, have_inv = false;
     // optional per-stage timing: events between stages of the last apply
@@ -81,6 +91,34 @@ __global__ void prep_kernel(Params p, const float *__restrict__ Y, float4 *x4, i
     cz = min(max(cz, 0), p.Mz - 1);
     keys[i] = cx + (cy + cz * p.My) * p.Mx;
     vals[i] = i;
+}
+
+// Marks the grid rows (y, z) that a particle's support touches (the points of build_tables), one bit a row, one thread
+// per particle and plane of its support: its run of rows is one or two words, set only where a bit is missing (most
+// rows are marked already, and a read is cheaper than an atomic).
+__global__ void mark_rows_kernel(Params p, const float *__restrict__ Y, unsigned *row_bits, int words) {
+    const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    const int i = static_cast<int>(t / p.ngd), kk = static_cast<int>(t - static_cast<long long>(i) * p.ngd);
+    if (i >= p.N) return;
+    auto place = [](float g, int n) { return min(max(static_cast<int>(g - n * floorf(g / n)), 0), n - 1); };
+    const float y = wrap_box(Y[3 * i + 1], p.Ly), z = wrap_box(Y[3 * i + 2], p.Lz);
+    unsigned *row = row_bits + static_cast<size_t>(place(rintf(z / p.dx) - p.ngd / 2 + kk, p.nz)) * words;
+    const float y0 = rintf(y / p.dx) - p.ngd / 2;
+    int word = -1;
+    unsigned bits = 0;
+    auto flush = [&] {
+        if (word >= 0 && (__ldcg(row + word) & bits) != bits) atomicOr(row + word, bits);
+    };
+    for (int jj = 0; jj < p.ngd; ++jj) {
+        const int r = place(y0 + jj, p.ny);
+        if ((r >> 5) != word) {
+            flush();
+            word = r >> 5;
+            bits = 0;
+        }
+        bits |= 1u << (r & 31);
+    }
+    flush();
 }
 
 __global__ void permute_kernel(Params p, const int *__restrict__ perm, const float4 *__restrict__ x4,
@@ -254,17 +292,41 @@ __device__ __forceinline__ void blob_pair(float r, float rsq, float sg, float sg
 }
 
 // Near-field correction + self correction, then the scatter to input order.
-// One thread per sorted particle, all 27 neighbour cells, pairs within Rc.
-__global__ void __launch_bounds__(128) correction_kernel(Params p, const float4 *__restrict__ xs,
-                                                         const float4 *__restrict__ fs, const int *__restrict__ keys,
-                                                         const int *__restrict__ cstart, const int *__restrict__ cend,
-                                                         const float4 *__restrict__ vgs, const int *__restrict__ perm,
-                                                         float *vout) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= p.N) return;
+// One warp per sorted particle: the lanes read the bounds of the 27 neighbour
+// cells, and the warp then walks the cells' particles as one list (candidate t
+// of the list: the cell whose run contains t), 32 at a time, evaluating the
+// pairs within Rc.  Bound by the latency of the chain cell bounds -> position ->
+// pair -> sum: one thread per particle ran it candidate by candidate (306 us for
+// 30,000 particles, a warp each 79).
+constexpr int kCorrWarps = 4;
+__global__ void __launch_bounds__(32 * kCorrWarps) correction_kernel(
+    Params p, const float4 *__restrict__ xs, const float4 *__restrict__ fs, const int *__restrict__ keys,
+    const int *__restrict__ cstart, const int *__restrict__ cend, const float4 *__restrict__ vgs,
+    const int *__restrict__ perm, float *vout) {
+    __shared__ int first[kCorrWarps][32], upto[kCorrWarps][32];  // per cell: first particle, candidates up to its end
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = blockIdx.x * kCorrWarps + w;
+    if (k >= p.N) return;  // uniform over the warp
     const float4 xi = xs[k];
     const int h = keys[k];
     const int cx = h % p.Mx, cy = (h / p.Mx) % p.My, cz = h / (p.Mx * p.My);
+    int start = 0, count = 0;
+    if (lane < 27) {
+        const int dz = lane / 9 - 1, dy = (lane / 3) % 3 - 1, dxc = lane % 3 - 1;
+        const int c = (cx + dxc + p.Mx) % p.Mx + ((cy + dy + p.My) % p.My + ((cz + dz + p.Mz) % p.Mz) * p.My) * p.Mx;
+        start = cstart[c];
+        count = max(0, cend[c] - start);
+    }
+    int sum = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += t;
+    }
+    first[w][lane] = start - (sum - count);  // candidate t of this cell is particle first + t
+    upto[w][lane] = sum;
+    const int total = __shfl_sync(0xffffffffu, sum, 31);
+    __syncwarp();
     const float pi = 3.14159265358979f;
     const float gam = 1.41421356237310f * p.Sigma, gamsq = gam * gam;
     const float gvf = 1.41421356237310f * p.sigma, gvfsq = gvf * gvf;
@@ -272,48 +334,50 @@ __global__ void __launch_bounds__(128) correction_kernel(Params p, const float4 
     const float gnorm_vf = 1.0f / powf(2.0f * pi * gvfsq, 1.5f);
     const float pd = p.pdmag, pdq = 0.25f * pd * pd;
     float vx = 0.0f, vy = 0.0f, vz = 0.0f;
-    for (int dz = -1; dz <= 1; ++dz) {
-        const int zc = (cz + dz + p.Mz) % p.Mz;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int yc = (cy + dy + p.My) % p.My;
-            for (int dxc = -1; dxc <= 1; ++dxc) {
-                const int xc = (cx + dxc + p.Mx) % p.Mx;
-                const int c = xc + (yc + zc * p.My) * p.Mx;
-                const int j1 = cend[c];
-                for (int j = cstart[c]; j < j1; ++j) {
-                    if (j == k) continue;
-                    const float4 xj = xs[j];
-                    float xij = xi.x - xj.x, yij = xi.y - xj.y, zij = xi.z - xj.z;
-                    // minimum image as the reference writes it (CUFCM_CORRECTION.cu:149-151)
-                    xij -= p.Lx * static_cast<float>(static_cast<int>(xij / (0.5f * p.Lx)));
-                    yij -= p.Ly * static_cast<float>(static_cast<int>(yij / (0.5f * p.Ly)));
-                    zij -= p.Lz * static_cast<float>(static_cast<int>(zij / (0.5f * p.Lz)));
-                    const float rsq = xij * xij + yij * yij + zij * zij;
-                    if (rsq >= p.Rcsq) continue;
-                    const float r = sqrtf(rsq);
-                    const float erfS = erff(0.5f * r / p.Sigma);
-                    const float gg = expf(-0.5f * rsq / gamsq) * gnorm;
-                    const float erfS_vf = erff(r / (1.41421356237310f * gvf));
-                    const float gg_vf = expf(-0.5f * rsq / gvfsq) * gnorm_vf;
-                    float A_vf, B_vf, A, B;
-                    blob_pair(r, rsq, gvf, gvfsq, gg_vf, erfS_vf, A_vf, B_vf);
-                    blob_pair(r, rsq, gam, gamsq, gg, erfS, A, B);
-                    const float r3 = r * rsq;
-                    const float QI = erfS / (4.0f * pi * r3) - (1.0f + gamsq / rsq) * gg;
-                    const float Qxx = -3.0f * erfS / (4.0f * pi * r3 * rsq) + (1.0f + 3.0f * gamsq / rsq) / rsq * gg;
-                    const float TI = (2.0f - rsq / gamsq) / gamsq * gg;
-                    const float Txx = gg / (gamsq * gamsq);
-                    const float t1 = A_vf - A - QI * pd - TI * pdq;
-                    const float t2 = B_vf - B - Qxx * pd - Txx * pdq;
-                    const float4 fj = fs[j];
-                    const float xf = xij * fj.x + yij * fj.y + zij * fj.z;
-                    vx += t1 * fj.x + t2 * xij * xf;
-                    vy += t1 * fj.y + t2 * yij * xf;
-                    vz += t1 * fj.z + t2 * zij * xf;
-                }
-            }
-        }
+    for (int t = lane; t < total; t += 32) {
+        int c = 0;  // the first cell with upto > t
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            if (upto[w][c + o - 1] <= t) c += o;
+        const int j = first[w][c] + t;
+        if (j == k) continue;
+        const float4 xj = xs[j];
+        float xij = xi.x - xj.x, yij = xi.y - xj.y, zij = xi.z - xj.z;
+        // minimum image as the reference writes it (CUFCM_CORRECTION.cu:149-151)
+        xij -= p.Lx * static_cast<float>(static_cast<int>(xij / (0.5f * p.Lx)));
+        yij -= p.Ly * static_cast<float>(static_cast<int>(yij / (0.5f * p.Ly)));
+        zij -= p.Lz * static_cast<float>(static_cast<int>(zij / (0.5f * p.Lz)));
+        const float rsq = xij * xij + yij * yij + zij * zij;
+        if (rsq >= p.Rcsq) continue;
+        const float r = sqrtf(rsq);
+        const float erfS = erff(0.5f * r / p.Sigma);
+        const float gg = expf(-0.5f * rsq / gamsq) * gnorm;
+        const float erfS_vf = erff(r / (1.41421356237310f * gvf));
+        const float gg_vf = expf(-0.5f * rsq / gvfsq) * gnorm_vf;
+        float A_vf, B_vf, A, B;
+        blob_pair(r, rsq, gvf, gvfsq, gg_vf, erfS_vf, A_vf, B_vf);
+        blob_pair(r, rsq, gam, gamsq, gg, erfS, A, B);
+        const float r3 = r * rsq;
+        const float QI = erfS / (4.0f * pi * r3) - (1.0f + gamsq / rsq) * gg;
+        const float Qxx = -3.0f * erfS / (4.0f * pi * r3 * rsq) + (1.0f + 3.0f * gamsq / rsq) / rsq * gg;
+        const float TI = (2.0f - rsq / gamsq) / gamsq * gg;
+        const float Txx = gg / (gamsq * gamsq);
+        const float t1 = A_vf - A - QI * pd - TI * pdq;
+        const float t2 = B_vf - B - Qxx * pd - Txx * pdq;
+        const float4 fj = fs[j];
+        const float xf = xij * fj.x + yij * fj.y + zij * fj.z;
+        vx += t1 * fj.x + t2 * xij * xf;
+        vy += t1 * fj.y + t2 * yij * xf;
+        vz += t1 * fj.z + t2 * zij * xf;
     }
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        vx += __shfl_down_sync(0xffffffffu, vx, o);
+        vy += __shfl_down_sync(0xffffffffu, vy, o);
+        vz += __shfl_down_sync(0xffffffffu, vz, o);
+    }
+    if (lane != 0) return;
     const float4 fi = fs[k];
     const float4 vg = vgs[k];
     const int o = perm[k];
@@ -366,6 +430,97 @@ int falloc(T **p, size_t n) {
     return CF_OK;
 }
 
+// The tables, flags and lists of fcm_fft.cuh for the handle's grid.
+int fft_setup(cf_fcm *h) {
+    fftk::Grid &g = h->g;
+    g.nx = h->nx;
+    g.ny = h->ny;
+    g.nz = h->nz;
+    g.mx = h->nx / 2;
+    g.ldx = (g.mx + 1 + fftk::kCols - 1) / fftk::kCols * fftk::kCols;
+    g.Lx = static_cast<float>(h->Lx);
+    g.Ly = static_cast<float>(h->Ly);
+    g.Lz = static_cast<float>(h->Lz);
+    // one table: per axis twiddles, frequencies, places; then the half-spectrum twiddles of x
+    const int len[3] = {g.mx, g.ny, g.nz};
+    fftk::Axis *axes[3] = {&g.x, &g.y, &g.z};
+    std::vector<char> host;
+    size_t off[3][3], off_wx;
+    auto put = [&](const void *src, size_t bytes) {
+        const size_t at = host.size();
+        host.resize(at + (bytes + 15) / 16 * 16);
+        std::memcpy(host.data() + at, src, bytes);
+        return at;
+    };
+    for (int a = 0; a < 3; ++a) {
+        const int n = len[a];
+        const std::vector<int> r = fftk::radices(n);
+        axes[a]->n = n;
+        axes[a]->ns = static_cast<int>(r.size());
+        std::copy(r.begin(), r.end(), axes[a]->radix);
+        const std::vector<float2> tw = fftk::twiddles(n, n);
+        const std::vector<int> freq = fftk::place_freq(n, r);
+        std::vector<int> place(n);
+        for (int q = 0; q < n; ++q) place[freq[q]] = q;
+        off[a][0] = put(tw.data(), n * sizeof(float2));
+        off[a][1] = put(freq.data(), n * sizeof(int));
+        off[a][2] = put(place.data(), n * sizeof(int));
+    }
+    const std::vector<float2> wx = fftk::twiddles(g.nx, g.mx + 1);
+    off_wx = put(wx.data(), wx.size() * sizeof(float2));
+    CF_CUDA(cudaMalloc(&h->fft_tables, host.size()));
+    CF_CUDA(cudaMemcpy(h->fft_tables, host.data(), host.size(), cudaMemcpyHostToDevice));
+    const char *t = static_cast<const char *>(h->fft_tables);
+    for (int a = 0; a < 3; ++a) {
+        axes[a]->tw = reinterpret_cast<const float2 *>(t + off[a][0]);
+        axes[a]->freq = reinterpret_cast<const int *>(t + off[a][1]);
+        axes[a]->place = reinterpret_cast<const int *>(t + off[a][2]);
+    }
+    g.wx = reinterpret_cast<const float2 *>(t + off_wx);
+    const size_t rows = static_cast<size_t>(g.ny) * g.nz, spec = 3 * static_cast<size_t>(g.ldx) * rows;
+    CF_CUDA(cudaMalloc(reinterpret_cast<void **>(&h->spec), spec * sizeof(float2)));
+    CF_CUDA(cudaMemset(h->spec, 0, spec * sizeof(float2)));  // the padding columns stay zero
+    g.words = (g.ny + 31) / 32;
+    const size_t bit_bytes = sizeof(unsigned) * g.words * static_cast<size_t>(g.nz);
+    h->flag_bytes = 16 + bit_bytes + g.nz;
+    CF_CUDA(cudaMalloc(reinterpret_cast<void **>(&h->flags), h->flag_bytes));
+    CF_CUDA(cudaMalloc(reinterpret_cast<void **>(&h->row_list), (rows + g.nz) * sizeof(int)));
+    g.counts = reinterpret_cast<int *>(h->flags);
+    g.row_bits = reinterpret_cast<unsigned *>(h->flags + 16);
+    g.plane_used = h->flags + 16 + bit_bytes;
+    g.rows = h->row_list;
+    g.planes = h->row_list + rows;
+    g.real = h->grid;
+    g.spec = reinterpret_cast<float2 *>(h->spec);
+    for (fftk::Kernel k : {fftk::pick_x(g.mx, false), fftk::pick_x(g.mx, true), fftk::pick_y(g.ny, false),
+                           fftk::pick_y(g.ny, true), fftk::pick_z(g.nz)})
+        CF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
+    return CF_OK;
+}
+
+int fft_launch(fftk::Kernel k, dim3 grid, int threads, size_t smem, cudaStream_t st, const fftk::Grid &g) {
+    k<<<grid, threads, smem, st>>>(g);
+    CF_CHECK_LAUNCH("fcm transform");
+    return CF_OK;
+}
+
+// Forward transform, projector and inverse transform of the used rows.  Blocks take rows and planes in turn (their
+// number is known on the device only): enough blocks for the whole grid's rows at small sizes, a few waves at large.
+int fft_solve(cf_fcm *h, cudaStream_t st) {
+    const fftk::Grid &g = h->g;
+    const int cols = g.ldx / fftk::kCols, rows = g.ny * g.nz;
+    const int xb = std::min((rows + fftk::kRowWarps - 1) / fftk::kRowWarps, 8 * h->num_sms);
+    const int yb = std::min(g.nz, std::max(1, 8 * h->num_sms / cols));
+    const int yt = std::min(256, std::max(64, (g.ny / g.y.radix[0] * 4 + 31) / 32 * 32));
+    const int zt = std::min(64 * fftk::kZPairs, std::max(64, (g.nz / g.z.radix[0] * fftk::kZPairs + 31) / 32 * 32));
+    CF_TRY(fft_launch(fftk::pick_x(g.mx, false), dim3(xb, 3), 256, fftk::x_smem(g), st, g));
+    CF_TRY(fft_launch(fftk::pick_y(g.ny, false), dim3(cols, yb, 3), yt, fftk::y_smem(g), st, g));
+    CF_TRY(fft_launch(fftk::pick_z(g.nz), dim3(g.ldx / (2 * fftk::kZPairs), g.ny), zt, fftk::z_smem(g), st, g));
+    CF_TRY(fft_launch(fftk::pick_y(g.ny, true), dim3(cols, yb, 3), yt, fftk::y_smem(g), st, g));
+    CF_TRY(fft_launch(fftk::pick_x(g.mx, true), dim3(xb, 3), 256, fftk::x_smem(g), st, g));
+    return CF_OK;
+}
+
 // The pipeline on device buffers: Y, F in the caller's [3N] layout, V out [3N].
 int fcm_run(cf_fcm *h, const float *dY, const float *dF, float *dV, cudaStream_t st) {
     const fcmk::Params p = params_of(h);
@@ -376,7 +531,22 @@ int fcm_run(cf_fcm *h, const float *dY, const float *dF, float *dV, cudaStream_t
         return CF_OK;
     };
     CF_TRY(mark(0));
-    CF_CUDA(cudaMemsetAsync(h->grid, 0, sizeof(float) * 3 * h->grid_size, st));
+    const int sms = h->num_sms;
+    if (h->own_fft) {
+        CF_CUDA(cudaMemsetAsync(h->flags, 0, h->flag_bytes, st));
+        const long long marks = static_cast<long long>(N) * h->ngd;
+        fcmk::mark_rows_kernel<<<static_cast<unsigned>((marks + 255) / 256), 256, 0, st>>>(
+            p, dY, const_cast<unsigned *>(h->g.row_bits), h->g.words);
+        CF_CHECK_LAUNCH("fcm mark_rows_kernel");
+        fftk::list_rows_kernel<<<h->nz, 256, 0, st>>>(h->g.row_bits, h->g.words, h->ny,
+                                                      const_cast<unsigned char *>(h->g.plane_used), h->row_list,
+                                                      const_cast<int *>(h->g.planes), const_cast<int *>(h->g.counts));
+        CF_CHECK_LAUNCH("fcm list_rows_kernel");
+        fftk::clear_rows_kernel<<<sms * 8, 256, 0, st>>>(h->g);
+        CF_CHECK_LAUNCH("fcm clear_rows_kernel");
+    } else {
+        CF_CUDA(cudaMemsetAsync(h->grid, 0, sizeof(float) * 3 * h->grid_size, st));
+    }
     CF_TRY(mark(1));
     fcmk::prep_kernel<<<nb, tb, 0, st>>>(p, dY, h->x4, h->keys, h->vals);
     CF_CHECK_LAUNCH("fcm prep_kernel");
@@ -393,16 +563,20 @@ int fcm_run(cf_fcm *h, const float *dY, const float *dF, float *dV, cudaStream_t
     fcmk::spread_kernel<<<wb, 128, 0, st>>>(p, h->xs, h->fs, h->grid);
     CF_CHECK_LAUNCH("fcm spread_kernel");
     CF_TRY(mark(3));
-    CF_TRY(cufft_status(cufftExecR2C(h->plan_fwd, h->grid, h->spec), "cufftExecR2C"));
-    const size_t sb = (h->fft_size + 255) / 256;
-    fcmk::stokes_kernel<<<static_cast<unsigned>(sb), 256, 0, st>>>(p, h->spec);
-    CF_CHECK_LAUNCH("fcm stokes_kernel");
-    CF_TRY(cufft_status(cufftExecC2R(h->plan_inv, h->spec, h->grid), "cufftExecC2R"));
+    if (h->own_fft) {
+        CF_TRY(fft_solve(h, st));
+    } else {
+        CF_TRY(cufft_status(cufftExecR2C(h->plan_fwd, h->grid, h->spec), "cufftExecR2C"));
+        const size_t sb = (h->fft_size + 255) / 256;
+        fcmk::stokes_kernel<<<static_cast<unsigned>(sb), 256, 0, st>>>(p, h->spec);
+        CF_CHECK_LAUNCH("fcm stokes_kernel");
+        CF_TRY(cufft_status(cufftExecC2R(h->plan_inv, h->spec, h->grid), "cufftExecC2R"));
+    }
     CF_TRY(mark(4));
     fcmk::gather_kernel<<<wb, 128, 0, st>>>(p, h->xs, h->grid, h->vgs);
     CF_CHECK_LAUNCH("fcm gather_kernel");
     CF_TRY(mark(5));
-    fcmk::correction_kernel<<<nb, tb, 0, st>>>(p, h->xs, h->fs, h->keys_sorted, h->cell_start, h->cell_end, h->vgs,
+    fcmk::correction_kernel<<<(N + fcmk::kCorrWarps - 1) / fcmk::kCorrWarps, 32 * fcmk::kCorrWarps, 0, st>>>(p, h->xs, h->fs, h->keys_sorted, h->cell_start, h->cell_end, h->vgs,
                                                h->perm, dV);
     CF_CHECK_LAUNCH("fcm correction_kernel");
     CF_TRY(mark(6));
@@ -461,10 +635,13 @@ extern "C" int cf_fcm_create(const cf_fcm_config *cfg, cf_fcm **out) {
                               __FILE__, __LINE__)))
             break;
         const size_t N = h->N;
-        if ((rc = falloc(&h->grid, 3 * h->grid_size)) || (rc = falloc(&h->spec, 3 * h->fft_size)) ||
-            (rc = falloc(&h->x4, N)) || (rc = falloc(&h->xs, N)) || (rc = falloc(&h->fs, N)) ||
-            (rc = falloc(&h->ys, 3 * N)) || (rc = falloc(&h->fsrc, 3 * N)) || (rc = falloc(&h->vout, 3 * N)) ||
-            (rc = falloc(&h->vgs, N)) || (rc = falloc(&h->keys, N)) || (rc = falloc(&h->keys_sorted, N)) ||
+        h->own_fft = fftk::supported(h->nx, h->ny, h->nz);
+        if ((rc = cuda_status(cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, cfg->device),
+                              "cudaDeviceGetAttribute", __FILE__, __LINE__)))
+            break;
+        if ((rc = falloc(&h->grid, 3 * h->grid_size)) || (rc = falloc(&h->x4, N)) || (rc = falloc(&h->xs, N)) || (rc = falloc(&h->fs, N)) ||
+            (rc = falloc(&h->ys, 3 * N)) || (rc = falloc(&h->fsrc, 3 * N)) || (rc = falloc(&h->vout, 3 * N)) || (rc = falloc(&h->vgs, N)) || (rc = falloc(&h->keys, N)) ||
+            (rc = falloc(&h->keys_sorted, N)) ||
             (rc = falloc(&h->vals, N)) || (rc = falloc(&h->perm, N)) || (rc = falloc(&h->cell_start, h->ncell)) ||
             (rc = falloc(&h->cell_end, h->ncell)))
             break;
@@ -476,6 +653,13 @@ extern "C" int cf_fcm_create(const cf_fcm_config *cfg, cf_fcm **out) {
         h->sort_tmp_bytes = tmp;
         if ((rc = cuda_status(cudaMalloc(&h->sort_tmp, std::max<size_t>(tmp, 1)), "cudaMalloc", __FILE__, __LINE__)))
             break;
+        if (h->own_fft) {
+            if ((rc = fft_setup(h))) break;
+            // the tables and zeros were written on the legacy stream
+            rc = cuda_status(cudaDeviceSynchronize(), "cudaDeviceSynchronize", __FILE__, __LINE__);
+            break;
+        }
+        if ((rc = falloc(&h->spec, 3 * h->fft_size))) break;
         // batched 3-D transforms of the three components, x fastest (cufftPlan3d(nz, ny, nx) in the reference)
         int n3[3] = {h->nz, h->ny, h->nx};
         if ((rc = cufft_status(cufftPlanMany(&h->plan_fwd, 3, n3, nullptr, 1, static_cast<int>(h->grid_size), nullptr,
@@ -510,9 +694,9 @@ extern "C" int cf_fcm_destroy(cf_fcm *h) {
         if (e) cudaEventDestroy(e);
     if (h->have_fwd) cufftDestroy(h->plan_fwd);
     if (h->have_inv) cufftDestroy(h->plan_inv);
-    for (void *p : {(void *)h->grid, (void *)h->spec, (void *)h->x4, (void *)h->xs, (void *)h->fs, (void *)h->ys,
-                    (void *)h->fsrc, (void *)h->vout, (void *)h->vgs, (void *)h->keys, (void *)h->keys_sorted,
-                    (void *)h->vals, (void *)h->perm, (void *)h->cell_start, (void *)h->cell_end, h->sort_tmp})
+    for (void *p : {(void *)h->grid, (void *)h->spec, (void *)h->x4, (void *)h->xs, (void *)h->fs, (void *)h->ys, (void *)h->fsrc, (void *)h->vout, (void *)h->vgs, (void *)h->keys, (void *)h->keys_sorted,
+                    (void *)h->vals, (void *)h->perm, (void *)h->cell_start, (void *)h->cell_end, h->sort_tmp,
+                    h->fft_tables, (void *)h->flags, (void *)h->row_list})
         if (p) cudaFree(p);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
