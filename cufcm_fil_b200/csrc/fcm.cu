@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <new>
 #include <vector>
 
@@ -39,9 +40,7 @@ struct cf_fcm {
     float *grid = nullptr;         // 3 real grids, component-major
     cufftComplex *spec = nullptr;  // 3 spectra
     float4 *x4 = nullptr, *xs = nullptr, *fs = nullptr;
-    float *ys = nullptr;           // caller-layout staging [3N] (host path)
-    float *fsrc = nullptr;         // [3N]
-    float *vout = nullptr;         // [3N]
+    cufil::HostStage stage;        // host path: positions, forces, velocities, [3N] each
     float4 *vgs = nullptr;         // gathered velocities, sorted order
     int *keys = nullptr, *keys_sorted = nullptr, *vals = nullptr, *perm = nullptr;
     int *cell_start = nullptr, *cell_end = nullptr;
@@ -583,6 +582,19 @@ int fcm_run(cf_fcm *h, const float *dY, const float *dF, float *dV, cudaStream_t
     return CF_OK;
 }
 
+// The pipeline on host positions and forces [3N].
+int fcm_host(cf_fcm *h, const float *Y, const float *F, float *V) {
+    const size_t b = sizeof(float) * 3 * static_cast<size_t>(h->N);
+    CF_CUDA(h->stage.put(0, Y, b, h->stream));
+    CF_CUDA(h->stage.put(b, F, b, h->stream));
+    CF_CUDA(h->stage.up(2 * b, h->stream));
+    CF_TRY(fcm_run(h, h->stage.at<float>(0), h->stage.at<float>(b), h->stage.at<float>(2 * b), h->stream));
+    CF_CUDA(h->stage.down(2 * b, b, h->stream));
+    CF_CUDA(cudaStreamSynchronize(h->stream));
+    CF_CUDA(h->stage.take(V, 2 * b, b, h->stream));
+    return CF_OK;
+}
+
 }  // namespace
 
 extern "C" int cf_fcm_create(const cf_fcm_config *cfg, cf_fcm **out) {
@@ -640,7 +652,7 @@ extern "C" int cf_fcm_create(const cf_fcm_config *cfg, cf_fcm **out) {
                               "cudaDeviceGetAttribute", __FILE__, __LINE__)))
             break;
         if ((rc = falloc(&h->grid, 3 * h->grid_size)) || (rc = falloc(&h->x4, N)) || (rc = falloc(&h->xs, N)) || (rc = falloc(&h->fs, N)) ||
-            (rc = falloc(&h->ys, 3 * N)) || (rc = falloc(&h->fsrc, 3 * N)) || (rc = falloc(&h->vout, 3 * N)) || (rc = falloc(&h->vgs, N)) || (rc = falloc(&h->keys, N)) ||
+            (rc = h->stage.alloc(9 * N * sizeof(float))) || (rc = falloc(&h->vgs, N)) || (rc = falloc(&h->keys, N)) ||
             (rc = falloc(&h->keys_sorted, N)) ||
             (rc = falloc(&h->vals, N)) || (rc = falloc(&h->perm, N)) || (rc = falloc(&h->cell_start, h->ncell)) ||
             (rc = falloc(&h->cell_end, h->ncell)))
@@ -694,10 +706,11 @@ extern "C" int cf_fcm_destroy(cf_fcm *h) {
         if (e) cudaEventDestroy(e);
     if (h->have_fwd) cufftDestroy(h->plan_fwd);
     if (h->have_inv) cufftDestroy(h->plan_inv);
-    for (void *p : {(void *)h->grid, (void *)h->spec, (void *)h->x4, (void *)h->xs, (void *)h->fs, (void *)h->ys, (void *)h->fsrc, (void *)h->vout, (void *)h->vgs, (void *)h->keys, (void *)h->keys_sorted,
+    for (void *p : {(void *)h->grid, (void *)h->spec, (void *)h->x4, (void *)h->xs, (void *)h->fs, (void *)h->vgs, (void *)h->keys, (void *)h->keys_sorted,
                     (void *)h->vals, (void *)h->perm, (void *)h->cell_start, (void *)h->cell_end, h->sort_tmp,
                     h->fft_tables, (void *)h->flags, (void *)h->row_list})
         if (p) cudaFree(p);
+    h->stage.release();
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return CF_OK;
@@ -728,13 +741,7 @@ extern "C" int cf_fcm_apply(cf_fcm *h, const float *Y, const float *F, float *V)
     clear_error();
     CF_REQUIRE(h && Y && F && V, "cf_fcm_apply: null argument");
     CF_CUDA(cudaSetDevice(h->cfg.device));
-    const size_t b = sizeof(float) * 3 * h->N;
-    CF_CUDA(cudaMemcpyAsync(h->ys, Y, b, cudaMemcpyHostToDevice, h->stream));
-    CF_CUDA(cudaMemcpyAsync(h->fsrc, F, b, cudaMemcpyHostToDevice, h->stream));
-    CF_TRY(fcm_run(h, h->ys, h->fsrc, h->vout, h->stream));
-    CF_CUDA(cudaMemcpyAsync(V, h->vout, b, cudaMemcpyDeviceToHost, h->stream));
-    CF_CUDA(cudaStreamSynchronize(h->stream));
-    return CF_OK;
+    return fcm_host(h, Y, F, V);
 }
 
 extern "C" int cf_fcm_apply_segments_blobs(cf_fcm *h, int n_seg, const float *x_segs, const float *x_blobs,

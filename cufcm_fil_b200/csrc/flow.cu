@@ -18,6 +18,7 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cstring>
 #include <new>
 
 struct cf_flow {
@@ -27,8 +28,7 @@ struct cf_flow {
     float4 *sx = nullptr, *sf = nullptr, *st = nullptr, *sb = nullptr;  // sources: centre, force, torque, body
     float4 *partial = nullptr;
     size_t partial_cap = 0;
-    float *hx_flow = nullptr, *hx_segs = nullptr, *hf_segs = nullptr, *hx_blobs = nullptr, *hf_blobs = nullptr,
-          *hx_bodies = nullptr, *hv_flow = nullptr;  // device staging of the host entry point
+    cufil::HostStage stage;  // host entry point: the call's arrays back to back, velocities last
     int max_bodies = 0;
 };
 
@@ -333,10 +333,9 @@ using namespace cufil;
 extern "C" int cf_flow_destroy(cf_flow *h) {
     if (!h) return CF_OK;
     cudaSetDevice(h->cfg.device);
-    for (void *p : {(void *)h->sx, (void *)h->sf, (void *)h->st, (void *)h->sb, (void *)h->partial,
-                    (void *)h->hx_flow, (void *)h->hv_flow, (void *)h->hx_segs, (void *)h->hf_segs,
-                    (void *)h->hx_blobs, (void *)h->hf_blobs, (void *)h->hx_bodies})
+    for (void *p : {(void *)h->sx, (void *)h->sf, (void *)h->st, (void *)h->sb, (void *)h->partial})
         if (p) cudaFree(p);
+    h->stage.release();
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return CF_OK;
@@ -369,13 +368,10 @@ extern "C" int cf_flow_create(const cf_flow_config *cfg, cf_flow **out) {
                          2 * static_cast<size_t>(cfg->max_flow);
         if ((rc = falloc(&h->sx, nsrc)) || (rc = falloc(&h->sf, nsrc)) || (rc = falloc(&h->st, nsrc)) ||
             (rc = falloc(&h->sb, nsrc)) || (rc = falloc(&h->partial, h->partial_cap)) ||
-            (rc = falloc(&h->hx_flow, 3 * static_cast<size_t>(cfg->max_flow))) ||
-            (rc = falloc(&h->hv_flow, 3 * static_cast<size_t>(cfg->max_flow))) ||
-            (rc = falloc(&h->hx_segs, 3 * static_cast<size_t>(cfg->max_seg))) ||
-            (rc = falloc(&h->hf_segs, 6 * static_cast<size_t>(cfg->max_seg))) ||
-            (rc = falloc(&h->hx_blobs, 3 * static_cast<size_t>(cfg->max_blob))) ||
-            (rc = falloc(&h->hf_blobs, 3 * static_cast<size_t>(cfg->max_blob))) ||
-            (rc = falloc(&h->hx_bodies, 3 * static_cast<size_t>(cfg->max_bodies))))
+            (rc = h->stage.alloc(sizeof(float) * (6 * static_cast<size_t>(cfg->max_flow) +
+                                                  9 * static_cast<size_t>(cfg->max_seg) +
+                                                  6 * static_cast<size_t>(cfg->max_blob) +
+                                                  3 * static_cast<size_t>(cfg->max_bodies)))))
             break;
     } while (0);
     if (rc != CF_OK) {
@@ -414,20 +410,24 @@ extern "C" int cf_flow_velocities(cf_flow *h, const float *x_flow, int n_flow, c
     CF_CUDA(cudaSetDevice(h->cfg.device));
     cudaStream_t st = h->stream;
     const int bodies = std::max(n_seg ? n_seg / n_seg_per_body : 0, n_blob ? n_blob / n_blob_per_body : 0);
-    if (n_flow) CF_CUDA(cudaMemcpyAsync(h->hx_flow, x_flow, sizeof(float) * 3 * n_flow, cudaMemcpyHostToDevice, st));
-    if (n_seg) {
-        CF_CUDA(cudaMemcpyAsync(h->hx_segs, x_segs, sizeof(float) * 3 * n_seg, cudaMemcpyHostToDevice, st));
-        CF_CUDA(cudaMemcpyAsync(h->hf_segs, f_segs, sizeof(float) * 6 * n_seg, cudaMemcpyHostToDevice, st));
-    }
-    if (n_blob) {
-        CF_CUDA(cudaMemcpyAsync(h->hx_blobs, x_blobs, sizeof(float) * 3 * n_blob, cudaMemcpyHostToDevice, st));
-        CF_CUDA(cudaMemcpyAsync(h->hf_blobs, f_blobs, sizeof(float) * 3 * n_blob, cudaMemcpyHostToDevice, st));
-    }
-    if (x_bodies && bodies)
-        CF_CUDA(cudaMemcpyAsync(h->hx_bodies, x_bodies, sizeof(float) * 3 * bodies, cudaMemcpyHostToDevice, st));
-    CF_TRY(flow_run(h, h->hx_flow, n_flow, h->hx_segs, h->hf_segs, n_seg, n_seg_per_body, h->hx_blobs, h->hf_blobs,
-                    n_blob, n_blob_per_body, x_bodies ? h->hx_bodies : nullptr, h->hv_flow, st));
-    if (n_flow) CF_CUDA(cudaMemcpyAsync(v_flow, h->hv_flow, sizeof(float) * 3 * n_flow, cudaMemcpyDeviceToHost, st));
+    const size_t nf3 = 3 * static_cast<size_t>(n_flow), ns3 = 3 * static_cast<size_t>(n_seg),
+                 nb3 = 3 * static_cast<size_t>(n_blob), nd3 = x_bodies ? 3 * static_cast<size_t>(bodies) : 0;
+    size_t at = 0;  // bytes
+    cudaError_t e = cudaSuccess;
+    auto put = [&](const float *src, size_t count) {
+        if (e == cudaSuccess) e = h->stage.put(at, src, count * sizeof(float), st);
+        float *d = h->stage.at<float>(at);
+        at += count * sizeof(float);
+        return d;
+    };
+    const float *dxf = put(x_flow, nf3), *dxs = put(x_segs, ns3), *dfs = put(f_segs, 2 * ns3), *dxb = put(x_blobs, nb3),
+                *dfb = put(f_blobs, nb3), *dxd = put(x_bodies, nd3);
+    CF_CUDA(e);
+    CF_CUDA(h->stage.up(at, st));
+    CF_TRY(flow_run(h, dxf, n_flow, dxs, dfs, n_seg, n_seg_per_body, dxb, dfb, n_blob, n_blob_per_body,
+                    x_bodies ? dxd : nullptr, h->stage.at<float>(at), st));
+    CF_CUDA(h->stage.down(at, nf3 * sizeof(float), st));
     CF_CUDA(cudaStreamSynchronize(st));
+    CF_CUDA(h->stage.take(v_flow, at, nf3 * sizeof(float), st));
     return CF_OK;
 }

@@ -8,15 +8,21 @@
 #include "rpy_kernels.cuh"
 
 #include <algorithm>
+#include <cstring>
 #include <functional>
 #include <new>
 #include <vector>
+
+using cufil::HostStage;
 
 struct cf_mobility {
     cf_mobility_config cfg{};
     int num_sms = CF_B200_SMS;
     cudaStream_t stream = nullptr;
-    // Device copies of the reference host layouts.
+    // Device copies of the reference host layouts: consecutive parts of one staging buffer, in the order x_segs,
+    // f_segs, x_blobs, f_blobs | v_segs, v_blobs, err.
+    HostStage stage;
+    size_t in_bytes = 0, out_bytes = 0;
     float *x_segs = nullptr, *f_segs = nullptr, *v_segs = nullptr;
     float *x_blobs = nullptr, *f_blobs = nullptr, *v_blobs = nullptr;
     // float4 particle records used by the kernels.
@@ -226,11 +232,18 @@ extern "C" int cf_mobility_create(const cf_mobility_config *cfg, cf_mobility **o
                               __FILE__, __LINE__)) != CF_OK)
             break;
         const size_t ns = cfg->n_seg, nb = cfg->n_blob;
-        if ((rc = dalloc(&h->x_segs, 3 * ns)) || (rc = dalloc(&h->f_segs, 6 * ns)) || (rc = dalloc(&h->v_segs, 6 * ns)) ||
-            (rc = dalloc(&h->x_blobs, 3 * nb)) || (rc = dalloc(&h->f_blobs, 3 * nb)) ||
-            (rc = dalloc(&h->v_blobs, 3 * nb)) || (rc = dalloc(&h->xs4, ns + nb)) || (rc = dalloc(&h->fs4, ns + nb)) ||
-            (rc = dalloc(&h->ts4, ns)) || (rc = dalloc(&h->err, 1)))
+        h->in_bytes = sizeof(float) * (9 * ns + 6 * nb);
+        h->out_bytes = sizeof(float) * (6 * ns + 3 * nb) + sizeof(int);
+        if ((rc = h->stage.alloc(h->in_bytes + h->out_bytes)) || (rc = dalloc(&h->xs4, ns + nb)) ||
+            (rc = dalloc(&h->fs4, ns + nb)) || (rc = dalloc(&h->ts4, ns)))
             break;
+        h->x_segs = h->stage.at<float>(0);
+        h->f_segs = h->x_segs + 3 * ns;
+        h->x_blobs = h->f_segs + 6 * ns;
+        h->f_blobs = h->x_blobs + 3 * nb;
+        h->v_segs = h->f_blobs + 3 * nb;
+        h->v_blobs = h->v_segs + 6 * ns;
+        h->err = reinterpret_cast<int *>(h->v_blobs + 3 * nb);
         h->xb4 = h->xs4 + ns;
         h->fb4 = h->fs4 + ns;
         // Partials buffer: the largest of the four block products' plans.
@@ -267,10 +280,9 @@ extern "C" int cf_mobility_destroy(cf_mobility *h) {
     if (!h) return CF_OK;
     cudaSetDevice(h->cfg.device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    for (void *p : {(void *)h->x_segs, (void *)h->f_segs, (void *)h->v_segs, (void *)h->x_blobs, (void *)h->f_blobs,
-                    (void *)h->v_blobs, (void *)h->xs4, (void *)h->fs4, (void *)h->ts4, (void *)h->scratch,
-                    (void *)h->err})
+    for (void *p : {(void *)h->xs4, (void *)h->fs4, (void *)h->ts4, (void *)h->scratch})
         if (p) cudaFree(p);
+    h->stage.release();
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return CF_OK;
@@ -381,14 +393,25 @@ extern "C" int cf_apply_mobility(cf_mobility *h, const float *x_segs, const floa
                                  const float *f_blobs, float *v_segs, float *v_blobs) {
     clear_error();
     CF_REQUIRE(h, "cf_apply_mobility: null handle");
-    CF_TRY(cf_copy_segment_positions_to_device(h, x_segs));
-    CF_TRY(cf_copy_blob_positions_to_device(h, x_blobs));
-    CF_TRY(cf_copy_segment_forces_to_device(h, f_segs));
-    CF_TRY(cf_copy_blob_forces_to_device(h, f_blobs));
-    CF_TRY(cf_evaluate_full_mobility(h));
-    CF_TRY(cf_copy_segment_velocities_to_host(h, v_segs));
-    CF_TRY(cf_copy_blob_velocities_to_host(h, v_blobs));
-    return cf_wait_for_device(h);
+    const size_t ns = h->cfg.n_seg, nb = h->cfg.n_blob;
+    CF_REQUIRE(!ns || (x_segs && f_segs && v_segs), "cf_apply_mobility: null segment argument");
+    CF_REQUIRE(!nb || (x_blobs && f_blobs && v_blobs), "cf_apply_mobility: null blob argument");
+    CF_CUDA(cudaSetDevice(h->cfg.device));
+    const HostStage &sg = h->stage;
+    const cudaStream_t st = h->stream;
+    CF_CUDA(sg.put(0, x_segs, 12 * ns, st));
+    CF_CUDA(sg.put(12 * ns, f_segs, 24 * ns, st));
+    CF_CUDA(sg.put(36 * ns, x_blobs, 12 * nb, st));
+    CF_CUDA(sg.put(36 * ns + 12 * nb, f_blobs, 12 * nb, st));
+    CF_CUDA(sg.up(h->in_bytes, st));
+    CF_TRY(apply_full(h, h->x_segs, h->x_blobs, h->f_segs, h->f_blobs, h->v_segs, h->v_blobs, st));
+    CF_CUDA(sg.down(h->in_bytes, h->out_bytes, st));
+    CF_CUDA(cudaStreamSynchronize(st));
+    CF_CUDA(sg.take(v_segs, h->in_bytes, 24 * ns, st));
+    CF_CUDA(sg.take(v_blobs, h->in_bytes + 24 * ns, 12 * nb, st));
+    int flags = 0;
+    CF_CUDA(sg.take(&flags, h->in_bytes + 24 * ns + 12 * nb, sizeof(int), st));
+    return flags ? check_device_flags(h) : CF_OK;
 }
 
 extern "C" int cf_apply_mobility_device(cf_mobility *h, const float *d_x_segs, const float *d_x_blobs,
