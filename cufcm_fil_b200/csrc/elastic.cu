@@ -752,79 +752,138 @@ __global__ void el_jacobian_kernel(ElDev d, int nt) {
 // In-place Gauss-Jordan inversion with partial pivoting of each filament's 6S x 6S block (FP64, held in
 // shared memory); a zero pivot column sets the non-finite flag.  Eight pivots (a panel of eight
 // columns) at a time, without moving rows:
-//   (a) every row's eight entries of the panel sit in one thread's registers.  Per pivot, each warp
-//       finds its largest unused entry (two 32-bit warp maxima over the bits of |a|) and publishes that
-//       row's entries; after one barrier every thread picks the largest of the warps' rows and updates
-//       its own row, which leaves the panel's columns of the partly inverted matrix;
-//   (b) the eight pivot rows are copied out, and every other column takes the rank-8 update
-//       A[r][c] = (r a pivot row ? 0 : A[r][c]) + sum_s P[r][s] A_old[p_s][c], P the panel's columns:
-//       a warp holds its share of the eight rows in registers and reads and writes each row once.
-// After the last panel, row p_k of A holds solution row k and column k belongs to equation p_k, so
-// inverse[k][p_j] = A[p_k][j].
+//   (a) every row's eight entries of the panel sit in one thread's registers, updated by the last panel;
+//   (b) per pivot, each warp finds its largest unused entry (a warp maximum over the high words of |a|)
+//       and publishes that row's entries; after one barrier every thread picks the largest of the warps'
+//       rows and updates its own row, which leaves the panel's columns P of the partly inverted matrix;
+//   (c) the eight pivot rows are copied out, and every other column takes the rank-8 update
+//       A[r][c] = (r a pivot row ? 0 : A[r][c]) + sum_s P[r][s] A_old[p_s][c].
+// The first warps (one row a thread) do (a) and (b) of a panel while the others do (c) of the panel
+// before on the remaining columns.  After the last panel, row p_k of A holds solution row k and column k
+// belongs to equation p_k, so inverse[k][p_j] = A[p_k][j].
 //
-// Bound by shared memory: the matrix moves twice per panel, 2 x 115 KB x 15 at S = 20, where one pivot
-// at a time moves it 120 times: 256 blocks of 120 x 120 (two waves) take 314 us, one at a time 800.
+// Bound by the chain of pivots (120 of about 450 cycles at S = 20: a division, a warp maximum, a barrier,
+// the published row).  256 blocks of 120 x 120 (two waves) take 200 us; 314 with (b) and (c) in turn and
+// one row at a time, 800 one pivot at a time.
 constexpr int kInvThreads = 512, kInvPanel = 8, kInvRowWarps = (6 * kMaxSeg + 31) / 32;
-__host__ __device__ constexpr size_t inv_smem_doubles(int n) { return static_cast<size_t>(n) * n + 2 * kInvPanel * n; }
+// The matrix in rows of n + 1 (no two rows of a warp start in one bank), two buffers of panel columns, the pivot rows.
+__host__ __device__ constexpr size_t inv_smem_doubles(int n) { return static_cast<size_t>(n) * (n + 1) + 3 * kInvPanel * n; }
 // Barrier among the first `threads` threads (whole warps).
 __device__ __forceinline__ void row_barrier(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 __global__ void __launch_bounds__(kInvThreads, 1) el_invert_kernel(ElDev d, int *flags) {
     extern __shared__ double A[];
     __shared__ double cand[2][kInvRowWarps][kInvPanel + 1];  // each warp's candidate row and 1 / pivot, by pivot parity
-    __shared__ unsigned long long key[2][kInvRowWarps];      // bits of its |pivot|
+    __shared__ unsigned key[2][kInvRowWarps];                // high word of its |pivot|
     __shared__ int crow[2][kInvRowWarps], piv_row[6 * kMaxSeg], singular_s;
-    __shared__ unsigned char rank_of[6 * kMaxSeg];           // position in the current panel of a pivot row, or 255
-    const int m = blockIdx.x, n = 6 * d.S;
-    double *P = A + static_cast<size_t>(n) * n;  // [n][8] panel columns
-    double *X = P + kInvPanel * n;               // [8][n] pivot rows before the update
+    __shared__ unsigned char pivot_of[2][6 * kMaxSeg];       // by panel parity: whether a row is one of its pivots
+    const int m = blockIdx.x, n = 6 * d.S, ld = n + 1;
+    double *const P0 = A + static_cast<size_t>(n) * ld;  // [2][n][8] panel columns, by panel parity
+    double *const X = P0 + 2 * kInvPanel * n;            // [8][n] pivot rows before the update
     double *J = d.jinv + static_cast<size_t>(m) * n * n;
-    for (int e = threadIdx.x; e < n * n / 2; e += blockDim.x)  // n * n is a multiple of 36
-        reinterpret_cast<double2 *>(A)[e] = reinterpret_cast<const double2 *>(J)[e];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int r = w; r < n; r += kInvThreads / 32)
+        for (int c = lane; c < n; c += 32) A[r * ld + c] = J[static_cast<size_t>(r) * n + c];
+    if (threadIdx.x < kInvRowWarps) key[0][threadIdx.x] = key[1][threadIdx.x] = 0u;
     if (threadIdx.x == 0) singular_s = 0;
     __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int row_warps = (n + 31) / 32, row = threadIdx.x;
     const bool holds = row < n;
     bool used = !holds;
-    for (int K = 0; K < n; K += kInvPanel) {
-        const int kb = min(kInvPanel, n - K);
-        if (w < row_warps) {  // (a), by the warps that hold the rows
-            double v[kInvPanel];
-            if (holds) rank_of[row] = 255;
+    // (c) for panel [K, K + kb): rows first, first + step, ... of every column but the panel's and [skip, skip + 8); the
+    // panel's take P.  128 columns at a time, four a lane, the pivot rows in registers, two rows for their latency.
+    auto update = [&](int first, int step, int K, int kb, int skip) {
+        const int par = (K / kInvPanel) & 1;
+        const double *P = P0 + par * kInvPanel * n;
+        constexpr int kSpan = 4;
+        for (int c0 = lane; c0 < n; c0 += 32 * kSpan) {
+            double x[kSpan][kInvPanel];
 #pragma unroll
-            for (int q = 0; q < kInvPanel; ++q) v[q] = (holds && q < kb) ? A[row * n + K + q] : 0.0;
+            for (int u = 0; u < kSpan; ++u)
+#pragma unroll
+                for (int t = 0; t < kInvPanel; ++t) x[u][t] = c0 + 32 * u < n ? X[t * n + c0 + 32 * u] : 0.0;
+            for (int r = first; r < n; r += 2 * step) {
+                const int r1 = min(r + step, n - 1);  // past the end: the last row, not stored
+                const bool own0 = pivot_of[par][r], own1 = pivot_of[par][r1];
+                double a0[kSpan], a1[kSpan];
+#pragma unroll
+                for (int u = 0; u < kSpan; ++u) {
+                    const int c = min(c0 + 32 * u, n - 1);
+                    a0[u] = A[r * ld + c];
+                    a1[u] = A[r1 * ld + c];
+                }
+#pragma unroll
+                for (int u = 0; u < kSpan; ++u) {
+                    a0[u] = own0 ? 0.0 : a0[u];
+                    a1[u] = own1 ? 0.0 : a1[u];
+                }
+#pragma unroll
+                for (int t = 0; t < kInvPanel; t += 2) {
+                    const double2 p0 = *reinterpret_cast<const double2 *>(P + r * kInvPanel + t);
+                    const double2 p1 = *reinterpret_cast<const double2 *>(P + r1 * kInvPanel + t);
+#pragma unroll
+                    for (int u = 0; u < kSpan; ++u) {
+                        a0[u] = fma(p0.y, x[u][t + 1], fma(p0.x, x[u][t], a0[u]));
+                        a1[u] = fma(p1.y, x[u][t + 1], fma(p1.x, x[u][t], a1[u]));
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kSpan; ++u) {
+                    const int c = c0 + 32 * u;
+                    if (c >= n || (c >= skip && c < skip + kInvPanel)) continue;
+                    const bool panel = c >= K && c < K + kb;
+                    A[r * ld + c] = panel ? P[r * kInvPanel + c - K] : a0[u];
+                    if (r + step < n) A[r1 * ld + c] = panel ? P[r1 * kInvPanel + c - K] : a1[u];
+                }
+            }
+        }
+    };
+    for (int K = 0; K < n; K += kInvPanel) {
+        const int kb = min(kInvPanel, n - K), now = (K / kInvPanel) & 1, last = now ^ 1;
+        if (w >= row_warps) {
+            if (K > 0) update(w - row_warps, kInvThreads / 32 - row_warps, K - kInvPanel, kInvPanel, K);
+        } else {
+            double v[kInvPanel];
+#pragma unroll
+            for (int q = 0; q < kInvPanel; ++q) v[q] = (holds && q < kb) ? A[row * ld + K + q] : 0.0;
+            if (K > 0 && holds) {  // (a) the last panel's update of these columns
+                const double *pr = P0 + last * kInvPanel * n + row * kInvPanel;
+                const bool own = pivot_of[last][row];
+#pragma unroll
+                for (int q = 0; q < kInvPanel; ++q) v[q] = own ? 0.0 : v[q];
+#pragma unroll
+                for (int t = 0; t < kInvPanel; ++t) {
+                    const double p = pr[t];
+#pragma unroll
+                    for (int q = 0; q < kInvPanel; ++q) v[q] = fma(p, q < kb ? X[t * n + K + q] : 0.0, v[q]);
+                }
+            }
+            if (holds) pivot_of[now][row] = 0;
             bool singular = false;
 #pragma unroll
-            for (int t = 0; t < kInvPanel; ++t) {
+            for (int t = 0; t < kInvPanel; ++t) {  // (b)
                 if (t >= kb || singular) continue;  // uniform over these warps
                 const int par = t & 1;
                 const double a = fabs(v[t]), inv_own = 1.0 / v[t];
-                const unsigned long long bits = (used || !(a == a)) ? 0ull : static_cast<unsigned long long>(__double_as_longlong(a));
-                const unsigned hi = static_cast<unsigned>(bits >> 32);
+                const unsigned hi = (used || !(a == a)) ? 0u : static_cast<unsigned>(__double2hiint(a));
                 const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-                const unsigned lo = hi == mh ? static_cast<unsigned>(bits) : 0u;
-                const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
-                const unsigned who = __ballot_sync(0xffffffffu, hi == mh && lo == ml && !used);
-                if (who != 0u && lane == __ffs(who) - 1) {
-                    key[par][w] = bits;
+                const unsigned who = __ballot_sync(0xffffffffu, hi == mh);
+                if (lane == __ffs(who) - 1) {
+                    key[par][w] = mh;
                     crow[par][w] = row;
 #pragma unroll
                     for (int q = 0; q < kInvPanel; ++q) cand[par][w][q] = v[q];
                     cand[par][w][kInvPanel] = inv_own;
-                } else if (who == 0u && lane == 0) {
-                    key[par][w] = 0ull;
                 }
                 row_barrier(32 * row_warps);
                 int best = 0;
-                unsigned long long bk = key[par][0];
-                for (int q = 1; q < row_warps; ++q) {
-                    const unsigned long long kq = key[par][q];
-                    if (kq > bk) {
-                        bk = kq;
-                        best = q;
-                    }
+                unsigned bk = key[par][0];
+#pragma unroll
+                for (int q = 1; q < kInvRowWarps; ++q) {  // a warp without rows keeps the key 0
+                    const unsigned kq = key[par][q];
+                    best = kq > bk ? q : best;
+                    bk = max(kq, bk);
                 }
-                if (bk == 0ull) {
+                if (bk == 0u) {
                     singular = true;
                     continue;
                 }
@@ -833,7 +892,7 @@ __global__ void __launch_bounds__(kInvThreads, 1) el_invert_kernel(ElDev d, int 
                 if (row == p) {
                     used = true;
                     piv_row[K + t] = p;
-                    rank_of[p] = static_cast<unsigned char>(t);
+                    pivot_of[now][p] = 1;
 #pragma unroll
                     for (int q = 0; q < kInvPanel; ++q) v[q] = q == t ? inv : v[q] * inv;
                 } else {
@@ -844,51 +903,26 @@ __global__ void __launch_bounds__(kInvThreads, 1) el_invert_kernel(ElDev d, int 
             }
             if (singular && row == 0) singular_s = 1;
             if (holds) {
-                double2 *o = reinterpret_cast<double2 *>(P + row * kInvPanel);
+                double2 *o = reinterpret_cast<double2 *>(P0 + now * kInvPanel * n + row * kInvPanel);
 #pragma unroll
                 for (int q = 0; q < kInvPanel; q += 2) o[q / 2] = make_double2(q < kb ? v[q] : 0.0, q + 1 < kb ? v[q + 1] : 0.0);
             }
         }
-        __syncthreads();  // piv_row, rank_of and P are complete
+        __syncthreads();  // the last panel's update, piv_row, pivot_of and P are complete
         if (singular_s) break;
-        for (int e = threadIdx.x; e < kInvPanel * n; e += blockDim.x) {
-            const int t = e / n, c = e - t * n;
-            X[e] = t < kb ? A[piv_row[K + t] * n + c] : 0.0;
-        }
-        __syncthreads();
-        constexpr int kSpan = 4;  // (b): 128 columns at a time, four a lane, the warp's share of X in registers
-        for (int c0 = lane; c0 < n; c0 += 32 * kSpan) {
-            double x[kSpan][kInvPanel];
-#pragma unroll
-            for (int u = 0; u < kSpan; ++u)
-#pragma unroll
-                for (int t = 0; t < kInvPanel; ++t) x[u][t] = c0 + 32 * u < n ? X[t * n + c0 + 32 * u] : 0.0;
-            for (int r = w; r < n; r += kInvThreads / 32) {
-                const bool own = rank_of[r] != 255;
-                const double2 *pr = reinterpret_cast<const double2 *>(P + r * kInvPanel);
-                const double2 p0 = pr[0], p1 = pr[1], p2 = pr[2], p3 = pr[3];
-                const double pv[kInvPanel] = {p0.x, p0.y, p1.x, p1.y, p2.x, p2.y, p3.x, p3.y};
-                double *Ar = A + r * n + c0;
-#pragma unroll
-                for (int u = 0; u < kSpan; ++u) {
-                    const int c = c0 + 32 * u;
-                    if (c < n) {
-                        double a = own ? 0.0 : Ar[32 * u];
-#pragma unroll
-                        for (int t = 0; t < kInvPanel; ++t) a = fma(pv[t], x[u][t], a);
-                        Ar[32 * u] = (c >= K && c < K + kb) ? P[r * kInvPanel + c - K] : a;
-                    }
-                }
-            }
-        }
+        for (int t = w; t < kInvPanel; t += kInvThreads / 32)
+            for (int c = lane; c < n; c += 32) X[t * n + c] = t < kb ? A[piv_row[K + t] * ld + c] : 0.0;
         __syncthreads();
     }
     if (singular_s) {
         if (threadIdx.x == 0) atomicOr(flags, kNonFinite);
         return;
     }
+    const int end = (n - 1) / kInvPanel * kInvPanel;
+    update(w, kInvThreads / 32, end, n - end, n);
+    __syncthreads();
     for (int r = w; r < n; r += kInvThreads / 32) {
-        const double *Ar = A + piv_row[r] * n;
+        const double *Ar = A + piv_row[r] * ld;
         for (int c = lane; c < n; c += 32) J[static_cast<size_t>(r) * n + piv_row[c]] = Ar[c];
     }
 }
