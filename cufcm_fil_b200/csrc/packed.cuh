@@ -4,7 +4,7 @@
 // two scalar ones, rounded the same, in one issue slot and with one read of
 // each operand pair.  The FP32 pipe is no faster for them (70.6 TFLOP/s either
 // way on independent fma chains), but a kernel that is held up by issue or by
-// register reads gains: the pair product of rpy_pairs.cuh 3.60 -> 3.01 ms per
+// register reads gains: the pair product of rpy_pairs.cuh 3.59 -> 2.81 ms per
 // 10^9 pairs.  Code for both is written once, over a real type T = float or F2.
 #pragma once
 

@@ -261,7 +261,7 @@ __device__ __forceinline__ void sym_tiles(const SymParams &p, const FreeSym6 &k,
     auto pair = [&](float *vj) {
         const float dx = xi.x - xs.x, dy = xi.y - xs.y, dz = xi.z - xs.z;
         if constexpr (!SI && !SJ) {
-            if constexpr (WALL) wall_pair_sym<float>(dx, dy, dz, xi.z, xs.z, fs, fi, vi, vj);
+            if constexpr (WALL) wall_pair_sym<float>(dx, dy, dz, xi.z, xs.z, wall_source(xs.z), fs, fi, vi, vj);
             else free_pair_sym<float>(dx, dy, dz, k.t, fs, fi, vi, vj);
         } else {
             if constexpr (WALL) wall_pair_sym6_f32<SI, SJ>(dx, dy, dz, xi.z, xs.z, fs, fi, vi, vj);
@@ -329,11 +329,13 @@ __global__ void __launch_bounds__(kThreads, kSym6CtasPerSm) rpy_sym6_kernel(SymP
 //
 // Every particle receives one partial per tile, as above: FP32 sums are of 32 terms.
 //
-// Bound by the FP32 pipe, at 81% of it (86 packed instructions for both directions of two pairs): a product of 20,480
-// segments above the wall takes 690 us; 880 us with one source a lane and its position and force rotating by shuffles.
-// The loop alone: 3.01 ms for 10^9 pairs, one scalar source 3.60, two rotating packed ones 3.13.
-constexpr int kSym3CtasPerSm = 4;
-using Sym3Smem = ulonglong2[3][64];
+// Bound by the FP32 pipe, at 81% of it (81 packed instructions above the wall for both directions of two pairs): a
+// product of 20,480 segments takes 663 us (389 without a wall); 880 us with one source a lane and its position and force
+// rotating by shuffles.  Five blocks an SM and eight steps unrolled: 678 with four blocks, 751 with sixteen steps (the
+// warps are at different steps, and the loop outgrows the instruction cache), 705 with two.
+constexpr int kSym3CtasPerSm = 5;
+template <bool WALL>
+using Sym3Smem = ulonglong2[WALL ? 4 : 3][64];
 
 __device__ __forceinline__ void sym3_unit(long long t, int nb, int &I, int &K) {
     const int nk = (nb + 1) / 2;
@@ -345,7 +347,7 @@ __device__ __forceinline__ void sym3_unit(long long t, int nb, int &I, int &K) {
 // store(particle, tile, velocity)
 template <bool WALL, class Store>
 __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const float4 *__restrict__ f, int n, int nb,
-                                           const FreeSym &k, int I, int K, int lane, Sym3Smem &sm, Store store) {
+                                           const FreeSym &k, int I, int K, int lane, Sym3Smem<WALL> &sm, Store store) {
     if (I >= nb) return;
     const unsigned full = 0xffffffffu;
     const int src_lane = (lane + 1) & 31;
@@ -371,36 +373,40 @@ __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const f
     sm[0][lane] = sm[0][lane + 32] = q0;
     sm[1][lane] = sm[1][lane + 32] = q1;
     sm[2][lane] = sm[2][lane + 32] = q2;
+    if constexpr (WALL) {
+        const WallSource<F2> z = wall_source(pack2(xa.z, xb.z));
+        sm[3][lane] = sm[3][lane + 32] = make_ulonglong2(z.p.v, z.q.v);
+    }
     __syncwarp();
     const F2 tx = splat<F2>(xi.x), ty = splat<F2>(xi.y), tz = splat<F2>(xi.z);
     const F2 fi[3] = {splat<F2>(fi4.x), splat<F2>(fi4.y), splat<F2>(fi4.z)};
     F2 vi[3] = {}, vj[3] = {};
-    auto pair = [&](F2 sx, F2 sy, F2 sz, const F2 *fj) {
-        if constexpr (WALL) wall_pair_sym<F2>(vsub(tx, sx), vsub(ty, sy), vsub(tz, sz), tz, sz, fj, fi, vi, vj);
-        else free_pair_sym<F2>(vsub(tx, sx), vsub(ty, sy), vsub(tz, sz), k, fj, fi, vi, vj);
+    // step `at - lane`; the particle itself, where it comes up, is replaced by an inert one
+    auto pair = [&](int at, bool self) {
+        const ulonglong2 a = sm[0][at], b = sm[1][at], c = sm[2][at];
+        F2 sx{a.x}, fj[3] = {F2{b.y}, F2{c.x}, F2{c.y}};
+        const F2 sy{a.y}, sz{b.x};
+        if (self) {
+            sx = pack2(-1.0e5f * static_cast<float>(lane + 1), unpack2(sx).y);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) vj[c].v = __shfl_sync(full, vj[c].v, src_lane);
+            for (int q = 0; q < 3; ++q) fj[q] = pack2(0.0f, unpack2(fj[q]).y);
+        }
+        const F2 dx = vsub(tx, sx), dy = vsub(ty, sy), dz = vsub(tz, sz);
+        if constexpr (WALL) {
+            const ulonglong2 d = sm[3][at];
+            wall_pair_sym<F2>(dx, dy, dz, tz, sz, WallSource<F2>{F2{d.x}, F2{d.y}}, fj, fi, vi, vj);
+        } else {
+            free_pair_sym<F2>(dx, dy, dz, k, fj, fi, vi, vj);
+        }
+#pragma unroll
+        for (int c3 = 0; c3 < 3; ++c3) vj[c3].v = __shfl_sync(full, vj[c3].v, src_lane);
     };
     if (!own) {
 #pragma unroll 8
-        for (int s = 0; s < 32; ++s) {
-            const ulonglong2 a = sm[0][lane + s], b = sm[1][lane + s], c = sm[2][lane + s];
-            const F2 fj[3] = {F2{b.y}, F2{c.x}, F2{c.y}};
-            pair(F2{a.x}, F2{a.y}, F2{b.x}, fj);
-        }
-    } else {
+        for (int s = 0; s < 32; ++s) pair(lane + s, false);
+    } else {  // at step 0 the own tile's half is the particle itself
 #pragma unroll 1
-        for (int s = 0; s < 32; ++s) {
-            const ulonglong2 a = sm[0][lane + s], b = sm[1][lane + s], c = sm[2][lane + s];
-            F2 sx{a.x}, fj[3] = {F2{b.y}, F2{c.x}, F2{c.y}};
-            if (s == 0) {
-                // at step 0 the own tile's half is the particle itself: an inert one instead
-                sx = pack2(-1.0e5f * static_cast<float>(lane + 1), unpack2(sx).y);
-#pragma unroll
-                for (int q = 0; q < 3; ++q) fj[q] = pack2(0.0f, unpack2(fj[q]).y);
-            }
-            pair(sx, F2{a.y}, F2{b.x}, fj);
-        }
+        for (int s = 0; s < 32; ++s) pair(lane + s, s == 0);
     }
     auto lo = [](F2 a) { return unpack2(a).x; };
     auto hi = [](F2 a) { return unpack2(a).y; };
@@ -414,7 +420,7 @@ __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const f
 
 template <bool WALL>
 __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_sym3_kernel(SymParams p) {
-    __shared__ Sym3Smem sm[kThreads / 32];
+    __shared__ Sym3Smem<WALL> sm[kThreads / 32];
     chain_wait();  // launched as a programmatic dependent of the packing launch
     if (p.gate && *p.gate == 0) return;
     FreeSym k{};
@@ -438,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_sym3_kernel(SymP
 // tile of the pair), so that both these writes and the per-segment reduction
 // that reads them are coalesced.
 __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_wall_sym_batch_kernel(SymBatchParams p) {
-    __shared__ Sym3Smem sm[kThreads / 32];
+    __shared__ Sym3Smem<true> sm[kThreads / 32];
     chain_wait();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
@@ -631,7 +637,7 @@ __global__ void __launch_bounds__(256) rpy_direct_kernel(DirectParams p) {
         const float px = xj[0], py = xj[1], pz = xj[2];
         if (j == i) continue;
         float drop[3] = {0.0f, 0.0f, 0.0f};
-        if constexpr (WALL) wall_pair_sym<float>(x - px, y - py, z - pz, z, pz, f, none, v, drop);
+        if constexpr (WALL) wall_pair_sym<float>(x - px, y - py, z - pz, z, pz, wall_source(pz), f, none, v, drop);
         else free_pair_sym<float>(x - px, y - py, z - pz, k, f, none, v, drop);
     }
 #pragma unroll

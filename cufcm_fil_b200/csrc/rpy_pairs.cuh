@@ -265,35 +265,44 @@ namespace cufil {
 //   b  =  w u (3/2 z_j + hz (u (2G + 5u) - 9P)) / 6 pi
 //   c  =  w u (3/2 z_j - 5 hz u^2) / 6 pi
 //   e  = -w u (3 z_j^2 + 3E + u (2 - 15E)) / 6 pi
-// 86 FP32 instructions and two reciprocal square roots for both directions; written with the reference's factors it
-// was 109, three and a division (a product of 20,480 segments took 994 us so, 880 without the division, both scalar).
+// The factor 1 / 6 pi is folded into the constants, and what depends on the source alone (WallSource) is formed once per
+// source, which leaves 81 FP32 instructions and two reciprocal square roots for both directions.  A product of 20,480
+// segments: 994 us with the reference's factors (109 instructions, three roots and a division), 880 without the division,
+// both scalar; packed 695 with 86 instructions, 663 with 81.
 template <class T>
-__device__ __forceinline__ void wall_pair_sym(T dx, T dy, T dz, T zi, T zj, const T *fj, const T *fi, T *vi, T *vj) {
+struct WallSource {
+    T p, q;  // 3/2 z_j / 6 pi, -3 z_j^2 / 6 pi
+};
+template <class T>
+__device__ __forceinline__ WallSource<T> wall_source(T zj) {
+    return {vmul(splat<T>(1.5f * RpyConst::inv6pi), zj), vmul(vmul(splat<T>(-3.0f * RpyConst::inv6pi), zj), zj)};
+}
+template <class T>
+__device__ __forceinline__ void wall_pair_sym(T dx, T dy, T dz, T zi, T zj, WallSource<T> z, const T *fj, const T *fi,
+                                              T *vi, T *vj) {
+    constexpr float c6 = RpyConst::inv6pi, c8 = RpyConst::inv8pi;
     auto k = [](float c) { return splat<T>(c); };
     const T q2 = vfma(dx, dx, vmul(dy, dy));
     // free space: A I + B d d^T (even in d)
     const T s = rsqrt_approx(vfma(dz, dz, q2));
     const T s2 = vmul(s, s);
-    const T g = vmul(k(RpyConst::inv8pi), s);
-    const T A = vmul(g, vfma(k(2.0f / 3.0f), s2, k(1.0f)));
-    const T B = vmul(vmul(g, s2), vfma(k(-2.0f), s2, k(1.0f)));
-    // image system; cw = -w / 6 pi, cu = cw u (the signs of the brackets below are turned accordingly)
+    const T A = vmul(s, vfma(k(2.0f / 3.0f * c8), s2, k(c8)));
+    const T B = vmul(vmul(s, s2), vfma(k(-2.0f * c8), s2, k(c8)));
+    // image system, every bracket over 6 pi
     const T hz = vadd(zi, zj);
     const T w = rsqrt_approx(vfma(hz, hz, q2));
-    const T u = vmul(w, w);
-    const T cw = vmul(k(-RpyConst::inv6pi), w), cu = vmul(cw, u);
+    const T u = vmul(w, w), wu = vmul(w, u);
     const T hu = vmul(hz, u), E = vmul(hz, hu);
-    const T P = vmul(vmul(zi, zj), u);
-    const T n5 = vfma(k(7.5f), E, k(-1.5f));  // -3/2 (1 - 5E)
-    const T u5 = vmul(k(5.0f), u);
-    const T G = vfma(u5, vfma(k(-3.5f), E, k(0.5f)), n5);
-    const T k0 = vfma(u, vfma(vmul(u, k(1.0f / 3.0f)), n5, vfma(k(-1.5f), E, k(0.5f))), vfma(k(1.5f), P, k(0.75f)));
-    const T AK = vfma(cw, k0, A);
-    const T a = vmul(cu, vfma(u, G, vfma(k(-4.5f), P, k(0.75f))));
-    const T z15 = vmul(k(-1.5f), zj);
-    const T b = vmul(cu, vfma(vmul(k(9.0f), P), hz, vfma(vmul(k(-1.0f), hu), vfma(k(2.0f), G, u5), z15)));
-    const T c = vmul(cu, vfma(u5, hu, z15));
-    const T e = vmul(cu, vfma(vmul(k(-2.0f), z15), zj, vfma(u, vfma(k(-15.0f), E, k(2.0f)), vmul(k(3.0f), E))));
+    const T P = vmul(vmul(zi, z.p), u);                                    // 3/2 P
+    const T n5 = vfma(k(-7.5f * c6), E, k(1.5f * c6));                     // 3/2 (1 - 5E)
+    const T u5 = vmul(k(-5.0f * c6), u);                                   // -5 u
+    const T H = vfma(u5, vfma(k(-3.5f), E, k(0.5f)), n5);                  // -G
+    const T k0 = vfma(u, vfma(n5, vfma(u, k(1.0f / 3.0f), k(-0.2f)), k(-0.2f * c6)), vsub(k(-0.75f * c6), P));
+    const T AK = vfma(w, k0, A);
+    const T a = vmul(wu, vfma(u, H, vfma(k(3.0f), P, k(-0.75f * c6))));
+    const T b = vmul(wu, vfma(vmul(k(-6.0f), P), hz, vfma(vmul(k(-1.0f), hu), vfma(k(2.0f), H, u5), z.p)));
+    const T c = vmul(wu, vfma(u5, hu, z.p));
+    const T e = vmul(wu, vadd(z.q, vfma(E, vfma(k(15.0f * c6), u, k(-3.0f * c6)), vmul(k(-2.0f * c6), u))));
     const T AKe = vadd(AK, e);
     // i <- j
     {

@@ -44,7 +44,7 @@ constexpr int kMinDotsChunk = 1024;
 
 // Launch shapes chosen by the autotuner (or the defaults).
 struct Tuning {
-    int pair_ctas_per_sm = 4;   // pair kernel residency target (its launch bound)
+    int pair_ctas_per_sm = 5;   // pair kernel residency target (its launch bound)
     int dots_chunk = 4096;      // rows per dot-product item
     int dots_blocks_per_sm = 2;
     int update_blocks_per_sm = 8;
