@@ -351,7 +351,7 @@ int fused_gradients(cf_mlp *h, const float *x, const float *t, int n, const mlpk
     a.db = h->db;
     a.loss = h->partial;
     a.scale = 1.0f / static_cast<float>(static_cast<long long>(n) * h->out);
-    CF_CUDA(launch_chained(mlpk::mlp_rows_kernel<true>, dim3(tiles), dim3(mlpk::kThreads), mlpk::kRowsSmem, st, a));
+    CF_CUDA(launch_chained(mlpk::mlp_rows_kernel<true>, dim3(tiles), dim3(mlpk::kRowThreads), mlpk::kRowsSmem, st, a));
     CF_CHECK_LAUNCH("mlp_rows_kernel");
     mlpk::GradArgs g{h->xt, h->a1t, h->a2t, h->dyt, h->dz2t, h->dz1t, h->gpart, h->nparam, h->in, h->hid, h->out, tiles,
                      splits};
@@ -386,7 +386,7 @@ int forward(cf_mlp *h, const float *x, int n, float *y, cudaStream_t st) {
         const bool shared = before(x, y + ny) && before(y, x + nx);
         a.y = shared ? h->Y : y;
         CF_CUDA(launch_chained(mlpk::mlp_rows_kernel<false>, dim3((n + mlpk::kRows - 1) / mlpk::kRows),
-                               dim3(mlpk::kThreads), mlpk::kRowsSmem, st, a));
+                               dim3(mlpk::kRowThreads), mlpk::kRowsSmem, st, a));
         CF_CHECK_LAUNCH("mlp_rows_kernel");
         if (shared) CF_CUDA(cudaMemcpyAsync(y, h->Y, ny * sizeof(float), cudaMemcpyDeviceToDevice, st));
         return CF_OK;

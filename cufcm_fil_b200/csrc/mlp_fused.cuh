@@ -21,9 +21,10 @@
 // What bounds it.  A pass over 1024 rows is 0.27 GFLOP and 0.9 MB: the time is
 // the chain of dependent steps (stage, multiply, read back, three times), so
 // each step moves its data once, 16 bytes at a time, and the next weights
-// arrive while the current product runs.  With 182 x 256 x 256 x 62: forward of 1024 rows 8.2 us a call (37 with three
-// GEMM launches and their activations in memory); loss and gradients of 2048 rows 57 + 17 + 6 us in the three kernels,
-// 119 us a call (947 with six GEMMs, those over K = 2048 rows unsplit, and serial column sums).
+// arrive while the current product runs.  With 182 x 256 x 256 x 62: forward of 1024 rows 7.9 us a call (37 with three
+// GEMM launches and their activations in memory); loss and gradients of 2048 rows 115 us a call (947 with six GEMMs,
+// those over K = 2048 rows unsplit, and serial column sums), of which the transfer of the gradients to the host is about
+// half.  Sixteen warps for the epilogues: eight took 8.2 and 119 us.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -38,7 +39,8 @@ constexpr int kRows = 128;      // rows of a block: the M of one tcgen05.mma
 constexpr int kMaxW = 256;      // widest input and hidden layer
 constexpr int kMaxOut = 128;    // widest output layer
 constexpr int kChunk = 128;     // image rows (output columns) of one weight chunk
-constexpr int kThreads = 256;   // two groups of four warps: each group every other block of 32 columns
+constexpr int kThreads = 256;
+constexpr int kRowThreads = 512, kGroups = kRowThreads / 128;  // groups of four warps: each every kGroups-th 32 columns
 constexpr uint32_t kCols = 256; // accumulator columns
 constexpr size_t kABytes = static_cast<size_t>(kRows) * kMaxW * 2;
 constexpr size_t kWBytes = static_cast<size_t>(kChunk) * kMaxW * 2;
@@ -101,7 +103,7 @@ __device__ __forceinline__ void store_image(__nv_bfloat16 *im, int row, int col0
 __device__ __forceinline__ void write_transposed(const __nv_bfloat16 *im, int kp, __nv_bfloat16 *out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nk = kp >> 3, total = (kRows / 8) * nk;  // core matrices, four at a time
-    for (int c0 = 4 * warp; c0 < total; c0 += 4 * (kThreads / 32)) {
+    for (int c0 = 4 * warp; c0 < total; c0 += 4 * (kRowThreads / 32)) {
         // core matrix c: feature group c / 16, row group c % 16, so four consecutive ones are 512 contiguous bytes
         const int c = c0 + (lane >> 3);
         const int fg = c >> 4, rg = c & 15;
@@ -132,11 +134,11 @@ __device__ __forceinline__ float column_sums(float *v, int lane) {
 
 // One block per 128 rows.  Thread 0 fetches the weight chunks (two buffers, the next chunk's copy issued as soon
 // as the product that read its buffer is done) and issues the products; all threads stage the input and run the
-// epilogues: warp w reads the accumulator rows 32 (w % 4) .. + 31, its group w / 4 every other block of 32 columns,
+// epilogues: warp w reads the accumulator rows 32 (w % 4) .. + 31, its group w / 4 every kGroups-th block of 32 columns,
 // the same assignment in every layer, so the ReLU masks of the backward pass stay in registers.  A bounded wait
 // that gives up ends the products: the outputs (or the gradients) are NaN then.
 template <bool TRAIN>
-__global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
+__global__ void __launch_bounds__(kRowThreads, 1) mlp_rows_kernel(RowArgs g) {
     extern __shared__ __align__(128) unsigned char dyn[];
     __nv_bfloat16 *As = reinterpret_cast<__nv_bfloat16 *>(dyn);
     __nv_bfloat16 *Ws[2] = {reinterpret_cast<__nv_bfloat16 *>(dyn + kABytes),
@@ -146,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
     __shared__ int alive;
     __shared__ float bias[2 * kMaxW + kMaxOut];
     __shared__ float csum[TRAIN ? 4 : 1][TRAIN ? kMaxW : 1];
-    __shared__ double lsum[kThreads / 32];
+    __shared__ double lsum[kRowThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp >> 2;
     const int tile = blockIdx.x, m0 = tile * kRows;
     const int row = 32 * (warp & 3) + lane;
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
         fetch(0);
         fetch(1);
     }
-    for (int j = threadIdx.x; j < 2 * kMaxW + kMaxOut; j += kThreads) {
+    for (int j = threadIdx.x; j < 2 * kMaxW + kMaxOut; j += kRowThreads) {
         const int l = j < kMaxW ? 0 : (j < 2 * kMaxW ? 1 : 2), c = j - l * kMaxW;
         const float *b = l == 0 ? g.b1 : (l == 1 ? g.b2 : g.b3);
         bias[j] = c < (l == 2 ? g.out : g.hid) ? b[c] : 0.0f;
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
         const int r8 = lane & 7, kg = lane >> 3;
         const int kblocks = inP / 32;  // 32 columns each
         const bool pairs = (g.in & 1) == 0 && (reinterpret_cast<uintptr_t>(g.x) & 7) == 0;
-        for (int it = warp; it < (kRows / 8) * kblocks; it += kThreads / 32) {
+        for (int it = warp; it < (kRows / 8) * kblocks; it += kRowThreads / 32) {
             const int r = 8 * (it / kblocks) + r8, k = 32 * (it % kblocks) + 8 * kg;
             const float *src = g.x + static_cast<size_t>(m0 + r) * g.in + k;
             float v[8];
@@ -266,12 +268,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
     };
 
     const float nan = __int_as_float(0x7fc00000);
-    uint32_t mask[2][4];
+    uint32_t mask[2][kMaxW / (32 * kGroups)];
     // hidden layers: bias, ReLU, the next image
     auto hidden = [&](int l) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int c0 = 32 * (2 * u + group);
+        for (int u = 0; u < kMaxW / (32 * kGroups); ++u) {
+            const int c0 = 32 * (kGroups * u + group);
             if (c0 >= hidP) continue;
             float v[32];
             tc::tmem_ld32(tc::tmem_addr(tmem, warp, c0), v);
@@ -290,8 +292,8 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
     // backward: ReLU mask, column sums, the next image
     auto hidden_back = [&](int l, int db0) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int c0 = 32 * (2 * u + group);
+        for (int u = 0; u < kMaxW / (32 * kGroups); ++u) {
+            const int c0 = 32 * (kGroups * u + group);
             if (c0 >= hidP) continue;
             float v[32];
             tc::tmem_ld32(tc::tmem_addr(tmem, warp, c0), v);
@@ -302,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
         }
         tc::fence_before_sync();
         __syncthreads();
-        for (int c = threadIdx.x; c < hidP; c += kThreads)
+        for (int c = threadIdx.x; c < hidP; c += kRowThreads)
             g.db[static_cast<size_t>(tile) * (2 * hidP + outP) + db0 + c] =
                 (csum[0][c] + csum[TRAIN ? 1 : 0][c]) + (csum[TRAIN ? 2 : 0][c] + csum[TRAIN ? 3 : 0][c]);
     };
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
         // the rows of y are contiguous: gathered in shared memory (the image is no longer needed), then copied
         float *ys = reinterpret_cast<float *>(dyn);
         const bool ok = alive != 0;
-        for (int c0 = 32 * group; c0 < outP; c0 += 64) {
+        for (int c0 = 32 * group; c0 < outP; c0 += 32 * kGroups) {
             float v[32];
             tc::tmem_ld32(tc::tmem_addr(tmem, warp, c0), v);
 #pragma unroll
@@ -334,10 +336,10 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
         __syncthreads();
         const int cnt = min(kRows, g.n - m0) * g.out;
         float *dst = g.y + static_cast<size_t>(m0) * g.out;
-        for (int e = threadIdx.x; e < cnt; e += kThreads) dst[e] = ys[e];
+        for (int e = threadIdx.x; e < cnt; e += kRowThreads) dst[e] = ys[e];
     } else {
         double ss = 0.0;
-        for (int c0 = 32 * group; c0 < outP; c0 += 64) {
+        for (int c0 = 32 * group; c0 < outP; c0 += 32 * kGroups) {
             float v[32];
             tc::tmem_ld32(tc::tmem_addr(tmem, warp, c0), v);
             const float *t = g.t + static_cast<size_t>(m0 + row) * g.out + c0;
@@ -358,12 +360,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
         if (lane == 0) lsum[warp] = ss;
         tc::fence_before_sync();
         __syncthreads();
-        for (int c = threadIdx.x; c < outP; c += kThreads)
+        for (int c = threadIdx.x; c < outP; c += kRowThreads)
             g.db[static_cast<size_t>(tile) * (2 * hidP + outP) + 2 * hidP + c] =
                 (csum[0][c] + csum[1][c]) + (csum[2][c] + csum[3][c]);
         if (threadIdx.x == 0) {
             double s = 0.0;
-            for (int w = 0; w < kThreads / 32; ++w) s += lsum[w];
+            for (int w = 0; w < kRowThreads / 32; ++w) s += lsum[w];
             g.loss[tile] = alive ? s : static_cast<double>(nan);
         }
         start(2 * ch + 1, ch);
@@ -379,10 +381,10 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_rows_kernel(RowArgs g) {
         write_transposed(As, hidP, g.dz1t + tileI * pad128(g.hid));
         if (!alive) {  // a product is missing: no gradient may look valid
             __syncthreads();
-            for (int c = threadIdx.x; c < 2 * hidP + outP; c += kThreads)
+            for (int c = threadIdx.x; c < 2 * hidP + outP; c += kRowThreads)
                 g.db[static_cast<size_t>(tile) * (2 * hidP + outP) + c] = nan;
             const __nv_bfloat16 bn = __float2bfloat16_rn(nan);
-            for (int e = threadIdx.x; e < kRows * hidP; e += kThreads) {
+            for (int e = threadIdx.x; e < kRows * hidP; e += kRowThreads) {
                 g.dz1t[tileI * pad128(g.hid) + e] = bn;
                 g.dz2t[tileI * pad128(g.hid) + e] = bn;
                 if (e < kRows * outP) g.dyt[tileI * outP + e] = bn;

@@ -67,3 +67,17 @@ def test_training_step_leaves_consistent_weights():
         p = net.params()
         assert rel(p, before) > 1e-3
         check(net, p, X, T, dims, exact=False)
+
+
+@pytest.mark.parametrize("n", [5, 300])
+def test_output_may_overlap_the_input(n):
+    rng = np.random.default_rng(n)
+    dims = (182, 256, 62)
+    X = rng.standard_normal((n, dims[0])).astype(np.float32)
+    with FilamentMLP(*dims, max_batch=512, seed=2) as net:
+        xd, yd = torch.tensor(X, device="cuda"), torch.zeros((n, dims[2]), device="cuda")
+        torch.cuda.synchronize()
+        net.forward(xd, yd)
+        net.forward(xd, xd.view(-1)[:n * dims[2]].view(n, dims[2]))
+        torch.cuda.synchronize()
+        assert torch.equal(xd.view(-1)[:n * dims[2]].view(n, dims[2]), yd)
