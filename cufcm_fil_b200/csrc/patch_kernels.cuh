@@ -435,18 +435,6 @@ __global__ void __launch_bounds__(256) gj_prep_kernel(PatchDev P, int K) {
     }
 }
 
-// 16-byte asynchronous copy global -> shared (zero-filled when !valid; src is
-// then not read but must still be a mapped address).  Both addresses 16-byte aligned.
-__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool valid) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 // One tile of round K's update: which tile of which patch, and its kind.
 struct GjTile {
     int p, n, row0, col0;
@@ -492,16 +480,15 @@ constexpr int kUpStage = 4 * tc::kOperandFloats;
 constexpr int kUpLd = kGjTile + 4;  // 16-byte rows
 constexpr size_t kUpdateSmem = (kUpStage + kGjTile * kUpLd) * sizeof(float);
 
-// Issues the 16-byte copies of a tile's operands into `stage` (contiguous blocks: 8 + 8 chunks per thread;
-// the pivot rows need B only).
-__device__ __forceinline__ void gj_issue_tile(const PatchDev &P, const GjTile &t, float *stage) {
-    float *Ab = stage, *Bb = stage + 2 * tc::kOperandFloats;
+// Starts the copies of a tile's operands into `stage` (one thread): each is one contiguous 32 KB block.  The pivot rows
+// need B only.
+__device__ __forceinline__ void gj_issue_tile(const PatchDev &P, const GjTile &t, float *stage, uint64_t *full) {
+    constexpr uint32_t kBytes = 2 * tc::kOperandFloats * sizeof(float);
     const float *csrc = P.csplit + (static_cast<size_t>(t.p) * P.T + t.row0 / kGjTile) * 2 * tc::kOperandFloats;
     const float *rsrc = P.rsplit + (static_cast<size_t>(t.p) * P.T + t.col0 / kGjTile) * 2 * tc::kOperandFloats;
-    for (int c = threadIdx.x; c < 2 * tc::kOperandFloats / 4; c += blockDim.x) {
-        cp_async16(Bb + 4 * c, rsrc + 4 * c, true);
-        if (!t.prow) cp_async16(Ab + 4 * c, csrc + 4 * c, true);
-    }
+    mbar_arrive_expect_tx(full, t.prow ? kBytes : 2 * kBytes);
+    bulk_g2s(stage + 2 * tc::kOperandFloats, rsrc, kBytes, full);
+    if (!t.prow) bulk_g2s(stage, csrc, kBytes, full);
 }
 
 // Round K, part (c), the 64x64 tiles of the upper block triangle:
@@ -520,11 +507,12 @@ __device__ __forceinline__ void gj_issue_tile(const PatchDev &P, const GjTile &t
 // while the operands land and its copies start as soon as the products have
 // read theirs, and the products go through shared memory so that the rows of A
 // are read and written 256 contiguous bytes at a time: a round of 16 patches of
-// 992 unknowns takes 33 us, 41 without, of which the chain diagonal tile ->
-// inversion is about 22.
+// 992 unknowns takes 31.6 us, 41 without (33.0 with 16-byte copies by every
+// thread instead of two bulk copies a tile), of which the chain diagonal tile ->
+// inversion is about 22 when it has its SM alone.
 // The block that takes a patch's diagonal tile (K + 1, K + 1) inverts it for
 // the next round right after its update, while the other blocks go on with the
-// rest.  A wait for the products that gives up (bounded) marks the tile's patch
+// rest.  A wait for copies or products that gives up (bounded) marks the tile's patch
 // unusable -- it falls back to the block-diagonal preconditioner -- and the
 // block computes no further products.  Dynamic shared memory: kUpdateSmem.
 __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, int T, int *counter) {
@@ -532,7 +520,7 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, in
     static_assert(kUpStage >= kInvWs, "the inversion reuses the stage");
     extern __shared__ __align__(128) float usm[];
     __shared__ int next_item[2];  // drawn ahead; drawn after an inversion
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bar, full;
     __shared__ uint32_t tbase;
     __shared__ int tc_ok, dead;
     chain_wait();
@@ -545,6 +533,7 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, in
     if (warp == 0) tc::tmem_alloc(&tbase, tc::kTmemCols);
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
+        mbar_init(&full, 1);
         fence_barrier_init();
         dead = 0;
     }
@@ -558,10 +547,9 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, in
     // this thread's output: rows tr + 16 k, columns tc4 .. + 3
     const int tr = threadIdx.x >> 4, tc4 = 4 * (threadIdx.x & 15);
     GjTile cur = gj_tile(P, K, T, item);
-    if (cur.valid) {
-        gj_issue_tile(P, cur, usm);
-        cp_async_commit();
-    }
+    uint32_t copies = 0;  // tiles whose operands were waited for
+    bool broken = false;  // such a wait gave up: nothing more is copied or multiplied
+    if (cur.valid && threadIdx.x == 0) gj_issue_tile(P, cur, usm, &full);
     for (;;) {
         int drawn = 0;
         if (threadIdx.x == 0 && !cur.diag) drawn = atomicAdd(counter, 1);
@@ -582,13 +570,13 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, in
                 }
         }
         if (threadIdx.x == 0) next_item[0] = drawn;
-        cp_async_wait<0>();
-        tc::fence_proxy_async();  // the operands are visible to the tensor cores
+        bool landed = true;
+        if (cur.valid && !broken) landed = mbar_wait_bounded(&full, copies++ & 1u);
         tc::fence_before_sync();
-        __syncthreads();
+        if (!__syncthreads_and(landed)) broken = true;
         tc::fence_after_sync();
         int next = next_item[0];
-        const bool stopped = dead != 0;
+        const bool stopped = dead != 0 || broken;
         if (cur.valid && !cur.prow && !stopped && threadIdx.x == 0) {
             tc::issue_tile_products(tmem, Ab, Ab + tc::kOperandFloats, Bb, Bb + tc::kOperandFloats);
             tc::commit(&bar);
@@ -613,11 +601,11 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, in
                 ++products;
             }
         }
+        tc::fence_proxy_async();
         __syncthreads();  // the stage has been read
         tc::fence_after_sync();
-        const bool product = cur.valid && !cur.prow, have = !product || (!stopped && tc_ok != 0);
-        if (nxt.valid) gj_issue_tile(P, nxt, usm);
-        cp_async_commit();
+        const bool product = cur.valid && !cur.prow, have = product ? !stopped && tc_ok != 0 : !broken;
+        if (nxt.valid && !broken && threadIdx.x == 0) gj_issue_tile(P, nxt, usm, &full);
         if (product && have) {
             // row m of the product lies in lane m % 16 of warps m / 16 and m / 16 + 4 (32 columns each)
             float v[32];
@@ -630,7 +618,7 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, in
             tc::fence_before_sync();
         }
         __syncthreads();
-        if (product && !have && threadIdx.x == 0) {
+        if (cur.valid && !have && threadIdx.x == 0) {
             P.ok[cur.p] = 0;
             dead = 1;
         }
@@ -681,15 +669,16 @@ __global__ void __launch_bounds__(256, 2) gj_update_kernel(PatchDev P, int K, in
             __syncthreads();  // inversion works in the stage, so the next tile is drawn and copied after it
             if (cur.valid) pivot_invert_patch(P, cur.p, K + 1, usm);
             if (threadIdx.x == 0) next_item[1] = atomicAdd(counter, 1);
+            tc::fence_proxy_async();
             __syncthreads();
             next = next_item[1];
             if (next < total) nxt = gj_tile(P, K, T, next);
-            if (nxt.valid) gj_issue_tile(P, nxt, usm);
-            cp_async_commit();
+            if (nxt.valid && !broken && threadIdx.x == 0) gj_issue_tile(P, nxt, usm, &full);
         }
         if (next >= total) break;
         cur = nxt;
     }
+    if (broken && threadIdx.x == 0) mbar_wait_bounded(&full, (copies - 1) & 1u);  // copies still in flight land first
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, tc::kTmemCols);
