@@ -197,7 +197,7 @@ struct SymParams {
     float4 *partial;
     int n, n6, nb;
     long long items;
-    float a, inv_mu;  // unbounded form: the common radius and 1 / viscosity
+    FreeSym6 k;       // unbounded form
     const int *gate;  // may be null: nothing is done where *gate is zero
 };
 
@@ -223,6 +223,9 @@ __device__ __forceinline__ void sym_load(const SymParams &p, int idx, int lane, 
         f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
+
+// First step of a tile against itself: its particles' neighbours along a filament come last.
+constexpr int kOwnStart = 4;
 
 // One pair of tiles.  SI, SJ: tile I, J holds particles with torques and spins (a tile that also holds others gives
 // those zero torques, and their spins are dropped).
@@ -275,25 +278,56 @@ __device__ __forceinline__ void sym_tiles(const SymParams &p, const FreeSym6 &k,
     auto store = [&](int q, int tile, const float *v, bool spins) {
         if (q >= p.n) return;
         float4 *o = place(q, tile);
-        o[0] = make_float4(v[0], v[1], v[2], 0.0f);
+        constexpr float scale = !SI && !SJ && WALL ? static_cast<float>(kPairScale) : 1.0f;
+        const float c = !SI && !SJ && !WALL ? k.c8 : scale;  // the force-only pairs come without their factor
+        o[0] = make_float4(c * v[0], c * v[1], c * v[2], 0.0f);
         if (spins && q < p.n6) o[1] = make_float4(v[3], v[4], v[5], 0.0f);
     };
-    if (I == J) {
-#pragma unroll 1
-        for (int step = 1; step < 32; ++step) {
-            rotate_source();
-            float drop[NJ] = {};
-            pair(drop);
+    // Tiles with force-only particles form sums of 16 terms: the first half's are set aside.  (Relative L2 error against
+    // FP64 in sets with 1,500 to 6,000 blobs 1.3 to 1.4e-7, the tile kernel's 1.3 to 2.1, sums of 32 1.5 to 1.8.  Between
+    // particles with torques sums of 32 are nearer than the tile kernel's, 1.1 to 1.4e-7 against 1.6 to 2.2, and the
+    // registers for shorter ones cost 8%.)
+    constexpr bool kSplit = !(SI && SJ);
+    float vi0[NI] = {}, vs0[NJ] = {};
+    auto set_aside = [&] {
+#pragma unroll
+        for (int c = 0; c < NI; ++c) {
+            vi0[c] = vi[c];
+            vi[c] = 0.0f;
         }
+#pragma unroll
+        for (int c = 0; c < NJ; ++c) {
+            vs0[c] = vs[c];
+            vs[c] = 0.0f;
+        }
+    };
+    if (I == J) {  // a filament's neighbours, the largest terms, come last: steps 4 .. 31, 1 .. 3
+#pragma unroll
+        for (int r = 0; r < kOwnStart; ++r) rotate_source();
+#pragma unroll 1
+        for (int step = kOwnStart; step < kOwnStart + 32; ++step) {
+            if (kSplit && step == kOwnStart + 16) set_aside();
+            float drop[NJ] = {};
+            if (step != 32) pair(drop);
+            rotate_source();
+        }
+#pragma unroll
+        for (int c = 0; c < NI; ++c) vi[c] += vi0[c];
         store(i, I, vi, SI);
     } else {
 #pragma unroll(SI || SJ ? 1 : 2)
         for (int step = 0; step < 32; ++step) {
+            if (kSplit && step == 16) set_aside();
             pair(vs);
             rotate_source();
 #pragma unroll
             for (int c = 0; c < NJ; ++c) rotate(vs[c]);
         }
+#pragma unroll
+        for (int c = 0; c < NI; ++c) vi[c] += vi0[c];
+#pragma unroll
+        for (int c = 0; c < NJ; ++c)
+            if (kSplit) vs[c] += __shfl_sync(full, vs0[c], lane ^ 16);  // set aside 16 lanes from home
         store(i, J, vi, SI);
         store(j, I, vs, SJ);
     }
@@ -305,8 +339,7 @@ template <bool WALL>
 __global__ void __launch_bounds__(kThreads, kSym6CtasPerSm) rpy_sym6_kernel(SymParams p) {
     chain_wait();  // launched as a programmatic dependent of the packing launch
     if (p.gate && *p.gate == 0) return;
-    FreeSym6 k{};
-    if constexpr (!WALL) k = free_sym6(p.a, p.inv_mu);
+    const FreeSym6 &k = p.k;
     const int lane = threadIdx.x & 31;
     const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
     for (long long t = static_cast<long long>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5); t < p.items;
@@ -327,10 +360,13 @@ __global__ void __launch_bounds__(kThreads, kSym6CtasPerSm) rpy_sym6_kernel(SymP
 // sources rotate.  In the units K = I / 2 the tile meets itself: those pairs are evaluated one-sided and a particle
 // never meets itself; an odd I leaves the other half empty there.
 //
-// Every particle receives one partial per tile, as above: FP32 sums are of 32 terms.
+// Every particle receives one partial per tile, as above, of two FP32 sums of 16 terms.  That is what the error against
+// FP64 depends on: 1.0e-7 (relative L2, cilia above the wall, 600 to 7,500 segments; 1.0e-7 without a wall, 1.0 to 1.3e-7
+// with blobs); 1.3, 1.3 and 1.7e-7 with one sum of 32 and the neighbours first.  Refining the reciprocal square roots did
+// not change it.
 //
 // Bound by the FP32 pipe, at 81% of it (81 packed instructions above the wall for both directions of two pairs): a
-// product of 20,480 segments takes 663 us (389 without a wall); 880 us with one source a lane and its position and force
+// product of 20,480 segments takes 664 us (393 without a wall); 880 us with one source a lane and its position and force
 // rotating by shuffles.  Five blocks an SM and eight steps unrolled: 678 with four blocks, 751 with sixteen steps (the
 // warps are at different steps, and the loop outgrows the instruction cache), 705 with two.
 constexpr int kSym3CtasPerSm = 5;
@@ -350,7 +386,7 @@ __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const f
                                            const FreeSym &k, int I, int K, int lane, Sym3Smem<WALL> &sm, Store store) {
     if (I >= nb) return;
     const unsigned full = 0xffffffffu;
-    const int src_lane = (lane + 1) & 31;
+    const int src_lane = (lane + 2) & 31;
     const bool own = K == I >> 1, odd_own = own && (I & 1);
     const int i = I * 32 + lane, ja = odd_own ? i : K * 64 + lane, jb = odd_own ? n : K * 64 + 32 + lane;
     auto load = [&](int idx, float apart, float4 &xv, float4 &fv) {
@@ -380,9 +416,10 @@ __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const f
     __syncwarp();
     const F2 tx = splat<F2>(xi.x), ty = splat<F2>(xi.y), tz = splat<F2>(xi.z);
     const F2 fi[3] = {splat<F2>(fi4.x), splat<F2>(fi4.y), splat<F2>(fi4.z)};
-    F2 vi[3] = {}, vj[3] = {};
+    // even and odd steps have their own sums, of 16 terms each; the sources' rotate by two lanes after each of theirs
+    F2 vi_[2][3] = {}, vj_[2][3] = {};
     // step `at - lane`; the particle itself, where it comes up, is replaced by an inert one
-    auto pair = [&](int at, bool self) {
+    auto pair = [&](int at, bool self, F2 *vi, F2 *vj) {
         const ulonglong2 a = sm[0][at], b = sm[1][at], c = sm[2][at];
         F2 sx{a.x}, fj[3] = {F2{b.y}, F2{c.x}, F2{c.y}};
         const F2 sy{a.y}, sz{b.x};
@@ -402,11 +439,27 @@ __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const f
         for (int c3 = 0; c3 < 3; ++c3) vj[c3].v = __shfl_sync(full, vj[c3].v, src_lane);
     };
     if (!own) {
-#pragma unroll 8
-        for (int s = 0; s < 32; ++s) pair(lane + s, false);
-    } else {  // at step 0 the own tile's half is the particle itself
+#pragma unroll 4
+        for (int s = 0; s < 32; s += 2) {
+            pair(lane + s, false, vi_[0], vj_[0]);
+            pair(lane + s + 1, false, vi_[1], vj_[1]);
+        }
+    } else {  // a filament's neighbours, the largest terms, come last (28 .. 31, 0 .. 3); at step 0 the own tile's half
+              // is the particle itself
 #pragma unroll 1
-        for (int s = 0; s < 32; ++s) pair(lane + s, s == 0);
+        for (int t = kOwnStart; t < kOwnStart + 32; t += 2) {
+            const int s = t & 31;
+            pair(lane + s, s == 0, vi_[0], vj_[0]);
+            pair(lane + s + 1, false, vi_[1], vj_[1]);
+        }
+    }
+    F2 vi[3], vj[3];
+    const int home = own ? kOwnStart : 0;  // the sources' sums end this far from home, the odd steps' one lane further
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        vi[c] = vadd(vi_[0][c], vi_[1][c]);
+        vj[c] = vadd(F2{__shfl_sync(full, vj_[0][c].v, (lane - home) & 31)},
+                     F2{__shfl_sync(full, vj_[1][c].v, (lane - home - 1) & 31)});
     }
     auto lo = [](F2 a) { return unpack2(a).x; };
     auto hi = [](F2 a) { return unpack2(a).y; };
@@ -423,8 +476,7 @@ __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_sym3_kernel(SymP
     __shared__ Sym3Smem<WALL> sm[kThreads / 32];
     chain_wait();  // launched as a programmatic dependent of the packing launch
     if (p.gate && *p.gate == 0) return;
-    FreeSym k{};
-    if constexpr (!WALL) k = free_sym(p.a, p.inv_mu);
+    const FreeSym &k = p.k.t;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
     auto store = [&](int q, int slot, float4 v) { p.partial[static_cast<size_t>(q) * p.nb + slot] = v; };
@@ -540,6 +592,7 @@ struct SetReduceParams {
     float *out, *out_b;
     int n, n_seg, n6, nb;
     float self_t, self_r;  // unbounded: 1 / (6 pi mu a), 1 / (8 pi mu a^3)
+    double scale;          // of the partials
 };
 template <bool WALL>
 __global__ void __launch_bounds__(256) rpy_set_reduce_kernel(SetReduceParams p) {
@@ -575,6 +628,7 @@ __global__ void __launch_bounds__(256) rpy_set_reduce_kernel(SetReduceParams p) 
         for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
     }
     if (lane != 0) return;
+    for (int c = 0; c < 6; ++c) v[c] *= p.scale;
     const float4 f4 = p.f[i];
     float f[6] = {f4.x, f4.y, f4.z, 0.f, 0.f, 0.f}, vs[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (six) {
@@ -614,7 +668,9 @@ struct DirectParams {
     const float *xs, *fs, *xb, *fb;
     float *vs, *vb;
     int ns, n;
-    float a, inv_mu, self_t;
+    FreeSym k;
+    float self_t;
+    double scale;
 };
 template <bool WALL>
 __global__ void __launch_bounds__(256) rpy_direct_kernel(DirectParams p) {
@@ -624,8 +680,6 @@ __global__ void __launch_bounds__(256) rpy_direct_kernel(DirectParams p) {
     const int target = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes, i = min(target, p.n - 1);
     auto position = [&](int q) { return q < p.ns ? p.xs + 3 * q : p.xb + 3 * (q - p.ns); };
     auto force = [&](int q) { return q < p.ns ? p.fs + 6 * q : p.fb + 3 * (q - p.ns); };
-    FreeSym k{};
-    if constexpr (!WALL) k = free_sym(p.a, p.inv_mu);
     const float *xi = position(i);
     const float x = xi[0], y = xi[1], z = xi[2];
     float v[3] = {0.0f, 0.0f, 0.0f};
@@ -638,7 +692,7 @@ __global__ void __launch_bounds__(256) rpy_direct_kernel(DirectParams p) {
         if (j == i) continue;
         float drop[3] = {0.0f, 0.0f, 0.0f};
         if constexpr (WALL) wall_pair_sym<float>(x - px, y - py, z - pz, z, pz, wall_source(pz), f, none, v, drop);
-        else free_pair_sym<float>(x - px, y - py, z - pz, k, f, none, v, drop);
+        else free_pair_sym<float>(x - px, y - py, z - pz, p.k, f, none, v, drop);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -657,7 +711,7 @@ __global__ void __launch_bounds__(256) rpy_direct_kernel(DirectParams p) {
         for (int c = 0; c < 3; ++c) self[c] = p.self_t * f[c];
     float *o = i < p.ns ? p.vs + 6 * static_cast<size_t>(i) : p.vb + 3 * static_cast<size_t>(i - p.ns);
     for (int c = 0; c < 3; ++c)
-        o[c] = static_cast<float>((part[w][c] + part[w + 1][c]) + (part[w + 2][c] + part[w + 3][c]) + self[c]);
+        o[c] = static_cast<float>(((part[w][c] + part[w + 1][c]) + (part[w + 2][c] + part[w + 3][c])) * p.scale + self[c]);
     if (i < p.ns)
         for (int c = 3; c < 6; ++c) o[c] = 0.0f;
 }
@@ -871,8 +925,7 @@ int rpy_launch_tiles(const RpyBlockDesc &d, const RpyPlan &plan, float4 *scratch
         p.n = d.nt;
         p.nb = plan.nb;
         p.items = plan.items;
-        p.a = d.at;
-        p.inv_mu = 1.0f / d.mu;
+        p.k = d.wall ? FreeSym6{} : free_sym6(d.at, d.mu);
         p.gate = d.gate;
         p.t = d.ts;
         p.n6 = plan.n6;
@@ -924,8 +977,12 @@ int rpy_launch_reduce_f32(const RpyBlockDesc &d, const RpyPlan &plan, const floa
 
 int rpy_direct_product(int wall, const float *x_segs, const float *f_segs, const float *x_blobs, const float *f_blobs,
                        int n_seg, int n_blob, float a, float mu, float *v_segs, float *v_blobs, cudaStream_t st) {
-    DirectParams p{x_segs, f_segs, x_blobs, f_blobs, v_segs, v_blobs, n_seg, n_seg + n_blob, a, 1.0f / mu,
-                   static_cast<float>(1.0 / (6.0 * 3.14159265358979323846 * mu * a))};
+    DirectParams p{x_segs, f_segs, x_blobs, f_blobs, v_segs, v_blobs, n_seg, n_seg + n_blob};
+    if (!wall) {
+        p.k = free_sym(a);
+        p.self_t = static_cast<float>(1.0 / (6.0 * 3.14159265358979323846 * mu * a));
+    }
+    p.scale = kPairScale / (wall ? 1.0 : mu);
     if (p.n <= 0) return CF_OK;
     const int per_block = 256 / (32 * kDirectWarps), blocks = (p.n + per_block - 1) / per_block;
     if (wall) rpy_direct_kernel<true><<<blocks, 256, 0, st>>>(p);
@@ -1003,6 +1060,7 @@ int rpy_set_product(const RpySetDesc &s, float4 *scratch, size_t scratch_cap, fl
     const double pi = 3.14159265358979323846;
     p.self_t = static_cast<float>(1.0 / (6.0 * pi * s.mu * s.a));
     p.self_r = static_cast<float>(1.0 / (8.0 * pi * s.mu * s.a * s.a * s.a));
+    p.scale = n6 ? 1.0 : kPairScale / (s.wall ? 1.0 : s.mu);
     auto kern = s.wall ? rpy_set_reduce_kernel<true> : rpy_set_reduce_kernel<false>;
     CF_CUDA(launch_chained(kern, dim3((s.n + 7) / 8), dim3(256), 0, st, p));
     CF_CHECK_LAUNCH("rpy_set_reduce_kernel");

@@ -63,6 +63,10 @@ RpyPlan rpy_plan_capped(int nt, int ns, int vd, int fd, int num_sms, int max_nsp
 // 2 nb n6 + nb (i - n6).
 RpyPlan rpy_plan_sym(int n, int n6, int num_sms);
 
+// The partials of the force-only symmetric kernels are 8 pi (without a wall 8 pi mu) times the velocities; who sums them
+// applies this.
+constexpr double kPairScale = 1.0 / (8.0 * 3.14159265358979323846);
+
 // The full product of one particle set on itself through the symmetric kernel: segments [0, n_seg) (with torques and
 // spins when seg_dof is 6) followed by blobs, the wall or equal radii `a`.  Velocities into v_segs [6 n_seg] (spins zero
 // for seg_dof 3) and v_blobs [3 (n - n_seg)].

@@ -265,44 +265,46 @@ namespace cufil {
 //   b  =  w u (3/2 z_j + hz (u (2G + 5u) - 9P)) / 6 pi
 //   c  =  w u (3/2 z_j - 5 hz u^2) / 6 pi
 //   e  = -w u (3 z_j^2 + 3E + u (2 - 15E)) / 6 pi
-// The factor 1 / 6 pi is folded into the constants, and what depends on the source alone (WallSource) is formed once per
-// source, which leaves 81 FP32 instructions and two reciprocal square roots for both directions.  A product of 20,480
+// What is added to vi and vj is 8 pi times that: the free-space factors are then 1 and 2/3, the image's 4/3 of the above,
+// and no rounded constant scales the sum (kPairScale, rpy_kernels.cuh, is applied to it in FP64).  What depends on the source alone
+// (WallSource) is formed once per source, which leaves 81 FP32 instructions and two reciprocal square roots for both
+// directions.  A product of 20,480
 // segments: 994 us with the reference's factors (109 instructions, three roots and a division), 880 without the division,
 // both scalar; packed 695 with 86 instructions, 663 with 81.
 template <class T>
 struct WallSource {
-    T p, q;  // 3/2 z_j / 6 pi, -3 z_j^2 / 6 pi
+    T p, q;  // 2 z_j, -4 z_j^2
 };
 template <class T>
 __device__ __forceinline__ WallSource<T> wall_source(T zj) {
-    return {vmul(splat<T>(1.5f * RpyConst::inv6pi), zj), vmul(vmul(splat<T>(-3.0f * RpyConst::inv6pi), zj), zj)};
+    const T p = vadd(zj, zj);
+    return {p, vmul(vmul(splat<T>(-1.0f), p), p)};
 }
 template <class T>
 __device__ __forceinline__ void wall_pair_sym(T dx, T dy, T dz, T zi, T zj, WallSource<T> z, const T *fj, const T *fi,
                                               T *vi, T *vj) {
-    constexpr float c6 = RpyConst::inv6pi, c8 = RpyConst::inv8pi;
     auto k = [](float c) { return splat<T>(c); };
     const T q2 = vfma(dx, dx, vmul(dy, dy));
     // free space: A I + B d d^T (even in d)
     const T s = rsqrt_approx(vfma(dz, dz, q2));
     const T s2 = vmul(s, s);
-    const T A = vmul(s, vfma(k(2.0f / 3.0f * c8), s2, k(c8)));
-    const T B = vmul(vmul(s, s2), vfma(k(-2.0f * c8), s2, k(c8)));
-    // image system, every bracket over 6 pi
+    const T A = vmul(s, vfma(k(2.0f / 3.0f), s2, k(1.0f)));
+    const T B = vmul(vmul(s, s2), vfma(k(-2.0f), s2, k(1.0f)));
+    // image system, every bracket times 4/3
     const T hz = vadd(zi, zj);
     const T w = rsqrt_approx(vfma(hz, hz, q2));
     const T u = vmul(w, w), wu = vmul(w, u);
     const T hu = vmul(hz, u), E = vmul(hz, hu);
-    const T P = vmul(vmul(zi, z.p), u);                                    // 3/2 P
-    const T n5 = vfma(k(-7.5f * c6), E, k(1.5f * c6));                     // 3/2 (1 - 5E)
-    const T u5 = vmul(k(-5.0f * c6), u);                                   // -5 u
-    const T H = vfma(u5, vfma(k(-3.5f), E, k(0.5f)), n5);                  // -G
-    const T k0 = vfma(u, vfma(n5, vfma(u, k(1.0f / 3.0f), k(-0.2f)), k(-0.2f * c6)), vsub(k(-0.75f * c6), P));
+    const T P = vmul(vmul(zi, z.p), u);                    // 2 P
+    const T n5 = vfma(k(-10.0f), E, k(2.0f));              // 2 (1 - 5E)
+    const T u5 = vmul(k(-20.0f / 3.0f), u);                // -20/3 u
+    const T H = vfma(u5, vfma(k(-3.5f), E, k(0.5f)), n5);  // -4/3 G
+    const T k0 = vfma(u, vfma(n5, vfma(u, k(1.0f / 3.0f), k(-0.2f)), k(-4.0f / 15.0f)), vsub(k(-1.0f), P));
     const T AK = vfma(w, k0, A);
-    const T a = vmul(wu, vfma(u, H, vfma(k(3.0f), P, k(-0.75f * c6))));
+    const T a = vmul(wu, vfma(u, H, vfma(k(3.0f), P, k(-1.0f))));
     const T b = vmul(wu, vfma(vmul(k(-6.0f), P), hz, vfma(vmul(k(-1.0f), hu), vfma(k(2.0f), H, u5), z.p)));
     const T c = vmul(wu, vfma(u5, hu, z.p));
-    const T e = vmul(wu, vadd(z.q, vfma(E, vfma(k(15.0f * c6), u, k(-3.0f * c6)), vmul(k(-2.0f * c6), u))));
+    const T e = vmul(wu, vadd(z.q, vfma(E, vfma(k(20.0f), u, k(-4.0f)), vmul(k(-8.0f / 3.0f), u))));
     const T AKe = vadd(AK, e);
     // i <- j
     {
@@ -332,13 +334,13 @@ __device__ __forceinline__ void wall_pair_sym(T dx, T dy, T dz, T zi, T zj, Wall
 // same for i <- j and j <- i, so one evaluation serves both.  Branches as in free_pair_f32 with ai = aj = a (far;
 // overlapping, with dmin = 0; coincident: the self mobility); the far one needs a single reciprocal square root,
 // and the others are a rare branch on top of it.
-//   a2 = a^2, c8 = 1 / (8 pi mu), c6 = 1 / (6 pi mu a)
+// What is added to vi and vj is 8 pi mu times the velocity (1 / 8 pi mu is applied to the sum in FP64).
 struct FreeSym {
-    float a4, k, c8, c6, ia;  // (2a)^2, 2 a^2 / 3, 1 / (8 pi mu), 1 / (6 pi mu a), 1 / a
+    float a4, k, c6, ia;  // (2a)^2, 2 a^2 / 3, 4 / (3 a), 1 / a
 };
-__device__ __forceinline__ FreeSym free_sym(float a, float inv_mu) {
-    const float pi = 3.14159265358979f;
-    return FreeSym{4.0f * a * a, a * a * (2.0f / 3.0f), inv_mu / (8.0f * pi), inv_mu / (6.0f * pi * a), 1.0f / a};
+inline FreeSym free_sym(double a) {
+    return FreeSym{static_cast<float>(4.0 * a * a), static_cast<float>(2.0 * a * a / 3.0), static_cast<float>(4.0 / (3.0 * a)),
+                   static_cast<float>(1.0 / a)};
 }
 // One overlapping pair's A and B.
 __device__ __forceinline__ void free_overlap(const FreeSym &q, float r2, float s, float &A, float &B) {
@@ -367,9 +369,8 @@ __device__ __forceinline__ void free_pair_sym(T dx, T dy, T dz, const FreeSym &q
     const T r2 = vfma(dx, dx, vfma(dy, dy, vmul(dz, dz)));
     const T s = rsqrt_approx(r2);
     const T s2 = vmul(s, s);
-    const T g = vmul(k(q.c8), s);
-    T A = vmul(g, vfma(k(q.k), s2, k(1.0f)));
-    T B = vmul(vmul(g, s2), vfma(k(-3.0f * q.k), s2, k(1.0f)));
+    T A = vmul(s, vfma(k(q.k), s2, k(1.0f)));
+    T B = vmul(vmul(s, s2), vfma(k(-3.0f * q.k), s2, k(1.0f)));
     free_near(q, r2, s, A, B);
     const T tj = vmul(B, vfma(dx, fj[0], vfma(dy, fj[1], vmul(dz, fj[2]))));
     const T ti = vmul(B, vfma(dx, fi[0], vfma(dy, fi[1], vmul(dz, fi[2]))));

@@ -145,20 +145,23 @@ __device__ __forceinline__ void wall_pair_sym6_f32(float dx, float dy, float dz,
 // the rare branch.  j <- i: d changes sign.
 struct FreeSym6 {
     FreeSym t;
+    float c8, c6;                  // 1 / (8 pi mu), 1 / (6 pi mu a)
     float c0, c1, p0, p1, p3, q0;  // touching: C = c0 - c1 r, P = p0 - p1 r + p3 r^3, Q = q0 (6 a^2 / r - r)
     float a2;
 };
-__device__ __forceinline__ FreeSym6 free_sym6(float a, float inv_mu) {
-    const float pi = 3.14159265358979f, a2 = a * a, a3 = a2 * a, a4 = a2 * a2, a6 = a3 * a3;
+inline FreeSym6 free_sym6(double a, double mu) {
+    const double pm = 3.14159265358979323846 * mu, a3 = a * a * a, a4 = a3 * a, a6 = a3 * a3;
     FreeSym6 q;
-    q.t = free_sym(a, inv_mu);
-    q.c0 = inv_mu / (16.0f * pi * a3);
-    q.c1 = 3.0f * inv_mu / (128.0f * pi * a4);
-    q.p0 = inv_mu / (8.0f * pi * a3);
-    q.p1 = 54.0f * inv_mu / (512.0f * pi * a4);
-    q.p3 = 5.0f * inv_mu / (512.0f * pi * a6);
-    q.q0 = 3.0f * inv_mu / (512.0f * pi * a6);
-    q.a2 = a2;
+    q.t = free_sym(a);
+    q.c8 = static_cast<float>(1.0 / (8.0 * pm));
+    q.c6 = static_cast<float>(1.0 / (6.0 * pm * a));
+    q.c0 = static_cast<float>(1.0 / (16.0 * pm * a3));
+    q.c1 = static_cast<float>(3.0 / (128.0 * pm * a4));
+    q.p0 = static_cast<float>(1.0 / (8.0 * pm * a3));
+    q.p1 = static_cast<float>(54.0 / (512.0 * pm * a4));
+    q.p3 = static_cast<float>(5.0 / (512.0 * pm * a6));
+    q.q0 = static_cast<float>(3.0 / (512.0 * pm * a6));
+    q.a2 = static_cast<float>(a * a);
     return q;
 }
 template <bool SI, bool SJ>
@@ -167,7 +170,7 @@ __device__ __forceinline__ void free_pair_sym6_f32(float dx, float dy, float dz,
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     const float s = rsqrtf(r2);
     const float s2 = s * s;
-    const float g = k.t.c8 * s;
+    const float g = k.c8 * s;
     float A = g * fmaf(k.t.k, s2, 1.0f);
     float C = g * s2;
     float B = C * fmaf(-3.0f * k.t.k, s2, 1.0f);
@@ -175,8 +178,8 @@ __device__ __forceinline__ void free_pair_sym6_f32(float dx, float dy, float dz,
     if (r2 <= k.t.a4) {
         const bool apart = r2 > 0.0f;
         const float r = apart ? r2 * s : 0.0f;
-        A = k.t.c6 * fmaf(-9.0f / 32.0f * k.t.ia, r, 1.0f);
-        B = apart ? k.t.c6 * k.t.ia * (3.0f / 32.0f) * s : 0.0f;
+        A = k.c6 * fmaf(-9.0f / 32.0f * k.t.ia, r, 1.0f);
+        B = apart ? k.c6 * k.t.ia * (3.0f / 32.0f) * s : 0.0f;
         C = fmaf(-k.c1, r, k.c0);
         P = fmaf(k.p3 * r, r2, fmaf(-k.p1, r, k.p0));
         Q = apart ? k.q0 * fmaf(6.0f * k.a2, s, -r) : 0.0f;

@@ -699,6 +699,7 @@ __global__ void __launch_bounds__(32 * kEpiWarps) saddle_epilogue_kernel(SimDev 
     double u[3] = {0.0, 0.0, 0.0};
     for (int w = 0; w < kEpiWarps; ++w)
         for (int c = 0; c < 3; ++c) u[c] += red[w][c][lane];
+    for (double &x : u) x *= kPairScale;
     const ArrayInfo &a = d.arr[b];
     const int m = i / d.nseg;
     const int lm = m - a.fil0;

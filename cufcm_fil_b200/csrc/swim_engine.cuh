@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(256) swim_rows_kernel(SwimParams p, const int 
         o[1] += q.y;
         o[2] += q.z;
     }
-    for (int c = 0; c < 3; ++c) o[c] = warp_sum(o[c]);
+    for (int c = 0; c < 3; ++c) o[c] = kPairScale * warp_sum(o[c]);  // mu = 1
     if (lane != 0) return;
     double r[3];
     swim_diff(p, i, r);
