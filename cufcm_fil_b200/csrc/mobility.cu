@@ -166,8 +166,9 @@ bool overlap(const float *a, size_t na, const float *b, size_t nb) {
     return na > 0 && nb > 0 && std::less<const float *>()(a, b + nb) && std::less<const float *>()(b, a + na);
 }
 
-// The full product from the callers' layouts (device).  The direct kernel reads inputs while others are written, so
-// velocities that share memory with an input take the packed way.
+// The full product from the callers' layouts (device).  Either way the handle's records then hold the call's particles,
+// as after the single copy calls, for the evaluations that may follow.  The direct kernel reads inputs while others are
+// written, so velocities that share memory with an input take the packed way.
 int eval_full(cf_mobility *h, float *v_segs, float *v_blobs, cudaStream_t st);
 int apply_full(cf_mobility *h, const float *x_segs, const float *x_blobs, const float *f_segs, const float *f_blobs,
                float *v_segs, float *v_blobs, cudaStream_t st) {
@@ -181,7 +182,7 @@ int apply_full(cf_mobility *h, const float *x_segs, const float *x_blobs, const 
         !shared(v_blobs, 3 * nb))
         return rpy_direct_product(c.wall, x_segs, f_segs, x_blobs, f_blobs, c.n_seg, c.n_blob,
                                   static_cast<float>(c.n_seg ? c.seg_radius : c.blob_radius), static_cast<float>(c.mu),
-                                  v_segs, v_blobs, st);
+                                  v_segs, v_blobs, h->xs4, h->fs4, st);
     CF_TRY(pack_sets_to_float4(x_segs, f_segs, x_blobs, f_blobs, c.n_seg, c.n_blob, h->xs4, h->fs4, h->ts4, st));
     return eval_full(h, v_segs, v_blobs, st);
 }

@@ -667,6 +667,7 @@ constexpr int kDirectWarps = 4;  // the last sum below is written for four
 struct DirectParams {
     const float *xs, *fs, *xb, *fb;
     float *vs, *vb;
+    float4 *x4, *f4;  // the particles' records, written for the evaluations that follow on the handle
     int ns, n;
     FreeSym k;
     float self_t;
@@ -705,6 +706,8 @@ __global__ void __launch_bounds__(256) rpy_direct_kernel(DirectParams p) {
     if (rank != 0 || target >= p.n) return;
     const float *fi = force(i);
     const float f[3] = {fi[0], fi[1], fi[2]};
+    p.x4[i] = make_float4(x, y, z, 0.0f);
+    p.f4[i] = make_float4(f[0], f[1], f[2], 0.0f);
     float self[3] = {0.0f, 0.0f, 0.0f};
     if constexpr (WALL) wall_self_f32<3, 3>(z, f, self);
     else
@@ -976,8 +979,9 @@ int rpy_launch_reduce_f32(const RpyBlockDesc &d, const RpyPlan &plan, const floa
 }
 
 int rpy_direct_product(int wall, const float *x_segs, const float *f_segs, const float *x_blobs, const float *f_blobs,
-                       int n_seg, int n_blob, float a, float mu, float *v_segs, float *v_blobs, cudaStream_t st) {
-    DirectParams p{x_segs, f_segs, x_blobs, f_blobs, v_segs, v_blobs, n_seg, n_seg + n_blob};
+                       int n_seg, int n_blob, float a, float mu, float *v_segs, float *v_blobs, float4 *x, float4 *force,
+                       cudaStream_t st) {
+    DirectParams p{x_segs, f_segs, x_blobs, f_blobs, v_segs, v_blobs, x, force, n_seg, n_seg + n_blob};
     if (!wall) {
         p.k = free_sym(a);
         p.self_t = static_cast<float>(1.0 / (6.0 * 3.14159265358979323846 * mu * a));

@@ -129,9 +129,11 @@ unsigned rpy_wait_limit();
 
 // The full product of a small set of force-only particles (the wall, or equal radii) in one launch, straight from and to
 // the reference's layouts: segments x [3 n_seg], f [6 n_seg], v [6 n_seg] (spins zero), blobs x, f, v [3 n_blob].
+// It leaves the set's float4 records in x and force, as pack_sets_to_float4 does.
 constexpr int kRpyDirectMax = 1280;  // largest n_seg + n_blob (see rpy_kernels.cu)
 int rpy_direct_product(int wall, const float *x_segs, const float *f_segs, const float *x_blobs, const float *f_blobs,
-                       int n_seg, int n_blob, float a, float mu, float *v_segs, float *v_blobs, cudaStream_t st);
+                       int n_seg, int n_blob, float a, float mu, float *v_segs, float *v_blobs, float4 *x, float4 *force,
+                       cudaStream_t st);
 
 // Packing helpers between the reference's AoS host layouts and float4 arrays.
 int pack_xyz_to_float4(const float *aos3, float4 *out, int n, cudaStream_t st);
