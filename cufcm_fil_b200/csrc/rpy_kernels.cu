@@ -213,13 +213,18 @@ __device__ __forceinline__ void sym_item(long long t, int nb, int &I, int &J) {
     J = r + static_cast<int>(t - start(r));
 }
 
+// Where lanes without a particle hold an inert one: far outside any system, since a pair at distance zero above the
+// wall is NaN even without a force (at 1e5, as it was, a real particle could meet one).  Where the square of such a
+// distance overflows, its reciprocal root is zero and the pair adds zero too.
+constexpr float kFarAway = 1.0e18f;
+
 __device__ __forceinline__ void sym_load(const SymParams &p, int idx, int lane, float4 &x, float4 &f) {
     if (idx < p.n) {
         x = p.x[idx];
         f = p.f[idx];
     } else {
         // inert padding: far from everything (and from each other), zero force
-        x = make_float4(1.0e5f * static_cast<float>(lane + 1), 0.0f, 1.0e4f, 0.0f);
+        x = make_float4(kFarAway * static_cast<float>(lane + 1), 0.0f, 1.0e4f, 0.0f);
         f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
@@ -394,14 +399,14 @@ __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const f
             xv = x[idx];
             fv = f[idx];
         } else {  // inert: far from everything and from each other, no force
-            xv = make_float4(1.0e5f * static_cast<float>(lane + 1), apart, 1.0e4f, 0.0f);
+            xv = make_float4(kFarAway * static_cast<float>(lane + 1), apart, 1.0e4f, 0.0f);
             fv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
     float4 xi, fi4, xa, fa, xb, fb;
     load(i, 0.0f, xi, fi4);
-    load(ja, 1.0e5f, xa, fa);
-    load(jb, 2.0e5f, xb, fb);
+    load(ja, kFarAway, xa, fa);
+    load(jb, 2.0f * kFarAway, xb, fb);
     const ulonglong2 q0 = make_ulonglong2(pack2(xa.x, xb.x).v, pack2(xa.y, xb.y).v),
                      q1 = make_ulonglong2(pack2(xa.z, xb.z).v, pack2(fa.x, fb.x).v),
                      q2 = make_ulonglong2(pack2(fa.y, fb.y).v, pack2(fa.z, fb.z).v);
@@ -424,7 +429,7 @@ __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const f
         F2 sx{a.x}, fj[3] = {F2{b.y}, F2{c.x}, F2{c.y}};
         const F2 sy{a.y}, sz{b.x};
         if (self) {
-            sx = pack2(-1.0e5f * static_cast<float>(lane + 1), unpack2(sx).y);
+            sx = pack2(-kFarAway, unpack2(sx).y);
 #pragma unroll
             for (int q = 0; q < 3; ++q) fj[q] = pack2(0.0f, unpack2(fj[q]).y);
         }
