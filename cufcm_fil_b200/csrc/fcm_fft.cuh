@@ -32,14 +32,13 @@
 #include <cmath>
 #include <vector>
 
+#include "fcm_plan.cuh"
 #include "packed.cuh"
 
 namespace cufil {
 namespace fftk {
 
-constexpr int kMaxStages = 10;
 constexpr int kCols = 8;       // kx columns of a block: 64 bytes of each row
-constexpr int kMaxLen = 1024;  // y and z: three columns blocks of 1024 points fit the shared memory
 
 // One axis: length, radices (forward order), twiddles exp(-2 pi i k / n), frequency of each place.
 struct Axis {
@@ -660,21 +659,6 @@ inline Kernel pick_z(int n) {
     }
 }
 
-// Radices of n (forward order, largest first); empty when n has a prime factor above 5 or fewer than two stages.
-inline std::vector<int> radices(int n) {
-    std::vector<int> r;
-    for (int p : {8, 5, 4, 3, 2})
-        while (n % p == 0) {
-            r.push_back(p);
-            n /= p;
-        }
-    if (n != 1) return {};
-    if (r.size() == 1 && r[0] == 8) r = {4, 2};
-    else if (r.size() == 1 && r[0] == 4) r = {2, 2};
-    if (r.size() < 2 || static_cast<int>(r.size()) > kMaxStages) return {};
-    return r;
-}
-
 // Frequency of each place after the forward stages.
 inline std::vector<int> place_freq(int n, const std::vector<int> &r) {
     std::vector<int> f(n);
@@ -704,18 +688,6 @@ inline int x_fixed(int mx) { return mx == 64 || mx == 128 || mx == 256 || mx == 
 inline size_t x_smem(const Grid &g) { return sizeof(float2) * (padded(g.mx) + 1) * (kRowWarps << x_lines(x_fixed(g.mx))); }
 inline size_t y_smem(const Grid &g) { return sizeof(float2) * kCols * padded(g.ny) + (g.ny + 15) / 16 * 16; }
 inline size_t z_smem(const Grid &g) { return sizeof(ulonglong2) * kZPairs * 3 * padded(g.nz) + (g.nz + 15) / 16 * 16; }
-
-// Whether a grid takes this path: every axis factors into the radices, the blocks fit the shared memory, and the
-// three grids with their spectra (24 bytes a point) outgrow the L2 cache.  Below that the library's passes stay in the
-// cache (128^3: 186 us a solve here and 212 there with particles on a sphere in the middle, 198 and 185 with particles
-// everywhere), and its inverse transform is up to 1.6e-5 off FP64 there, by which results would move.  Above, us here
-// and there: 180^3 361 and 606 on a sphere, 531 and 567 everywhere; 200^3 387, 726 and 598, 689; 256^3 527, 939 and
-// 958, 930; 320^3 908, 2420 and 1877, 2427.
-constexpr long long kMinPoints = 5500000;
-inline bool supported(int nx, int ny, int nz) {
-    return static_cast<long long>(nx) * ny * nz >= kMinPoints && nx % 2 == 0 && nx <= 2 * kMaxLen && ny <= kMaxLen &&
-           nz <= kMaxLen && !radices(nx / 2).empty() && !radices(ny).empty() && !radices(nz).empty();
-}
 
 }  // namespace fftk
 }  // namespace cufil
