@@ -64,7 +64,8 @@ RpyPlan rpy_plan_capped(int nt, int ns, int vd, int fd, int num_sms, int max_nsp
 RpyPlan rpy_plan_sym(int n, int n6, int num_sms);
 
 // The partials of the force-only symmetric kernels are 8 pi (without a wall 8 pi mu) times the velocities; who sums them
-// applies this.
+// applies this.  Those with torques are velocities and spins, without a wall in lengths of a power of two near a radius far from 1
+// (rpy_set_product scales back); neither holds the self blocks.
 constexpr double kPairScale = 1.0 / (8.0 * 3.14159265358979323846);
 
 // The full product of one particle set on itself through the symmetric kernel: segments [0, n_seg) (with torques and

@@ -5,7 +5,7 @@
 // wall_pair_f32 / free_pair_f32 <6, 6> (rpy_pairs.cuh).
 //
 // With d = x_i - x_j, d' = (dx, dy, hz), hz = z_i + z_j, and the symmetric
-// coefficients of wall_pair_sym_f32 for velocities from forces:
+// coefficients of wall_pair_sym for velocities from forces:
 //   spin of i from the force F on j
 //     (tau_j F1 + Y dy, -tau_j F0 - Y dx, kappa (F0 dy - F1 dx)),  Y = (p_j - kappa) F2 - (d'.F) s_j
 //   velocity of i from the torque T on j, the transpose of j's spin from a force on i, with X = dx T1 - dy T0
@@ -141,7 +141,7 @@ __device__ __forceinline__ void wall_pair_sym6_f32(float dx, float dy, float dz,
 
 // Equal spheres of radius a without a wall:
 //   v_i = A F + B (d.F) d + C T x d,   w_i = C F x d + P T + Q (d.T) d,
-// far (r > 2a): A, B as free_pair_sym_f32, C = c8 / r^3, P = -C / 2, Q = 3 C / (2 r^2); touching spheres (Zuk et al.) in
+// far (r > 2a): A, B as free_pair_sym, C = c8 / r^3, P = -C / 2, Q = 3 C / (2 r^2); touching spheres (Zuk et al.) in
 // the rare branch.  j <- i: d changes sign.
 struct FreeSym6 {
     FreeSym t;

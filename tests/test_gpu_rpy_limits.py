@@ -1,5 +1,7 @@
 """Products of one set of equal particles at the limits of single precision: particles at the places of the inert ones
-that fill a tile.  Against the FP64 oracle; tolerance 1e-5 relative L2 (the mobility contract)."""
+that fill a tile, and spheres of a few nanometres in SI units, where fifth powers of a distance leave the range.
+Against the FP64 oracle; tolerance 1e-5 relative L2 (the mobility contract), velocities and spins apart where their
+units differ."""
 import numpy as np
 import pytest
 
@@ -31,5 +33,19 @@ def test_far_places_are_not_special(cuda, dof, n_seg, n_blob, wall):
         xs[320 + lane, 0] = -1e5 * (lane + 1)
     vs, vb, vs64, vb64 = product(xs, fs, xb, fb, wall=wall, seg_dof=dof)
     assert oracle.rel_l2(vs, vs64) <= TOL
+    if n_blob:
+        assert oracle.rel_l2(vb, vb64) <= TOL
+
+
+@pytest.mark.parametrize("a", [1e-9, 1e-8, 1e-6, 1.0, 1e4])
+@pytest.mark.parametrize("n_seg,n_blob", [(600, 0), (500, 70)])
+def test_sets_with_torques_in_other_units(cuda, n_seg, n_blob, a):
+    xs, fs, xb, fb = particles(n_seg, n_blob, 6, False, seed=9)
+    xs, xb = (xs * a).astype(np.float32), (xb * a).astype(np.float32)
+    fs[:, 3:] *= np.float32(a)  # torques in units of force times radius
+    kw = dict(wall=False, seg_dof=6, seg_radius=a, blob_radius=a, mu=1e-3)
+    vs, vb, vs64, vb64 = product(xs, fs, xb, fb, **kw)
+    assert oracle.rel_l2(vs[:, :3], vs64[:, :3]) <= TOL
+    assert oracle.rel_l2(vs[:, 3:], vs64[:, 3:]) <= TOL
     if n_blob:
         assert oracle.rel_l2(vb, vb64) <= TOL
