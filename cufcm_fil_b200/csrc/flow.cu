@@ -57,10 +57,11 @@ __device__ __forceinline__ float inv_sqrt(float x) {
 
 // One source at one flow point.  With d = x - x_s, p = dx fx + dy fy and R = (dx, dy, z + z_s), the terms are
 // gathered by vector so that the pair takes about 55 multiply-adds and two reciprocal square roots:
-//   direct   f / r + ((d.f) d + t x d) / r^3
+//   direct   (f + ((d.f) d + t x d) / r^2) / r
 //   image    -f / R - (R.f) R / R^3
 //            + 2 z_s / R^5 (z (3 a R - R^2 f*) + R^2 (p e_z + f_z (dx, dy, 0))),   f* = (fx, fy, -fz), a = R.f*
-// xs.w holds 2 z_s.
+// xs.w holds 2 z_s.  The direct terms form no cube of 1 / r: it leaves FP32 below r = 1.4e-13 (a flow point on a blob up
+// to the rounding of cos(pi / 2)) and above 4e12, where the velocity itself does not.
 template <bool SEG, bool WALL, bool NET>
 __device__ __forceinline__ void flow_pair(float xi, float yi, float zi, float z3, const float4 &xs, const float4 &f,
                                           const float4 &t, const float4 &xb, float &vx, float &vy, float &vz) {
@@ -68,20 +69,20 @@ __device__ __forceinline__ void flow_pair(float xi, float yi, float zi, float z3
     const float q2 = fmaf(dx, dx, dy * dy);
     const float p = fmaf(dx, f.x, dy * f.y);
     const float rm1 = inv_sqrt(fmaf(dz, dz, q2));
-    const float rm3 = rm1 * rm1 * rm1;
+    const float rm2 = rm1 * rm1;
     const float df = fmaf(dz, f.z, p);
     if constexpr (SEG) {  // with the rotlet of the segment torque
         const float cx = fmaf(t.y, dz, fmaf(-t.z, dy, df * dx));
         const float cy = fmaf(t.z, dx, fmaf(-t.x, dz, df * dy));
         const float cz = fmaf(t.x, dy, fmaf(-t.y, dx, df * dz));
-        vx = fmaf(rm3, cx, fmaf(rm1, f.x, vx));
-        vy = fmaf(rm3, cy, fmaf(rm1, f.y, vy));
-        vz = fmaf(rm3, cz, fmaf(rm1, f.z, vz));
+        vx = fmaf(rm1, fmaf(rm2, cx, f.x), vx);
+        vy = fmaf(rm1, fmaf(rm2, cy, f.y), vy);
+        vz = fmaf(rm1, fmaf(rm2, cz, f.z), vz);
     } else {
-        const float g = rm3 * df;
-        vx = fmaf(g, dx, fmaf(rm1, f.x, vx));
-        vy = fmaf(g, dy, fmaf(rm1, f.y, vy));
-        vz = fmaf(g, dz, fmaf(rm1, f.z, vz));
+        const float g = rm2 * df;
+        vx = fmaf(rm1, fmaf(g, dx, f.x), vx);
+        vy = fmaf(rm1, fmaf(g, dy, f.y), vy);
+        vz = fmaf(rm1, fmaf(g, dz, f.z), vz);
     }
     if constexpr (SEG && WALL) {  // Blake's image system (no blobs: half-space data)
         const float Rz = zi + xs.z;
@@ -101,10 +102,10 @@ __device__ __forceinline__ void flow_pair(float xi, float yi, float zi, float z3
     if constexpr (NET) {  // minus a Stokeslet of the same force at the source's body
         const float ex = xi - xb.x, ey = yi - xb.y, ez = zi - xb.z;
         const float qm1 = inv_sqrt(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
-        const float g = -(qm1 * qm1 * qm1) * fmaf(ex, f.x, fmaf(ey, f.y, ez * f.z));
-        vx = fmaf(g, ex, fmaf(-qm1, f.x, vx));
-        vy = fmaf(g, ey, fmaf(-qm1, f.y, vy));
-        vz = fmaf(g, ez, fmaf(-qm1, f.z, vz));
+        const float g = (qm1 * qm1) * fmaf(ex, f.x, fmaf(ey, f.y, ez * f.z));
+        vx = fmaf(-qm1, fmaf(g, ex, f.x), vx);
+        vy = fmaf(-qm1, fmaf(g, ey, f.y), vy);
+        vz = fmaf(-qm1, fmaf(g, ez, f.z), vz);
     }
 }
 
