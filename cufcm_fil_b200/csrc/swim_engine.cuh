@@ -808,12 +808,13 @@ __global__ void __launch_bounds__(256) swim_combine_kernel(const SwimCtl *ctl, d
 
 __global__ void swim_set_step_kernel(LoopCtl *lc, int nt) { lc->nt = nt; }
 
-// sol as ctl->apply says, and the rates that the next step advances with.
+// sol as ctl->apply says, and the rates that the next step advances with; both stay as they are where the body matrix
+// could not be inverted (no solve took place).
 __global__ void swim_finish_kernel(SwimParams p, const SwimCtl *ctl, const double *z, double *sol, int n,
                                    double *phase_dot, double *angle_dot) {
     chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || ctl->singular) return;
     const int a = ctl->apply;
     double v = sol[i];
     if (a == 1) v += z[i];
