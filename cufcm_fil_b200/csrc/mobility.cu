@@ -11,7 +11,6 @@
 #include <cstring>
 #include <functional>
 #include <new>
-#include <vector>
 
 using cufil::HostStage;
 
@@ -189,7 +188,9 @@ int apply_full(cf_mobility *h, const float *x_segs, const float *x_blobs, const 
 
 int eval_full(cf_mobility *h, float *v_segs, float *v_blobs, cudaStream_t st) {
     const cf_mobility_config &c = h->cfg;
-    if (c.n_seg > 0 && c.n_blob > 0 && one_set(c)) {  // the four blocks in one symmetric product
+    if (c.n_seg > 0 && c.n_blob > 0 && one_set(c) &&
+        rpy_plan_sym(c.n_seg + c.n_blob, set_n6(c), h->num_sms).scratch_float4 <= h->scratch_cap) {
+        // the four blocks in one symmetric product
         RpySetDesc d{c.wall, c.seg_dof, c.n_seg, c.n_seg + c.n_blob, h->xs4, h->fs4, h->ts4,
                      static_cast<float>(c.seg_radius), static_cast<float>(c.mu)};
         return rpy_set_product(d, h->scratch, h->scratch_cap, v_segs, v_blobs, h->num_sms, st);
@@ -247,17 +248,28 @@ extern "C" int cf_mobility_create(const cf_mobility_config *cfg, cf_mobility **o
         h->err = reinterpret_cast<int *>(h->v_blobs + 3 * nb);
         h->xb4 = h->xs4 + ns;
         h->fb4 = h->fs4 + ns;
-        // Partials buffer: the largest of the four block products' plans.
+        // Partials buffer: the largest of the products' plans.  Where the symmetric products' of sets with torques or of
+        // both kinds of particles do not fit the device's free memory, the tile kernel serves those.
         const int sd = cfg->seg_dof, n_s = cfg->n_seg, n_b = cfg->n_blob;
         const int n6 = set_n6(*cfg);
-        std::vector<RpyPlan> plans = {rpy_plan(n_s, n_s, sd, sd, h->num_sms), rpy_plan(n_s, n_b, sd, 3, h->num_sms),
-                                      rpy_plan(n_b, n_b, 3, 3, h->num_sms), rpy_plan(n_b, n_s, 3, sd, h->num_sms),
-                                      rpy_plan_sym(n_b, 0, h->num_sms)};
-        if (n6 == 0 || rpy_set_symmetric(n_s, n6)) plans.push_back(rpy_plan_sym(n_s, n6, h->num_sms));
-        if (n_s > 0 && n_b > 0 && one_set(*cfg)) plans.push_back(rpy_plan_sym(n_s + n_b, n6, h->num_sms));
-        h->scratch_cap = 1;
-        for (const RpyPlan &pl : plans) h->scratch_cap = std::max(h->scratch_cap, pl.scratch_float4);
-        if ((rc = dalloc(&h->scratch, h->scratch_cap))) break;
+        size_t blocks = 1, sets = 0;
+        auto need = [](size_t &cap, const RpyPlan &pl) { cap = std::max(cap, pl.scratch_float4); };
+        need(blocks, rpy_plan(n_s, n_s, sd, sd, h->num_sms));
+        need(blocks, rpy_plan(n_s, n_b, sd, 3, h->num_sms));
+        need(blocks, rpy_plan(n_b, n_b, 3, 3, h->num_sms));
+        need(blocks, rpy_plan(n_b, n_s, 3, sd, h->num_sms));
+        need(blocks, rpy_plan_sym(n_b, 0, h->num_sms));
+        if (n6 == 0) need(blocks, rpy_plan_sym(n_s, 0, h->num_sms));
+        else if (rpy_set_symmetric(n_s, n6)) need(sets, rpy_plan_sym(n_s, n6, h->num_sms));
+        if (n_s > 0 && n_b > 0 && one_set(*cfg)) need(sets, rpy_plan_sym(n_s + n_b, n6, h->num_sms));
+        h->scratch_cap = std::max(blocks, sets);
+        rc = dalloc(&h->scratch, h->scratch_cap);
+        if (rc == CF_ENOMEM && sets > blocks) {
+            cudaGetLastError();
+            h->scratch_cap = blocks;
+            rc = dalloc(&h->scratch, h->scratch_cap);
+        }
+        if (rc) break;
         if ((rc = cuda_status(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream), "cudaMemsetAsync", __FILE__,
                               __LINE__)))
             break;

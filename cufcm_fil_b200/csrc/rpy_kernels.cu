@@ -1102,6 +1102,7 @@ int rpy_block_product(const RpyBlockDesc &d, float4 *scratch, size_t scratch_cap
                       int stride, int mode, int num_sms, cudaStream_t st) {
     if (d.nt <= 0) return CF_OK;
     RpyPlan plan = rpy_plan_for(d, num_sms);
+    if (plan.sym && plan.scratch_float4 > scratch_cap) plan = rpy_plan(d.nt, d.ns, d.vd, d.fd, num_sms);
     if (plan.scratch_float4 > scratch_cap)
         return set_error(CF_EINVAL, "rpy: scratch too small (%zu < %zu float4)", scratch_cap, plan.scratch_float4);
     if (plan.sym && mode == kOutWrite && (stride == 6 || (stride == 3 && d.vd == 3))) {
