@@ -3,7 +3,6 @@
 #pragma once
 
 #include <cuda_runtime.h>
-#include <cstring>
 #include <cstdio>
 #include <cstdarg>
 #include <cstdlib>
@@ -60,51 +59,6 @@ inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     cfg.numAttrs = chained_launches() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
-
-// Device buffer behind a host entry point and, up to kPinnedMax, a page-locked host buffer of the same layout: the
-// call's arrays are gathered into one copy each way.  (A copy from the caller's pageable memory is staged by CUDA, array
-// by array: a swimmer's product of 3,180 segments and its blobs took 200 us so, 138 this way, a flow field of 16,000
-// points 291 and 256.)  Above the limit the copy itself is what costs and page-locking would slow the handle's
-// creation, so the arrays are copied as they are.  Offsets and sizes in bytes.
-struct HostStage {
-    static constexpr size_t kPinnedMax = size_t{4} << 20;
-    char *host = nullptr, *dev = nullptr;
-    int alloc(size_t bytes) {
-        bytes = bytes > 0 ? bytes : 1;
-        cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&dev), bytes);
-        if (e == cudaSuccess && bytes <= kPinnedMax) e = cudaMallocHost(reinterpret_cast<void **>(&host), bytes);
-        return cuda_status(e, "staging buffers", __FILE__, __LINE__);
-    }
-    void release() {
-        if (host) cudaFreeHost(host);
-        if (dev) cudaFree(dev);
-        host = dev = nullptr;
-    }
-    template <typename T>
-    T *at(size_t off) const { return reinterpret_cast<T *>(dev + off); }
-    // put() the inputs, then up() their whole range; after the work, down() the results' range, synchronize, take().
-    cudaError_t put(size_t off, const void *src, size_t bytes, cudaStream_t st) const {
-        if (!bytes) return cudaSuccess;
-        if (!host) return cudaMemcpyAsync(dev + off, src, bytes, cudaMemcpyHostToDevice, st);
-        std::memcpy(host + off, src, bytes);
-        return cudaSuccess;
-    }
-    cudaError_t up(size_t bytes, cudaStream_t st) const {
-        return host && bytes ? cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
-    }
-    cudaError_t down(size_t off, size_t bytes, cudaStream_t st) const {
-        return host && bytes ? cudaMemcpyAsync(host + off, dev + off, bytes, cudaMemcpyDeviceToHost, st) : cudaSuccess;
-    }
-    cudaError_t take(void *dst, size_t off, size_t bytes, cudaStream_t st) const {
-        if (!bytes) return cudaSuccess;
-        if (host) {
-            std::memcpy(dst, host + off, bytes);
-            return cudaSuccess;
-        }
-        cudaError_t e = cudaMemcpyAsync(dst, dev + off, bytes, cudaMemcpyDeviceToHost, st);
-        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
-    }
-};
 
 }  // namespace cufil
 

@@ -19,6 +19,7 @@
 // results scattered straight back to input order instead of a second sort.
 #include "common.cuh"
 #include "fcm_fft.cuh"
+#include "host_stage.cuh"
 
 #include <cub/cub.cuh>
 #include <cufft.h>
@@ -585,6 +586,7 @@ int fcm_run(cf_fcm *h, const float *dY, const float *dF, float *dV, cudaStream_t
 // The pipeline on host positions and forces [3N].
 int fcm_host(cf_fcm *h, const float *Y, const float *F, float *V) {
     const size_t b = sizeof(float) * 3 * static_cast<size_t>(h->N);
+    h->stage.open();
     CF_CUDA(h->stage.put(0, Y, b, h->stream));
     CF_CUDA(h->stage.put(b, F, b, h->stream));
     CF_CUDA(h->stage.up(2 * b, h->stream));
@@ -652,8 +654,8 @@ extern "C" int cf_fcm_create(const cf_fcm_config *cfg, cf_fcm **out) {
                               "cudaDeviceGetAttribute", __FILE__, __LINE__)))
             break;
         if ((rc = falloc(&h->grid, 3 * h->grid_size)) || (rc = falloc(&h->x4, N)) || (rc = falloc(&h->xs, N)) || (rc = falloc(&h->fs, N)) ||
-            (rc = h->stage.alloc(9 * N * sizeof(float))) || (rc = falloc(&h->vgs, N)) || (rc = falloc(&h->keys, N)) ||
-            (rc = falloc(&h->keys_sorted, N)) ||
+            (rc = cuda_status(h->stage.alloc(9 * N * sizeof(float)), "staging buffer", __FILE__, __LINE__)) ||
+            (rc = falloc(&h->vgs, N)) || (rc = falloc(&h->keys, N)) || (rc = falloc(&h->keys_sorted, N)) ||
             (rc = falloc(&h->vals, N)) || (rc = falloc(&h->perm, N)) || (rc = falloc(&h->cell_start, h->ncell)) ||
             (rc = falloc(&h->cell_end, h->ncell)))
             break;

@@ -16,9 +16,9 @@
 // SM, FP32 sums of one tile under a TwoSum accumulation, and an FP64 reduction
 // of the split partials in a fixed order (deterministic, no atomics).
 #include "common.cuh"
+#include "host_stage.cuh"
 
 #include <algorithm>
-#include <cstring>
 #include <new>
 
 struct cf_flow {
@@ -369,10 +369,11 @@ extern "C" int cf_flow_create(const cf_flow_config *cfg, cf_flow **out) {
                          2 * static_cast<size_t>(cfg->max_flow);
         if ((rc = falloc(&h->sx, nsrc)) || (rc = falloc(&h->sf, nsrc)) || (rc = falloc(&h->st, nsrc)) ||
             (rc = falloc(&h->sb, nsrc)) || (rc = falloc(&h->partial, h->partial_cap)) ||
-            (rc = h->stage.alloc(sizeof(float) * (6 * static_cast<size_t>(cfg->max_flow) +
-                                                  9 * static_cast<size_t>(cfg->max_seg) +
-                                                  6 * static_cast<size_t>(cfg->max_blob) +
-                                                  3 * static_cast<size_t>(cfg->max_bodies)))))
+            (rc = cuda_status(h->stage.alloc(sizeof(float) * (6 * static_cast<size_t>(cfg->max_flow) +
+                                                              9 * static_cast<size_t>(cfg->max_seg) +
+                                                              6 * static_cast<size_t>(cfg->max_blob) +
+                                                              3 * static_cast<size_t>(cfg->max_bodies))),
+                              "staging buffer", __FILE__, __LINE__)))
             break;
     } while (0);
     if (rc != CF_OK) {
@@ -413,6 +414,7 @@ extern "C" int cf_flow_velocities(cf_flow *h, const float *x_flow, int n_flow, c
     const int bodies = std::max(n_seg ? n_seg / n_seg_per_body : 0, n_blob ? n_blob / n_blob_per_body : 0);
     const size_t nf3 = 3 * static_cast<size_t>(n_flow), ns3 = 3 * static_cast<size_t>(n_seg),
                  nb3 = 3 * static_cast<size_t>(n_blob), nd3 = x_bodies ? 3 * static_cast<size_t>(bodies) : 0;
+    h->stage.open();
     size_t at = 0;  // bytes
     cudaError_t e = cudaSuccess;
     auto put = [&](const float *src, size_t count) {

@@ -19,6 +19,7 @@
 // attaches) run on the fused kernels of mlp_fused.cuh instead: the same
 // products of the same BF16 operands, one launch forward, three for a gradient.
 #include "common.cuh"
+#include "host_stage.cuh"
 #include "mlp_fused.cuh"
 #include "tc_tf32.cuh"
 
@@ -241,7 +242,7 @@ struct cf_mlp {
     __nv_bfloat16 *xt = nullptr, *a1t = nullptr, *a2t = nullptr, *dyt = nullptr, *dz2t = nullptr, *dz1t = nullptr;
     float *gpart = nullptr, *db = nullptr;
     int max_tiles = 0;
-    float *h_grads = nullptr;  // pinned: gradients, then the loss partials
+    cufil::PinnedBuffer pinned;  // the gradients on their way to the caller
     cudaStream_t stream = nullptr;
     std::vector<void *> allocations;
 };
@@ -290,7 +291,6 @@ int alloc_fused(cf_mlp *h) {
     CF_TRY(mlp_alloc(h, &h->gpart, static_cast<size_t>(grad_splits(h->max_tiles)) * h->nparam));
     CF_TRY(mlp_alloc(h, &h->db, static_cast<size_t>(h->max_tiles) * (2 * hidP + outP)));
     CF_TRY(mlp_alloc(h, &h->partial, h->max_tiles));
-    CF_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h->h_grads), h->nparam * sizeof(float) + 8));
     CF_CUDA(cudaFuncSetAttribute(mlpk::mlp_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(mlpk::kRowsSmem)));
     CF_CUDA(cudaFuncSetAttribute(mlpk::mlp_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -524,7 +524,6 @@ extern "C" int cf_mlp_create(int in_dim, int hidden, int out_dim, int max_batch,
     if (rc != CF_OK) {
         std::string msg = cf_last_error();
         for (void *q : h->allocations) cudaFree(q);
-        if (h->h_grads) cudaFreeHost(h->h_grads);
         if (h->stream) cudaStreamDestroy(h->stream);
         delete h;
         return set_error(rc, "%s", msg.c_str());
@@ -538,7 +537,7 @@ extern "C" int cf_mlp_destroy(cf_mlp *h) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (void *q : h->allocations) cudaFree(q);
-    if (h->h_grads) cudaFreeHost(h->h_grads);
+    h->pinned.release();
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return CF_OK;
@@ -562,11 +561,12 @@ extern "C" int cf_mlp_gradients(cf_mlp *h, const float *x, const float *t, int n
     double l = 0.0;
     if (h->fused) {
         CF_TRY(fused_gradients(h, x, t, n, nullptr));
-        if (grads)
-            CF_CUDA(cudaMemcpyAsync(h->h_grads, h->grads, sizeof(float) * h->nparam, cudaMemcpyDeviceToHost, h->stream));
+        const size_t bytes = sizeof(float) * h->nparam;
+        void *via = grads ? h->pinned.open(bytes) : nullptr;
+        if (grads) CF_CUDA(cudaMemcpyAsync(via ? via : grads, h->grads, bytes, cudaMemcpyDeviceToHost, h->stream));
         CF_TRY(fused_loss(h, n, &l));  // waits for the stream
         if (loss) *loss = l;
-        if (grads) std::memcpy(grads, h->h_grads, sizeof(float) * h->nparam);
+        if (via) std::memcpy(grads, via, bytes);
         return CF_OK;
     }
     CF_TRY(backward(h, x, t, n, &l));

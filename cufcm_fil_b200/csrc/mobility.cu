@@ -5,10 +5,10 @@
 // but one device, one stream per handle, no device-wide synchronisation, and
 // float4 particle records repacked once per copy.
 #include "common.cuh"
+#include "host_stage.cuh"
 #include "rpy_kernels.cuh"
 
 #include <algorithm>
-#include <cstring>
 #include <functional>
 #include <new>
 
@@ -236,8 +236,8 @@ extern "C" int cf_mobility_create(const cf_mobility_config *cfg, cf_mobility **o
         const size_t ns = cfg->n_seg, nb = cfg->n_blob;
         h->in_bytes = sizeof(float) * (9 * ns + 6 * nb);
         h->out_bytes = sizeof(float) * (6 * ns + 3 * nb) + sizeof(int);
-        if ((rc = h->stage.alloc(h->in_bytes + h->out_bytes)) || (rc = dalloc(&h->xs4, ns + nb)) ||
-            (rc = dalloc(&h->fs4, ns + nb)) || (rc = dalloc(&h->ts4, ns)))
+        if ((rc = cuda_status(h->stage.alloc(h->in_bytes + h->out_bytes), "staging buffer", __FILE__, __LINE__)) ||
+            (rc = dalloc(&h->xs4, ns + nb)) || (rc = dalloc(&h->fs4, ns + nb)) || (rc = dalloc(&h->ts4, ns)))
             break;
         h->x_segs = h->stage.at<float>(0);
         h->f_segs = h->x_segs + 3 * ns;
@@ -410,8 +410,9 @@ extern "C" int cf_apply_mobility(cf_mobility *h, const float *x_segs, const floa
     CF_REQUIRE(!ns || (x_segs && f_segs && v_segs), "cf_apply_mobility: null segment argument");
     CF_REQUIRE(!nb || (x_blobs && f_blobs && v_blobs), "cf_apply_mobility: null blob argument");
     CF_CUDA(cudaSetDevice(h->cfg.device));
-    const HostStage &sg = h->stage;
+    HostStage &sg = h->stage;
     const cudaStream_t st = h->stream;
+    sg.open();
     CF_CUDA(sg.put(0, x_segs, 12 * ns, st));
     CF_CUDA(sg.put(12 * ns, f_segs, 24 * ns, st));
     CF_CUDA(sg.put(36 * ns, x_blobs, 12 * nb, st));
