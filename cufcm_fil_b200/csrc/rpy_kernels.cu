@@ -982,6 +982,7 @@ int rpy_prepare(const RpyBlockDesc &d, const RpyPlan &plan) {
 
 int rpy_launch_reduce_f32(const RpyBlockDesc &d, const RpyPlan &plan, const float4 *scratch, float *out_f,
                           int stride, int mode, cudaStream_t st, const int *dev_err) {
+    if (plan.sym) return set_error(CF_EINVAL, "rpy: a symmetric plan's partials are not a block's");
     if (d.nt <= 0) return CF_OK;
     ReduceParams p;
     p.partial = scratch;

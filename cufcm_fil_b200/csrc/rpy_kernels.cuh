@@ -120,7 +120,9 @@ enum RpyOut : int { kOutWrite = 0, kOutAdd = 1 };
 // vd..stride-1 are zeroed in write mode (the reference writes all six
 // entries of a segment velocity, cuda_functions.cu:460-469).
 // With dev_err given, every output of the launch is a quiet NaN when that
-// word is non-zero (a tile block gave up waiting for its sources).
+// word is non-zero (a tile block gave up waiting for its sources).  A symmetric
+// plan is refused: its partials have other factors and lack the self blocks
+// (kPairScale); rpy_set_product sums them, or a kernel of the caller's.
 int rpy_launch_reduce_f32(const RpyBlockDesc &d, const RpyPlan &plan, const float4 *scratch, float *out_f,
                           int stride, int mode, cudaStream_t st, const int *dev_err = nullptr);
 
