@@ -5,7 +5,7 @@
 // each operand pair.  The FP32 pipe is no faster for them (70.6 TFLOP/s either
 // way on independent fma chains), but a kernel that is held up by issue or by
 // register reads gains: the pair product of rpy_pairs.cuh 3.59 -> 2.81 ms per
-// 10^9 pairs.  Code for both is written once, over a real type T = float or F2.
+// 10^9 pairs.  Code for both is written once, over a real type T = float, F1 or F2.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -49,8 +49,21 @@ __device__ __forceinline__ float vadd(float a, float b) { return a + b; }
 __device__ __forceinline__ float vsub(float a, float b) { return a - b; }
 __device__ __forceinline__ float vmul(float a, float b) { return a * b; }
 __device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
+// One value, rounded after every operation as each half of F2 is (a plain float may be contracted).  Products that are
+// added are written as vfma: the compiler contracts packed ones that are not.
+struct F1 {
+    float v;
+};
+__device__ __forceinline__ F1 vadd(F1 a, F1 b) { return {__fadd_rn(a.v, b.v)}; }
+__device__ __forceinline__ F1 vsub(F1 a, F1 b) { return {__fsub_rn(a.v, b.v)}; }
+__device__ __forceinline__ F1 vmul(F1 a, F1 b) { return {__fmul_rn(a.v, b.v)}; }
+__device__ __forceinline__ F1 vfma(F1 a, F1 b, F1 c) { return {__fmaf_rn(a.v, b.v, c.v)}; }
 template <class T>
 __device__ __forceinline__ T splat(float c);
+template <>
+__device__ __forceinline__ F1 splat<F1>(float c) {
+    return {c};
+}
 template <>
 __device__ __forceinline__ float splat<float>(float c) {
     return c;
@@ -60,6 +73,7 @@ __device__ __forceinline__ F2 splat<F2>(float c) {
     return pack2(c, c);
 }
 __device__ __forceinline__ float rsqrt_approx(float a) { return rsqrtf(a); }
+__device__ __forceinline__ F1 rsqrt_approx(F1 a) { return {rsqrtf(a.v)}; }
 __device__ __forceinline__ F2 rsqrt_approx(F2 a) {
     const float2 v = unpack2(a);
     return pack2(rsqrtf(v.x), rsqrtf(v.y));

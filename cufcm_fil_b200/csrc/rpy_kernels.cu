@@ -493,9 +493,82 @@ __device__ __forceinline__ void sym3_tiles(const float4 *__restrict__ x, const f
     if (jb < n) store(jb, I, make_float4(hi(vj[0]), hi(vj[1]), hi(vj[2]), 0.0f));
 }
 
-template <bool WALL>
+// The same sums from one source a lane: a warp takes the tiles I <= J alone, the sources and their accumulators rotate by
+// shuffles.  Every operation and every order of summation is that of sym3_tiles, so the partials are the same bit for bit
+// (an array's step does not depend on what else is in its batch); for launches too small to fill the SMs, where the
+// latency of a unit's chain is what counts.
+template <bool WALL, class Store>
+__device__ __forceinline__ void sym1_tiles(const float4 *__restrict__ x, const float4 *__restrict__ f, int n,
+                                           const FreeSym &k, int I, int J, int lane, Store store) {
+    const unsigned full = 0xffffffffu;
+    const int i = I * 32 + lane, j = J * 32 + lane;
+    auto load = [&](int idx, float apart, float4 &xv, float4 &fv) {
+        if (idx < n) {
+            xv = x[idx];
+            fv = f[idx];
+        } else {
+            xv = make_float4(kFarAway * static_cast<float>(lane + 1), apart, 1.0e4f, 0.0f);
+            fv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    float4 xi, fi4, xs, fs;
+    load(i, 0.0f, xi, fi4);
+    load(j, kFarAway, xs, fs);
+    const bool near = I >> 1 == J >> 1;  // the units K = I / 2: they start at kOwnStart
+    const int start = near ? kOwnStart : 0;
+    const F1 tx{xi.x}, ty{xi.y}, tz{xi.z}, fi[3] = {{fi4.x}, {fi4.y}, {fi4.z}};
+    auto from = [&](float &v, int by) { v = __shfl_sync(full, v, (lane + by) & 31); };
+    auto rotate = [&](int by) {
+        from(xs.x, by);
+        from(xs.y, by);
+        from(xs.z, by);
+        from(fs.x, by);
+        from(fs.y, by);
+        from(fs.z, by);
+    };
+    F1 vi_[2][3] = {}, vj_[2][3] = {};
+    auto pair = [&](F1 *vi, F1 *vj) {
+        const F1 sx{xs.x}, sy{xs.y}, sz{xs.z}, fj[3] = {{fs.x}, {fs.y}, {fs.z}};
+        const F1 dx = vsub(tx, sx), dy = vsub(ty, sy), dz = vsub(tz, sz);
+        if constexpr (WALL) wall_pair_sym<F1>(dx, dy, dz, tz, sz, wall_source(sz), fj, fi, vi, vj);
+        else free_pair_sym<F1>(dx, dy, dz, k, fj, fi, vi, vj);
+        rotate(1);
+    };
+    auto both = [&](F1 *vi, F1 *vj) {
+        pair(vi, vj);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) from(vj[c].v, 2);
+    };
+    if (near) rotate(kOwnStart);
+    if (I != J) {
+#pragma unroll 2
+        for (int t = 0; t < 32; t += 2) {
+            both(vi_[0], vj_[0]);
+            both(vi_[1], vj_[1]);
+        }
+    } else {
+#pragma unroll 1
+        for (int t = kOwnStart; t < kOwnStart + 32; t += 2) {
+            F1 drop[3] = {};
+            if (t != 32) pair(vi_[0], drop);  // not with itself
+            else rotate(1);
+            pair(vi_[1], drop);
+        }
+    }
+    F1 vi[3], vj[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        vi[c] = vadd(vi_[0][c], vi_[1][c]);
+        vj[c] = vadd(F1{__shfl_sync(full, vj_[0][c].v, (lane - start) & 31)},
+                     F1{__shfl_sync(full, vj_[1][c].v, (lane - start - 1) & 31)});
+    }
+    if (i < n) store(i, J, make_float4(vi[0].v, vi[1].v, vi[2].v, 0.0f));
+    if (j < n && I != J) store(j, I, make_float4(vj[0].v, vj[1].v, vj[2].v, 0.0f));
+}
+
+template <bool WALL, bool PACKED>
 __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_sym3_kernel(SymParams p) {
-    __shared__ Sym3Smem<WALL> sm[kThreads / 32];
+    __shared__ Sym3Smem<WALL> sm[PACKED ? kThreads / 32 : 1];
     chain_wait();  // launched as a programmatic dependent of the packing launch
     if (p.gate && *p.gate == 0) return;
     const FreeSym &k = p.k.t;
@@ -504,8 +577,13 @@ __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_sym3_kernel(SymP
     auto store = [&](int q, int slot, float4 v) { p.partial[static_cast<size_t>(q) * p.nb + slot] = v; };
     for (long long t = static_cast<long long>(blockIdx.x) * (kThreads / 32) + w; t < p.items; t += nwarps) {
         int I, K;
-        sym3_unit(t, p.nb, I, K);
-        sym3_tiles<WALL>(p.x, p.f, p.n, p.nb, k, I, K, lane, sm[w], store);
+        if constexpr (PACKED) {
+            sym3_unit(t, p.nb, I, K);
+            sym3_tiles<WALL>(p.x, p.f, p.n, p.nb, k, I, K, lane, sm[w], store);
+        } else {
+            sym_item(t, p.nb, I, K);
+            sym1_tiles<WALL>(p.x, p.f, p.n, k, I, K, lane, store);
+        }
     }
 }
 
@@ -517,8 +595,9 @@ __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_sym3_kernel(SymP
 // stored slot-major per array, partial[poff + slot * n + i] (slot = the other
 // tile of the pair), so that both these writes and the per-segment reduction
 // that reads them are coalesced.
+template <bool PACKED>
 __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_wall_sym_batch_kernel(SymBatchParams p) {
-    __shared__ Sym3Smem<true> sm[kThreads / 32];
+    __shared__ Sym3Smem<true> sm[PACKED ? kThreads / 32 : 1];
     chain_wait();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long nwarps = static_cast<long long>(gridDim.x) * (kThreads / 32);
@@ -532,11 +611,17 @@ __global__ void __launch_bounds__(kThreads, kSym3CtasPerSm) rpy_wall_sym_batch_k
         const int b = lo;
         if (p.active && !p.active[b]) continue;
         const int n = p.n[b], nb = p.nb[b];
+        const float4 *x = p.x + p.seg0[b], *f = p.f + p.seg0[b];
         float4 *partial = p.partial + p.poff[b];
         auto store = [&](int q, int slot, float4 v) { partial[static_cast<size_t>(slot) * n + q] = v; };
         int I, K;
-        sym3_unit(t - p.item0[b], nb, I, K);
-        sym3_tiles<true>(p.x + p.seg0[b], p.f + p.seg0[b], n, nb, FreeSym{}, I, K, lane, sm[w], store);
+        if constexpr (PACKED) {
+            sym3_unit(t - p.item0[b], nb, I, K);
+            sym3_tiles<true>(x, f, n, nb, FreeSym{}, I, K, lane, sm[w], store);
+        } else {
+            sym_item(t - p.item0[b], nb, I, K);
+            sym1_tiles<true>(x, f, n, FreeSym{}, I, K, lane, store);
+        }
     }
 }
 
@@ -859,7 +944,8 @@ RpyPlan rpy_plan_sym(int n, int n6, int num_sms) {
     pl.ti = 1;
     const int nb = std::max(1, (n + 31) / 32);
     pl.nb = nb;
-    pl.items = n6 > 0 ? static_cast<long long>(nb) * (nb + 1) / 2 : rpy_sym_items(nb);
+    pl.packed = n6 == 0 && rpy_sym_packed(rpy_sym_items(nb, false), num_sms);
+    pl.items = rpy_sym_items(nb, pl.packed);
     const int per_sm = n6 > 0 ? kSym6CtasPerSm : kSym3CtasPerSm;
     const long long max_warps = static_cast<long long>(std::max(1, num_sms)) * per_sm * (kThreads / 32);
     const long long per_warp = (pl.items + max_warps - 1) / max_warps;  // balanced: every warp does per_warp items
@@ -956,8 +1042,10 @@ int rpy_launch_tiles(const RpyBlockDesc &d, const RpyPlan &plan, float4 *scratch
         p.gate = d.gate;
         p.t = d.ts;
         p.n6 = plan.n6;
-        auto kern = d.wall ? (plan.n6 ? rpy_sym6_kernel<true> : rpy_sym3_kernel<true>)
-                           : (plan.n6 ? rpy_sym6_kernel<false> : rpy_sym3_kernel<false>);
+        auto kern = d.wall ? (plan.n6 ? rpy_sym6_kernel<true>
+                                      : plan.packed ? rpy_sym3_kernel<true, true> : rpy_sym3_kernel<true, false>)
+                           : (plan.n6 ? rpy_sym6_kernel<false>
+                                      : plan.packed ? rpy_sym3_kernel<false, true> : rpy_sym3_kernel<false, false>);
         if (unit != 1.0) kern = rpy_sym6_kernel<false, true>;
         CF_CUDA(launch_chained(kern, dim3(plan.grid), dim3(kThreads), 0, st, p));
         CF_CHECK_LAUNCH("rpy_sym kernel");
@@ -1144,7 +1232,8 @@ namespace cufil {
 
 int rpy_launch_sym_batch(const SymBatchParams &p, int grid, cudaStream_t st) {
     if (p.items <= 0) return CF_OK;
-    CF_CUDA(launch_chained(rpy_wall_sym_batch_kernel, dim3(grid), dim3(kThreads), 0, st, p));
+    auto kern = p.packed ? rpy_wall_sym_batch_kernel<true> : rpy_wall_sym_batch_kernel<false>;
+    CF_CUDA(launch_chained(kern, dim3(grid), dim3(kThreads), 0, st, p));
     return CF_OK;
 }
 

@@ -40,7 +40,8 @@ struct RpyPlan {
     int sym;       // 1: symmetric warp-tile kernel (a set on itself)
     int n6;        // symmetric: the first n6 particles have torques and spins
     int nb;        // symmetric: 32-particle tiles
-    long long items;  // symmetric: tile pairs of the upper triangle
+    bool packed;      // symmetric: what the items are (rpy_sym_items); false with torques
+    long long items;  // symmetric: work items
     int grid;      // symmetric: CTAs
     int ti;        // targets per thread
     int tiles;     // target tiles (gridDim.x)
@@ -94,7 +95,7 @@ int rpy_launch_tiles(const RpyBlockDesc &d, const RpyPlan &plan, float4 *scratch
 // Batched symmetric wall products (segments on segments, 3x3) of B independent
 // particle sets stored back to back.  Per array b: particles [seg0[b], seg0[b]+n[b])
 // of x/f, nb[b] = ceil(n[b]/32) tiles, partials at partial + poff[b] laid out
-// slot-major, [tile * n[b] + i], and rpy_sym_items(nb[b]) work items [item0[b], item0[b+1]) (item0[B] == items).
+// slot-major, [tile * n[b] + i], and rpy_sym_items(nb[b], packed) work items [item0[b], item0[b+1]) (item0[B] == items).
 struct SymBatchParams {
     const float4 *x;
     const float4 *f;
@@ -103,13 +104,20 @@ struct SymBatchParams {
     const long long *poff, *item0;
     const int *active;  // may be null: every array active
     int B;
+    bool packed;        // what the items are (rpy_sym_items)
     long long items;
 };
 int rpy_launch_sym_batch(const SymBatchParams &p, int grid, cudaStream_t st);
-// Work items of a force-only set of nb tiles.
-__host__ __device__ constexpr long long rpy_sym_items(int nb) {
-    return static_cast<long long>((nb + 1) / 2) * ((nb + 1) / 2 + 1);
+// Work items of a force-only set of nb tiles: 32 targets x 64 sources in packed arithmetic, or pairs of tiles.
+__host__ __device__ constexpr long long rpy_sym_items(int nb, bool packed) {
+    return packed ? static_cast<long long>((nb + 1) / 2) * ((nb + 1) / 2 + 1) : static_cast<long long>(nb) * (nb + 1) / 2;
 }
+// Whether a launch over that many pairs of tiles takes the packed units.  Below about thirteen an SM the SMs are not full
+// and the launch lasts as long as one unit, which a pair of tiles, half the work, makes shorter; the results are the same
+// bit for bit.  A step by pairs and packed, us: one array of 4 cilia (6 pairs) 209 and 217, of 30 (190) 226 and 236, of 48
+// (465) 231 and 240, 100 arrays of 6 (1,000) 347 and 362, 8 of 30 (1,520) 258 and 264; one of 100 (2,016) 244 and 241, 4 of
+// 64 (3,280) 279 and 264.
+constexpr bool rpy_sym_packed(long long tile_pairs, int num_sms) { return tile_pairs > 13LL * num_sms; }
 // Largest useful grid of the batched kernel (one resident wave).
 int rpy_sym_batch_max_grid(int num_sms);
 

@@ -304,8 +304,8 @@ __device__ __forceinline__ void wall_pair_sym(T dx, T dy, T dz, T zi, T zj, Wall
     const T a = vmul(wu, vfma(u, H, vfma(k(3.0f), P, k(-1.0f))));
     const T b = vmul(wu, vfma(vmul(k(-6.0f), P), hz, vfma(vmul(k(-1.0f), hu), vfma(k(2.0f), H, u5), z.p)));
     const T c = vmul(wu, vfma(u5, hu, z.p));
-    const T e = vmul(wu, vadd(z.q, vfma(E, vfma(k(20.0f), u, k(-4.0f)), vmul(k(-8.0f / 3.0f), u))));
-    const T AKe = vadd(AK, e);
+    const T e = vadd(z.q, vfma(E, vfma(k(20.0f), u, k(-4.0f)), vmul(k(-8.0f / 3.0f), u)));  // over w u
+    const T AKe = vfma(wu, e, AK);
     // i <- j
     {
         const T p = vfma(dx, fj[0], vmul(dy, fj[1]));
@@ -351,6 +351,7 @@ __device__ __forceinline__ void free_overlap(const FreeSym &q, float r2, float s
 __device__ __forceinline__ void free_near(const FreeSym &q, float r2, float s, float &A, float &B) {
     if (r2 <= q.a4) free_overlap(q, r2, s, A, B);
 }
+__device__ __forceinline__ void free_near(const FreeSym &q, F1 r2, F1 s, F1 &A, F1 &B) { free_near(q, r2.v, s.v, A.v, B.v); }
 __device__ __forceinline__ void free_near(const FreeSym &q, F2 r2, F2 s, F2 &A, F2 &B) {
     const float2 r = unpack2(r2);
     if (fminf(r.x, r.y) <= q.a4) {

@@ -693,7 +693,7 @@ int engine_init(Engine *e, const cf_sim_config *cfgs, int B) {
     // placement of every array in the batch
     e->arr.resize(B);
     int fil = 0, seg = 0, mi_max = 1;
-    long long voff = 0, poff = 0, item0 = 0;
+    long long voff = 0, poff = 0, tile_pairs = 0, item0 = 0;
     std::vector<int> fil_arr, rb_arr, h_seg0(B), h_n(B), h_nb(B);
     std::vector<long long> h_poff(B), h_item0(B);
     for (int b = 0; b < B; ++b) {
@@ -718,15 +718,19 @@ int engine_init(Engine *e, const cf_sim_config *cfgs, int B) {
         h_n[b] = a.N;
         h_nb[b] = a.nb;
         h_poff[b] = a.poff;
-        h_item0[b] = item0;
         fil += a.F;
         seg += a.N;
         voff += a.vlen;
         poff += static_cast<long long>(a.N) * a.nb;
-        item0 += rpy_sym_items(a.nb);
+        tile_pairs += rpy_sym_items(a.nb, false);
         mi_max = std::max(mi_max, a.max_iter);
     }
     CF_REQUIRE(voff < (1LL << 31), "cf_batch_create: the batch vectors exceed 2^31 rows");
+    const bool packed = rpy_sym_packed(tile_pairs, e->num_sms);
+    for (int b = 0; b < B; ++b) {
+        h_item0[b] = item0;
+        item0 += rpy_sym_items(h_nb[b], packed);
+    }
     d.B = B;
     d.F = fil;
     d.nseg = ns;
@@ -853,6 +857,7 @@ int engine_init(Engine *e, const cf_sim_config *cfgs, int B) {
     p.active = d.active;
     p.B = B;
     p.items = item0;
+    p.packed = packed;
 
     CF_CUDA(cudaMemset(d.iter_log, 0, sizeof(int) * static_cast<size_t>(B) * kIterLogCap));
     CF_CUDA(cudaMemset(d.ctl, 0, sizeof(GmresCtl) * B));
