@@ -17,6 +17,7 @@
 // work list of every array, and arrays whose GMRES stopped are masked out of
 // the remaining iterations.  A single array (cf_sim) is a batch of one.
 #include "common.cuh"
+#include "host_stage.cuh"
 #include "rpy_kernels.cuh"
 #include "sim_kernels.cuh"
 #include "patch_kernels.cuh"

@@ -69,7 +69,9 @@ struct cf_swim {
     double *part = nullptr;           // block partials of the sums that span blocks
     unsigned int *counter = nullptr;  // their arrival counter (zero between launches)
     cufil::swim::SwimCtl *ctl = nullptr;
-    cufil::swim::SwimReport *h_rep = nullptr;  // pinned: control records and body velocity read back
+    cufil::swim::SwimReport *h_rep = nullptr;  // control records and body velocity read back: page-locked, or own_rep
+    cufil::swim::SwimReport own_rep{};         // in the first step, where each read back waits
+    cufil::PinnedBuffer pinned;
     cudaEvent_t ev[2] = {};
     int last_iters = 0, last_status = CF_OK;
     double last_relres = 0.0;
@@ -987,7 +989,7 @@ void swim_release(cf_swim *h) {
     cudaSetDevice(h->device);
     for (void *p : h->allocations) cudaFree(p);
     h->allocations.clear();
-    if (h->h_rep) cudaFreeHost(h->h_rep);
+    h->pinned.release();
     h->h_rep = nullptr;
     for (cudaEvent_t &e : h->ev) {
         if (e) cudaEventDestroy(e);
@@ -1125,14 +1127,13 @@ extern "C" int cf_swim_create(const cf_swim_config *cfg, cf_swim **out) {
         if ((rc = cuda_status(cudaMemset(h->counter, 0, sizeof(unsigned int)), "cudaMemset", __FILE__, __LINE__)) ||
             (rc = cuda_status(cudaMemset(h->ctl, 0, sizeof(SwimCtl)), "cudaMemset", __FILE__, __LINE__)) ||
             (rc = cuda_status(cudaMemset(h->rhs, 0, sizeof(double) * nv), "cudaMemset", __FILE__, __LINE__)) ||
-            (rc = cuda_status(cudaMallocHost(reinterpret_cast<void **>(&h->h_rep), sizeof(SwimReport)),
-                              "cudaMallocHost", __FILE__, __LINE__)) ||
             (rc = cuda_status(cudaEventCreateWithFlags(&h->ev[0], cudaEventDisableTiming), "cudaEventCreate", __FILE__,
                               __LINE__)) ||
             (rc = cuda_status(cudaEventCreateWithFlags(&h->ev[1], cudaEventDisableTiming), "cudaEventCreate", __FILE__,
                               __LINE__)))
             break;
         d.Rfil = h->Rfil;
+        h->h_rep = &h->own_rep;
         RpyBlockDesc bd{};
         bd.wall = 0;
         bd.vd = 3;
@@ -1169,6 +1170,8 @@ extern "C" int cf_swim_step(cf_swim *h, int nt, int *iters, double *relres) {
     CF_CUDA(cudaSetDevice(h->device));
     cudaStream_t st = h->stream;
     SimDev &d = h->d;
+    void *locked = h->pinned.open(sizeof(SwimReport));
+    h->h_rep = locked ? static_cast<SwimReport *>(locked) : &h->own_rep;
     BodyState body;
     for (int c = 0; c < 3; ++c) body.x[c] = h->bx[c];
     for (int c = 0; c < 4; ++c) body.q[c] = h->bq[c];
