@@ -82,21 +82,6 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Block-wide sum (blockDim.x a multiple of 32); the result is valid in thread 0.
-__device__ __forceinline__ double block_sum(double v, double *sm32) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    v = warp_sum(v);
-    __syncthreads();
-    if (lane == 0) sm32[wid] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (wid == 0) {
-        r = lane < static_cast<int>(blockDim.x >> 5) ? sm32[lane] : 0.0;
-        r = warp_sum(r);
-    }
-    return r;
-}
-
 // ------------------------------------------------------------ FP64 rotations
 // Quaternions (scalar first) and the Lie-group maps of src/general/quaternion.cpp,
 // written from their definitions.
@@ -483,7 +468,7 @@ __global__ void __launch_bounds__(kBarThreads) el_barrier_kernel(ElDev d) {
         for (int q = 0; q < 4; ++q) {
             const int jj = 4 * threadIdx.x + q;
             p[q] = jj < nj ? d.x4[j0 + jj] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            // a NaN position is kept: the test below then rejects it, as it rejects NaN distances
+            // a NaN position is kept: its distances pass the tests below, and the force is NaN
             in[q] = jj < nj && !(p[q].x < lo[0] || p[q].x > hi[0] || p[q].y < lo[1] || p[q].y > hi[1] || p[q].z < lo[2] ||
                                  p[q].z > hi[2]);
             kept += in[q] ? 1 : 0;
@@ -762,9 +747,10 @@ __global__ void el_jacobian_kernel(ElDev d, int nt) {
 // before on the remaining columns.  After the last panel, row p_k of A holds solution row k and column k
 // belongs to equation p_k, so inverse[k][p_j] = A[p_k][j].
 //
-// Bound by the chain of pivots (120 of about 450 cycles at S = 20: a division, a warp maximum, a barrier,
-// the published row).  256 blocks of 120 x 120 (two waves) take 200 us; 314 with (b) and (c) in turn and
-// one row at a time, 800 one pivot at a time.
+// Bound by the chain of pivots (a division, a warp maximum, a barrier, the published row), which (c) beside it slows: of
+// a block's 182,000 cycles at S = 20 the row warps' (a) and (b) take 134,000, 1,100 a pivot, while the others' (c) takes
+// 110,000; copying the pivot rows out takes 13,500, the last update with the store 17,000, the load 14,000.  256 blocks of
+// 120 x 120 (two waves) take 200 us; 314 with (b) and (c) in turn and one row at a time, 800 one pivot at a time.
 constexpr int kInvThreads = 512, kInvPanel = 8, kInvRowWarps = (6 * kMaxSeg + 31) / 32;
 // The matrix in rows of n + 1 (no two rows of a warp start in one bank), two buffers of panel columns, the pivot rows.
 __host__ __device__ constexpr size_t inv_smem_doubles(int n) { return static_cast<size_t>(n) * (n + 1) + 3 * kInvPanel * n; }
@@ -1073,8 +1059,8 @@ ElDev dev(const cf_elastic *h) {
 
 int grid_for(int n, int t) { return std::max(1, (n + t - 1) / t); }
 
-// with `update`, that update of the state; forces, barrier forces, the 6x6 wall mobility and the residual into e; the flags word is
-// cleared first and left on the device.
+// with `update`, that update of the state; forces, barrier forces, the 6x6 wall mobility and the residual into e; the flags
+// word is cleared first and left on the device.
 int evaluate(cf_elastic *h, int nt, const double *update, double *e) {
     cudaStream_t st = h->stream;
     const ElDev d = dev(h);
@@ -1097,7 +1083,8 @@ int evaluate(cf_elastic *h, int nt, const double *update, double *e) {
     bd.as = 1.0f;
     bd.mu = 1.0f;
     // The tile kernel, not the symmetric one: the tethering and inextensibility multipliers carry the product's FP32
-    // rounding amplified a thousandfold, so another order of summation would move the forces by more than 2e-5.
+    // rounding amplified a thousandfold, and another order of summation moved the forces by up to 3.3e-5.  Which of the two
+    // is nearer to a step whose product is FP64 was not measured; the symmetric one would take 0.24 ms off a step of 1.7.
     const RpyPlan plan = rpy_plan(h->N, h->N, 6, 6, h->num_sms);
     CF_TRY(rpy_launch_tiles(bd, plan, h->scratch, h->flags + 1, st));
     CF_TRY(rpy_launch_reduce_f32(bd, plan, h->scratch, h->v, 6, kOutWrite, st, h->flags + 1));

@@ -13,10 +13,10 @@
 // particles everywhere this is the full transform.
 //
 // What bounds it.  Every pass moves each value once, 64 bytes or more at a
-// time (z: read, three transforms forward, projector, three back, write), so
-// the passes run at the memory's or the shared memory's rate; a library
-// transform of the whole grid takes six passes and the projector a seventh,
-// on every point.  At 512^3 with 28% of the planes used (10,000 blobs and 20,000
+// time (z: read, three transforms forward, projector, three back, write).  The
+// x and y passes run near the memory's rate, z at the latency of its chain of
+// stages (z_kernel); a library transform of the whole grid takes six passes and
+// the projector a seventh, on every point.  At 512^3 with 28% of the planes used (10,000 blobs and 20,000
 // segments on a sphere, and their neighbourhood) the five passes take 88 + 207 +
 // 851 + 172 + 82 us, the library's two transforms, the projector and the clearing
 // of whole grids 5.8 ms.

@@ -15,9 +15,10 @@
 //   dZ1 = (dZ2 W2^T) o [A1 > 0]   dW1 = X^T dZ1    db1 = colsum dZ1
 // then one Adam step on FP32 master weights.  Reductions (loss, bias
 // gradients) are fixed-order: results do not depend on the launch.
-// Networks of widths in, H <= 256 and out <= 128 (every one the implicit step
-// attaches) run on the fused kernels of mlp_fused.cuh instead: the same
-// products of the same BF16 operands, one launch forward, three for a gradient.
+// Networks of widths in, H <= 256 and out <= 128 (for the implicit step, whose
+// input has 9 values a segment and two more, those of up to 28 segments a
+// filament) run on the fused kernels of mlp_fused.cuh instead: the same products
+// of the same BF16 operands, one launch forward, three for a gradient.
 #include "common.cuh"
 #include "host_stage.cuh"
 #include "mlp_fused.cuh"

@@ -146,14 +146,6 @@ __device__ __forceinline__ void block_gemm64(const float *L, const float *R, flo
     }
 }
 
-// The pivot block D (rows and columns [k0, k0 + b) of A, padded with the identity to 64 x 64) into M.
-__device__ __forceinline__ void load_pivot_block(const float *A, int n, int k0, int b, float *M) {
-    for (int e = threadIdx.x; e < kGjBlock * kGjBlock; e += blockDim.x) {
-        const int r = e >> 6, c = e & 63;
-        M[r * kInvLd + c] = (r < b && c < b) ? A[static_cast<size_t>(k0 + r) * patch_ld(n) + k0 + c] : (r == c ? 1.0f : 0.0f);
-    }
-}
-
 // Part (a) of a round: inverts pivot block K of patch p (rows and columns
 // [64K, 64K + b)) into its dinv block, zero-padded to 64 x 64; called by all
 // 256 threads of a block.  The 64x64 block D (padded with the identity beyond
@@ -173,6 +165,10 @@ __device__ __forceinline__ void load_pivot_block(const float *A, int n, int k0, 
 // with bank conflicts, four 128-bit loads per sixteen FMAs, where a 4 x 4 tile
 // reads two without; and each warp eliminating its own panel moved sixteen
 // values per pivot by shuffles.  The Newton products take 7 700.
+// The reciprocals are the hardware's approximation: |D X - I| of random and of mobility blocks (condition 2 to 1e4) has
+// the same mean over 148 blocks, 2.4e-8 to 1.2e-5, as with correctly rounded ones and as in the elimination before, within
+// 1%; the inverses of whole patches likewise (80a apart, one step forth and back: 5.4e-5, 5.5e-5 and 5.2e-5 of 40 blocks of
+// 62, 5.7, 5.5 and 5.7e-5 of 24 filaments in patches of 3), and so the solver's iterations on colliding cilia.
 // A: the patch matrix (n x n), dv: its dinv block, ok: its flag, ws: shared
 // memory of at least kInvWs floats.
 constexpr int kInvWs = 2 * kGjBlock * kInvLd;

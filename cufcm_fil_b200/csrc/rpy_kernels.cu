@@ -1237,6 +1237,4 @@ int rpy_launch_sym_batch(const SymBatchParams &p, int grid, cudaStream_t st) {
     return CF_OK;
 }
 
-int rpy_sym_batch_max_grid(int num_sms) { return std::max(1, num_sms) * kSym3CtasPerSm; }
-
 }  // namespace cufil

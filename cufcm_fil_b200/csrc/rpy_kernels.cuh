@@ -118,8 +118,6 @@ __host__ __device__ constexpr long long rpy_sym_items(int nb, bool packed) {
 // (465) 231 and 240, 100 arrays of 6 (1,000) 347 and 362, 8 of 30 (1,520) 258 and 264; one of 100 (2,016) 244 and 241, 4 of
 // 64 (3,280) 279 and 264.
 constexpr bool rpy_sym_packed(long long tile_pairs, int num_sms) { return tile_pairs > 13LL * num_sms; }
-// Largest useful grid of the batched kernel (one resident wave).
-int rpy_sym_batch_max_grid(int num_sms);
 
 // Output modes of the reduction.
 enum RpyOut : int { kOutWrite = 0, kOutAdd = 1 };

@@ -901,7 +901,8 @@ int engine_init(Engine *e, const cf_sim_config *cfgs, int B) {
     t0.dots_chunk = static_cast<int>(std::min<long long>(4096, std::max<long long>(kMinDotsChunk, chunk)));
     // default update tile: the tallest that still gives every resident block one.  Tall tiles have a thread sum all the
     // basis vectors of its row, with no exchange between the threads; small systems need short ones to fill the SMs.
-    // A step of 64 arrays (5.8e5 rows): 8.7 ms with 256 rows, 9.3 with 32; of one array (1.6e4 rows, 32) unchanged.
+    // A step of 64 arrays (5.8e5 rows) on the device: 8.7 ms with 256 rows, 9.3 with 32; of one array (1.6e4 rows, 32)
+    // unchanged.
     for (int rows = 64; rows <= 256 && d.nrows / rows >= 1LL * e->num_sms * t0.update_blocks_per_sm; rows *= 2)
         t0.update_rows = rows;
     CF_TRY(apply_tuning(e, t0));

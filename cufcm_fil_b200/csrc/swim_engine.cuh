@@ -254,8 +254,8 @@ __device__ __forceinline__ void swim_range(const SwimParams &p, int blk, int &lo
     }
 }
 
-// Totals over the blocks of NV values each left in part[block][NV], by the block that arrives last; value c in
-// thread c * (kSwT / NV) ... handled by warp c % 4, in a fixed order, into out[c] (shared).
+// Totals over the blocks of NV values each left in part[block][NV], by the block that arrives last: value c by warp
+// c % (kSwT / 32), in a fixed order, into out[c] (shared).
 template <int NV>
 __device__ __forceinline__ bool swim_totals(double *part, unsigned int *counter, int *flag, double *out) {
     if (!arrive_last(counter, gridDim.x, flag)) return false;
