@@ -122,7 +122,7 @@ __device__ __forceinline__ void two_sum3(float *hi, float *lo, float ax, float a
 
 // grid (ceil(nf / (128 TI)), nsplit): block (x, y) sums sources [y*split, (y+1)*split)
 // of its 128 TI flow points.  Sources [0, nseg_src) are segments, the rest blobs.
-// Bound by the FP32 pipe: 16,000 points and 5,120 segments (8.2e7 pairs above the wall) take 176 us, about 51 TFLOP/s;
+// Bound by the FP32 pipe: 16,000 points and 5,120 segments (8.2e7 pairs above the wall) take 168 us, about 53 TFLOP/s;
 // term by term with divisions and square roots, in tiles of 256 at four blocks an SM, it was 425 us.  Four points a
 // thread leave too few warps (201 us).
 template <bool WALL, bool NET, int TI>
