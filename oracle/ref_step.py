@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import subprocess
 import tempfile
+import unittest
 from dataclasses import dataclass
 from pathlib import Path
 
@@ -32,6 +33,13 @@ def binary(variant: str) -> Path:
 
 def available(variant: str = "step_dyn_f64") -> bool:
     return binary(variant).exists()
+
+
+def _built(variant: str) -> str:
+    """Path of a built harness; a test that reaches one that is not built is skipped, as those that ask available() are."""
+    if not available(variant):
+        raise unittest.SkipTest(f"reference step binary {variant} not built (oracle/ref_build.py)")
+    return str(binary(variant))
 
 
 def _tag(nseg: int, seg_sep: float) -> str:
@@ -59,7 +67,7 @@ def wgf_tables(nseg: int = 20, seg_sep: float = 2.6, timeout: float = 600.0):
     with tempfile.TemporaryDirectory() as tmp:
         d = Path(tmp)
         (d / "input" / "forcing").mkdir(parents=True)
-        subprocess.run([str(binary("step_wgf_f64")), "wgf", str(nseg), repr(float(seg_sep)), "out.bin"], cwd=d,
+        subprocess.run([_built("step_wgf_f64"), "wgf", str(nseg), repr(float(seg_sep)), "out.bin"], cwd=d,
                        check=True, capture_output=True, timeout=timeout)
         f = d / "input" / "forcing"
         qp = _read_vec(f / _forcing_name("phase_generalised_forces", nseg, seg_sep))
@@ -100,7 +108,7 @@ def run(*, nfil: int, fil_x_dim: int, spacing: float, phase0, angle0, steps: int
             f"{s.shape[0]} {s.shape[1]} " + " ".join(repr(float(x)) for x in s.ravel()))
         ic = np.concatenate([np.asarray(phase0, float), np.asarray(angle0, float)])
         (d / "psi.dat").write_text("0 0 " + " ".join(repr(float(x)) for x in ic))
-        cmd = [str(binary(variant)), "run", str(nseg), str(F), str(int(fil_x_dim)), repr(float(spacing)),
+        cmd = [_built(variant), "run", str(nseg), str(F), str(int(fil_x_dim)), repr(float(spacing)),
                repr(float(seg_sep)), repr(float(spring_factor)), str(int(steps)), "psi.dat", "out.bin"]
         if write:
             cmd.append("write")
@@ -174,7 +182,7 @@ def run_body(*, fil_normals, blob_normals, ar: float, phase0, angle0, steps: int
         _write_seeds(d, B, blob_normals)
         ic = np.concatenate([np.asarray(phase0, float), np.asarray(angle0, float)])
         (d / "psi.dat").write_text("0 0 " + " ".join(repr(float(x)) for x in ic))
-        cmd = [str(binary("step_body_f64")), "run", str(nseg), str(F), str(B), repr(float(ar)), repr(float(seg_sep)),
+        cmd = [_built("step_body_f64"), "run", str(nseg), str(F), str(B), repr(float(ar)), repr(float(seg_sep)),
                repr(float(spring_factor)), str(int(steps)), "psi.dat", "out.bin"]
         subprocess.run(cmd, cwd=d, check=True, capture_output=True, timeout=timeout)
         width = 2 + 7 * F + 13
@@ -201,7 +209,7 @@ def run_elastic(*, nfil: int, fil_x_dim: int, spacing: float, steps: int, nseg: 
     CILIA_IC_TYPE 0, FP64), run by ref_elastic_harness.cu; DT = period / 300."""
     with tempfile.TemporaryDirectory() as tmp:
         d = Path(tmp)
-        cmd = [str(binary("elastic_f64")), "run", str(nseg), str(int(nfil)), str(int(fil_x_dim)), repr(float(spacing)),
+        cmd = [_built("elastic_f64"), "run", str(nseg), str(int(nfil)), str(int(fil_x_dim)), repr(float(spacing)),
                repr(float(seg_sep)), repr(float(period)), str(int(steps)), "out.bin"]
         subprocess.run(cmd, cwd=d, check=True, capture_output=True, timeout=timeout)
         N = int(nfil) * nseg
@@ -215,7 +223,7 @@ def elastic_jacobian(*, nseg: int = 20, seg_sep: float = 2.6, period: float = 36
     first evaluation of step 0, from the reference's own invert_approx_jacobian."""
     with tempfile.TemporaryDirectory() as tmp:
         d = Path(tmp)
-        cmd = [str(binary("elastic_f64")), "jac", str(nseg), repr(float(seg_sep)), repr(float(period)), "out.bin"]
+        cmd = [_built("elastic_f64"), "jac", str(nseg), repr(float(seg_sep)), repr(float(period)), "out.bin"]
         subprocess.run(cmd, cwd=d, check=True, capture_output=True, timeout=600)
         raw = np.fromfile(d / "out.bin")
     n = 6 * nseg
