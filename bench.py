@@ -893,6 +893,10 @@ def run_reference(args):
         return
     import oracle
     from oracle import ref_step
+    missing = [v for v in ("step_wgf_f64", "step_dyn_f64") if not ref_step.available(v)]
+    if missing:
+        print(json.dumps({"impl": "reference", "unavailable": f"step code not built: {', '.join(missing)} (oracle/ref_build.py)"}))
+        return
     inp = workload_inputs(s_table_from="reference")
     F = NX * NX
     # The reference's own prescribed-cilia step code (mobility_solver.cpp, filament.cpp, ...: host GMRES, its
